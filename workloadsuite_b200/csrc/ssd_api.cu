@@ -11,6 +11,7 @@ namespace {
 
 constexpr int kAbiVersion = 3;
 constexpr int kSmCount = 148;  // B200
+constexpr int kShortSequence = 32;   // tokens; one staged piece of the fp32 scan
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -46,11 +47,9 @@ int resolve_kernel(const SsdArgs* a) {
   if (a->kernel == SSD_KERNEL_TCGEN05) return SSD_KERNEL_TCGEN05;
   // (states that are only 4-byte aligned go to the fp32 scan, which moves them element by element)
   const bool st16 = aligned16(a->initial_state) && aligned16(a->final_state);
-  return ssd::tc_supports(*a) && st16 ? SSD_KERNEL_TCGEN05 : SSD_KERNEL_SCAN_F32;
+  // A tile of the tensor-core kernel takes as long for one token as for 128; a few tokens are quicker in the fp32 scan.
+  return ssd::tc_supports(*a) && st16 && a->seqlen >= kShortSequence ? SSD_KERNEL_TCGEN05 : SSD_KERNEL_SCAN_F32;
 }
-
-// The two-head kernel whenever the heads of a B/C group come in pairs, else one head per CTA.
-bool use_tc2(const SsdArgs* a) { return ssd::tc2_supports(*a); }
 
 int tile_tokens(int kernel) { return kernel == SSD_KERNEL_TCGEN05 ? 128 : ssd::scan_f32_tile_tokens(); }
 
@@ -60,7 +59,7 @@ void resolve_segments(const SsdArgs* a, int kernel, int* nseg, int* seg_len) {
   int want = a->nsegments;
   if (want <= 0) {
     if (kernel == SSD_KERNEL_TCGEN05) {
-      want = use_tc2(a) ? ssd::tc2_default_segments(*a) : ssd::tc_default_segments(*a);
+      want = ssd::tc2_default_segments(*a);
     } else {
       const int64_t units = (int64_t)a->batch * a->nheads;
       // Two passes cost about 1.5x the work of one, so split only when the
@@ -114,7 +113,7 @@ bool z_vector_friendly(const SsdArgs* a) {
 bool states_aligned16(const SsdArgs* a) { return aligned16(a->initial_state) && aligned16(a->final_state); }
 
 int launch_kernel(int kernel, const SsdArgs* a, const ssd::ScanParams& prm, cudaStream_t stream) {
-  if (kernel == SSD_KERNEL_TCGEN05) return use_tc2(a) ? ssd::launch_tc2(*a, prm, stream) : ssd::launch_tc(*a, prm, stream);
+  if (kernel == SSD_KERNEL_TCGEN05) return ssd::launch_tc2(*a, prm, stream);
   return ssd::launch_scan_f32(prm, a->dtype, stream);
 }
 
@@ -154,7 +153,7 @@ int ssd_b200_plan(const SsdArgs* args, int32_t* kernel_out, int32_t* nsegments_o
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
   int launches = 1;
   if (nseg > 1) {
-    const bool chained = kernel == SSD_KERNEL_TCGEN05 && use_tc2(args) && ssd::tc2_chain_mode(*args, nseg) != 0;
+    const bool chained = kernel == SSD_KERNEL_TCGEN05 && ssd::tc2_chain_mode(*args, nseg) != 0;
     launches = chained ? 1 : (state_only ? 2 : 3);
     if (!chained && (args->flags & SSD_FLAG_REUSE_SEGMENTS)) launches -= 1;
   }
@@ -172,7 +171,7 @@ size_t ssd_b200_workspace_bytes(const SsdArgs* args) {
   if (nseg <= 1) return 0;
   const size_t units = (size_t)args->batch * args->nheads;
   const size_t np = (size_t)args->dstate * args->headdim;
-  if (kernel == SSD_KERNEL_TCGEN05 && use_tc2(args) && ssd::tc2_chain_mode(*args, nseg) != 0) {
+  if (kernel == SSD_KERNEL_TCGEN05 && ssd::tc2_chain_mode(*args, nseg) != 0) {
     // chained / look-back mode: one slot per CTA and head of the pair -- state, log-decay sum, ready flag
     const size_t slots = 2 * (size_t)kSmCount;
     return align_up(slots * np * sizeof(float), 256) + 2 * align_up(slots * sizeof(float), 256);
@@ -221,7 +220,7 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
   const size_t need = ssd_b200_workspace_bytes(args);
   if (!args->workspace || args->workspace_bytes < need) return SSD_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(args->workspace) & 255) return SSD_ERR_MISALIGNED;
-  const int chain_mode = (kernel == SSD_KERNEL_TCGEN05 && use_tc2(args)) ? ssd::tc2_chain_mode(*args, nseg) : 0;
+  const int chain_mode = kernel == SSD_KERNEL_TCGEN05 ? ssd::tc2_chain_mode(*args, nseg) : 0;
   if (chain_mode != 0) {
     // one launch: the pieces of a sequence pass their state through the workspace, one slot per CTA and head
     const size_t slots = 2 * (size_t)kSmCount;
@@ -293,10 +292,9 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
   if (rc != SSD_OK) return rc;
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
   if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false);
-  // skip and gate of model_ref.py:116-118: fused into the two-head tensor-core kernel, a kernel of their own otherwise
+  // skip and gate of model_ref.py:116-118: fused into the tensor-core kernel, a kernel of their own otherwise
   const int kernel = resolve_kernel(args);
-  const bool fuse = kernel == SSD_KERNEL_TCGEN05 && ssd::tc_supports(*args) && use_tc2(args) &&
-                    z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
+  const bool fuse = kernel == SSD_KERNEL_TCGEN05 && ssd::tc_supports(*args) && z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
   rc = forward_impl(args, stream_v, fuse);
   if (rc != SSD_OK || fuse) return rc;
   ssd::ScanParams ep;

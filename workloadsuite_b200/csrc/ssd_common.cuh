@@ -86,13 +86,8 @@ int launch_fold(const float* states, int64_t st_unit_stride, int64_t st_seg_stri
                 float* out_final, float* out_ld, int upto, float* incoming, int64_t units, int64_t np,
                 cudaStream_t stream);
 
-// tcgen05 kernel family (ssd_tcgen05.cu)
+// tensor-core kernel (ssd_tc2.cu)
 bool tc_supports(const SsdArgs& a);
-int tc_default_segments(const SsdArgs& a);
-int launch_tc(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);
-
-// two-heads-per-CTA tcgen05 kernel (ssd_tc2.cu): needs an even number of heads per B/C group
-bool tc2_supports(const SsdArgs& a);
 int tc2_default_segments(const SsdArgs& a);
 int tc2_chain_mode(const SsdArgs& a, int nseg);   // 1: chained, 2: look-back (one launch each); 0: two passes + fold
 int launch_tc2(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);

@@ -1,28 +1,29 @@
-// Two-head tensor-core SSD forward for sm_100a (the fast path when the heads of a
-// group come in pairs).  One persistent CTA per SM walks work items (a run of
-// 128-token tiles of one (batch, head pair) sequence) in order.
+// Tensor-core SSD forward for sm_100a: one persistent CTA per SM walks work items (a run of 128-token tiles of one
+// sequence of two heads) as one unbroken pipeline of tiles.
 //
-// The two heads of a pair read the same B and C (model_ref.py:97-99), so B, C and
-// G = C.B^T (model_ref.py:143) are loaded/computed once per tile and shared.  The two
-// heads' Xd tiles and 16-bit state copies lie one 64-column block apart in shared
-// memory, so S = B^T.[Xd0|Xd1] and C.[H0|H1] are single N = 128 MMAs as well (an N = 64
-// MMA occupies the tensor pipe as long as an N = 128 one).  Each head has its own
-// compute warpgroup (one thread per tile row / TMEM lane).  Per head and tile k, in
-// the order the warpgroup runs them inside one loop iteration:
-//   a. H <- exp(cs_last) H + S(k)         (model_ref.py:150,156)   S = B^T.Xd from step c of the previous iteration
-//   e. Y(k-1) -> global                    (:162)                   the P.X MMA of tile k-1 ran under step a
-//   c. tile k+1: prefix sum (:135), Xd = exp(cs_last - cs_l) x~ (:144,148) -> smem -> S MMA; the rows of Xd are dealt
-//      to the four warps unevenly (the row's scale goes through shared memory), the warps with fewer blocks of P in
-//      step d taking more
-//   d. P(k) = G o exp(segsum) o causal     (:139-145) -> TMEM as the A operand of Y += P.X
-//   b. Y(k) <- exp(cs_l) * (C.H)           (:160-161) scaled in place in TMEM (the C.H MMA ran under steps c, d)
-//      16-bit copy of H(k+1) -> smem for the next C.H MMA
-// Warp 0 is the TMA producer, warp 1 issues the G MMAs, warp 2 the S and C.H MMAs,
-// warp 3 the two heads' P.X MMAs (one thread each, blocking on the mbarriers in the
-// order the warpgroups raise them); warps 4-7 and 8-11 are the compute warpgroups.
-// tcgen05.mma holds its issuing thread for about as long as the MMA runs (77-160
-// cycles per 128xNx16 step, depending on the operand layouts), which is why the three
-// MMA streams have a thread each.  All waits are bounded.
+// The two heads of a pair read the same B and C (model_ref.py:97-99), so B, C and G = C.B^T (model_ref.py:143) are
+// loaded and computed once per tile and shared, and S = B^T.[Xd0|Xd1] and C.[H0|H1] are single N = 128 MMAs.  A group
+// with an odd number of heads leaves the second half of its last pair empty (zeros in, nothing out).
+//
+// Roles (512 threads):
+//   warp 0        TMA producer
+//   warp 1        MMA issuer: P.X(t) per head, then S(t+1), G(t+1), C.H(t+1)
+//   warps 2, 3    prefix sum of the log-decay (model_ref.py:135) and every factor derived from it, one head each, up to
+//                 two tiles ahead; the other roles read the factors from shared memory
+//   warps 4-7     head 0, warps 8-11 head 1: thread = tile row = TMEM lane.  Per iteration, in this order:
+//     A. P(t)   = G o exp(segsum) o causal  (:139-145)  -> TMEM, the A operand of Yd = P.X
+//     B. Xd(t+1) = exp(cs_last - cs) x~     (:144,148)  -> shared memory -> S = B^T.Xd
+//     D. 16-bit copy of the state entering tile t+1     -> shared memory -> Yo = C.H   (:160-161)
+//     E. H <- exp(cs_last) H + S(t+1)       (:150,156)  in fp32 registers
+//   warps 12-15   Y(t) = Yd + exp(cs) Yo (:162) [+ skip and gate, :116-118] -> shared memory -> TMA store, both heads
+//
+// What bounds it.  A 128xNx16 tcgen05.mma takes 62 cycles at N = 128 and 55 at N = 64 (any operand layout), so the
+// four contractions of a tile pair need 2 430 tensor-pipe cycles; HBM needs 2 800 cycles per SM for its 64 KB of X
+// and Y.  The state recurrence is the only true chain.  Tensor memory (512 columns) is what limits overlap: G 128,
+// Yo 128, Yd 128 and 128 columns that S and P take turns in -- S(t+1) is consumed (step E) before P(t+1) is written
+// (step A), and S(t+1) is issued once P.X(t) has read P(t).  Keeping Yo and Yd apart means that nothing has to be
+// scaled in place between C.H and P.X, and that C.H(t+1) and the reloads of B and C run under steps A, B and D.
+// All waits are bounded.
 #include <cuda.h>
 
 #include <algorithm>
@@ -38,20 +39,24 @@ namespace {
 using namespace ptx;
 using namespace tc;
 
-constexpr int kThreads2 = 384;
+constexpr int kThreads2 = 512;
 constexpr int kSms = 148;
-constexpr int kXStages = 3;   // X tiles in flight per head; a consumed stage doubles as the Y staging buffer
 
 template <int N>
 struct Layout2 {
   static constexpr int NB = N / 64;
-  static constexpr int oB = 0;
-  static constexpr int oC = oB + NB * kBlk;
-  static constexpr int oX = oC + NB * kBlk;     // [head][stage], kXStages stages
-  static constexpr int oXd = oX + 2 * kXStages * kBlk;   // [head]
-  static constexpr int oH = oXd + 2 * kBlk;      // [head], N rows of 128 B
+  // B and C tiles in flight, and X tiles (one head each) in flight; an X slot whose tile is consumed doubles as the Y
+  // staging buffer.  n = 64 leaves room for more of both.
+  static constexpr int kBC = N == 128 ? 1 : 2;
+  static constexpr int kXSlots = N == 128 ? 5 : 6;
+  static constexpr int oB = 0;                           // [stage]
+  static constexpr int oC = oB + kBC * NB * kBlk;        // [stage]
+  static constexpr int oX = oC + kBC * NB * kBlk;        // [slot]
+  static constexpr int oXd = oX + kXSlots * kBlk;        // [head]
+  static constexpr int oH = oXd + 2 * kBlk;              // [head], N rows of 128 B
   static constexpr int oMisc = oH + 2 * N * 128;
-  static constexpr int kBytes = oMisc + 3072;   // no slack: the dynamic segment must start 1024-byte aligned
+  static constexpr int kMiscBytes = 10240;
+  static constexpr int kBytes = oMisc + kMiscBytes;   // no slack: the dynamic segment must start 1024-byte aligned
 };
 
 // Work list of this CTA.
@@ -64,153 +69,234 @@ struct Layout2 {
 //  - Look-back mode (sp.chain == 2), for fewer sequences than CTAs: the same even cut, but a piece cannot wait
 //    for the full scan of the piece before it (the pieces of one sequence would run one after the other).
 //    Instead every CTA first scans the LAST piece of its range from a zero state, state and log-decay sum only
-//    (about 0.4 of the full work; item 0, skipped when that piece ends its sequence), and publishes the pair.
-//    Then it walks its pieces like the chained mode; a piece that starts inside a sequence folds the published
-//    pairs of the CTAs before it, back to the one that holds the sequence's first tile (the recurrence is linear:
-//    H_in = sum_c exp(sum of the log-decays after c) F_c), and stops early once the decay factor has underflowed.
+//    (item 0, skipped when that piece ends its sequence), and publishes the pair.  Then it walks its pieces like
+//    the chained mode; a piece that starts inside a sequence folds the published pairs of the CTAs before it, back
+//    to the one that holds the sequence's first tile (the recurrence is linear: H_in = sum_c exp(sum of the
+//    log-decays after c) F_c), skipping those whose decay factor has underflowed.
 // Computed once per CTA (thread 0, into shared memory): the 64-bit divisions are bulky code.
 struct Work {
-  int count;
-  int lo, hi, nt, pl;   // chained mode: global tile range, tiles per sequence, last sequence of the range
-  int hp, hpg;          // head pairs per batch entry, heads per B/C group
-  int pre;              // look-back mode: 1 when item 0 is the state-only scan of the range's last piece
-  int ytot;             // tiles of all Y-producing items
+  int total;            // tiles of all items
+  int npre;             // the first npre of them produce a state only
+  int lo, hi, nt, first;   // chained modes: global tile range, tiles per sequence, first tile of item 0's sequence
+  int from;             // look-back mode: the CTA that holds the first tile of the range's first sequence
+  int hpg, ppg;         // heads per B/C group, head pairs per group
+  // item 0 as (pair of the group, group, batch entry, segment), and the step from one item to the next in the same
+  // mixed-radix digits: the walk needs no division
+  int d0[4], step[4];
+};
+
+// Factors of one tile of one head, written by the prefix-sum warp.
+struct alignas(16) Factors {
+  float cs2[T];       // cs * log2(e)
+  float cf[T];        // exp(cs at the end of the row's 32-block - cs of the row) * dt: the row's factor as a column of P
+  float dg[T];        // diagonal blocks: at columns 4i cs * log2(e) - log2(dt), at the three after it the ratio to the column before
+  uint16_t xs[T];     // exp(cs_last - cs) * dt, the 16-bit scale of the row of X being turned into Xd
+  float tot;          // cs_last
 };
 
 struct Misc2 {
   Work work;
-  uint64_t full_b, full_c, empty_b, empty_c;
-  uint64_t full_x[2][kXStages], empty_x[2][kXStages];
-  uint64_t bar_g;
-  uint64_t bar_yo, bar_s, bar_y[2];   // tcgen05.commit arrivals (the S and C.H MMAs serve both heads at once)
-  uint64_t bar_xd, bar_h, bar_e;      // one arrival per compute warp of either head (8)
-  uint64_t bar_p[2];                  // one arrival per compute warp of the head (4)
-  uint64_t bar_drain[3];              // give-up path: the MMAs of issuing warp 1 / 2 / 3 have all completed
+  Factors f[2][2];                    // [head][tile parity]
+  uint64_t full_b[2], full_c[2], empty_b[2], empty_c[2];   // [stage]
+  uint64_t full_x[6], empty_x[6];
+  uint64_t full_f[2][2], empty_f[2][2];   // factors [head][tile parity]
+  uint64_t bar_g, bar_s, bar_ch, bar_y[2];   // tcgen05.commit arrivals (S and C.H serve both heads at once)
+  uint64_t bar_xd, bar_h, bar_e;      // one arrival per warp and head (8)
+  uint64_t bar_p[2];                  // one arrival per warp of the head (4)
+  uint64_t bar_drain;                 // all MMAs issued have completed
   uint32_t tmem_base;
   long long wait_clocks;     // bound of every wait (SM clock cycles)
   volatile int abort_flag;   // 0, or the status code of the first wait that gave up (every role then leaves)
-  float wsum[2][4];
-  // Double-buffered by tile parity: step c writes the next tile's values while step d still reads this tile's.
-  alignas(16) float cf[2][2][T];   // [head][parity][row]: exp(cs at the end of the row's 32-block - cs of the row)
-  float cend[2][2][4];             // [head][parity][block]: cs * log2(e) at the end of each 32-row block
-  uint16_t xs[2][T];               // [head][row]: the 16-bit scale exp(cs_last - cs_row) * dt of the row of X being turned into Xd
 };
 
-static_assert(sizeof(Misc2) <= 3072, "Misc2 outgrew its shared-memory slot");
-static_assert(Layout2<128>::kBytes <= 232448, "shared memory budget of one SM exceeded");
+static_assert(sizeof(Misc2) <= Layout2<128>::kMiscBytes, "Misc2 outgrew its shared-memory slot");
+static_assert(Layout2<128>::kBytes <= 232448 && Layout2<64>::kBytes <= 232448, "shared memory budget of one SM exceeded");
 
 struct Tc2Params {
   ScanParams sp;
-  int nitems;   // (batch * nheads / 2) * nseg
-  int upairs;   // batch * nheads / 2
+  int nitems;   // upairs * nseg
+  int upairs;   // batch * head pairs
+  int ppg;      // head pairs per B/C group
 };
 
-// One work item: `ntiles` tiles of one (batch, head pair) sequence from token t_begin on.  in_slot / out_slot are
-// the scratch slots the state is taken from / handed to when the item is an inner piece of a sequence that
-// continues on a neighbouring CTA (-1: the sequence starts / ends here).
-struct Item {
-  int seg, bi, h0, gi, t_begin, ntiles, in_slot, out_slot;
-  int yflag;      // this item produces Y (0: state and log-decay sum only)
-  int fold_from;  // look-back mode: first CTA whose published pair enters the fold (-1: none), up to in_slot
-  int ends_seq;   // the item holds the last tile of its sequence: it writes the caller's final state
-};
+// Item `i` of the (segment, batch, group, pair) grid as digits.
+__device__ __forceinline__ void digits(int i, const Tc2Params& prm, int (&d)[4]) {
+  d[0] = i % prm.ppg; i /= prm.ppg;
+  d[1] = i % prm.sp.ngroups; i /= prm.sp.ngroups;
+  d[2] = i % prm.sp.batch; d[3] = i / prm.sp.batch;
+}
 
-__device__ __forceinline__ void work_list(const Tc2Params& prm, Work* out) {
-  Work wk;
-  wk.lo = wk.hi = wk.pl = 0;
-  wk.nt = 1;
-  wk.hp = prm.sp.nheads >> 1;
-  wk.hpg = prm.sp.nheads / prm.sp.ngroups;
-  if (prm.sp.chain) {
-    wk.nt = prm.sp.seqlen / T;
+__device__ __forceinline__ void work_list(const Tc2Params& prm, Work& wk) {
+  const ScanParams& sp = prm.sp;
+  wk.nt = (sp.seqlen + T - 1) / T;
+  wk.hpg = sp.nheads / sp.ngroups;
+  wk.ppg = prm.ppg;
+  wk.npre = sp.compute_y ? 0 : 0x7fffffff;
+  wk.lo = wk.hi = wk.first = wk.from = 0;
+  if (sp.chain) {
     const long long total = (long long)prm.upairs * wk.nt;
     wk.lo = (int)((long long)blockIdx.x * total / gridDim.x);
     wk.hi = (int)((long long)(blockIdx.x + 1) * total / gridDim.x);
-    wk.pl = wk.hi > wk.lo ? (wk.hi - 1) / wk.nt : 0;
-    wk.count = wk.hi > wk.lo ? wk.pl - wk.lo / wk.nt + 1 : 0;
-    wk.pre = (prm.sp.chain == 2 && wk.hi > wk.lo && wk.hi % wk.nt != 0) ? 1 : 0;
-    wk.count += wk.pre;
-  } else {
-    wk.pre = 0;
-    wk.count = (int)blockIdx.x < prm.nitems ? (prm.nitems - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-  }
-  wk.ytot = 0;
-  *out = wk;
-}
-
-__device__ __forceinline__ Item work_item(const Tc2Params& prm, const Work& wk, int i) {
-  const ScanParams& sp = prm.sp;
-  Item it;
-  int u2;
-  it.yflag = sp.compute_y;
-  it.fold_from = -1;
-  it.ends_seq = 1;
-  if (sp.chain) {
-    const bool pre = wk.pre && i == 0;        // look-back mode: the state-only scan of the last piece
-    u2 = wk.pl - (pre ? 0 : i - wk.pre);
-    const int first = u2 * wk.nt, start = max(wk.lo, first), end = min(wk.hi, first + wk.nt);
-    it.seg = 0;
-    it.t_begin = (start - first) * T;
-    it.ntiles = end - start;
-    it.in_slot = start > first ? (int)blockIdx.x - 1 : -1;
-    it.out_slot = end < first + wk.nt ? (int)blockIdx.x : -1;
-    it.ends_seq = end == first + wk.nt;
-    if (sp.chain == 2) {
-      if (pre) {
-        it.yflag = 0;
-        it.in_slot = -1;                      // from a zero state
-      } else {
-        it.out_slot = -1;                     // only the state-only scan publishes
-        if (it.in_slot >= 0) {
-          // the CTA that holds the sequence's first tile: the largest c with lo(c) <= first
-          const long long total = (long long)prm.upairs * wk.nt;
-          int c = (int)((((long long)first + 1) * gridDim.x - 1) / total);
-          while (c > 0 && (long long)c * total / gridDim.x > first) --c;
-          while ((long long)(c + 1) * total / gridDim.x <= first) ++c;
-          it.fold_from = c;
-        }
-      }
+    wk.total = wk.hi - wk.lo;
+    const int last = (wk.hi - 1) / wk.nt;     // (every CTA has at least one tile)
+    wk.first = last * wk.nt;
+    if (sp.chain == 2 && wk.hi % wk.nt != 0) {
+      wk.npre = wk.hi - max(wk.lo, wk.first);
+      wk.total += wk.npre;
     }
+    // the largest c with lo(c) <= first tile of the range's first sequence
+    const int first = wk.lo / wk.nt * wk.nt;
+    int c = (int)((((long long)first + 1) * gridDim.x - 1) / total);
+    while (c > 0 && (long long)c * total / gridDim.x > first) --c;
+    while ((long long)(c + 1) * total / gridDim.x <= first) ++c;
+    wk.from = c;
+    digits(last, prm, wk.d0);
+    wk.step[0] = -1;
+    wk.step[1] = wk.step[2] = wk.step[3] = 0;
   } else {
-    const int item = blockIdx.x + i * gridDim.x;
-    it.seg = item / prm.upairs;
-    u2 = item - it.seg * prm.upairs;
-    it.t_begin = it.seg * sp.seg_len;
-    it.ntiles = (min(sp.seqlen, it.t_begin + sp.seg_len) - it.t_begin) / T;
-    it.in_slot = it.out_slot = -1;
+    wk.total = 0;
+    for (int i = blockIdx.x; i < prm.nitems; i += gridDim.x) {
+      const int t = i / prm.upairs * sp.seg_len;
+      wk.total += (min(sp.seqlen, t + sp.seg_len) - t + T - 1) / T;
+    }
+    digits(blockIdx.x, prm, wk.d0);
+    digits(gridDim.x, prm, wk.step);
   }
-  it.bi = u2 / wk.hp;
-  it.h0 = 2 * (u2 - it.bi * wk.hp);
-  it.gi = it.h0 / wk.hpg;
-  return it;
 }
 
-// Bounded wait on an mbarrier phase; false when it gave up (or another role already had).
-__device__ __forceinline__ bool wait2(uint64_t* bar, uint32_t parity, Misc2* m, int code, int32_t* status) {
-  if (mbar_try_wait(bar, parity)) return true;   // the common case in steady state: no clock read, no sleep
+// Walks the tiles of all items of this CTA, in order.  An item is a run of `ntiles` tiles of one (batch, head pair)
+// sequence from token t_begin on.
+struct Cursor {
+  int t0, left;           // first token of the current tile, tiles of the item after it
+  int t_begin, ntiles;
+  int q, g, b, seg;       // pair of the group, group, batch entry, segment
+  int first;              // chained modes: first tile of the sequence in the laid-out order
+  int item;
+  __device__ __forceinline__ Cursor() : left(0), item(-1) {}
+  __device__ __forceinline__ void next(const Tc2Params& prm, const Work& wk) {
+    if (__builtin_expect(left > 0, 1)) {
+      --left;
+      t0 += T;
+      return;
+    }
+    const ScanParams& sp = prm.sp;
+    if (++item == 0) {
+      q = wk.d0[0]; g = wk.d0[1]; b = wk.d0[2]; seg = wk.d0[3];
+      first = wk.first;
+    } else if (!(item == 1 && sp.chain == 2 && wk.npre > 0)) {   // (after the state-only scan: the same piece again)
+      first -= wk.nt;
+      int c = 0;
+      q += wk.step[0];
+      if (q >= prm.ppg) { q -= prm.ppg; c = 1; }
+      if (q < 0) { q += prm.ppg; c = -1; }
+      g += wk.step[1] + c;
+      c = 0;
+      if (g >= sp.ngroups) { g -= sp.ngroups; c = 1; }
+      if (g < 0) { g += sp.ngroups; c = -1; }
+      b += wk.step[2] + c;
+      c = 0;
+      if (b >= sp.batch) { b -= sp.batch; c = 1; }
+      seg += wk.step[3] + c;
+    }
+    if (sp.chain) {
+      const int start = max(wk.lo, first), end = min(wk.hi, first + wk.nt);
+      t_begin = (start - first) * T;
+      ntiles = end - start;
+    } else {
+      t_begin = seg * sp.seg_len;
+      ntiles = (min(sp.seqlen, t_begin + sp.seg_len) - t_begin + T - 1) / T;
+    }
+    t0 = t_begin;
+    left = ntiles - 1;
+  }
+  __device__ __forceinline__ bool first_tile() const { return left == ntiles - 1; }
+  __device__ __forceinline__ int head(const Work& wk) const { return g * wk.hpg + 2 * q; }   // first of the pair
+  __device__ __forceinline__ bool live(const Work& wk, int h) const { return 2 * q + h < wk.hpg; }
+};
+
+// Waits.  The tile loop has to stay inside the instruction cache (about 24 KB: a loop that outgrows it runs at five to
+// ten cycles per instruction), so a wait is only "until the phase is over, or the CTA has given up", and one thread --
+// the TMA producer, whose waits depend on everybody's progress -- holds the clock (guarded_wait).  A role that was
+// released that way runs through its remaining tiles without waiting, on whatever is in the buffers, and leaves.
+// (The phase before a fresh barrier's first counts as over: the parity of "free" in the first round.)
+__device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, const Misc2* m) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .u32 a;\n"
+      "AGAIN:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra DONE;\n\t"
+      "ld.volatile.shared.u32 a, [%2];\n\tsetp.eq.u32 p, a, 0;\n\t@p bra AGAIN;\n"
+      "DONE:\n\t}"
+      ::"r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<int*>(&m->abort_flag)))
+      : "memory");
+  __syncwarp();   // (what follows may be a warp-wide instruction)
+}
+// False when the CTA has given up; gives up with `code` when the bound runs out (twice that of the wait for another
+// CTA's hand-over: everything inside the CTA may be waiting behind that one, and the cause should be what reports).
+__device__ __forceinline__ bool guarded_wait(uint64_t* bar, uint32_t parity, Misc2* m, int code) {
   const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {   // (try_wait parks the thread for a short, hardware-chosen time by itself)
+  while (!mbar_try_wait(bar, parity)) {
     if (m->abort_flag) return false;
-    // (twice the bound of the wait for another CTA's hand-over: everything inside the CTA may be waiting behind
-    //  that one, and the wait that is the cause should be the one that reports)
     if (clock64() - t0 > 2 * m->wait_clocks) {
       m->abort_flag = code;   // reported to the caller's status word at kernel end
       return false;
     }
   }
-  return true;
+  return m->abort_flag == 0;
+}
+// (the same for all lanes of the warp)
+__device__ __forceinline__ bool given_up(const Misc2* m) { return __any_sync(0xffffffffu, m->abort_flag != 0) != 0; }
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+  return r != 0;
 }
 
-// Last act of an MMA-issuing thread: tensor memory is freed at the end of the kernel, so the MMAs this thread
-// has issued must have completed by then -- also when the roles that would have waited for them gave up
-// (bounded, like every wait).
-__device__ __forceinline__ void drain_mmas(Misc2* m, int which) {
-  umma_commit(&m->bar_drain[which]);
-  const long long t0 = clock64();
-  while (!mbar_try_wait(&m->bar_drain[which], 0))
-    if (clock64() - t0 > m->wait_clocks) break;
+// D <- A . B over STEPS k-steps of 16: four MMAs in line (instruction cache), the operands advancing by `ai` / `bi` inside
+// the four and by `ao` / `bo` from one four to the next (descriptor units).
+template <int STEPS>
+__device__ __forceinline__ void issue(uint32_t d, uint64_t a, uint32_t ai, uint32_t ao, uint64_t b, uint32_t bi, uint32_t bo,
+                                      uint32_t id) {
+#pragma unroll 1
+  for (int o = 0; o < STEPS; o += 4) {
+    umma_ss(d, a, b, id, o);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) umma_ss(d, a + i * ai, b + i * bi, id, 1);
+    a += ao;
+    b += bo;
+  }
 }
 
+// Products of fp32 pairs (one instruction for two elements).
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair(uint32_t a, uint32_t b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+template <typename T16>
+__device__ __forceinline__ uint32_t pack_pair(uint64_t v) {
+  const float2 f = unpair(v);
+  return pack2<T16>(f.x, f.y);
+}
 
 // EPI: apply the skip and gate of model_ref.py:116-118 to Y on its way out (sp.D / sp.Z; either may be null).
 template <typename T16, int N, bool EPI>
@@ -222,6 +308,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   constexpr int NB = L::NB;
   constexpr int KN = N / 16;
   constexpr int KT = T / 16;
+  constexpr int BC = L::kBC;
+  constexpr int XS = L::kXSlots;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   Misc2* m = reinterpret_cast<Misc2*>(smem + L::oMisc);
@@ -234,301 +322,331 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   //  hand-over, so the CTA that continues its sequence runs into the bound of its wait)
   if (sp.inject_lost_handover && sp.chain && blockIdx.x == 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool want_y = sp.compute_y != 0;
   int32_t* status = sp.status;
 
   if (tid == 0) {
-    mbar_init(&m->full_b, 1); mbar_init(&m->full_c, 1);
-    // B is released by the G MMA and the S MMA; C by the G MMA and the C.H MMA
-    mbar_init(&m->empty_b, want_y ? 2 : 1); mbar_init(&m->empty_c, 2);   // (a state-only item inside a Y launch: the S issuer commits twice)
-    mbar_init(&m->bar_g, 1);
-    mbar_init(&m->bar_yo, 1); mbar_init(&m->bar_s, 1);
+    for (int s = 0; s < BC; ++s) {
+      mbar_init(&m->full_b[s], 1); mbar_init(&m->full_c[s], 1);
+      mbar_init(&m->empty_b[s], 1); mbar_init(&m->empty_c[s], 1);
+    }
+    // an X slot is handed back by four warps: those that read out Y from it, or those that made Xd of a state-only tile
+    for (int s = 0; s < XS; ++s) { mbar_init(&m->full_x[s], 1); mbar_init(&m->empty_x[s], 4); }
+    mbar_init(&m->bar_g, 1); mbar_init(&m->bar_s, 1); mbar_init(&m->bar_ch, 1);
     mbar_init(&m->bar_xd, 8); mbar_init(&m->bar_h, 8); mbar_init(&m->bar_e, 8);
     for (int h = 0; h < 2; ++h) {
-      // an X stage is handed back by the head's warpgroup once it is done with it (in Y mode: after the stage
-      // has served as the source of the TMA store of Y)
-      for (int s = 0; s < kXStages; ++s) {
-        mbar_init(&m->full_x[h][s], 1);
-        mbar_init(&m->empty_x[h][s], 4);   // Y items: the thread that issued the TMA store of Y arrives for all four
-      }
       mbar_init(&m->bar_y[h], 1);
-      mbar_init(&m->bar_p[h], 4);   // one arrival per compute warp (lane 0, after a warp barrier)
+      mbar_init(&m->bar_p[h], 4);
+      // factors are released by the head's four warps (P) and the four read-out warps
+      for (int s = 0; s < 2; ++s) { mbar_init(&m->full_f[h][s], 1); mbar_init(&m->empty_f[h][s], 8); }
     }
-    for (int i = 0; i < 3; ++i) mbar_init(&m->bar_drain[i], 1);
+    mbar_init(&m->bar_drain, 1);
     m->abort_flag = 0;
     m->wait_clocks = sp.wait_clocks;
-    work_list(prm, &m->work);
-    for (int i = 0; i < m->work.count; ++i) {
-      const Item wi = work_item(prm, m->work, i);
-      if (wi.yflag) m->work.ytot += wi.ntiles;
-    }
+    work_list(prm, m->work);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&m->tmem_base, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tb = m->tmem_base;
-  const uint32_t tG = tb;
+  constexpr uint32_t tG = 0, tSP = 128, tYo = 256, tYd = 384;   // (all 512 columns are ours: the allocation starts at 0)
   const uint32_t sB = smem_u32(smem + L::oB), sC = smem_u32(smem + L::oC), sX = smem_u32(smem + L::oX);
   const uint32_t sXd = smem_u32(smem + L::oXd), sH = smem_u32(smem + L::oH);
-
+  const Work& wk = m->work;
+  const uint32_t total = m->tmem_base == 0 ? (uint32_t)wk.total : 0u, npre = (uint32_t)wk.npre;
+  // One arrival per warp: every lane has issued its fences, the warp barrier orders their writes before
+  // lane 0's arrive (128 per-thread arrivals on one mbarrier cost several hundred cycles per hand-off).
+  auto warp_arrive = [&](uint64_t* bar) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+  };
+  // Registers: 128 x 512 at launch, re-divided 64 | 168 | 168 | 112 (the sum may not exceed what was launched).
   if (warp < 4) {
-    setmaxnreg_dec<72>();   // 128*72 + 256*216 = 384*168: the CTA can only re-divide its own allocation
+    setmaxnreg_dec<64>();
     if (warp == 0 && lane == 0) {
       // ---------------------------------------------------------------- TMA producer
       prefetch_tmap(&tmX); prefetch_tmap(&tmB); prefetch_tmap(&tmC); prefetch_tmap(&tmY);
       bool ok = true;
-      uint32_t it = 0;    // running tile ordinal of this CTA
-      uint32_t ity = 0;   // ... counting the tiles of Y-producing items only (C is loaded for those)
-      const Work wk = m->work;
-      for (int wi = 0; wi < wk.count && ok; ++wi) {
-        const Item w = work_item(prm, wk, wi);
-        for (int j = 0; j < w.ntiles && ok; ++j, ++it) {
-          const int t0 = w.t_begin + j * T;
-          const uint32_t st = it % kXStages, use = it / kXStages;
-          for (int h = 0; h < 2 && ok; ++h) {
-            if (use > 0) ok = wait2(&m->empty_x[h][st], (use - 1) & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status);
-            if (!ok) break;
-            mbar_expect_tx(&m->full_x[h][st], kBlk);
-            tma_load_4d(smem + L::oX + (kXStages * h + st) * kBlk, &tmX, &m->full_x[h][st], 0, w.h0 + h, t0, w.bi);
-          }
+      uint32_t xi = 0, xph = 0;              // next X slot and how often the ring has been walked (parity)
+      uint32_t bs = 0, bph = 0, cs = 0, cph = 0;   // the same for B and C
+      Cursor c;
+#pragma unroll 1
+      for (uint32_t n = 0; n < total && ok; ++n) {
+        c.next(prm, wk);
+        // X of both heads, B, then C (not for a state-only tile).  B before C: the B tile is free earlier, and the S MMA
+        // that waits for it is on the state's chain.
+#pragma unroll 1
+        for (int k = 0; k < (n < npre ? 3 : 4); ++k) {
+          const CUtensorMap* tm = k < 2 ? &tmX : k == 2 ? &tmB : &tmC;
+          uint64_t* full = k < 2 ? &m->full_x[xi] : k == 2 ? &m->full_b[bs] : &m->full_c[cs];
+          uint64_t* empty = k < 2 ? &m->empty_x[xi] : k == 2 ? &m->empty_b[bs] : &m->empty_c[cs];
+          const uint32_t ph = k < 2 ? xph : k == 2 ? bph : cph;
+          uint32_t dst = k < 2 ? sX + xi * kBlk : k == 2 ? sB + bs * (NB * kBlk) : sC + cs * (NB * kBlk);
+          const int blocks = k < 2 ? 1 : NB;
+          ok = guarded_wait(empty, ph ^ 1, m, STATUS_WAIT_TIMEOUT_MMA);
           if (!ok) break;
-          // B before C: the B tile is free as soon as the previous tile's G and S MMAs are done, the C tile only once
-          // its C.H MMA is, which waits for the read-out of the tile before; the S MMA of this tile must not wait that long.
-          if (it > 0) ok = wait2(&m->empty_b, (it - 1) & 1, m, STATUS_WAIT_TIMEOUT_MMA, status);
-          if (!ok) break;
-          mbar_expect_tx(&m->full_b, NB * kBlk);
-#pragma unroll
-          for (int kb = 0; kb < NB; ++kb)
-            tma_load_4d(smem + L::oB + kb * kBlk, &tmB, &m->full_b, 64 * kb, w.gi, t0, w.bi);
-          if (!ok) break;
-          if (w.yflag) {
-            if (ity > 0) ok = wait2(&m->empty_c, (ity - 1) & 1, m, STATUS_WAIT_TIMEOUT_MMA, status);
-            if (!ok) break;
-            mbar_expect_tx(&m->full_c, NB * kBlk);
-#pragma unroll
-            for (int kb = 0; kb < NB; ++kb)
-              tma_load_4d(smem + L::oC + kb * kBlk, &tmC, &m->full_c, 64 * kb, w.gi, t0, w.bi);
-            ++ity;
+          mbar_expect_tx(full, blocks * kBlk);
+#pragma unroll 1
+          for (int kb = 0; kb < blocks; ++kb, dst += kBlk)
+            tma_load_5d(dst, tm, full, 64 * kb, k < 2 ? 2 * c.q + k : 0, c.g, c.t0, c.b);
+          if (k < 2) {
+            if (++xi == XS) { xi = 0; xph ^= 1; }
+          } else if (k == 2) {
+            if (++bs == BC) { bs = 0; bph ^= 1; }
+          } else {
+            if (++cs == BC) { cs = 0; cph ^= 1; }
           }
         }
       }
-      if (m->abort_flag && it > 0) {
-        // let copies already in flight land before the CTA gives its shared memory back
-        const uint32_t k = it - 1;
+      if (ok) ok = guarded_wait(&m->bar_drain, 0, m, STATUS_WAIT_TIMEOUT_SYNC);   // (every MMA of the CTA: keeps the clock to the end)
+      if (!ok) {
+        // let copies already in flight land before the CTA gives its shared memory back (a millisecond)
         const long long c0 = clock64();
-        while (clock64() - c0 < 2000000LL) {
-          const uint32_t xs = k % kXStages, xp = (k / kXStages) & 1;
-          if (mbar_try_wait(&m->full_b, k & 1) && mbar_try_wait(&m->full_x[0][xs], xp) &&
-              mbar_try_wait(&m->full_x[1][xs], xp) && (ity == 0 || mbar_try_wait(&m->full_c, (ity - 1) & 1)))
-            break;
-        }
+        while (clock64() - c0 < 2000000LL) { }
       }
-    } else if (warp == 1 && lane == 0) {
-      // ---------------------------------------------------------------- MMA issuer for G = C.B^T (shared by the heads)
-      if (want_y) {
-        constexpr int fmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
-        constexpr uint32_t idG = umma_idesc(128, 128, fmt, 0, 0);
-        constexpr uint64_t dK = umma_desc_base(16, 1024);
-        const Work wk = m->work;
-        bool ok = true;
-        uint32_t it = 0, k = 0;   // tile ordinal over all items / over the Y-producing ones
-        for (int wi = 0; wi < wk.count && ok; ++wi) {
-          const Item w = work_item(prm, wk, wi);
-          if (!w.yflag) { it += w.ntiles; continue; }
-        for (int j = 0; j < w.ntiles && ok; ++j, ++it, ++k) {
-          // both heads are done reading G(k-1); B and C of tile k have landed
-          if (k > 0)
-            ok = wait2(&m->bar_p[0], (k - 1) & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status) &&
-                 wait2(&m->bar_p[1], (k - 1) & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status);
-          ok = ok && wait2(&m->full_c, k & 1, m, STATUS_WAIT_TIMEOUT_TMA, status) &&
-               wait2(&m->full_b, it & 1, m, STATUS_WAIT_TIMEOUT_TMA, status);
-          if (!ok) break;
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < KN; ++kk) {
-            const uint32_t off = (kk >> 2) * kBlk + (kk & 3) * 32;
-            umma_ss(tG, umma_desc(dK, sC + off), umma_desc(dK, sB + off), idG, kk > 0);
-          }
-          umma_commit(&m->bar_g);
-          umma_commit(&m->empty_c);
-          umma_commit(&m->empty_b);
-        }
-        }
-      }
-      drain_mmas(m, 0);
-    } else if (warp == 2 && lane == 0) {
-      // ---------------------------------------------------------------- MMA issuer for S = B^T.[Xd0|Xd1] and Y = C.[H0|H1]
-      // The two heads' Xd (and state copies) lie one 64-column block apart in shared memory, so one
-      // N = 128 MMA serves both heads; it costs the tensor pipe what the N = 64 one does.
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- MMA issuer (one elected thread issues)
       constexpr int fmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
-      constexpr uint32_t idKM = umma_idesc(128, 128, fmt, 0, 1);
-      constexpr uint32_t idMM = umma_idesc(128, 128, fmt, 1, 1);
+      constexpr uint32_t idKK = umma_idesc(128, 128, fmt, 0, 0);   // G
+      constexpr uint32_t idMM = umma_idesc(128, 128, fmt, 1, 1);   // S
+      constexpr uint32_t idKM = umma_idesc(128, 128, fmt, 0, 1);   // C.H
+      constexpr uint32_t idPX = umma_idesc(128, 64, fmt, 0, 1);    // P.X
       constexpr uint64_t dK = umma_desc_base(16, 1024);
-      constexpr uint64_t dMN = umma_desc_base(kBlk, 1024);       // B tile; [Xd0|Xd1]
-      constexpr uint64_t dMNh = umma_desc_base(N * 128, 1024);   // [H0|H1]
-      const uint32_t tS = tb + 128, tY = tb + 256;
-      bool ok = true;
-      uint32_t k0 = 0;   // running tile ordinal of the item's first tile
-      uint32_t ky = 0;   // tile ordinal over the Y-producing items
-      const Work wk = m->work;
-      for (int wi = 0; wi < wk.count && ok; ++wi) {
-        const Item w = work_item(prm, wk, wi);
-        const int nt = w.ntiles;
+      constexpr uint64_t dMN = umma_desc_base(kBlk, 1024);         // B tile; [Xd0|Xd1]; X
+      constexpr uint64_t dMNh = umma_desc_base(N * 128, 1024);     // [H0|H1]
+      constexpr uint32_t kKi = 32 >> 4, kKo = kBlk >> 4, kMi = 2048 >> 4, kMo = 8192 >> 4;   // K-major / MN-major operand steps
+      uint32_t xi = 0;             // X slot of the tile whose P.X is next
+      uint32_t ky = 0;             // Y-producing tiles whose G and C.H have been issued; P.X of the last of them is due
 #pragma unroll 1
-        for (int j = 0; j < nt && ok; ++j) {
-          const uint32_t k = k0 + j;
-          // S <- B^T . Xd
-          ok = wait2(&m->full_b, k & 1, m, STATUS_WAIT_TIMEOUT_TMA, status) &&
-               wait2(&m->bar_xd, k & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status);
-          if (!ok) break;
-          tc_fence_after();
+      for (uint32_t n = 0;; ++n) {
+        if (n > 0) {
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            if (ky > 0) {
+              wait(&m->bar_p[h], (ky - 1) & 1, m);   // (its warps have seen X arrive)
+              tc_fence_after();
+              if (elect_one()) {
+                uint32_t pa = tSP + 64 * h;
+                uint64_t xb = umma_desc(dMN, sX + xi * kBlk);
+#pragma unroll 1
+                for (int o = 0; o < KT; o += 4) {
+                  umma_ts(tYd + 64 * h, pa, xb, idPX, o);
 #pragma unroll
-          for (int kk = 0; kk < KT; ++kk)
-            umma_ss(tS, umma_desc(dMN, sB + kk * 2048), umma_desc(dMN, sXd + kk * 2048), idMM, kk > 0);
+                  for (int i = 1; i < 4; ++i) umma_ts(tYd + 64 * h, pa + 8 * i, xb + i * kMi, idPX, 1);
+                  pa += 32;
+                  xb += kMo;
+                }
+                umma_commit(&m->bar_y[h]);
+              }
+            }
+            if (++xi == XS) xi = 0;
+          }
+        }
+        if (n == total) break;
+        const uint32_t s = n % BC, sc = ky % BC;
+        const uint32_t sBs = sB + s * (NB * kBlk), sCs = sC + sc * (NB * kBlk);
+        // S <- B^T . Xd, into the columns that P of the tile before was read from; then, for a tile that produces Y,
+        // G <- C . B^T (both heads have read G of the tile before: their P is done) and
+        // Yo <- C . H (both heads' Yo and Yd of the tile before have been read out).
+        wait(&m->full_b[s], (n / BC) & 1, m);
+        wait(&m->bar_xd, n & 1, m);
+        wait(&m->bar_y[1], (ky & 1) ^ 1, m);   // (its commit covers head 0's MMAs too)
+        tc_fence_after();
+        if (elect_one()) {
+          issue<KT>(tSP, umma_desc(dMN, sBs), kMi, kMo, umma_desc(dMN, sXd), kMi, kMo, idMM);
           umma_commit(&m->bar_s);
-          umma_commit(&m->empty_b);
-          if (!w.yflag) {
-            // (a state-only item inside a Y launch: no G MMA reads this B tile, its arrival is made here)
-            if (want_y) umma_commit(&m->empty_b);
-            continue;
-          }
-          // Y <- C . H
-          ok = wait2(&m->full_c, ky & 1, m, STATUS_WAIT_TIMEOUT_TMA, status) &&
-               wait2(&m->bar_h, ky & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status);
-          if (ok && ky > 0) ok = wait2(&m->bar_e, (ky - 1) & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status);
-          if (!ok) break;
-          ++ky;
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < KN; ++kk) {
-            const uint32_t off = (kk >> 2) * kBlk + (kk & 3) * 32;
-            umma_ss(tY, umma_desc(dK, sC + off), umma_desc(dMNh, sH + kk * 2048), idKM, kk > 0);
-          }
-          umma_commit(&m->bar_yo);
-          umma_commit(&m->empty_c);
+          if (n < npre) umma_commit(&m->empty_b[s]);
         }
-        k0 += nt;
+        if (n < npre) continue;
+        wait(&m->full_c[sc], (ky / BC) & 1, m);
+        tc_fence_after();
+        if (elect_one()) {
+          issue<KN>(tG, umma_desc(dK, sCs), kKi, kKo, umma_desc(dK, sBs), kKi, kKo, idKK);
+          umma_commit(&m->bar_g);
+          umma_commit(&m->empty_b[s]);
+        }
+        wait(&m->bar_h, ky & 1, m);
+        wait(&m->bar_e, (ky & 1) ^ 1, m);
+        tc_fence_after();
+        if (elect_one()) {
+          issue<KN>(tYo, umma_desc(dK, sCs), kKi, kKo, umma_desc(dMNh, sH), kMi, kMo, idKM);
+          umma_commit(&m->bar_ch);
+          umma_commit(&m->empty_c[sc]);
+        }
+        ++ky;
       }
-      drain_mmas(m, 1);
-    } else if (warp == 3 && lane == 0) {
-      // ---------------------------------------------------------------- MMA issuer for Y_h += P_h . X_h, head 0 then head 1
-      if (want_y) {
-        constexpr int fmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
-        constexpr uint32_t idKM = umma_idesc(128, 64, fmt, 0, 1);
-        constexpr uint64_t dMN = umma_desc_base(kBlk, 1024);
-        const Work wk = m->work;
-        bool ok = true;
-        uint32_t it = 0, k = 0;   // tile ordinal over all items / over the Y-producing ones
-        for (int wi = 0; wi < wk.count && ok; ++wi) {
-          const Item w = work_item(prm, wk, wi);
-          if (!w.yflag) { it += w.ntiles; continue; }
+      // Tensor memory is freed at the end of the kernel: the MMAs issued here must have completed by then (bounded).
+      if (elect_one()) {
+        umma_commit(&m->bar_drain);
+        const long long t0 = clock64();
+        while (!mbar_try_wait(&m->bar_drain, 0))
+          if (clock64() - t0 > m->wait_clocks) break;
+      }
+      __syncwarp();
+    } else if (warp >= 2) {
+      // ---------------------------------------------------------------- prefix sums (warp 2: head 0, warp 3: head 1)
+      // Lane i owns tokens i, 32 + i, 64 + i, 96 + i; the next tile's values are on their way while this one's are used.
+      const int h = warp - 2;
+      const bool has_dt = sp.dt != nullptr;
+      float an[4];
+      T16 dn[4];
+      const float* Ag = nullptr;
+      const T16* Dg = nullptr;
+      Cursor c;
 #pragma unroll 1
-        for (int j = 0; j < w.ntiles && ok; ++j, ++it, ++k) {
-          const uint32_t st = it % kXStages;
-#pragma unroll 1
-          for (int h = 0; h < 2 && ok; ++h) {
-            ok = wait2(&m->bar_p[h], k & 1, m, STATUS_WAIT_TIMEOUT_SYNC, status) &&
-                 wait2(&m->full_x[h][st], (it / kXStages) & 1, m, STATUS_WAIT_TIMEOUT_TMA, status);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t tY = tb + 256 + 64 * h, tP = tb + 384 + 64 * h;
+      for (uint32_t k = 0; k <= total; ++k) {
+        float a0 = an[0], a1 = an[1], a2 = an[2], a3 = an[3];
+        T16 d0 = dn[0], d1 = dn[1], d2 = dn[2], d3 = dn[3];
+        if (k < total) {
+          c.next(prm, wk);
+          const int t = c.t0 + lane;
+          const int in = c.live(wk, h) ? sp.seqlen - t : 0;   // past the end: decay 1 and x = 0, the state stays as it is
+          if (__builtin_expect(c.first_tile(), 0)) {          // (later tiles of the item: where the last one ended)
+            const int head = c.head(wk) + h;
+            Ag = sp.A + c.b * sp.as[0] + head * sp.as[2] + t * sp.as[1];
+            Dg = static_cast<const T16*>(sp.dt) + c.b * sp.dts[0] + head * sp.dts[2] + t * sp.dts[1];
+          }
 #pragma unroll
-            for (int kk = 0; kk < KT; ++kk)
-              umma_ts(tY, tP + 8 * kk, umma_desc(dMN, sX + (kXStages * h + st) * kBlk + kk * 2048), idKM, 1);
-            umma_commit(&m->bar_y[h]);
+          for (int e = 0; e < 4; ++e) {
+            an[e] = 0.f;
+            dn[e] = Cvt<T16>::from_f(1.f);
+            if (32 * e < in) {
+              an[e] = *Ag;
+              if (has_dt) dn[e] = *Dg;
+            }
+            Ag += 32 * sp.as[1];
+            Dg += 32 * sp.dts[1];
           }
         }
+        if (k == 0) continue;
+        const uint32_t n = k - 1, par = n & 1;
+        wait(&m->empty_f[h][par], ((n >> 1) & 1) ^ 1, m);
+        Factors& f = m->f[h][par];
+        float base = 0.f, keep[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int b32 = 0; b32 < 4; ++b32) {
+          const int r = 32 * b32 + lane;
+          float cs = a0;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, cs, d);
+            if (lane >= d) cs += t;
+          }
+          cs += base;
+          base = __shfl_sync(0xffffffffu, cs, 31);   // at the end of the 32-token block
+          const float dt = Cvt<T16>::to_f(d0);
+          const float cs2 = cs * kLog2e;
+          f.cs2[r] = cs2;
+          f.cf[r] = ex2(base * kLog2e - cs2) * dt;
+          // dt multiplies the columns of P instead of the rows of X (P.(dt o x) = (P o dt_s).x), so the X tile stays as
+          // loaded (clamped: dt == 0 must not break the chain of ratios; the clamped column then weighs 2^-60, i.e.
+          // nothing).  The ratios are clamped too: one above the diagonal may overflow, it is masked out by a select.
+          const float cc = cs2 - fmaxf(lg2(dt), -60.f);   // (lg2(1) is 0)
+          const float ratio = ex2(fminf(__shfl_up_sync(0xffffffffu, cc, 1) - cc, 126.f));
+          f.dg[r] = (lane & 3) == 0 ? cc : ratio;
+          keep[0] = keep[1]; keep[1] = keep[2]; keep[2] = keep[3]; keep[3] = cs;
+          a0 = a1; a1 = a2; a2 = a3;
+          const T16 t16 = d0;
+          d0 = d1; d1 = d2; d2 = d3; d3 = t16;       // (back where they were after four steps)
         }
+#pragma unroll 1
+        for (int b32 = 0; b32 < 4; ++b32) {
+          f.xs[32 * b32 + lane] = (uint16_t)pack2<T16>(ex2((base - keep[0]) * kLog2e) * Cvt<T16>::to_f(d0), 0.f);
+          keep[0] = keep[1]; keep[1] = keep[2]; keep[2] = keep[3];
+          d0 = d1; d1 = d2; d2 = d3;
+        }
+        if (lane == 0) f.tot = base;
+        warp_arrive(&m->full_f[h][par]);
       }
-      drain_mmas(m, 2);
     }
-  } else {
-    // ------------------------------------------------------------------ compute warpgroups (warps 4-7: head 0, 8-11: head 1)
-    setmaxnreg_inc<216>();
+  } else if (warp < 12) {
+    // ------------------------------------------------------------------ warps 4-7: head 0, 8-11: head 1
+    setmaxnreg_inc<168>();
     const int h = (warp - 4) >> 2;
-    const int lane_base = (warp & 3) * 32;
-    const int l = lane_base + lane;
     const int q = warp & 3;
+    const int lane_base = q * 32;
+    const int l = lane_base + lane;
     const uint32_t tlane = (uint32_t)lane_base << 16;
     const uint32_t swz = (uint32_t)(l & 7);
     const bool owns_state = lane_base < N;
-    const uint32_t tS = tb + 128 + 64 * h, tY = tb + 256 + 64 * h, tP = tb + 384 + 64 * h;
+    const uint32_t tS = tSP + 64 * h, tP = tSP + 64 * h;
     const uint32_t sHh = sH + h * (N * 128), sXdh = sXd + h * kBlk;
-    const int bar_id = 1 + h;
 
-    uint32_t it = 0;    // running tile ordinal of this CTA
-    uint32_t ity = 0;   // ... counting the tiles of Y-producing items only
-    bool ok = true;
-    auto cwait = [&](uint64_t* bar, uint32_t parity, int code) {
-      return __all_sync(0xffffffffu, wait2(bar, parity, m, code, status)) != 0;
-    };
-    // One arrival per warp: every lane has issued its fences, the warp barrier orders their writes before
-    // lane 0's arrive (128 per-thread arrivals on one mbarrier cost several hundred cycles per hand-off).
-    auto warp_arrive = [&](uint64_t* bar) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar);
-    };
-
-    float H[P];
-    float cs = 0.f, tot = 0.f, cs2 = 0.f;   // of the tile whose P / Y is being produced
-    // dt multiplies the columns of P instead of the rows of X (P.(dt o x) = (P o dt_s).x), so the X tile stays as
-    // loaded: this row's value as a column of the diagonal mask block is cs2 - log2(dt) (clamped: dt == 0 must not
-    // break the chain of per-token factors there; the clamped column then weighs 2^-60, i.e. nothing).
-    float cs2c = 0.f;
-    // log-decay / dt of this thread's row in the next tile to be scanned.  dt stays as loaded (16 bits) until the scan uses
-    // it one iteration later: a conversion right behind the load would hold the warp for the whole memory latency.
-    float a_next = 0.f;
-    T16 dt_next = Cvt<T16>::from_f(1.f);
-    bool next_prefetched = false;
-    bool store_pending = false;    // (thread l == 0) a TMA store of Y is in flight from X stage store_stage
-    uint32_t store_stage = 0;
+    uint64_t H[P / 2];               // fp32 pairs
+#pragma unroll
+    for (int e = 0; e < P / 2; ++e) H[e] = 0;
+    float asum0 = 0.f;               // log-decay summed over the earlier pieces of the sequence
     float asum = 0.f, acomp = 0.f;   // compensated (Kahan) sum of the tile totals; FP64 is slow on this part
 
-    // prefix sum of the log-decay over the 128 rows (model_ref.py:135); publishes cs*log2(e) for the P step
-    auto scan_tile = [&](float a, float dtv, uint32_t par, float& cs_o, float& tot_o, float& cs2_o,
-                         float& cs2c_o) {
-      float v = a;
+    // A. P = (C B^T) o exp(segsum), causal -> TMEM (A operand, 16-bit pairs).  Decay mask per 32-token column block J of
+    // this warp's 32 rows (block q is the diagonal one):
+    //   J == q: exp2(cs_l - cs_s), causal, one ex2 per four columns and the ratios between neighbours;
+    //   J <  q: exp(cs_l - cs_s) = rf_J[l] * cf[s] with both factors <= 1 for non-positive log-decays
+    //           (rf_J[l] = exp(cs_l - cs_end(J)), cf[s] = exp(cs_end(J) - cs_s)): two multiplies;
+    //   J >  q: zero.
+    auto make_p = [&](const Factors& f) {
+      const float cs2 = f.cs2[l];
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        uint32_t g[16];
+        tmem_ld16(tG + tlane + 32 * q + 16 * half, g);
+        const float4* dv = reinterpret_cast<const float4*>(&f.dg[32 * q + 16 * half]);
+        const int ln = lane - 16 * half;
+        tmem_ld_wait();
+        uint32_t pk[8];
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, v, d);
-        if (lane >= d) v += t;
+        for (int e4 = 0; e4 < 4; ++e4) {
+          const float4 d = dv[e4];
+          const float w0 = ex2(cs2 - d.x), w1 = w0 * d.y, w2 = w1 * d.z, w3 = w2 * d.w;
+          const float v0 = __uint_as_float(g[4 * e4]) * w0, v1 = __uint_as_float(g[4 * e4 + 1]) * w1;
+          const float v2 = __uint_as_float(g[4 * e4 + 2]) * w2, v3 = __uint_as_float(g[4 * e4 + 3]) * w3;
+          pk[2 * e4] = pack2<T16>(4 * e4 <= ln ? v0 : 0.f, 4 * e4 + 1 <= ln ? v1 : 0.f);
+          pk[2 * e4 + 1] = pack2<T16>(4 * e4 + 2 <= ln ? v2 : 0.f, 4 * e4 + 3 <= ln ? v3 : 0.f);
+        }
+        tmem_st8(tP + tlane + 16 * q + 8 * half, pk);
       }
-      if (lane == 31) m->wsum[h][q] = v;
-      named_bar_sync(bar_id, 128);
-      const float w0 = m->wsum[h][0], w1 = m->wsum[h][1], w2 = m->wsum[h][2], w3 = m->wsum[h][3];
-      cs_o = v + ((q > 0 ? w0 : 0.f) + (q > 1 ? w1 : 0.f) + (q > 2 ? w2 : 0.f));
-      tot_o = (w0 + w1 + w2) + w3;
-      cs2_o = cs_o * kLog2e;
-      // column factor of the factored decay mask: exp(cs at the end of this row's 32-token block - cs_row)
-      // (times dt of the row: the factor belongs to the row as a column of P)
-      m->cf[h][par][l] = ex2(__shfl_sync(0xffffffffu, cs2_o, 31) - cs2_o) * dtv;
-      cs2c_o = cs2_o - fmaxf(__log2f(dtv), -60.f);
-      if (lane == 31) m->cend[h][par][q] = cs2_o;
-      // the row's scale for Xd (model_ref.py:144,148), for whichever thread turns that row of X into Xd
-      m->xs[h][l] = (uint16_t)pack2<T16>(ex2((tot_o - cs_o) * kLog2e) * dtv, 0.f);
-      named_bar_sync(bar_id, 128);
+#pragma unroll 1
+      for (int J = 0; J < q; ++J) {   // strictly below the diagonal
+        uint32_t g[32];
+        tmem_ld32(tG + tlane + 32 * J, g);
+        const float rf = ex2(cs2 - f.cs2[32 * J + 31]);
+        const uint64_t rf2 = pair(rf, rf);
+        const ulonglong2* fv = reinterpret_cast<const ulonglong2*>(&f.cf[32 * J]);
+        tmem_ld_wait();
+        uint32_t pk[16];
+#pragma unroll
+        for (int e4 = 0; e4 < 8; ++e4) {
+          const ulonglong2 c = fv[e4];
+          pk[2 * e4] = pack_pair<T16>(mul_pair(pair(g[4 * e4], g[4 * e4 + 1]), mul_pair(rf2, c.x)));
+          pk[2 * e4 + 1] = pack_pair<T16>(mul_pair(pair(g[4 * e4 + 2], g[4 * e4 + 3]), mul_pair(rf2, c.y)));
+        }
+        tmem_st16(tP + tlane + 16 * J, pk);
+      }
+      if (q < 3) {
+        uint32_t pz[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) pz[e] = 0u;
+#pragma unroll 1
+        for (int J = q + 1; J < 4; ++J) tmem_st16(tP + tlane + 16 * J, pz);
+      }
     };
-    // Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148) from X stage `st` into this head's Xd buffer, in packed
-    // 16-bit arithmetic as the reference does it.  The rows are not dealt out evenly: the mask step that follows gives
-    // warp q (rows 32q..32q+31 of the causal P) q + 1 blocks of 32 columns to fill, and the four warps meet at the next
-    // tile's prefix sum, so the warps with fewer mask blocks take more rows here.  Eight lanes share a row (one 16-byte
-    // piece each), a warp moves four rows per instruction ("a quad": 32 quads per tile).
-    auto make_xd = [&](uint32_t st, bool with_mask) {
+    // B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148) from X slot at `xb` into this head's Xd buffer, in packed
+    // 16-bit arithmetic as the reference does it.  The rows are not dealt out evenly: warp q has q + 1 blocks of P to
+    // fill, so the warps with fewer blocks take more rows here.  Eight lanes share a row (one 16-byte piece each), a
+    // warp moves four rows per instruction ("a quad": 32 quads per tile).
+    auto make_xd = [&](uint32_t xb, const Factors& f, bool with_mask) {
       // first quad of warp 0..3 and the end, one byte each: 0 14 24 30 32 when all four warps also update and copy the
       // state (N = 128), 0 10 18 26 32 when only warps 0 and 1 do
       constexpr uint64_t kFirst = N == 128 ? 0x201E180E00ull : 0x201A120A00ull;
       const int qb = with_mask ? (int)((kFirst >> (8 * q)) & 0xff) : 8 * q;
       const int qe = with_mask ? (int)((kFirst >> (8 * q + 8)) & 0xff) : 8 * q + 8;
-      const uint32_t xb = sX + (kXStages * h + st) * kBlk;
       const uint32_t sub = (uint32_t)lane >> 3, pc = (uint32_t)lane & 7u;
 #pragma unroll 1
       for (int qd = qb; qd < qe; qd += 2) {   // (every share is an even number of quads)
         const uint32_t r0 = 4 * qd + sub, r1 = r0 + 4;
         const uint32_t o0 = r0 * 128 + ((pc ^ (r0 & 7u)) << 4), o1 = r1 * 128 + ((pc ^ (r1 & 7u)) << 4);
         const uint4 a0 = lds128(xb + o0), a1 = lds128(xb + o1);
-        const uint32_t s0 = m->xs[h][r0], s1 = m->xs[h][r1];
+        const uint32_t s0 = f.xs[r0], s1 = f.xs[r1];
         const uint32_t d0 = s0 | (s0 << 16), d1 = s1 | (s1 << 16);
         uint4 v;
         v.x = mul2<T16>(a0.x, d0); v.y = mul2<T16>(a0.y, d0); v.z = mul2<T16>(a0.z, d0); v.w = mul2<T16>(a0.w, d0);
@@ -542,466 +660,316 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint4 v;
-          v.x = pack2<T16>(H[8 * c + 0], H[8 * c + 1]); v.y = pack2<T16>(H[8 * c + 2], H[8 * c + 3]);
-          v.z = pack2<T16>(H[8 * c + 4], H[8 * c + 5]); v.w = pack2<T16>(H[8 * c + 6], H[8 * c + 7]);
+          v.x = pack_pair<T16>(H[4 * c]); v.y = pack_pair<T16>(H[4 * c + 1]);
+          v.z = pack_pair<T16>(H[4 * c + 2]); v.w = pack_pair<T16>(H[4 * c + 3]);
           sts128(sHh + l * 128 + ((c ^ swz) << 4), v);
         }
       }
     };
-
-    // ---- e. Y -> global, for the tile whose P.X MMA was started one step earlier (its latency is spent in the
-    //      next tile's state update).  Returns false when a wait gave up.
-    bool y_pending = false;
-    uint32_t y_it = 0, y_ity = 0;
-    int y_hi = 0, y_t0 = 0, y_bi = 0;
-    float y_dskip = 0.f;   // (EPI) D of the head whose tile is queued: loaded when the tile is queued, used a tile later
-    auto finish_y = [&]() -> bool {
-      // (EPI) the gate rows of this warp's 32 tokens, fetched ahead of the wait for the MMA.  Eight lanes read one
-      // 128-byte row per load (whole lines), four rows per instruction; the rows reach their threads through the
-      // staging buffer below.
-      uint4 zr[8];
-      if constexpr (EPI) {
-        if (sp.Z) {
-          const T16* zbase = static_cast<const T16*>(sp.Z) + y_bi * sp.zs[0] + y_hi * sp.zs[2] + 8 * (lane & 7);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int row = lane_base + 4 * i + (lane >> 3);
-            zr[i] = __ldg(reinterpret_cast<const uint4*>(zbase + (int64_t)(y_t0 + row) * sp.zs[1]));
-          }
-          // the next tile's gate rows as far as L2 (one row per lane), so that the loads above find them there
-          if (y_t0 + T + lane_base + lane < sp.seqlen)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T16*>(sp.Z) + y_bi * sp.zs[0] + y_hi * sp.zs[2] +
-                                                         (int64_t)(y_t0 + T + lane_base + lane) * sp.zs[1]));
-        }
-      }
-      if (!cwait(&m->bar_y[h], y_ity & 1, STATUS_WAIT_TIMEOUT_MMA)) return false;
-      tc_fence_after();
-      // The X stage of that tile is dead (its P.X MMA is complete): stage the 16-bit Y rows there; one
-      // thread then hands the whole tile to the TMA engine.
-      const uint32_t xst = y_it % kXStages;
-      const uint32_t ystage = sX + (kXStages * h + xst) * kBlk;
-      {
-        uint32_t y0[32], y1[32];
-        tmem_ld32(tY + tlane, y0);
-        tmem_ld32(tY + tlane + 32, y1);
-        tmem_ld_wait();
-        tc_fence_before();
-        warp_arrive(&m->bar_e);   // the Y accumulator is read out: the next tile's C.H may overwrite it
-        if constexpr (EPI) {
-          // Y <- (Y + x * D) * silu(z) (model_ref.py:116-118) in fp32; x is this thread's row of the X tile, still in
-          // the stage that the Y rows go to; silu(z) = z * (0.5 + 0.5 tanh(z / 2)), the tanh on 16-bit pairs.
-          const bool gate = sp.Z != nullptr;
-          if (sp.D) {
-            const float dskip = y_dskip;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const uint4 xr = lds128(ystage + l * 128 + ((c ^ swz) << 4));
-              const uint32_t xw[4] = {xr.x, xr.y, xr.z, xr.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                uint32_t* yy = (c < 4) ? &y0[8 * c + 2 * e] : &y1[8 * (c - 4) + 2 * e];
-                const float2 xf = unpack2<T16>(xw[e]);
-                yy[0] = __float_as_uint(fmaf(xf.x, dskip, __uint_as_float(yy[0])));
-                yy[1] = __float_as_uint(fmaf(xf.y, dskip, __uint_as_float(yy[1])));
-              }
-            }
-          }
-          if (gate) {
-            // x is consumed: the warp's gate rows go through its 32 rows of the stage to the threads that own them
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int row = lane_base + 4 * i + (lane >> 3);
-              sts128(ystage + row * 128 + ((((uint32_t)lane & 7u) ^ ((uint32_t)row & 7u)) << 4), zr[i]);
-            }
-            __syncwarp();
-            const uint32_t half2 = pack2<T16>(0.5f, 0.5f);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const uint4 zq = lds128(ystage + l * 128 + ((c ^ swz) << 4));
-              const uint32_t zw[4] = {zq.x, zq.y, zq.z, zq.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                uint32_t* yy = (c < 4) ? &y0[8 * c + 2 * e] : &y1[8 * (c - 4) + 2 * e];
-                // silu(z) = z * (0.5 + 0.5 tanh(z / 2)) on the packed 16-bit pair, as the reference forms it in
-                // half precision (model_ref.py:118); the product with Y is taken in fp32
-                const uint32_t sg = fma2<T16>(tanh2<T16>(mul2<T16>(zw[e], half2)), half2, half2);
-                const float2 gf = unpack2<T16>(mul2<T16>(zw[e], sg));
-                yy[0] = __float_as_uint(__uint_as_float(yy[0]) * gf.x);
-                yy[1] = __float_as_uint(__uint_as_float(yy[1]) * gf.y);
-              }
+    // (bounded) wait until the four warps of head h of CTAs `from` .. `to` have published.  Every warp asks for itself: a
+    // barrier among the four would hang where one of them has given up.
+    auto wait_published = [&](int to, int from) {
+      if (lane == 0) {
+        const long long c0 = clock64();
+        for (int c = to; c >= from && !m->abort_flag; --c) {
+          while (true) {
+            int f;
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + 2 * c + h) : "memory");
+            if (f >= 4 || m->abort_flag) break;
+            if (clock64() - c0 > m->wait_clocks) {
+              m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
+              break;
             }
           }
         }
+      }
+      __syncwarp();
+    };
+    // The state entering an item.
+    Cursor c;
+    auto enter_item = [&](bool wy) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint4 o;
-          o.x = pack2<T16>(__uint_as_float(y0[8 * c + 0]), __uint_as_float(y0[8 * c + 1]));
-          o.y = pack2<T16>(__uint_as_float(y0[8 * c + 2]), __uint_as_float(y0[8 * c + 3]));
-          o.z = pack2<T16>(__uint_as_float(y0[8 * c + 4]), __uint_as_float(y0[8 * c + 5]));
-          o.w = pack2<T16>(__uint_as_float(y0[8 * c + 6]), __uint_as_float(y0[8 * c + 7]));
-          sts128(ystage + l * 128 + ((c ^ swz) << 4), o);
+      for (int e = 0; e < P / 2; ++e) H[e] = 0;
+      asum0 = asum = acomp = 0.f;
+      const bool look_back = sp.chain == 2;
+      const bool cut_front = sp.chain && c.t_begin > 0 && !(look_back && !wy);   // (the look-back scan starts from zero)
+      const bool init = sp.init && c.live(wk, h) && !(look_back && !wy) && (!cut_front || look_back);
+      // Chained: what the CTA before this one handed over.  Look-back: fold the pairs (state from zero, log-decay
+      // sum) that the CTAs from .. before this one published for their pieces of this sequence, newest first:
+      // H_in = sum_c exp(log-decay after c) F_c (+ the same for the caller's initial state).
+      int p = cut_front ? (int)blockIdx.x - 1 : 0;
+      const int from = cut_front ? (look_back ? wk.from : p) : 1;
+      if (cut_front) wait_published(p, from);
+#pragma unroll 1
+      for (;; --p) {
+        const float* src;
+        if (p >= from) {
+          src = sp.chain_state + (2 * p + h) * (int64_t)(N * P);
+        } else {
+          if (!init) break;
+          src = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride;
         }
+        const float wgt = ex2(asum0 * kLog2e);   // asum0: log-decay between the end of the piece being added and this item
+        if (owns_state && wgt != 0.f) {          // (an underflowed piece adds nothing)
+          const float4* I = reinterpret_cast<const float4*>(src + (int64_t)l * P);
+          const uint64_t w2 = pair(wgt, wgt);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint4 o;
-          o.x = pack2<T16>(__uint_as_float(y1[8 * c + 0]), __uint_as_float(y1[8 * c + 1]));
-          o.y = pack2<T16>(__uint_as_float(y1[8 * c + 2]), __uint_as_float(y1[8 * c + 3]));
-          o.z = pack2<T16>(__uint_as_float(y1[8 * c + 4]), __uint_as_float(y1[8 * c + 5]));
-          o.w = pack2<T16>(__uint_as_float(y1[8 * c + 6]), __uint_as_float(y1[8 * c + 7]));
-          sts128(ystage + l * 128 + (((4 + c) ^ swz) << 4), o);
+          for (int e = 0; e < P / 4; ++e) {
+            const float4 v = __ldcg(I + e);      // (may be written by another SM: bypass L1)
+            H[2 * e] = fma_pair(w2, pair(v.x, v.y), H[2 * e]);
+            H[2 * e + 1] = fma_pair(w2, pair(v.z, v.w), H[2 * e + 1]);
+          }
+        }
+        if (p < from) break;
+        asum0 += __ldcg(sp.chain_ld + 2 * p + h);
+      }
+    };
+    // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
+    auto leave_item = [&](bool wy) {
+      const bool cut_back = sp.chain && c.t_begin / T + c.ntiles < wk.nt;
+      const bool publish = cut_back && !(sp.chain == 2 && wy);   // (look-back: only the state-only scan publishes)
+      const int64_t slot = 2 * (int64_t)blockIdx.x + h;
+      const int64_t unit = (int64_t)c.b * sp.nheads + c.head(wk) + h;
+      const int seg = sp.chain ? 0 : c.seg;
+      if (publish ? given_up(m) : (cut_back || !c.live(wk, h))) return;
+      float* to = publish ? sp.chain_state + slot * (N * P)
+                          : (sp.fin ? sp.fin + unit * sp.fin_unit_stride + seg * sp.fin_seg_stride : nullptr);
+      float* ld = publish ? sp.chain_ld + slot
+                          : (sp.fin_ld ? sp.fin_ld + unit * sp.finld_unit_stride + seg * sp.finld_seg_stride : nullptr);
+      if (to && owns_state) {
+        ulonglong2* F = reinterpret_cast<ulonglong2*>(to + (int64_t)l * P);
+#pragma unroll
+        for (int e = 0; e < P / 4; ++e) F[e] = make_ulonglong2(H[2 * e], H[2 * e + 1]);
+      }
+      if (ld && l == 0) *ld = asum0 + asum;
+      if (publish) {
+        // Each warp publishes its own rows: a release-add by lane 0 after a warp barrier orders the
+        // whole warp's stores before the count, and nobody has to wait for the stores to land.
+        __syncwarp();
+        if (lane == 0) {
+          const int one = 1;
+          asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + slot), "r"(one) : "memory");
         }
       }
-      fence_proxy_async();         // staged rows -> visible to the TMA engine
-      named_bar_sync(bar_id, 128);
-      if (l == 0) {
-        // The previous store must be done reading its stage before the producer may refill it.
-        if (store_pending) {
-          bulk_wait_read_all();
-          mbar_arrive_n(&m->empty_x[h][store_stage], 4);
-        }
-        tma_store_4d(&tmY, ystage, 0, y_hi, y_t0, y_bi);
-        bulk_commit();
-        store_pending = true;
-        store_stage = xst;
-      }
-      y_pending = false;
-      return true;
     };
 
-    const Work wk = m->work;
-    // (one pass more than there are items: an empty item whose only iteration reads out the last Y tile, so that
-    //  the read-out code exists once)
-    for (int wi = 0; wi <= wk.count && ok; ++wi) {
-      Item w = {};
-      if (wi < wk.count) w = work_item(prm, wk, wi);
-      if (w.ntiles == 0 && wi < wk.count) continue;
-      const int hi = w.h0 + h;
-      const bool wy = w.yflag != 0;   // this item produces Y (a look-back launch starts with a state-only item)
-      const int64_t unit = (int64_t)w.bi * sp.nheads + hi;
-      const float* Ag = sp.A + w.bi * sp.as[0] + hi * sp.as[2];
-      const T16* Dg = sp.dt ? static_cast<const T16*>(sp.dt) + w.bi * sp.dts[0] + hi * sp.dts[2] : nullptr;
-
-      float asum0 = 0.f;   // log-decay summed over the earlier segments of a chained sequence
-      asum = 0.f;
-      acomp = 0.f;
-      if (!next_prefetched && w.ntiles > 0) {   // (the first item of this CTA; later items were prefetched during their predecessor)
-        a_next = Ag[(int64_t)(w.t_begin + l) * sp.as[1]];
-        dt_next = Dg ? Dg[(int64_t)(w.t_begin + l) * sp.dts[1]] : Cvt<T16>::from_f(1.f);
+    bool cur_y = false;
+    uint32_t xi = h, xph = 0;   // X slot of the tile being prepared
+    uint32_t ky = 0;            // Y-producing tiles prepared
+#pragma unroll 1
+    for (uint32_t n = 0;; ++n) {   // tile n is prepared, P of tile n - 1 is made
+      if (cur_y) {
+        wait(&m->bar_g, (ky - 1) & 1, m);
+        tc_fence_after();
+        const uint32_t par = (n - 1) & 1;
+        make_p(m->f[h][par]);
+        tmem_st_wait();
+        tc_fence_before();
+        warp_arrive(&m->bar_p[h]);
+        if (lane == 0) mbar_arrive(&m->empty_f[h][par]);
       }
-      next_prefetched = false;
-
-      // Iteration j = -1 only prepares tile 0 (state copy, prefix sum, Xd); iteration j >= 0 finishes
-      // tile j (steps a, b, d, e) and prepares tile j + 1 (step c) in between, so that the S MMA of the
-      // next tile runs under steps d and e.  One copy of each step keeps the loop inside the
-      // instruction cache.
-#pragma unroll 1
-      for (int j = -1; j < w.ntiles && ok; ++j) {
-        const int t0 = w.t_begin + j * T;
-        const bool have_next = (j + 1 < w.ntiles);
-        if (j >= 0) {
-          // ---- a. state: H <- exp(cs_last) H + S
-          ok = cwait(&m->bar_s, it & 1, STATUS_WAIT_TIMEOUT_MMA);
-          if (!ok) break;
-          tc_fence_after();
-          {
-            const float yk = tot - acomp, tk = asum + yk;
-            acomp = (tk - asum) - yk;
-            asum = tk;
-          }
-          if (owns_state) {
-            const float g = ex2(tot * kLog2e);
-            uint32_t sv0[32], sv1[32];
-            tmem_ld32(tS + tlane, sv0);
-            tmem_ld32(tS + tlane + 32, sv1);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) H[e] = fmaf(H[e], g, __uint_as_float(sv0[e]));
-#pragma unroll
-            for (int e = 0; e < 32; ++e) H[32 + e] = fmaf(H[32 + e], g, __uint_as_float(sv1[e]));
-          }
-        }
-        // ---- state leaving the item: it is final once the last tile's update (step a) is done, so it is
-        //      handed over here, ahead of the rest of that tile; the next item's first log-decays are fetched too
-        if (j >= 0 && !have_next) {
-          const bool hand_over = w.out_slot >= 0;
-          if (hand_over) {
-            const int64_t slot = 2 * w.out_slot + h;
-            if (owns_state) {
-              float4* F = reinterpret_cast<float4*>(sp.chain_state + slot * (int64_t)(N * P) + (int64_t)l * P);
-    #pragma unroll
-              for (int j = 0; j < P / 4; ++j) F[j] = make_float4(H[4 * j], H[4 * j + 1], H[4 * j + 2], H[4 * j + 3]);
-            }
-            if (l == 0) sp.chain_ld[slot] = asum0 + asum;
-            // Each warp publishes its own rows: a release-add by lane 0 after a warp barrier orders the
-            // whole warp's stores before the count, and nobody has to wait for the stores to land.
-            __syncwarp();
-            if (lane == 0) {
-              const int one = 1;
-              asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + slot), "r"(one) : "memory");
-            }
-          } else if (w.ends_seq) {
-            // last (or only) segment of the sequence: the caller's outputs
-            const int fseg = sp.chain ? 0 : w.seg;
-            if (sp.fin && owns_state) {
-              float4* F = reinterpret_cast<float4*>(sp.fin + unit * sp.fin_unit_stride + fseg * sp.fin_seg_stride +
-                                                    (int64_t)l * P);
-    #pragma unroll
-              for (int j = 0; j < P / 4; ++j) F[j] = make_float4(H[4 * j], H[4 * j + 1], H[4 * j + 2], H[4 * j + 3]);
-            }
-            if (sp.fin_ld && l == 0)
-              sp.fin_ld[unit * sp.finld_unit_stride + fseg * sp.finld_seg_stride] = asum0 + asum;
-          }
-          if (wi + 1 < wk.count) {
-            const Item wn = work_item(prm, wk, wi + 1);
-            if (wn.ntiles > 0) {
-              const int hn = wn.h0 + h;
-              a_next = sp.A[wn.bi * sp.as[0] + hn * sp.as[2] + (int64_t)(wn.t_begin + l) * sp.as[1]];
-              if (sp.dt)
-                dt_next = static_cast<const T16*>(sp.dt)[wn.bi * sp.dts[0] + hn * sp.dts[2] +
-                                                          (int64_t)(wn.t_begin + l) * sp.dts[1]];
-              next_prefetched = true;
-            }
-          }
-        }
-        if (y_pending) {   // (j == -1: the previous item's last tile)
-          ok = finish_y();
-          if (!ok) break;
-        }
-        // ---- c. next tile: prefix sum and Xd (the S MMA that read the Xd buffer was waited for in step a)
-        float cs_n = 0.f, tot_n = 0.f, cs2_n = 0.f, cs2c_n = 0.f;
-        if (have_next) {
-          const uint32_t itn = (j >= 0) ? it + 1 : it;
-          const float a = a_next, dtv = Cvt<T16>::to_f(dt_next);
-          if (j + 2 < w.ntiles) {
-            a_next = Ag[(int64_t)(t0 + 2 * T + l) * sp.as[1]];
-            if (Dg) dt_next = Dg[(int64_t)(t0 + 2 * T + l) * sp.dts[1]];
-          }
-          scan_tile(a, dtv, itn & 1, cs_n, tot_n, cs2_n, cs2c_n);
-          ok = cwait(&m->full_x[h][itn % kXStages], (itn / kXStages) & 1, STATUS_WAIT_TIMEOUT_TMA);
-          if (!ok) break;
-          make_xd(itn % kXStages, wy);
-          fence_proxy_async();
-          warp_arrive(&m->bar_xd);
-          if (!wy) warp_arrive(&m->empty_x[h][itn % kXStages]);   // nothing else reads X of a state-only item
-        }
-        // ---- state entering the item (after the first tile's Xd is on its way to the S MMA: the wait for a
-        //      chained predecessor and the state load then overlap that MMA)
-        if (j == -1 && w.ntiles > 0) {
-          if (w.in_slot >= 0 && sp.chain == 2) {
-            // Look-back: fold the pairs (state from zero, log-decay sum) that the CTAs fold_from..in_slot published
-            // for their pieces of this sequence, newest first: H_in = sum_c exp(log-decay after c) F_c (+ the same
-            // for the caller's initial state).  Wait (bounded) until all of them are there.
-            if (l == 0) {
-              const long long c0 = clock64();
-              for (int c = w.in_slot; c >= w.fold_from && !m->abort_flag; --c) {
-                while (true) {
-                  int f;
-                  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + 2 * c + h) : "memory");
-                  if (f >= 4) break;   // all four warps of that CTA's warpgroup have published
-                  if (m->abort_flag) break;
-                  if (clock64() - c0 > m->wait_clocks) {
-                    m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
-                    break;
-                  }
-                }
-              }
-            }
-            named_bar_sync(bar_id, 128);
-            if (m->abort_flag) { ok = false; break; }
-#pragma unroll
-            for (int e = 0; e < P; ++e) H[e] = 0.f;
-            float dsum = 0.f;   // log-decay between the end of the piece being added and the start of this one
-            for (int c = w.in_slot; c >= w.fold_from; --c) {
-              const int64_t slot = 2 * c + h;
-              const float wgt = ex2(dsum * kLog2e);
-              if (owns_state && wgt != 0.f) {   // (a piece whose weight has underflowed adds nothing)
-                const float4* I = reinterpret_cast<const float4*>(sp.chain_state + slot * (int64_t)(N * P) + (int64_t)l * P);
-#pragma unroll
-                for (int e = 0; e < P / 4; ++e) {
-                  const float4 v = __ldcg(I + e);   // written by another SM: bypass L1
-                  H[4 * e] = fmaf(wgt, v.x, H[4 * e]); H[4 * e + 1] = fmaf(wgt, v.y, H[4 * e + 1]);
-                  H[4 * e + 2] = fmaf(wgt, v.z, H[4 * e + 2]); H[4 * e + 3] = fmaf(wgt, v.w, H[4 * e + 3]);
-                }
-              }
-              dsum += __ldcg(sp.chain_ld + slot);
-            }
-            if (sp.init && owns_state) {
-              const float wgt = ex2(dsum * kLog2e);
-              const float4* I = reinterpret_cast<const float4*>(sp.init + unit * sp.init_unit_stride + (int64_t)l * P);
-#pragma unroll
-              for (int e = 0; e < P / 4; ++e) {
-                const float4 v = I[e];
-                H[4 * e] = fmaf(wgt, v.x, H[4 * e]); H[4 * e + 1] = fmaf(wgt, v.y, H[4 * e + 1]);
-                H[4 * e + 2] = fmaf(wgt, v.z, H[4 * e + 2]); H[4 * e + 3] = fmaf(wgt, v.w, H[4 * e + 3]);
-              }
-            }
-            asum0 = dsum;
-          } else if (w.in_slot >= 0) {
-            // wait (bounded) for the previous segment of this unit, which another CTA may still be finishing
-            const int64_t slot = 2 * w.in_slot + h;
-            if (l == 0) {
-              const long long c0 = clock64();
-              while (true) {
-                int f;
-                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + slot) : "memory");
-                if (f >= 4) break;   // all four warps of the predecessor's warpgroup have published
-                if (m->abort_flag) break;
-                if (clock64() - c0 > m->wait_clocks) {
-                  m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
-                  break;
-                }
-              }
-            }
-            named_bar_sync(bar_id, 128);
-            if (m->abort_flag) { ok = false; break; }
-            if (owns_state) {
-              const float4* I = reinterpret_cast<const float4*>(sp.chain_state + slot * (int64_t)(N * P) + (int64_t)l * P);
-    #pragma unroll
-              for (int j = 0; j < P / 4; ++j) {
-                const float4 v = __ldcg(I + j);   // written by another SM: bypass L1
-                H[4 * j] = v.x; H[4 * j + 1] = v.y; H[4 * j + 2] = v.z; H[4 * j + 3] = v.w;
-              }
-            } else {
-    #pragma unroll
-              for (int j = 0; j < P; ++j) H[j] = 0.f;
-            }
-            asum0 = __ldcg(sp.chain_ld + slot);
-          } else if (sp.init && owns_state && !(sp.chain == 2 && !wy)) {   // (the look-back scan starts from zero)
-            const float4* I = reinterpret_cast<const float4*>(sp.init + unit * sp.init_unit_stride +
-                                                              w.seg * sp.init_seg_stride + (int64_t)l * P);
-    #pragma unroll
-            for (int j = 0; j < P / 4; ++j) {
-              const float4 v = I[j];
-              H[4 * j] = v.x; H[4 * j + 1] = v.y; H[4 * j + 2] = v.z; H[4 * j + 3] = v.w;
-            }
-          } else {
-    #pragma unroll
-            for (int j = 0; j < P; ++j) H[j] = 0.f;
-          }
-        }
-        if (l == 0 && store_pending) {
-          // the Y store issued in the previous tile's step e has finished reading its stage by now: hand it back
-          bulk_wait_read_all();
-          mbar_arrive_n(&m->empty_x[h][store_stage], 4);
-          store_pending = false;
-        }
-        if (j >= 0) {
-          if (wy) {
-            // ---- d. P = (C B^T) o exp(segsum), causal -> TMEM (A operand, 16-bit pairs)
-            ok = cwait(&m->bar_g, ity & 1, STATUS_WAIT_TIMEOUT_MMA);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t par = it & 1;
-            // Decay mask per 32-token column block J of this warp's 32 rows (block q is the diagonal one):
-            //   J == q: exp2(cs_l - cs_s), causal, one ex2 per element;
-            //   J <  q: exp(cs_l - cs_s) = rf_J[l] * cf[s] with both factors <= 1 for non-positive
-            //           log-decays (rf_J[l] = exp(cs_l - cs_end(J)), cf[s] = exp(cs_end(J) - cs_s)): two multiplies;
-            //   J >  q: zero, written once (nothing else ever writes those TMEM columns).
-            {
-              // diagonal block first: its TMEM load is in flight while the factors are fetched
-              uint32_t gd[32];
-              tmem_ld32(tG + tlane + 32 * q, gd);
-              tmem_ld_wait();
-              // One ex2 per four columns: exp(cs_l - cs_{s+1}) = exp(cs_l - cs_s) * exp(-a_{s+1}), the per-token
-              // factor exp(-a) coming from the lane that owns the row (clamped: an entry above the diagonal may
-              // overflow, it is masked out by a select, never multiplied into anything that is kept).
-              const float einv = ex2(fminf(__shfl_up_sync(0xffffffffu, cs2c, 1) - cs2c, 126.f));
-              uint32_t pk[16];
-#pragma unroll
-              for (int e4 = 0; e4 < 8; ++e4) {
-                const float c0 = __shfl_sync(0xffffffffu, cs2c, 4 * e4);   // the column's value: from the lane owning that row
-                const float f1 = __shfl_sync(0xffffffffu, einv, 4 * e4 + 1), f2 = __shfl_sync(0xffffffffu, einv, 4 * e4 + 2);
-                const float f3 = __shfl_sync(0xffffffffu, einv, 4 * e4 + 3);
-                const float w0 = ex2(cs2 - c0), w1 = w0 * f1, w2 = w1 * f2, w3 = w2 * f3;
-                const float v0 = __uint_as_float(gd[4 * e4]) * w0, v1 = __uint_as_float(gd[4 * e4 + 1]) * w1;
-                const float v2 = __uint_as_float(gd[4 * e4 + 2]) * w2, v3 = __uint_as_float(gd[4 * e4 + 3]) * w3;
-                pk[2 * e4] = pack2<T16>(4 * e4 <= lane ? v0 : 0.f, 4 * e4 + 1 <= lane ? v1 : 0.f);
-                pk[2 * e4 + 1] = pack2<T16>(4 * e4 + 2 <= lane ? v2 : 0.f, 4 * e4 + 3 <= lane ? v3 : 0.f);
-              }
-              tmem_st16(tP + tlane + 16 * q, pk);
-            }
-#pragma unroll 1
-            for (int J = 0; J < q; ++J) {   // strictly below the diagonal
-              uint32_t gv[32];
-              tmem_ld32(tG + tlane + 32 * J, gv);
-              const float rf = ex2(cs2 - m->cend[h][par][J]);
-              float4 fq[8];
-              const float4* fv = reinterpret_cast<const float4*>(&m->cf[h][par][32 * J]);
-#pragma unroll
-              for (int e4 = 0; e4 < 8; ++e4) fq[e4] = fv[e4];
-              tmem_ld_wait();
-              uint32_t pk[16];
-#pragma unroll
-              for (int e4 = 0; e4 < 8; ++e4) {
-                const float w0 = rf * fq[e4].x, w1 = rf * fq[e4].y, w2 = rf * fq[e4].z, w3 = rf * fq[e4].w;
-                pk[2 * e4] = pack2<T16>(__uint_as_float(gv[4 * e4]) * w0, __uint_as_float(gv[4 * e4 + 1]) * w1);
-                pk[2 * e4 + 1] = pack2<T16>(__uint_as_float(gv[4 * e4 + 2]) * w2, __uint_as_float(gv[4 * e4 + 3]) * w3);
-              }
-              tmem_st16(tP + tlane + 16 * J, pk);
-            }
-            if (ity == 0) {
-              uint32_t pz[16];
-#pragma unroll
-              for (int e = 0; e < 16; ++e) pz[e] = 0u;
-#pragma unroll 1
-              for (int J = q + 1; J < 4; ++J) tmem_st16(tP + tlane + 16 * J, pz);
-            }
-            // ---- b. Y <- exp(cs_l) * (C.H) in place (after P: the C.H MMA could only start once the previous
-            //      tile's Y had been read out, so it runs under step d); the P.X MMA accumulates on top
-            ok = cwait(&m->bar_yo, ity & 1, STATUS_WAIT_TIMEOUT_MMA);
-            if (!ok) break;
-            tc_fence_after();
-            const float el = ex2(cs2);
-            {
-              uint32_t y0[32], y1[32];
-              tmem_ld32(tY + tlane, y0);
-              tmem_ld32(tY + tlane + 32, y1);
-              tmem_ld_wait();
-#pragma unroll
-              for (int e = 0; e < 32; ++e) y0[e] = __float_as_uint(__uint_as_float(y0[e]) * el);
-              tmem_st32(tY + tlane, y0);
-#pragma unroll
-              for (int e = 0; e < 32; ++e) y1[e] = __float_as_uint(__uint_as_float(y1[e]) * el);
-              tmem_st32(tY + tlane + 32, y1);
-            }
-            tmem_st_wait();
-            tc_fence_before();
-            warp_arrive(&m->bar_p[h]);   // P is written and Y is scaled: the P.X MMA may run
-          }
-        }
-        // (all C.H MMAs that read the state copy have been waited for: the previous item's in its step b)
-        if (wy && have_next) {
-          store_hb();
-          fence_proxy_async();
-          warp_arrive(&m->bar_h);
-        }
-        if (j >= 0) {
-          if (wy) {
-            y_pending = true;
-            y_it = it; y_ity = ity; y_hi = hi; y_t0 = t0; y_bi = w.bi;
-            if constexpr (EPI) {
-              if (sp.D) y_dskip = sp.D[hi];
-            }
-            ++ity;
-          }
-          ++it;
-        }
-        cs = cs_n; tot = tot_n; cs2 = cs2_n; cs2c = cs2c_n;
+      if (n == total) break;
+      c.next(prm, wk);
+      const bool wy = n >= npre;   // this tile produces Y (a look-back launch starts with a state-only item)
+      const uint32_t par = n & 1;
+      const Factors& f = m->f[h][par];
+      wait(&m->full_f[h][par], (n >> 1) & 1, m);
+      wait(&m->full_x[xi], xph, m);
+      make_xd(sX + xi * kBlk, f, wy);   // (the S MMA that read the Xd buffer was waited for in step E)
+      fence_proxy_async();
+      warp_arrive(&m->bar_xd);
+      if (!wy && lane == 0) mbar_arrive(&m->empty_x[xi]);   // nothing else reads X of a state-only tile
+      xi += 2;
+      if (xi >= XS) { xi -= XS; xph ^= 1; }
+      // D. (after Xd is on its way: the wait for another CTA's state and its load overlap the S MMA)
+      if (__builtin_expect(c.first_tile(), 0)) enter_item(wy);
+      if (wy) {
+        wait(&m->bar_ch, (ky & 1) ^ 1, m);   // the C.H MMA has read the copy before this one
+        store_hb();
+        fence_proxy_async();
+        warp_arrive(&m->bar_h);
+        ++ky;
       }
-      if (!ok) break;
-
+      // E. H <- exp(cs_last) H + S
+      const float tot = f.tot;
+      if (!wy) warp_arrive(&m->empty_f[h][par]);
+      const float gs = ex2(tot * kLog2e);
+      {
+        const float yk = tot - acomp, tk = asum + yk;
+        acomp = (tk - asum) - yk;
+        asum = tk;
+      }
+      wait(&m->bar_s, n & 1, m);
+      tc_fence_after();
+      if (owns_state) {
+        const uint64_t g2 = pair(gs, gs);
+        uint32_t s0[32], s1[32];
+        tmem_ld32(tS + tlane, s0);
+        tmem_ld32(tS + tlane + 32, s1);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) H[e] = fma_pair(H[e], g2, pair(s0[2 * e], s0[2 * e + 1]));
+#pragma unroll
+        for (int e = 0; e < 16; ++e) H[16 + e] = fma_pair(H[16 + e], g2, pair(s1[2 * e], s1[2 * e + 1]));
+      }
+      if (__builtin_expect(c.left == 0, 0)) leave_item(wy);
+      cur_y = wy;
     }
-    if (l == 0) bulk_wait_all();   // the Y tiles this thread stored must have landed before the CTA exits
+  } else {
+    // ------------------------------------------------------------------ warps 12-15: read-out of Y, both heads
+    setmaxnreg_dec<112>();
+    const int lane_base = (warp & 3) * 32;
+    const int l = lane_base + lane;
+    const uint32_t tlane = (uint32_t)lane_base << 16;
+    const uint32_t swz = (uint32_t)(l & 7);
+    Cursor c;
+    uint32_t xi = 0;
+    uint32_t ky = 0;
+    int pending = -1;    // (lane 0) X slot that this warp's last TMA store still reads
+#pragma unroll 1
+    for (uint32_t n = 0; n < total; ++n) {
+      c.next(prm, wk);
+      if (n < npre) {    // (takes its turn in the factors' ring all the same)
+        for (int h = 0; h < 2; ++h) {
+          wait(&m->full_f[h][n & 1], (n >> 1) & 1, m);
+          if (lane == 0) mbar_arrive(&m->empty_f[h][n & 1]);
+        }
+        xi += 2;
+        if (xi >= XS) xi -= XS;
+        continue;
+      }
+      const int t0 = c.t0;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const bool live = c.live(wk, h);
+        // (EPI) the gate rows of this warp's 32 tokens, fetched ahead of the wait for the MMA.  Four lanes read half a
+        // 128-byte row per load, eight rows per instruction; the rows reach their threads through the staging buffer below.
+        uint4 zr[8];
+        float dskip = 0.f;
+        if constexpr (EPI) {
+          if (sp.D && live) dskip = sp.D[c.head(wk) + h];
+          if (sp.Z && live) {
+            const T16* zbase = static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] + (c.head(wk) + h) * sp.zs[2] + 8 * (lane & 3);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int tok = t0 + lane_base + 8 * i + (lane >> 2);
+              if (tok < sp.seqlen) {
+                const uint4* zp = reinterpret_cast<const uint4*>(zbase + (int64_t)tok * sp.zs[1]);
+                zr[i] = __ldg(zp);
+                zr[4 + i] = __ldg(zp + 4);
+              }
+            }
+          }
+        }
+        wait(&m->full_f[h][n & 1], (n >> 1) & 1, m);
+        const float el = ex2(m->f[h][n & 1].cs2[l]);
+        warp_arrive(&m->empty_f[h][n & 1]);
+        wait(&m->bar_y[h], ky & 1, m);
+        tc_fence_after();
+        if (lane == 0 && pending >= 0) {
+          bulk_wait_read_all();
+          mbar_arrive(&m->empty_x[pending]);
+        }
+        const uint64_t el2 = pair(el, el);
+        // The X tile is dead (its P.X MMA is complete): the 16-bit Y rows are staged in its slot.
+        const uint32_t ystage = sX + xi * kBlk;
+        const uint32_t yrow = ystage + l * 128;
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          uint32_t o[32], d[32];
+          tmem_ld32(tYo + 64 * h + tlane + 32 * half, o);
+          tmem_ld32(tYd + 64 * h + tlane + 32 * half, d);
+          tmem_ld_wait();
+          if (half == 1) {
+            tc_fence_before();
+            warp_arrive(&m->bar_e);   // both accumulators are read out
+          }
+          uint64_t y[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) y[e] = fma_pair(pair(o[2 * e], o[2 * e + 1]), el2, pair(d[2 * e], d[2 * e + 1]));
+          if constexpr (EPI) {
+            // Y <- (Y + x * D) * silu(z) (model_ref.py:116-118) in fp32; x is this thread's row of the X tile, still in
+            // the slot that the Y rows go to; silu(z) = z * (0.5 + 0.5 tanh(z / 2)), the tanh on 16-bit pairs.
+            if (sp.D && live) {
+              const uint64_t ds = pair(dskip, dskip);
+#pragma unroll
+              for (int cc = 0; cc < 4; ++cc) {
+                const uint4 xr = lds128(yrow + (((4 * half + cc) ^ swz) << 4));
+                const uint32_t xw[4] = {xr.x, xr.y, xr.z, xr.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 xf = unpack2<T16>(xw[e]);
+                  y[4 * cc + e] = fma_pair(pair(xf.x, xf.y), ds, y[4 * cc + e]);
+                }
+              }
+            }
+            if (sp.Z && live) {
+              // x of this half is consumed: the warp's gate rows go through its 32 rows of the slot to the threads that
+              // own them (four lanes hold the four 16-byte pieces of one row's half)
+              __syncwarp();
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int row = lane_base + 8 * i + (lane >> 2);
+                sts128(ystage + row * 128 + (((4 * half + (lane & 3)) ^ (row & 7)) << 4), half ? zr[4 + i] : zr[i]);
+              }
+              __syncwarp();
+              const uint32_t half2 = pack2<T16>(0.5f, 0.5f);
+#pragma unroll
+              for (int cc = 0; cc < 4; ++cc) {
+                const uint4 zq = lds128(yrow + (((4 * half + cc) ^ swz) << 4));
+                const uint32_t zw[4] = {zq.x, zq.y, zq.z, zq.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  // silu(z) = z * (0.5 + 0.5 tanh(z / 2)) on the packed 16-bit pair, as the reference forms it in
+                  // half precision (model_ref.py:118); the product with Y is taken in fp32
+                  const uint32_t sg = fma2<T16>(tanh2<T16>(mul2<T16>(zw[e], half2)), half2, half2);
+                  const float2 gf = unpack2<T16>(mul2<T16>(zw[e], sg));
+                  y[4 * cc + e] = mul_pair(y[4 * cc + e], pair(gf.x, gf.y));
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) {
+            uint4 v;
+            v.x = pack_pair<T16>(y[4 * cc]); v.y = pack_pair<T16>(y[4 * cc + 1]);
+            v.z = pack_pair<T16>(y[4 * cc + 2]); v.w = pack_pair<T16>(y[4 * cc + 3]);
+            sts128(yrow + (((4 * half + cc) ^ swz) << 4), v);
+          }
+        }
+        fence_proxy_async();         // staged rows -> visible to the TMA engine
+        __syncwarp();
+        if (lane == 0) {
+          // each warp hands its own 32 rows to the TMA engine; rows past the end of the sequence are clipped
+          if (live && t0 + lane_base < sp.seqlen) {
+            tma_store_5d(&tmY, ystage + lane_base * 128, 0, 2 * c.q + h, c.g, t0 + lane_base, c.b);
+            bulk_commit();
+          }
+          pending = (int)xi;
+        }
+        if (++xi == XS) xi = 0;
+      }
+      ++ky;
+    }
+    if (lane == 0) {
+      if (pending >= 0) {
+        bulk_wait_read_all();
+        mbar_arrive(&m->empty_x[pending]);
+      }
+      bulk_wait_all();   // the Y rows this warp stored must have landed before the CTA exits
+    }
   }
 
   // ---------------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && m->abort_flag && status) atomicCAS(status, 0, (int)m->abort_flag);
+  if (tid == 0 && status) {
+    if (m->tmem_base != 0) atomicCAS(status, 0, (int)STATUS_TMEM_ALLOC);
+    if (m->abort_flag) atomicCAS(status, 0, (int)m->abort_flag);
+  }
   if (warp == 0) {
     __syncwarp();
-    tmem_dealloc(tb, 512);
+    tmem_dealloc(m->tmem_base, 512);
   }
 }
 
@@ -1013,18 +981,27 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return SSD_ERR_CUDA;
   // chained mode: the tiles of all sequences are dealt out evenly, every CTA gets at least one
-  const long long tiles = (long long)prm.upairs * (prm.sp.seqlen / T);
+  const long long tiles = (long long)prm.upairs * ((prm.sp.seqlen + T - 1) / T);
   const int grid = prm.sp.chain ? (int)std::min<long long>(tiles, kSms) : std::min(prm.nitems, kSms);
   kern<<<grid, kThreads2, smem, stream>>>(tx, tb, tc, ty, prm);
   return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
 
+// Head pairs over the whole batch; a group with an odd number of heads has a half-empty pair.
+int64_t unit_pairs(const SsdArgs& a) { return (int64_t)a.batch * a.ngroups * ((a.nheads / a.ngroups + 1) / 2); }
+
 }  // namespace
 
-bool tc2_supports(const SsdArgs& a) {
-  if (!tc_supports(a)) return false;
-  const int hpg = a.nheads / a.ngroups;
-  return a.nheads % 2 == 0 && hpg % 2 == 0;
+bool tc_supports(const SsdArgs& a) {
+  if (a.dtype != SSD_DTYPE_F16 && a.dtype != SSD_DTYPE_BF16) return false;
+  if (a.headdim != P || (a.dstate != 64 && a.dstate != 128)) return false;
+  if (!ok16(a.X) || !ok16(a.B) || !stride_ok(a.x_stride) || !stride_ok(a.b_stride)) return false;
+  const bool state_only = (a.flags & SSD_FLAG_STATE_ONLY) != 0;
+  if (!state_only) {
+    if (!a.C || !a.Y) return true;  // shape query without pointers (kernel_name / workspace_bytes)
+    if (!ok16(a.C) || !ok16(a.Y) || !stride_ok(a.c_stride) || !stride_ok(a.y_stride)) return false;
+  }
+  return true;
 }
 
 // Rounds of `items` equal work items over the persistent grid, as a fraction of the ideal.
@@ -1043,14 +1020,14 @@ static double round_efficiency(int64_t items) {
 //      states, which a sequence-sharded forward makes around its exchange.
 int tc2_chain_mode(const SsdArgs& a, int nseg) {
   if (nseg <= 1) return 0;
-  const int64_t upairs = (int64_t)a.batch * a.nheads / 2;
+  const int64_t upairs = unit_pairs(a);
   if (upairs >= kSms) return 1;
   return (a.flags & (SSD_FLAG_STATE_ONLY | SSD_FLAG_REUSE_SEGMENTS)) ? 0 : 2;
 }
 
 int tc2_default_segments(const SsdArgs& a) {
-  const int64_t upairs = (int64_t)a.batch * a.nheads / 2;
-  const int tiles = a.seqlen / T;
+  const int64_t upairs = unit_pairs(a);
+  const int tiles = (a.seqlen + T - 1) / T;
   // whole sequences already fill the rounds of the persistent grid well: no cuts; else the even deal (any count
   // above one selects it, the cut points follow from the grid)
   if (upairs >= kSms) return (round_efficiency(upairs) >= 0.97 || tiles < 2) ? 1 : 2;
@@ -1083,14 +1060,17 @@ int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
   if (sp.seg_len % T != 0) return SSD_ERR_UNSUPPORTED;
   Tc2Params prm;
   prm.sp = sp;
-  prm.upairs = a.batch * (a.nheads / 2);
+  prm.ppg = (a.nheads / a.ngroups + 1) / 2;
+  const int64_t upairs = unit_pairs(a);
+  if (upairs * sp.nseg > 0x7fffffffLL || upairs * ((a.seqlen + T - 1) / T) > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
+  prm.upairs = (int)upairs;
   prm.nitems = prm.upairs * sp.nseg;
   CUtensorMap tx, tb, tc, ty;
-  if (!make_map(&tx, a.X, a.dtype, a.headdim, a.nheads, a.seqlen, a.batch, a.x_stride)) return SSD_ERR_CUDA;
-  if (!make_map(&tb, a.B, a.dtype, a.dstate, a.ngroups, a.seqlen, a.batch, a.b_stride)) return SSD_ERR_CUDA;
+  if (!make_map(&tx, a.X, a, P, a.nheads / a.ngroups, a.x_stride, T)) return SSD_ERR_CUDA;
+  if (!make_map(&tb, a.B, a, a.dstate, 1, a.b_stride, T)) return SSD_ERR_CUDA;
   if (sp.compute_y) {
-    if (!make_map(&tc, a.C, a.dtype, a.dstate, a.ngroups, a.seqlen, a.batch, a.c_stride)) return SSD_ERR_CUDA;
-    if (!make_map(&ty, a.Y, a.dtype, a.headdim, a.nheads, a.seqlen, a.batch, a.y_stride)) return SSD_ERR_CUDA;
+    if (!make_map(&tc, a.C, a, a.dstate, 1, a.c_stride, T)) return SSD_ERR_CUDA;
+    if (!make_map(&ty, a.Y, a, P, a.nheads / a.ngroups, a.y_stride, 32)) return SSD_ERR_CUDA;
   } else {
     tc = tb;
     ty = tx;

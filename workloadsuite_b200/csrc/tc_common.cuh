@@ -120,16 +120,19 @@ inline EncodeFn encode_fn() {
   return fn;
 }
 
-// [b, s, heads, inner] 16-bit tensor viewed innermost-first; box = 64 inner x 1 head x 128 tokens x 1 batch.
-inline bool make_map(CUtensorMap* tm, const void* base, int dtype, int inner, int heads, int s, int b, const int64_t* st) {
+// [b, s, groups * per_group, inner] 16-bit tensor viewed as (inner, rows of a group, groups, s, b), so that a pair of heads
+// that reaches past its group reads zeros there instead of the next group's first head; box = 64 inner x 1 x `rows` tokens.
+inline bool make_map(CUtensorMap* tm, const void* base, const SsdArgs& a, int inner, int per_group, const int64_t* st, int rows) {
   EncodeFn fn = encode_fn();
   if (!fn) return false;
-  const cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)heads, (cuuint64_t)s, (cuuint64_t)b};
-  const cuuint64_t strides[3] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[1] * 2, (cuuint64_t)st[0] * 2};
-  const cuuint32_t box[4] = {64, 1, (cuuint32_t)T, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUtensorMapDataType dt = dtype == SSD_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  return fn(tm, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const cuuint64_t dims[5] = {(cuuint64_t)inner, (cuuint64_t)per_group, (cuuint64_t)a.ngroups, (cuuint64_t)a.seqlen,
+                              (cuuint64_t)a.batch};
+  const cuuint64_t strides[4] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[2] * 2 * per_group, (cuuint64_t)st[1] * 2,
+                                 (cuuint64_t)st[0] * 2};
+  const cuuint32_t box[5] = {64, 1, 1, (cuuint32_t)rows, 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUtensorMapDataType dt = a.dtype == SSD_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  return fn(tm, dt, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
