@@ -9,17 +9,19 @@
 //   warp 0        TMA producer
 //   warp 1        MMA issuer: P.X(t) per head, then S(t+1), G(t+1), C.H(t+1)
 //   warps 2, 3    prefix sum of the log-decay (model_ref.py:135) and every factor derived from it, one head each, up to
-//                 two tiles ahead; the other roles read the factors from shared memory
+//                 four tiles ahead; the other roles read the factors from shared memory
 //   warps 4-7     head 0, warps 8-11 head 1: thread = tile row = TMEM lane.  Per iteration, in this order:
 //     A. P(t)   = G o exp(segsum) o causal  (:139-145)  -> TMEM, the A operand of Yd = P.X
-//     B. Xd(t+1) = exp(cs_last - cs) x~     (:144,148)  -> shared memory -> S = B^T.Xd
 //     D. 16-bit copy of the state entering tile t+1     -> shared memory -> Yo = C.H   (:160-161)
 //     E. H <- exp(cs_last) H + S(t+1)       (:150,156)  in fp32 registers
-//   warps 12-15   Y(t) = Yd + exp(cs) Yo (:162) [+ skip and gate, :116-118] -> shared memory -> TMA store, both heads
+//   warps 12-15   both heads, in this order:
+//     B. Xd(t+1) = exp(cs_last - cs) x~     (:144,148)  -> shared memory -> S = B^T.Xd
+//     Y(t) = Yd + exp(cs) Yo (:162) [+ skip and gate, :116-118] -> shared memory -> TMA store
 //
 // What bounds it.  A 128xNx16 tcgen05.mma takes 62 cycles at N = 128 and 55 at N = 64 (any operand layout), so the
 // four contractions of a tile pair need 2 430 tensor-pipe cycles; HBM needs 2 800 cycles per SM for its 64 KB of X
-// and Y.  The state recurrence is the only true chain.  Tensor memory (512 columns) is what limits overlap: G 128,
+// and Y.  The loop that sets the period is A -> P.X -> S -> E -> A, which is
+// why Xd has other warps than P (with B in the warps of A, D and E a tile took 5 400 cycles).  Tensor memory (512 columns) is what limits overlap: G 128,
 // Yo 128, Yd 128 and 128 columns that S and P take turns in -- S(t+1) is consumed (step E) before P(t+1) is written
 // (step A), and S(t+1) is issued once P.X(t) has read P(t).  Keeping Yo and Yd apart means that nothing has to be
 // scaled in place between C.H and P.X, and that C.H(t+1) and the reloads of B and C run under steps A, B and D.
@@ -55,7 +57,7 @@ struct Layout2 {
   static constexpr int oXd = oX + kXSlots * kBlk;        // [head]
   static constexpr int oH = oXd + 2 * kBlk;              // [head], N rows of 128 B
   static constexpr int oMisc = oH + 2 * N * 128;
-  static constexpr int kMiscBytes = 10240;
+  static constexpr int kMiscBytes = 16384;
   static constexpr int kBytes = oMisc + kMiscBytes;   // no slack: the dynamic segment must start 1024-byte aligned
 };
 
@@ -94,14 +96,17 @@ struct alignas(16) Factors {
   float tot;          // cs_last
 };
 
+constexpr int kFactors = 4;   // tiles that the prefix sums may be ahead
+
 struct Misc2 {
   Work work;
-  Factors f[2][2];                    // [head][tile parity]
+  Factors f[2][kFactors];             // [head][tile ordinal % kFactors]
   uint64_t full_b[2], full_c[2], empty_b[2], empty_c[2];   // [stage]
   uint64_t full_x[6], empty_x[6];
-  uint64_t full_f[2][2], empty_f[2][2];   // factors [head][tile parity]
+  uint64_t full_f[2][kFactors], empty_f[2][kFactors];
   uint64_t bar_g, bar_s, bar_ch, bar_y[2];   // tcgen05.commit arrivals (S and C.H serve both heads at once)
-  uint64_t bar_xd, bar_h, bar_e;      // one arrival per warp and head (8)
+  uint64_t bar_h, bar_e, bar_u;       // one arrival per warp and head (8); bar_u: S of a state-only tile is consumed
+  uint64_t bar_xd;                    // one arrival per warp of the read-out group (4)
   uint64_t bar_p[2];                  // one arrival per warp of the head (4)
   uint64_t bar_drain;                 // all MMAs issued have completed
   uint32_t tmem_base;
@@ -332,12 +337,12 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // an X slot is handed back by four warps: those that read out Y from it, or those that made Xd of a state-only tile
     for (int s = 0; s < XS; ++s) { mbar_init(&m->full_x[s], 1); mbar_init(&m->empty_x[s], 4); }
     mbar_init(&m->bar_g, 1); mbar_init(&m->bar_s, 1); mbar_init(&m->bar_ch, 1);
-    mbar_init(&m->bar_xd, 8); mbar_init(&m->bar_h, 8); mbar_init(&m->bar_e, 8);
+    mbar_init(&m->bar_xd, 4); mbar_init(&m->bar_h, 8); mbar_init(&m->bar_e, 8); mbar_init(&m->bar_u, 8);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&m->bar_y[h], 1);
       mbar_init(&m->bar_p[h], 4);
       // factors are released by the head's four warps (P) and the four read-out warps
-      for (int s = 0; s < 2; ++s) { mbar_init(&m->full_f[h][s], 1); mbar_init(&m->empty_f[h][s], 8); }
+      for (int s = 0; s < kFactors; ++s) { mbar_init(&m->full_f[h][s], 1); mbar_init(&m->empty_f[h][s], 8); }
     }
     mbar_init(&m->bar_drain, 1);
     m->abort_flag = 0;
@@ -423,7 +428,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
             if (ky > 0) {
-              wait(&m->bar_p[h], (ky - 1) & 1, m);   // (its warps have seen X arrive)
+              wait(&m->bar_p[h], (ky - 1) & 1, m);   // (X is there: Xd was made of it)
               tc_fence_after();
               if (elect_one()) {
                 uint32_t pa = tSP + 64 * h;
@@ -451,6 +456,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         wait(&m->full_b[s], (n / BC) & 1, m);
         wait(&m->bar_xd, n & 1, m);
         wait(&m->bar_y[1], (ky & 1) ^ 1, m);   // (its commit covers head 0's MMAs too)
+        if (n > 0 && n <= npre) wait(&m->bar_u, (n - 1) & 1, m);
         tc_fence_after();
         if (elect_one()) {
           issue<KT>(tSP, umma_desc(dMN, sBs), kMi, kMo, umma_desc(dMN, sXd), kMi, kMo, idMM);
@@ -485,8 +491,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       __syncwarp();
     } else if (warp >= 2) {
       // ---------------------------------------------------------------- prefix sums (warp 2: head 0, warp 3: head 1)
-      // Lane i owns tokens i, 32 + i, 64 + i, 96 + i.  Nothing is fetched ahead into registers (this warp is up to two
-      // tiles ahead of the others as it is), the next tile's lines only as far as L2.
+      // Lane i owns tokens i, 32 + i, 64 + i, 96 + i; nothing is fetched for the tile after (this warp is ahead as it is).
       const int h = warp - 2;
       const int64_t as32 = 32 * sp.as[1], ds32 = 32 * sp.dts[1];
       const float* Ag = nullptr;
@@ -495,24 +500,31 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll 1
       for (uint32_t n = 0; n < total; ++n) {
         c.next(prm, wk);
-        int in = c.live(wk, h) ? sp.seqlen - c.t0 - lane : 0;   // past the end: decay 1 and x = 0, the state stays as it is
+        const int in = c.live(wk, h) ? sp.seqlen - c.t0 - lane : 0;   // past the end: decay 1 and x = 0, the state stays as it is
         if (__builtin_expect(c.first_tile(), 0)) {              // (later tiles of the item: where the last one ended)
           const int head = c.head(wk) + h, t = c.t0 + lane;
           Ag = sp.A + c.b * sp.as[0] + head * sp.as[2] + t * sp.as[1];
           Dg = static_cast<const T16*>(sp.dt) + c.b * sp.dts[0] + head * sp.dts[2] + t * sp.dts[1];
         }
-        const uint32_t par = n & 1;
-        wait(&m->empty_f[h][par], ((n >> 1) & 1) ^ 1, m);
-        Factors& f = m->f[h][par];
+        float a[4];
+        T16 d[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          a[e] = 32 * e < in ? Ag[e * as32] : 0.f;
+          d[e] = sp.dt && 32 * e < in ? Dg[e * ds32] : Cvt<T16>::from_f(1.f);
+        }
+        Ag += 4 * as32;
+        Dg += 4 * ds32;
+        const uint32_t slot = n % kFactors;
+        wait(&m->empty_f[h][slot], ((n / kFactors) & 1) ^ 1, m);
+        Factors& f = m->f[h][slot];
         float base = 0.f;
 #pragma unroll 1
         for (int b32 = 0; b32 < T; b32 += 32) {
-          float cs = in > 0 ? *Ag : 0.f;
-          const float dt = sp.dt && in > 0 ? Cvt<T16>::to_f(*Dg) : 1.f;
-          if (in > T) asm volatile("prefetch.global.L2 [%0];" ::"l"(Ag + 4 * as32));
-          Ag += as32;
-          Dg += ds32;
-          in -= 32;
+          float cs = a[0];
+          const float dt = Cvt<T16>::to_f(d[0]);
+          a[0] = a[1]; a[1] = a[2]; a[2] = a[3];
+          d[0] = d[1]; d[1] = d[2]; d[2] = d[3];
 #pragma unroll
           for (int d = 1; d < 32; d <<= 1) {
             const float t = __shfl_up_sync(0xffffffffu, cs, d);
@@ -536,7 +548,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         for (int b32 = 0; b32 < T; b32 += 32)      // exp(cs_last - cs) dt = exp(cs_last - cs at the block's end) cf
           f.xs[b32 + lane] = (uint16_t)pack2<T16>(ex2(base * kLog2e - f.cs2[b32 + 31]) * f.cf[b32 + lane], 0.f);
         if (lane == 0) f.tot = base;
-        warp_arrive(&m->full_f[h][par]);
+        warp_arrive(&m->full_f[h][slot]);
       }
     }
   } else if (warp < 12) {
@@ -550,7 +562,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     const uint32_t swz = (uint32_t)(l & 7);
     const bool owns_state = lane_base < N;
     const uint32_t tS = tSP + 64 * h, tP = tSP + 64 * h;
-    const uint32_t sHh = sH + h * (N * 128), sXdh = sXd + h * kBlk;
+    const uint32_t sHh = sH + h * (N * 128);
 
     uint64_t H[P / 2];               // fp32 pairs
 #pragma unroll
@@ -610,31 +622,6 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         for (int J = q + 1; J < 4; ++J) tmem_st16(tP + tlane + 16 * J, pz);
       }
     };
-    // B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148) from X slot at `xb` into this head's Xd buffer, in packed
-    // 16-bit arithmetic as the reference does it.  The rows are not dealt out evenly: warp q has q + 1 blocks of P to
-    // fill, so the warps with fewer blocks take more rows here.  Eight lanes share a row (one 16-byte piece each), a
-    // warp moves four rows per instruction ("a quad": 32 quads per tile).
-    auto make_xd = [&](uint32_t xb, const Factors& f, bool with_mask) {
-      // first quad of warp 0..3 and the end, one byte each: 0 14 24 30 32 when all four warps also update and copy the
-      // state (N = 128), 0 10 18 26 32 when only warps 0 and 1 do
-      constexpr uint64_t kFirst = N == 128 ? 0x201E180E00ull : 0x201A120A00ull;
-      const int qb = with_mask ? (int)((kFirst >> (8 * q)) & 0xff) : 8 * q;
-      const int qe = with_mask ? (int)((kFirst >> (8 * q + 8)) & 0xff) : 8 * q + 8;
-      const uint32_t sub = (uint32_t)lane >> 3, pc = (uint32_t)lane & 7u;
-#pragma unroll 1
-      for (int qd = qb; qd < qe; qd += 2) {   // (every share is an even number of quads)
-        const uint32_t r0 = 4 * qd + sub, r1 = r0 + 4;
-        const uint32_t o0 = r0 * 128 + ((pc ^ (r0 & 7u)) << 4), o1 = r1 * 128 + ((pc ^ (r1 & 7u)) << 4);
-        const uint4 a0 = lds128(xb + o0), a1 = lds128(xb + o1);
-        const uint32_t s0 = f.xs[r0], s1 = f.xs[r1];
-        const uint32_t d0 = s0 | (s0 << 16), d1 = s1 | (s1 << 16);
-        uint4 v;
-        v.x = mul2<T16>(a0.x, d0); v.y = mul2<T16>(a0.y, d0); v.z = mul2<T16>(a0.z, d0); v.w = mul2<T16>(a0.w, d0);
-        sts128(sXdh + o0, v);
-        v.x = mul2<T16>(a1.x, d1); v.y = mul2<T16>(a1.y, d1); v.z = mul2<T16>(a1.z, d1); v.w = mul2<T16>(a1.w, d1);
-        sts128(sXdh + o1, v);
-      }
-    };
     auto store_hb = [&]() {
       if (owns_state) {
 #pragma unroll
@@ -665,21 +652,37 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       }
       __syncwarp();
     };
-    // The state entering an item.
+    // The state entering an item: zero or the caller's, unless the item continues a sequence that another CTA works on.
+    // Called as soon as the state of the item before has left, so that the loads are in flight during step A.
     Cursor c;
+    bool fold = false;               // the state entering comes (also) from other CTAs: fold_item() before it is used
     auto enter_item = [&](bool wy) {
-#pragma unroll
-      for (int e = 0; e < P / 2; ++e) H[e] = 0;
       asum0 = asum = acomp = 0.f;
+      const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
+      fold = sp.chain && c.t_begin > 0 && !from_zero;
+      if (sp.init && c.live(wk, h) && !from_zero && !fold && owns_state) {
+        const ulonglong2* I = reinterpret_cast<const ulonglong2*>(
+            sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride + (int64_t)l * P);
+#pragma unroll
+        for (int e = 0; e < P / 4; ++e) {
+          const ulonglong2 v = I[e];
+          H[2 * e] = v.x;
+          H[2 * e + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < P / 2; ++e) H[e] = 0;
+      }
+    };
+    // Chained: what the CTA before this one handed over.  Look-back: fold the pairs (state from zero, log-decay
+    // sum) that the CTAs from .. before this one published for their pieces of this sequence, newest first:
+    // H_in = sum_c exp(log-decay after c) F_c (+ the same for the caller's initial state).
+    auto fold_item = [&]() {
       const bool look_back = sp.chain == 2;
-      const bool cut_front = sp.chain && c.t_begin > 0 && !(look_back && !wy);   // (the look-back scan starts from zero)
-      const bool init = sp.init && c.live(wk, h) && !(look_back && !wy) && (!cut_front || look_back);
-      // Chained: what the CTA before this one handed over.  Look-back: fold the pairs (state from zero, log-decay
-      // sum) that the CTAs from .. before this one published for their pieces of this sequence, newest first:
-      // H_in = sum_c exp(log-decay after c) F_c (+ the same for the caller's initial state).
-      int p = cut_front ? (int)blockIdx.x - 1 : 0;
-      const int from = cut_front ? (look_back ? wk.from : p) : 1;
-      if (cut_front) wait_published(p, from);
+      const bool init = sp.init && c.live(wk, h) && look_back;
+      int p = (int)blockIdx.x - 1;
+      const int from = look_back ? wk.from : p;
+      wait_published(p, from);
 #pragma unroll 1
       for (;; --p) {
         const float* src;
@@ -734,35 +737,31 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     };
 
     bool cur_y = false;
-    uint32_t xi = h, xph = 0;   // X slot of the tile being prepared
     uint32_t ky = 0;            // Y-producing tiles prepared
+    if (total > 0) {
+      c.next(prm, wk);
+      enter_item(npre == 0);
+    }
 #pragma unroll 1
     for (uint32_t n = 0;; ++n) {   // tile n is prepared, P of tile n - 1 is made
       if (cur_y) {
         wait(&m->bar_g, (ky - 1) & 1, m);
         tc_fence_after();
-        const uint32_t par = (n - 1) & 1;
-        make_p(m->f[h][par]);
+        const uint32_t slot = (n - 1) % kFactors;
+        make_p(m->f[h][slot]);
         tmem_st_wait();
         tc_fence_before();
         warp_arrive(&m->bar_p[h]);
-        if (lane == 0) mbar_arrive(&m->empty_f[h][par]);
+        if (lane == 0) mbar_arrive(&m->empty_f[h][slot]);
       }
       if (n == total) break;
-      c.next(prm, wk);
       const bool wy = n >= npre;   // this tile produces Y (a look-back launch starts with a state-only item)
-      const uint32_t par = n & 1;
-      const Factors& f = m->f[h][par];
-      wait(&m->full_f[h][par], (n >> 1) & 1, m);
-      wait(&m->full_x[xi], xph, m);
-      make_xd(sX + xi * kBlk, f, wy);   // (the S MMA that read the Xd buffer was waited for in step E)
-      fence_proxy_async();
-      warp_arrive(&m->bar_xd);
-      if (!wy && lane == 0) mbar_arrive(&m->empty_x[xi]);   // nothing else reads X of a state-only tile
-      xi += 2;
-      if (xi >= XS) { xi -= XS; xph ^= 1; }
-      // D. (after Xd is on its way: the wait for another CTA's state and its load overlap the S MMA)
-      if (__builtin_expect(c.first_tile(), 0)) enter_item(wy);
+      const uint32_t slot = n % kFactors;
+      // D. 16-bit copy of the state for C.H
+      if (__builtin_expect(fold, 0)) {
+        fold_item();
+        fold = false;
+      }
       if (wy) {
         wait(&m->bar_ch, (ky & 1) ^ 1, m);   // the C.H MMA has read the copy before this one
         store_hb();
@@ -771,8 +770,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         ++ky;
       }
       // E. H <- exp(cs_last) H + S
-      const float tot = f.tot;
-      if (!wy) warp_arrive(&m->empty_f[h][par]);
+      wait(&m->full_f[h][slot], (n / kFactors) & 1, m);
+      const float tot = m->f[h][slot].tot;
       const float gs = ex2(tot * kLog2e);
       {
         const float yk = tot - acomp, tk = asum + yk;
@@ -792,28 +791,86 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll
         for (int e = 0; e < 16; ++e) H[16 + e] = fma_pair(H[16 + e], g2, pair(s1[2 * e], s1[2 * e + 1]));
       }
-      if (__builtin_expect(c.left == 0, 0)) leave_item(wy);
+      if (!wy) {
+        tc_fence_before();
+        warp_arrive(&m->bar_u);
+        if (lane == 0) mbar_arrive(&m->empty_f[h][slot]);
+      }
+      const bool last = c.left == 0;
+      if (__builtin_expect(last, 0)) leave_item(wy);
+      if (n + 1 < total) c.next(prm, wk);
+      if (__builtin_expect(last && n + 1 < total, 0)) enter_item(n + 1 >= npre);
       cur_y = wy;
     }
   } else {
-    // ------------------------------------------------------------------ warps 12-15: read-out of Y, both heads
+    // ------------------------------------------------------------------ warps 12-15: Xd, and read-out of Y, both heads
     setmaxnreg_dec<112>();
-    const int lane_base = (warp & 3) * 32;
+    const int q = warp & 3;
+    const int lane_base = q * 32;
     const int l = lane_base + lane;
     const uint32_t tlane = (uint32_t)lane_base << 16;
     const uint32_t swz = (uint32_t)(l & 7);
+    // B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148), in packed 16-bit arithmetic as the reference does it.
+    // Eight lanes share a row (one 16-byte piece each), a warp moves four rows per instruction.
+    auto make_xd = [&](uint32_t xb, uint32_t xd, const Factors& f) {
+      uint32_t r = 32 * q + ((uint32_t)lane >> 3);
+      const uint32_t pc = (uint32_t)lane & 7u;
+#pragma unroll 1
+      for (int i = 0; i < 2; ++i, r += 16) {
+        uint4 a[4];
+        uint32_t sc[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] = lds128(xb + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4));
+          sc[k] = f.xs[r + 4 * k];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t d = sc[k] | (sc[k] << 16);
+          uint4 v;
+          v.x = mul2<T16>(a[k].x, d); v.y = mul2<T16>(a[k].y, d); v.z = mul2<T16>(a[k].z, d); v.w = mul2<T16>(a[k].w, d);
+          sts128(xd + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4), v);
+        }
+      }
+    };
     Cursor c;
-    uint32_t xi = 0;
+    uint32_t bi = 0, bph = 0;   // X slot of the next tile to make Xd of
+    uint32_t xi = 0;            // X slot of the tile being read out
     uint32_t ky = 0;
     int pending = -1;    // (lane 0) X slot that this warp's last TMA store still reads
+    auto release = [&]() {
+      if (lane == 0 && pending >= 0) {
+        bulk_wait_read_all();
+        mbar_arrive(&m->empty_x[pending]);
+        pending = -1;
+      }
+    };
 #pragma unroll 1
-    for (uint32_t n = 0; n < total; ++n) {
-      c.next(prm, wk);
-      if (n < npre) {    // (takes its turn in the factors' ring all the same)
+    for (uint32_t k = 0; k <= total; ++k) {   // Xd of tile k, Y of tile k - 1
+      if (k < total) {
+        if (k > 0) wait(&m->bar_s, (k - 1) & 1, m);   // the S MMA has read the Xd before this one
+#pragma unroll 1
         for (int h = 0; h < 2; ++h) {
-          wait(&m->full_f[h][n & 1], (n >> 1) & 1, m);
-          if (lane == 0) mbar_arrive(&m->empty_f[h][n & 1]);
+          wait(&m->full_f[h][k % kFactors], (k / kFactors) & 1, m);
+          wait(&m->full_x[bi], bph, m);
+          make_xd(sX + bi * kBlk, sXd + h * kBlk, m->f[h][k % kFactors]);
+          if (k < npre) {   // nothing else reads X and the factors of a state-only tile
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(&m->empty_x[bi]);
+              mbar_arrive(&m->empty_f[h][k % kFactors]);
+            }
+          }
+          if (++bi == XS) { bi = 0; bph ^= 1; }
         }
+        fence_proxy_async();
+        warp_arrive(&m->bar_xd);
+        release();
+      }
+      if (k == 0) continue;
+      const uint32_t n = k - 1, slot = n % kFactors;
+      c.next(prm, wk);
+      if (n < npre) {
         xi += 2;
         if (xi >= XS) xi -= XS;
         continue;
@@ -841,15 +898,11 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             }
           }
         }
-        wait(&m->full_f[h][n & 1], (n >> 1) & 1, m);
-        const float el = ex2(m->f[h][n & 1].cs2[l]);
-        warp_arrive(&m->empty_f[h][n & 1]);
+        const float el = ex2(m->f[h][slot].cs2[l]);
+        warp_arrive(&m->empty_f[h][slot]);
         wait(&m->bar_y[h], ky & 1, m);
         tc_fence_after();
-        if (lane == 0 && pending >= 0) {
-          bulk_wait_read_all();
-          mbar_arrive(&m->empty_x[pending]);
-        }
+        release();
         const uint64_t el2 = pair(el, el);
         // The X tile is dead (its P.X MMA is complete): the 16-bit Y rows are staged in its slot.
         const uint32_t ystage = sX + xi * kBlk;
@@ -931,13 +984,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       }
       ++ky;
     }
-    if (lane == 0) {
-      if (pending >= 0) {
-        bulk_wait_read_all();
-        mbar_arrive(&m->empty_x[pending]);
-      }
-      bulk_wait_all();   // the Y rows this warp stored must have landed before the CTA exits
-    }
+    release();
+    if (lane == 0) bulk_wait_all();   // the Y rows this warp stored must have landed before the CTA exits
   }
 
   // ---------------------------------------------------------------------- teardown
