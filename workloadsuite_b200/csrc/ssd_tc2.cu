@@ -92,7 +92,6 @@ struct alignas(16) Factors {
   float cs2[T];       // cs * log2(e)
   float cf[T];        // exp(cs at the end of the row's 32-block - cs of the row) * dt: the row's factor as a column of P
   float dg[T];        // diagonal blocks: at columns 4i cs * log2(e) - log2(dt), at the three after it the ratio to the column before
-  uint16_t xs[T];     // exp(cs_last - cs) * dt, the 16-bit scale of the row of X being turned into Xd
   float tot;          // cs_last
 };
 
@@ -100,6 +99,7 @@ constexpr int kFactors = 4;   // tiles that the prefix sums may be ahead
 
 struct Misc2 {
   Work work;
+  uint4 causal[17][2];                // the first j of 16 columns kept, as masks of 16-bit pairs
   Factors f[2][kFactors];             // [head][tile ordinal % kFactors]
   uint64_t full_b[2], full_c[2], empty_b[2], empty_c[2];   // [stage]
   uint64_t full_x[6], empty_x[6];
@@ -351,6 +351,13 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&m->tmem_base, 512);
+  if (warp == 1 && lane < 17) {
+    uint32_t k[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) k[e] = (2 * e < lane ? 0xffffu : 0u) | (2 * e + 1 < lane ? 0xffff0000u : 0u);
+    m->causal[lane][0] = make_uint4(k[0], k[1], k[2], k[3]);
+    m->causal[lane][1] = make_uint4(k[4], k[5], k[6], k[7]);
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -491,63 +498,72 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       __syncwarp();
     } else if (warp >= 2) {
       // ---------------------------------------------------------------- prefix sums (warp 2: head 0, warp 3: head 1)
-      // Lane i owns tokens i, 32 + i, 64 + i, 96 + i; nothing is fetched for the tile after (this warp is ahead as it is).
+      // Lane i owns tokens 4i .. 4i+3; nothing is fetched for the tile after (this warp is ahead as it is).
       const int h = warp - 2;
-      const int64_t as32 = 32 * sp.as[1], ds32 = 32 * sp.dts[1];
       const float* Ag = nullptr;
       const T16* Dg = nullptr;
       Cursor c;
 #pragma unroll 1
       for (uint32_t n = 0; n < total; ++n) {
         c.next(prm, wk);
-        const int in = c.live(wk, h) ? sp.seqlen - c.t0 - lane : 0;   // past the end: decay 1 and x = 0, the state stays as it is
+        const int in = c.live(wk, h) ? sp.seqlen - c.t0 - 4 * lane : 0;   // past the end: decay 1 and x = 0, the state stays as it is
         if (__builtin_expect(c.first_tile(), 0)) {              // (later tiles of the item: where the last one ended)
-          const int head = c.head(wk) + h, t = c.t0 + lane;
+          const int head = c.head(wk) + h, t = c.t0 + 4 * lane;
           Ag = sp.A + c.b * sp.as[0] + head * sp.as[2] + t * sp.as[1];
           Dg = static_cast<const T16*>(sp.dt) + c.b * sp.dts[0] + head * sp.dts[2] + t * sp.dts[1];
         }
-        float a[4];
-        T16 d[4];
+        float a[4], dt[4];
+        {
+          const float* p = Ag;
+          const T16* q = Dg;
+          T16 d[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          a[e] = 32 * e < in ? Ag[e * as32] : 0.f;
-          d[e] = sp.dt && 32 * e < in ? Dg[e * ds32] : Cvt<T16>::from_f(1.f);
+          for (int e = 0; e < 4; ++e, p += sp.as[1], q += sp.dts[1]) {
+            a[e] = 0.f;
+            d[e] = Cvt<T16>::from_f(1.f);
+            if (e < in) a[e] = *p;
+            if (e < in && sp.dt) d[e] = *q;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) dt[e] = Cvt<T16>::to_f(d[e]);
         }
-        Ag += 4 * as32;
-        Dg += 4 * ds32;
+        Ag += T * sp.as[1];
+        Dg += T * sp.dts[1];
+        float cs = a[0] + a[1] + a[2] + a[3];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const float t = __shfl_up_sync(0xffffffffu, cs, d);
+          if (lane >= d) cs += t;
+        }
+        float c2[4];                                       // cs * log2(e)
+        {
+          float r = __shfl_up_sync(0xffffffffu, cs, 1);
+          if (lane == 0) r = 0.f;
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            r += a[e];
+            c2[e] = r * kLog2e;
+          }
+          c2[3] = cs * kLog2e;
+        }
+        const float ce = __shfl_sync(0xffffffffu, c2[3], lane | 7);   // at the end of the 32-token block
         const uint32_t slot = n % kFactors;
         wait(&m->empty_f[h][slot], ((n / kFactors) & 1) ^ 1, m);
         Factors& f = m->f[h][slot];
-        float base = 0.f;
-#pragma unroll 1
-        for (int b32 = 0; b32 < T; b32 += 32) {
-          float cs = a[0];
-          const float dt = Cvt<T16>::to_f(d[0]);
-          a[0] = a[1]; a[1] = a[2]; a[2] = a[3];
-          d[0] = d[1]; d[1] = d[2]; d[2] = d[3];
+        if (lane == 31) f.tot = cs;
+        reinterpret_cast<float4*>(f.cs2)[lane] = make_float4(c2[0], c2[1], c2[2], c2[3]);
+        float cf[4], cc[4];
 #pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const float t = __shfl_up_sync(0xffffffffu, cs, d);
-            if (lane >= d) cs += t;
-          }
-          cs += base;
-          base = __shfl_sync(0xffffffffu, cs, 31);   // at the end of the 32-token block
-          const float cs2 = cs * kLog2e;
-          const int r = b32 + lane;
-          f.cs2[r] = cs2;
-          f.cf[r] = ex2(base * kLog2e - cs2) * dt;
+        for (int e = 0; e < 4; ++e) {
+          cf[e] = ex2(ce - c2[e]) * dt[e];
           // dt multiplies the columns of P instead of the rows of X (P.(dt o x) = (P o dt_s).x), so the X tile stays as
           // loaded (clamped: dt == 0 must not break the chain of ratios; the clamped column then weighs 2^-60, i.e.
-          // nothing).  The ratios are clamped too: one above the diagonal may overflow, it is masked out by a select.
-          const float cc = cs2 - fmaxf(lg2(dt), -60.f);   // (lg2(1) is 0)
-          const float ratio = ex2(fminf(__shfl_up_sync(0xffffffffu, cc, 1) - cc, 126.f));
-          f.dg[r] = (lane & 3) == 0 ? cc : ratio;
+          // nothing).  The ratios are clamped too: one above the diagonal may overflow, it is masked out.
+          cc[e] = c2[e] - fmaxf(lg2(dt[e]), -60.f);        // (lg2(1) is 0)
         }
-        __syncwarp();
-#pragma unroll 1
-        for (int b32 = 0; b32 < T; b32 += 32)      // exp(cs_last - cs) dt = exp(cs_last - cs at the block's end) cf
-          f.xs[b32 + lane] = (uint16_t)pack2<T16>(ex2(base * kLog2e - f.cs2[b32 + 31]) * f.cf[b32 + lane], 0.f);
-        if (lane == 0) f.tot = base;
+        reinterpret_cast<float4*>(f.cf)[lane] = make_float4(cf[0], cf[1], cf[2], cf[3]);
+        reinterpret_cast<float4*>(f.dg)[lane] =
+            make_float4(cc[0], ex2(fminf(cc[0] - cc[1], 126.f)), ex2(fminf(cc[1] - cc[2], 126.f)), ex2(fminf(cc[2] - cc[3], 126.f)));
         warp_arrive(&m->full_f[h][slot]);
       }
     }
@@ -583,7 +599,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         uint32_t g[16];
         tmem_ld16(tG + tlane + 32 * q + 16 * half, g);
         const float4* dv = reinterpret_cast<const float4*>(&f.dg[32 * q + 16 * half]);
-        const int ln = lane - 16 * half;
+        const uint4* keep = m->causal[max(0, min(16, lane - 16 * half + 1))];
         tmem_ld_wait();
         uint32_t pk[8];
 #pragma unroll
@@ -592,9 +608,12 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           const float w0 = ex2(cs2 - d.x), w1 = w0 * d.y, w2 = w1 * d.z, w3 = w2 * d.w;
           const float v0 = __uint_as_float(g[4 * e4]) * w0, v1 = __uint_as_float(g[4 * e4 + 1]) * w1;
           const float v2 = __uint_as_float(g[4 * e4 + 2]) * w2, v3 = __uint_as_float(g[4 * e4 + 3]) * w3;
-          pk[2 * e4] = pack2<T16>(4 * e4 <= ln ? v0 : 0.f, 4 * e4 + 1 <= ln ? v1 : 0.f);
-          pk[2 * e4 + 1] = pack2<T16>(4 * e4 + 2 <= ln ? v2 : 0.f, 4 * e4 + 3 <= ln ? v3 : 0.f);
+          pk[2 * e4] = pack2<T16>(v0, v1);
+          pk[2 * e4 + 1] = pack2<T16>(v2, v3);
         }
+        const uint4 k0 = keep[0], k1 = keep[1];
+        pk[0] &= k0.x; pk[1] &= k0.y; pk[2] &= k0.z; pk[3] &= k0.w;
+        pk[4] &= k1.x; pk[5] &= k1.y; pk[6] &= k1.z; pk[7] &= k1.w;
         tmem_st8(tP + tlane + 16 * q + 8 * half, pk);
       }
 #pragma unroll 1
@@ -815,18 +834,19 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     auto make_xd = [&](uint32_t xb, uint32_t xd, const Factors& f) {
       uint32_t r = 32 * q + ((uint32_t)lane >> 3);
       const uint32_t pc = (uint32_t)lane & 7u;
+      const float g = ex2((f.tot * kLog2e) - f.cs2[32 * q + 31]);   // (cf goes as far as the end of the 32-row block)
 #pragma unroll 1
       for (int i = 0; i < 2; ++i, r += 16) {
         uint4 a[4];
-        uint32_t sc[4];
+        float sc[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           a[k] = lds128(xb + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4));
-          sc[k] = f.xs[r + 4 * k];
+          sc[k] = f.cf[r + 4 * k] * g;
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint32_t d = sc[k] | (sc[k] << 16);
+          const uint32_t d = pack2<T16>(sc[k], sc[k]);
           uint4 v;
           v.x = mul2<T16>(a[k].x, d); v.y = mul2<T16>(a[k].y, d); v.z = mul2<T16>(a[k].z, d); v.w = mul2<T16>(a[k].w, d);
           sts128(xd + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4), v);
@@ -863,6 +883,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           }
           if (++bi == XS) { bi = 0; bph ^= 1; }
         }
+        wait(&m->full_b[k % BC], (k / BC) & 1, m);   // (for the S MMA, which waits for this group only)
         fence_proxy_async();
         warp_arrive(&m->bar_xd);
         release();
