@@ -62,7 +62,8 @@ enum {
   SSD_FLAG_INJECT_LOST_HANDOVER = 8 /* testing the give-up path: in a launch whose sequences are handed from CTA to
                                     CTA, the first CTA leaves without working, so the CTA that continues its
                                     sequence runs into the bound of its wait (wait_limit_ms), reports status 6 and
-                                    returns; Y and the states of that launch are then incomplete */
+                                    returns; Y and the states of that launch are then incomplete */,
+  SSD_FLAG_D_IN_DTYPE = 16      /* D points to [h] elements of `dtype` (the layer's own parameter), not fp32 */
 };
 
 /*
@@ -109,7 +110,7 @@ typedef struct SsdArgs {
   /* Optional fused epilogue of SSDLayer.forward after the core (model_ref.py:116-118):
    *   Y <- (Y + x * D[head]) * silu(z)
    * with x the X input, evaluated in fp32 and rounded once.  D == NULL skips the skip term, Z == NULL the gate. */
-  const float* D;               /* [h]        fp32, or NULL            model_ref.py:116 */
+  const float* D;               /* [h]        fp32 (SSD_FLAG_D_IN_DTYPE: `dtype`), or NULL   model_ref.py:116 */
   const void*  Z;               /* [b,s,h,p]  dtype, or NULL           model_ref.py:118 */
   int64_t z_stride[3];          /* b, s, h */
 } SsdArgs;
@@ -220,6 +221,25 @@ int ssd_b200_dt_prologue(const void* dt_raw, int64_t stride_b, int64_t stride_l,
 int ssd_b200_step(const void* x, const float* a, const void* B, const void* C, const void* dt, const float* D,
                   const void* z, float* state, void* y, int32_t batch, int32_t nheads, int32_t headdim,
                   int32_t dstate, int32_t ngroups, int32_t dtype, void* stream);
+
+/* The same with the layer's tensors where they lie: strides in elements (batch, head or group; innermost axis contiguous,
+ * state and y contiguous), so that columns of a projection's output need no copies, and D in `dtype` when d_in_dtype is
+ * not 0 (else fp32). */
+typedef struct SsdStepArgs {
+  const void* x;
+  const float* a;
+  const void* B;
+  const void* C;
+  const void* dt;               /* or NULL */
+  const void* D;                /* or NULL */
+  const void* z;                /* or NULL */
+  float* state;
+  void* y;
+  int32_t batch, nheads, headdim, dstate, ngroups, dtype;
+  int32_t d_in_dtype, reserved;
+  int64_t x_stride[2], a_stride[2], b_stride[2], c_stride[2], dt_stride[2], z_stride[2];
+} SsdStepArgs;
+int ssd_b200_step_strided(const SsdStepArgs* args, void* stream);
 
 /* Whole forward with HOST buffers: copies X/A/B/C (and dt, initial_state when
  * given) from host memory, runs the forward and copies Y (and final_state) back,

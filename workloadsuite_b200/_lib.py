@@ -6,6 +6,7 @@ nvcc, and if that is impossible the import of the compute functions fails.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 from pathlib import Path
 
@@ -25,6 +26,7 @@ FLAG_STATE_ONLY = 1
 FLAG_REUSE_SEGMENTS = 2
 FLAG_SEPARATE_EPILOGUE = 4
 FLAG_INJECT_LOST_HANDOVER = 8
+FLAG_D_IN_DTYPE = 16
 
 # every symbol include/ssd_b200.h declares
 EXPORTS = (
@@ -33,7 +35,7 @@ EXPORTS = (
     "ssd_b200_static_scratch_capacity", "ssd_b200_forward_static_scratch", "ssd_b200_plan",
     "ssd_b200_conv1d_silu", "ssd_b200_dt_prologue",
     "ssd_b200_xchg_create", "ssd_b200_xchg_connect", "ssd_b200_xchg_buffer", "ssd_b200_xchg_all_gather",
-    "ssd_b200_xchg_destroy", "ssd_b200_step",
+    "ssd_b200_xchg_destroy", "ssd_b200_step", "ssd_b200_step_strided",
 )
 XCHG_HANDLE_BYTES = 64
 
@@ -104,6 +106,8 @@ def load(build_if_missing: bool = True) -> C.CDLL:
                                          C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]
     lib.ssd_b200_step.restype = C.c_int
     lib.ssd_b200_step.argtypes = [C.c_void_p] * 9 + [C.c_int32] * 6 + [C.c_void_p]
+    lib.ssd_b200_step_strided.restype = C.c_int
+    lib.ssd_b200_step_strided.argtypes = [C.c_void_p, C.c_void_p]
     lib.ssd_b200_xchg_create.restype = C.c_int
     lib.ssd_b200_xchg_create.argtypes = [C.c_size_t, C.c_int32, C.POINTER(C.c_void_p), C.c_void_p]
     lib.ssd_b200_xchg_connect.restype = C.c_int
@@ -119,6 +123,24 @@ def load(build_if_missing: bool = True) -> C.CDLL:
         raise RuntimeError(f"libssd_b200 ABI version {got}, binding expects {ABI_VERSION}; rebuild the library")
     _LIB = lib
     return lib
+
+
+_FAST = None
+
+
+def fast():
+    """The binding module ``ssd_b200_torch`` (``csrc/torch_binding.cpp``), bound to the loaded library."""
+    global _FAST
+    if _FAST is None:
+        lib = load()
+        spec = importlib.util.spec_from_file_location("ssd_b200_torch", str(_build.TORCH_LIB))
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        addr = lambda f: C.cast(f, C.c_void_p).value
+        mod.init(addr(lib.ssd_b200_forward), addr(lib.ssd_b200_workspace_bytes), addr(lib.ssd_b200_step_strided),
+                 addr(lib.ssd_b200_conv1d_silu), addr(lib.ssd_b200_dt_prologue))
+        _FAST = mod
+    return _FAST
 
 
 def strerror(code: int) -> str:

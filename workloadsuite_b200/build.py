@@ -1,9 +1,10 @@
-"""Build the sm_100a shared library ``lib/libssd_b200.so`` in-tree with nvcc.
+"""Build the sm_100a shared library ``lib/libssd_b200.so`` in-tree with nvcc, and ``lib/ssd_b200_torch.so``, the
+short way from PyTorch tensors to it, with the host compiler.
 
     python -m workloadsuite_b200.build [--force] [--verbose]
 
 nvcc cross-compiles without a GPU.  The library is a plain C-ABI ``.so``
-(``include/ssd_b200.h``); it does not link against PyTorch.
+(``include/ssd_b200.h``); it does not link against PyTorch, the small binding module does.
 """
 from __future__ import annotations
 
@@ -20,6 +21,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libssd_b200.so"
+TORCH_LIB = LIB_DIR / "ssd_b200_torch.so"
 STAMP = LIB_DIR / "libssd_b200.stamp"
 
 NVCC_FLAGS = [
@@ -63,7 +65,24 @@ def source_fingerprint() -> str:
 
 
 def is_current() -> bool:
-    return LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == _fingerprint()
+    return LIB.exists() and TORCH_LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == _fingerprint()
+
+
+def _start_torch_binding():
+    """Compiles ``csrc/torch_binding.cpp`` (a CPython module on PyTorch's C++ API) in the background."""
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [os.environ.get("CXX") or shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", str(ROOT / "include"), "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
+           "-I", str(cuda / "include"), "-I", sysconfig.get_paths()["include"],
+           str(CSRC / "torch_binding.cpp"), "-o", str(TORCH_LIB),
+           "-L", str(root / "lib"), f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -83,15 +102,16 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(obj)
     failed = False
+    procs.append((CSRC / "torch_binding.cpp", _start_torch_binding()))
     for src, pr in procs:
         out, _ = pr.communicate()
         if pr.returncode != 0:
             failed = True
-            sys.stderr.write(f"--- nvcc failed on {src.name}\n{out}\n")
+            sys.stderr.write(f"--- compilation failed: {src.name}\n{out}\n")
         elif verbose or out.strip():
             sys.stderr.write(f"--- {src.name}\n{out}\n")
     if failed:
-        raise RuntimeError("nvcc compilation failed")
+        raise RuntimeError("compilation failed")
     link = [nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-gencode", "arch=compute_100a,code=sm_100a",
             "-lcudart_static", "-lcuda", "-Xcompiler", "-fPIC"]
     subprocess.run(link, check=True)

@@ -82,6 +82,7 @@ void fill_params(const SsdArgs* a, ssd::ScanParams* p) {
   std::memset(p, 0, sizeof(*p));
   p->X = a->X; p->A = a->A; p->B = a->B; p->C = a->C; p->dt = a->dt; p->Y = a->Y;
   p->D = a->D; p->Z = a->Z;
+  p->d_in_dtype = (a->flags & SSD_FLAG_D_IN_DTYPE) ? 1 : 0;
   p->status = a->status;
   p->batch = a->batch; p->seqlen = a->seqlen; p->nheads = a->nheads; p->p = a->headdim; p->n = a->dstate;
   p->ngroups = a->ngroups;

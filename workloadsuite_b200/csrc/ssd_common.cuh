@@ -52,8 +52,9 @@ struct ScanParams {
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], zeroed before the launch
   // Optional epilogue Y <- (Y + x * D[head]) * silu(z) (model_ref.py:116-118); either pointer may be null.
-  const float* D;         // [h]
+  const float* D;         // [h], fp32 or (d_in_dtype) elements of the tensors' type
   const void* Z;          // [b,s,h,p], strides zs
+  int d_in_dtype;
   int64_t xs[3], as[3], bs[3], cs[3], dts[3], ys[3], zs[3];
 };
 
@@ -70,6 +71,12 @@ template <> struct Cvt<__nv_bfloat16> {
   static __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
   static __device__ __forceinline__ __nv_bfloat16 from_f(float v) { return __float2bfloat16_rn(v); }
 };
+
+// D[head] of the skip term.
+template <typename T>
+__device__ __forceinline__ float load_skip(const ScanParams& p, int head) {
+  return p.d_in_dtype ? Cvt<T>::to_f(reinterpret_cast<const T*>(p.D)[head]) : p.D[head];
+}
 
 // Launchers implemented in the kernel translation units.  Each returns an
 // SSD_ERR_* code and enqueues on `stream`.

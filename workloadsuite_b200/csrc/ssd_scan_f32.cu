@@ -16,7 +16,7 @@ namespace ssd {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kTile = 32;  // tokens staged in shared memory per step
+constexpr int kTile = 32;  // tokens staged in shared memory per step: a multiple of this, see tile_tokens()
 
 template <typename T>
 __device__ __forceinline__ void load8(const T* src, float* dst);
@@ -83,6 +83,7 @@ __device__ __forceinline__ void stage_rows(const T* src, int64_t row_stride, int
                                            bool vec_ok, int tid) {
   if (vec_ok) {
     const int per_row = width >> 3;
+#pragma unroll 4
     for (int i = tid; i < rows * per_row; i += kThreads) {
       const int r = i / per_row, c = (i - r * per_row) << 3;
       load8<T>(src + r * row_stride + c, dst + r * width + c);
@@ -96,17 +97,17 @@ __device__ __forceinline__ void stage_rows(const T* src, int64_t row_stride, int
 }
 
 template <typename T, int NS, int P>
-__global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams prm) {
+__global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams prm, const int tile) {
   constexpr int SL = kThreads / P;  // lanes sharing one state column
   constexpr int NS4 = NS / 4;
   extern __shared__ __align__(16) float smem[];
   const int n = prm.n;
-  float* Xs = smem;                  // [kTile][P]   x_t * dt_t
-  float* Bs = Xs + kTile * P;        // [kTile][n]
-  float* Cs = Bs + kTile * n;        // [kTile][n]
-  float* Ys = Cs + kTile * n;        // [kTile][P]
-  float* dec = Ys + kTile * P;       // [kTile]  exp(a_t)
-  float* araw = dec + kTile;         // [kTile]  a_t
+  float* Xs = smem;                  // [tile][P]   x_t * dt_t
+  float* Bs = Xs + tile * P;         // [tile][n]
+  float* Cs = Bs + tile * n;         // [tile][n]
+  float* Ys = Cs + tile * n;         // [tile][P]
+  float* dec = Ys + tile * P;        // [tile]  exp(a_t)
+  float* araw = dec + tile;          // [tile]  a_t
 
   const int unit = blockIdx.x;
   const int seg = blockIdx.y;
@@ -142,8 +143,8 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
   }
   double asum = 0.0;
 
-  for (int t0 = t_begin; t0 < t_end; t0 += kTile) {
-    const int rows = min(kTile, t_end - t0);
+  for (int t0 = t_begin; t0 < t_end; t0 += tile) {
+    const int rows = min(tile, t_end - t0);
     __syncthreads();  // previous tile fully consumed (Ys stored, Xs/Bs/Cs read)
     stage_rows<T>(Xg + (int64_t)t0 * prm.xs[1], prm.xs[1], rows, P, Xs, vec_ok, tid);
     stage_rows<T>(Bg + (int64_t)t0 * prm.bs[1], prm.bs[1], rows, n, Bs, vec_ok, tid);
@@ -161,7 +162,10 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
       }
       __syncthreads();
     }
+    // (several tokens in line: only the state's fma chain links them, the shared-memory reads and the shuffles of one token
+    //  run under those of the others)
     if (prm.compute_y) {
+#pragma unroll 4
       for (int t = 0; t < rows; ++t) {
         const float x = Xs[t * P + j];
         const float d = dec[t];
@@ -188,6 +192,7 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
         if (sl == 0) Ys[t * P + j] = y;
       }
     } else {
+#pragma unroll 4
       for (int t = 0; t < rows; ++t) {
         const float x = Xs[t * P + j];
         const float d = dec[t];
@@ -265,16 +270,30 @@ __global__ void ssd_fold_kernel(const float* states, int64_t st_unit_stride, int
   }
 }
 
+size_t smem_bytes(int tile, int p, int n) { return sizeof(float) * (size_t)(2 * tile * p + 2 * tile * n + 2 * tile); }
+
+// Tokens per step.  A step costs a round trip to memory and three barriers whatever its length, which other CTAs of the SM
+// cover where there are some: so the longest step (up to 128 tokens) that still leaves room for as many CTAs as an SM
+// gets, or for four.
+int tile_tokens(const ScanParams& prm, int p) {
+  const int64_t ctas = (int64_t)prm.batch * prm.nheads * prm.nseg;
+  const int64_t per_sm = std::min<int64_t>(4, (ctas + 147) / 148);
+  int tile = kTile;
+  while (tile < 128 && tile < prm.seg_len && per_sm * (smem_bytes(2 * tile, p, prm.n) + 1024) <= 227 * 1024) tile *= 2;
+  return tile;
+}
+
 template <typename T, int NS, int P>
 int launch_one(const ScanParams& prm, cudaStream_t stream) {
-  const size_t smem = sizeof(float) * (size_t)(2 * kTile * P + 2 * kTile * prm.n + 2 * kTile);
+  const int tile = tile_tokens(prm, P);
+  const size_t smem = smem_bytes(tile, P, prm.n);
   auto kern = ssd_scan_f32_kernel<T, NS, P>;
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SSD_ERR_CUDA;
   }
   dim3 grid((unsigned)(prm.batch * prm.nheads), (unsigned)prm.nseg);
-  kern<<<grid, kThreads, smem, stream>>>(prm);
+  kern<<<grid, kThreads, smem, stream>>>(prm, tile);
   return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
 
@@ -333,7 +352,7 @@ ssd_epilogue_kernel(const ScanParams p) {
     T* y = static_cast<T*>(p.Y) + b * p.ys[0] + (int64_t)t * p.ys[1] + hh * p.ys[2] + 8 * v;
     const T* x = static_cast<const T*>(p.X) + b * p.xs[0] + (int64_t)t * p.xs[1] + hh * p.xs[2] + 8 * v;
     const T* z = p.Z ? static_cast<const T*>(p.Z) + b * p.zs[0] + (int64_t)t * p.zs[1] + hh * p.zs[2] + 8 * v : nullptr;
-    const float d = p.D ? p.D[hh] : 0.f;
+    const float d = p.D ? load_skip<T>(p, hh) : 0.f;
     // eight elements per thread, moved as whole 16-byte (32-byte for fp32) vectors when the rows allow it
     T yv[8], xv[8], zv[8];
     constexpr int kVecs = sizeof(T) * 8 / 16;

@@ -3,9 +3,11 @@
 //   H[b,h] <- exp(a[b,h]) * H[b,h] + B[b,g] (x) (dt[b,h] * x[b,h])        H is [n, p] fp32
 //   y[b,h] <- C[b,g] . H[b,h]   (+ x * D[h], then * silu(z), as model_ref.py:116-118, when given)
 // HBM-bound: the fp32 state is read and written once (2 * n * p * 4 bytes per (b, h)); everything else is small.
-// One CTA per (batch, head): thread (r, c) owns four state columns 4c..4c+3 of the rows r, r + 16, ... ; all of its
-// state loads are issued before the first use (n / 16 sixteen-byte loads in flight per thread), y is reduced over
-// the sixteen row groups through shared memory.
+// One CTA of 128 threads per (batch, head) and half of the columns (columns are independent, rows are what y sums over):
+// thread (r, c) owns four state columns of the rows r, r + 16, ...; all of its state loads are issued before the first
+// use (n / 16 sixteen-byte loads in flight per thread), y is reduced over the sixteen row groups through shared memory.
+// Half-size CTAs because the whole grid is a few waves at most: the tail is shorter, and a small model's heads reach
+// twice the SMs.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -18,42 +20,54 @@
 namespace ssd {
 namespace {
 
-constexpr int kStepThreads = 256;
-constexpr int kHeadDim = 64;    // four columns per thread, sixteen threads per state row
-constexpr int kMaxRowsPerThread = 16;   // dstate <= 256
+constexpr int kHeadDim = 64;
+constexpr int kCols = 32;                       // columns of a CTA
+constexpr int kLanes = kCols / 4;               // threads per state row
+constexpr int kStepThreads = 16 * kLanes;
+constexpr int kMaxRowsPerThread = 16;           // dstate <= 256
 
 template <typename T, int ROWS>   // ROWS = dstate / 16
 __global__ void __launch_bounds__(kStepThreads)
-ssd_step_kernel(const T* __restrict__ x, const float* __restrict__ a, const T* __restrict__ B, const T* __restrict__ C,
-                const T* __restrict__ dt, const float* __restrict__ D, const T* __restrict__ z, float* __restrict__ state,
-                T* __restrict__ y, int nheads, int ngroups) {
-  __shared__ float ypart[16][kHeadDim];
+ssd_step_kernel(const SsdStepArgs p) {
+  __shared__ float ypart[16][kCols];
   __shared__ float bs[16 * ROWS], cs[16 * ROWS];
-  const int n = 16 * ROWS;
-  const int unit = blockIdx.x;               // b * nheads + h
-  const int b = unit / nheads, h = unit - b * nheads;
-  const int g = h / (nheads / ngroups);
-  const int tid = threadIdx.x, r = tid >> 4, c = tid & 15;
-  float4* S = reinterpret_cast<float4*>(state + (int64_t)unit * n * kHeadDim) + c;
+  constexpr int n = 16 * ROWS;
+  const int unit = blockIdx.x >> 1;          // b * nheads + h
+  const int col0 = (blockIdx.x & 1) * kCols;
+  const int b = unit / p.nheads, h = unit - b * p.nheads;
+  const int g = h / (p.nheads / p.ngroups);
+  const int tid = threadIdx.x, r = tid / kLanes, c = tid % kLanes;
+  float4* S = reinterpret_cast<float4*>(p.state + (int64_t)unit * n * kHeadDim + col0) + c;
   float4 hv[ROWS];
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) hv[i] = S[(int64_t)(i * 16 + r) * (kHeadDim / 4)];   // all loads first
-  const T* Bg = B + ((int64_t)b * ngroups + g) * n;
-  const T* Cg = C + ((int64_t)b * ngroups + g) * n;
+  const T* Bg = static_cast<const T*>(p.B) + b * p.b_stride[0] + g * p.b_stride[1];
+  const T* Cg = static_cast<const T*>(p.C) + b * p.c_stride[0] + g * p.c_stride[1];
   for (int i = tid; i < n; i += kStepThreads) {
     bs[i] = Cvt<T>::to_f(Bg[i]);
     cs[i] = Cvt<T>::to_f(Cg[i]);
   }
-  const T* xr = x + (int64_t)unit * kHeadDim + 4 * c;
-  float xv[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) xv[e] = Cvt<T>::to_f(xr[e]);
+  const T* xr = static_cast<const T*>(p.x) + b * p.x_stride[0] + h * p.x_stride[1] + col0;
+  const bool has_dt = p.dt != nullptr;
+  const float dtv = has_dt ? Cvt<T>::to_f(static_cast<const T*>(p.dt)[b * p.dt_stride[0] + h * p.dt_stride[1]]) : 1.f;
+  const float av = p.a[b * p.a_stride[0] + h * p.a_stride[1]];
   // x * dt in the layer's precision, as the reference forms it (model_ref.py:144)
   float xd[4];
-  const float dtv = dt ? Cvt<T>::to_f(dt[unit]) : 1.f;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) xd[e] = dt ? Cvt<T>::to_f(Cvt<T>::from_f(xv[e] * dtv)) : xv[e];
-  const float decay = __expf(a[unit]);
+  for (int e = 0; e < 4; ++e) {
+    const float xv = Cvt<T>::to_f(xr[4 * c + e]);
+    xd[e] = has_dt ? Cvt<T>::to_f(Cvt<T>::from_f(xv * dtv)) : xv;
+  }
+  // what the epilogue needs, fetched while the state is on its way
+  float xs = 0.f, ds = 0.f, zs = 0.f;
+  if (tid < kCols) {
+    if (p.D) {
+      xs = Cvt<T>::to_f(xr[tid]);
+      ds = p.d_in_dtype ? Cvt<T>::to_f(static_cast<const T*>(p.D)[h]) : static_cast<const float*>(p.D)[h];
+    }
+    if (p.z) zs = Cvt<T>::to_f(static_cast<const T*>(p.z)[b * p.z_stride[0] + h * p.z_stride[1] + col0 + tid]);
+  }
+  const float decay = __expf(av);
   __syncthreads();
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -67,35 +81,25 @@ ssd_step_kernel(const T* __restrict__ x, const float* __restrict__ a, const T* _
     acc[0] = fmaf(cn, v.x, acc[0]); acc[1] = fmaf(cn, v.y, acc[1]);
     acc[2] = fmaf(cn, v.z, acc[2]); acc[3] = fmaf(cn, v.w, acc[3]);
   }
-#pragma unroll
-  for (int e = 0; e < 4; ++e) ypart[r][4 * c + e] = acc[e];
+  *reinterpret_cast<float4*>(&ypart[r][4 * c]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
   __syncthreads();
-  if (tid < kHeadDim) {
+  if (tid < kCols) {
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < 16; ++k) s += ypart[k][tid];
-    const int64_t o = (int64_t)unit * kHeadDim + tid;
-    if (D) s = fmaf(Cvt<T>::to_f(x[o]), D[h], s);
-    if (z) {
-      const float zz = Cvt<T>::to_f(z[o]);
-      s *= zz / (1.f + __expf(-zz));
-    }
-    y[o] = Cvt<T>::from_f(s);
+    if (p.D) s = fmaf(xs, ds, s);
+    if (p.z) s *= zs / (1.f + __expf(-zs));
+    static_cast<T*>(p.y)[(int64_t)unit * kHeadDim + col0 + tid] = Cvt<T>::from_f(s);
   }
 }
 
 template <typename T>
-int launch_step(const void* x, const float* a, const void* B, const void* C, const void* dt, const float* D,
-                const void* z, float* state, void* y, int batch, int nheads, int dstate, int ngroups,
-                cudaStream_t stream) {
-  const int units = batch * nheads;
+int launch_step(const SsdStepArgs& p, cudaStream_t stream) {
   auto go = [&](auto kern) {
-    kern<<<units, kStepThreads, 0, stream>>>(static_cast<const T*>(x), a, static_cast<const T*>(B),
-                                             static_cast<const T*>(C), static_cast<const T*>(dt), D,
-                                             static_cast<const T*>(z), state, static_cast<T*>(y), nheads, ngroups);
+    kern<<<2 * p.batch * p.nheads, kStepThreads, 0, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? (int)SSD_OK : (int)SSD_ERR_CUDA;
   };
-  switch (dstate / 16) {
+  switch (p.dstate / 16) {
     case 1: return go(ssd_step_kernel<T, 1>);
     case 2: return go(ssd_step_kernel<T, 2>);
     case 4: return go(ssd_step_kernel<T, 4>);
@@ -108,24 +112,28 @@ int launch_step(const void* x, const float* a, const void* B, const void* C, con
 }  // namespace
 }  // namespace ssd
 
+extern "C" int ssd_b200_step_strided(const SsdStepArgs* p, void* stream) {
+  if (!p || !p->x || !p->a || !p->B || !p->C || !p->state || !p->y) return SSD_ERR_NULL_POINTER;
+  if (p->batch <= 0 || p->nheads <= 0 || p->headdim <= 0 || p->dstate <= 0 || p->ngroups <= 0 || p->nheads % p->ngroups != 0)
+    return SSD_ERR_BAD_SHAPE;
+  if (p->headdim != ssd::kHeadDim || p->dstate % 16 != 0 || p->dstate / 16 > ssd::kMaxRowsPerThread)
+    return SSD_ERR_UNSUPPORTED;
+  if ((int64_t)p->batch * p->nheads > 0x3fffffffLL) return SSD_ERR_TOO_LARGE;
+  if (reinterpret_cast<uintptr_t>(p->state) & 15) return SSD_ERR_MISALIGNED;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (p->dtype) {
+    case SSD_DTYPE_F32: return ssd::launch_step<float>(*p, s);
+    case SSD_DTYPE_F16: return ssd::launch_step<__half>(*p, s);
+    case SSD_DTYPE_BF16: return ssd::launch_step<__nv_bfloat16>(*p, s);
+    default: return SSD_ERR_UNSUPPORTED;
+  }
+}
+
 extern "C" int ssd_b200_step(const void* x, const float* a, const void* B, const void* C, const void* dt,
                              const float* D, const void* z, float* state, void* y, int32_t batch, int32_t nheads,
                              int32_t headdim, int32_t dstate, int32_t ngroups, int32_t dtype, void* stream) {
-  if (!x || !a || !B || !C || !state || !y) return SSD_ERR_NULL_POINTER;
-  if (batch <= 0 || nheads <= 0 || headdim <= 0 || dstate <= 0 || ngroups <= 0 || nheads % ngroups != 0)
-    return SSD_ERR_BAD_SHAPE;
-  if (headdim != ssd::kHeadDim || dstate % 16 != 0 || dstate / 16 > ssd::kMaxRowsPerThread) return SSD_ERR_UNSUPPORTED;
-  if ((int64_t)batch * nheads > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
-  if (reinterpret_cast<uintptr_t>(state) & 15) return SSD_ERR_MISALIGNED;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  switch (dtype) {
-    case SSD_DTYPE_F32:
-      return ssd::launch_step<float>(x, a, B, C, dt, D, z, state, y, batch, nheads, dstate, ngroups, s);
-    case SSD_DTYPE_F16:
-      return ssd::launch_step<__half>(x, a, B, C, dt, D, z, state, y, batch, nheads, dstate, ngroups, s);
-    case SSD_DTYPE_BF16:
-      return ssd::launch_step<__nv_bfloat16>(x, a, B, C, dt, D, z, state, y, batch, nheads, dstate, ngroups, s);
-    default:
-      return SSD_ERR_UNSUPPORTED;
-  }
+  const int64_t h = nheads, p = headdim, g = ngroups, n = dstate;
+  const SsdStepArgs s = {x, a, B, C, dt, D, z, state, y, batch, nheads, headdim, dstate, ngroups, dtype, 0, 0,
+                         {h * p, p}, {h, 1}, {g * n, n}, {g * n, n}, {h, 1}, {h * p, p}};
+  return ssd_b200_step_strided(&s, stream);
 }

@@ -905,7 +905,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         uint4 zr[8];
         float dskip = 0.f;
         if constexpr (EPI) {
-          if (sp.D && live) dskip = sp.D[c.head(wk) + h];
+          if (sp.D && live) dskip = load_skip<T16>(sp, c.head(wk) + h);
           if (sp.Z && live) {
             const T16* zbase = static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] + (c.head(wk) + h) * sp.zs[2] + 8 * (lane & 3);
 #pragma unroll

@@ -17,17 +17,13 @@ _DTYPES = {torch.float32: _lib.DTYPE_F32, torch.float16: _lib.DTYPE_F16, torch.b
 _KERNELS = {None: _lib.KERNEL_AUTO, "auto": _lib.KERNEL_AUTO, "scan_f32": _lib.KERNEL_SCAN_F32,
             "tcgen05": _lib.KERNEL_TCGEN05}
 
-_workspaces: dict = {}
-_status: dict = {}
+
+def _index(device) -> int:
+    return torch.cuda.current_device() if device.index is None else device.index
 
 
 def _status_word(device) -> torch.Tensor:
-    key = (device.type, device.index)
-    st = _status.get(key)
-    if st is None:
-        st = torch.zeros(1024, dtype=torch.int32, device=device)
-        _status[key] = st
-    return st
+    return _lib.fast().status_word(_index(device))
 
 
 def device_status(device="cuda:0", clear: bool = True) -> int:
@@ -149,12 +145,7 @@ def _fill(args, X, A, B, Cm, dt, initial_states, Y, final_state, final_ld, chunk
 def _workspace(device, nbytes: int) -> Optional[torch.Tensor]:
     if nbytes == 0:
         return None
-    key = (device.type, device.index)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    return _lib.fast().workspace(_index(device), nbytes)
 
 
 def ssd_forward(
@@ -218,6 +209,12 @@ def ssd_forward(
     that runs into the bound writes a code to the device status word (``device_status``) and returns.
     ``inject_lost_handover`` exists to test that path: see ``SSD_FLAG_INJECT_LOST_HANDOVER``.
     """
+    if (kernel is None and not nsegments and not wait_limit_ms and out_final_state is None
+            and not (state_only or reuse_segments or return_logdecay or separate_epilogue or inject_lost_handover)):
+        got = _lib.fast().forward(X, A, B, C_, chunk, dt, initial_states, D, z, out, bool(return_final_state))
+        if got is not None:
+            return got
+    # whatever needs a copy, a rarer option or an exception
     if not X.is_cuda:
         raise RuntimeError("ssd_forward needs CUDA tensors (there is no CPU path); see ssd_forward_host")
     b, s, h, p, g, n = _check(X, A, B, C_, dt, initial_states)
@@ -291,6 +288,9 @@ def conv1d_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     ``nn.Conv1d(d, d, k, groups=d)`` parameter [d,1,k] (or [d,k]); bias [d] or None.  Returns [b,l,d] contiguous
     in x's dtype (fp32 accumulation, one rounding).
     """
+    got = _lib.fast().conv1d_silu(x, weight, bias, out)
+    if got is not None:
+        return got
     if not x.is_cuda:
         raise RuntimeError("conv1d_silu needs CUDA tensors (there is no CPU path)")
     if x.dim() != 3 or x.stride(2) != 1 or x.dtype not in _DTYPES:
@@ -322,6 +322,9 @@ def dt_prologue(dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor], A_log: to
     """``dt = softplus(dt_raw + dt_bias)`` and ``A_dt = -exp(A_log) * dt.float()`` (``model_ref.py:94, 102-103``) in one
     pass on the current CUDA stream.  dt_raw [b,l,h] with a contiguous head axis (a column slice of the projection
     output is fine); dt_bias [h] or None; A_log [h] float32.  Returns (dt [b,l,h] in dt_raw's dtype, A_dt float32)."""
+    got = _lib.fast().dt_prologue(dt_raw, dt_bias, A_log)
+    if got is not None:
+        return got
     if not dt_raw.is_cuda:
         raise RuntimeError("dt_prologue needs CUDA tensors (there is no CPU path)")
     if dt_raw.dim() != 3 or dt_raw.stride(2) != 1 or dt_raw.dtype not in _DTYPES:
@@ -357,6 +360,9 @@ def ssd_step(x: torch.Tensor, a: torch.Tensor, B: torch.Tensor, C_: torch.Tensor
     state float32 [b,h,n,p] (what ``ssd_forward(..., return_final_state=True)`` returns).  Returns y [b,h,p].
     Equal, within the kernels' tolerances, to ``ssd_forward`` over a one-token sequence with ``initial_states=state``.
     """
+    got = _lib.fast().step(x, a, B, C_, state, dt, D, z, out)
+    if got is not None:
+        return got
     if not x.is_cuda:
         raise RuntimeError("ssd_step needs CUDA tensors (there is no CPU path)")
     if x.dim() != 3 or B.dim() != 3 or state.dim() != 4 or x.dtype not in _DTYPES:
