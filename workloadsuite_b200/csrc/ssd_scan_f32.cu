@@ -9,6 +9,7 @@
 // conflict-free float4 broadcasts and y_t is finished by a shuffle over the SL
 // lanes that share a column.
 #include <algorithm>
+#include <type_traits>
 #include "ssd_common.cuh"
 
 namespace ssd {
@@ -81,7 +82,15 @@ __device__ __forceinline__ void store8<float>(float* dst, const float* src) {
 template <typename T>
 __device__ __forceinline__ void stage_rows(const T* src, int64_t row_stride, int rows, int width, float* dst,
                                            bool vec_ok, int tid) {
-  if (vec_ok) {
+  if (sizeof(T) == 4 && vec_ok) {   // no conversion: asynchronous copies, waited for once all tensors' are under way
+    const int per_row = width >> 2;
+    for (int i = tid; i < rows * per_row; i += kThreads) {
+      const int r = i / per_row, c = (i - r * per_row) << 2;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * width + c)),
+                   "l"(src + r * row_stride + c)
+                   : "memory");
+    }
+  } else if (vec_ok) {
     const int per_row = width >> 3;
 #pragma unroll 4
     for (int i = tid; i < rows * per_row; i += kThreads) {
@@ -96,12 +105,31 @@ __device__ __forceinline__ void stage_rows(const T* src, int64_t row_stride, int
   }
 }
 
-template <typename T, int NS, int P>
+// Sums v[0..U) over the SL lanes of an aligned group; lane sl is left with the sums of elements sl * U / SL + i in v[i].
+template <int U, int SL>
+__device__ __forceinline__ void reduce_scatter(float (&v)[U], int sl) {
+  int left = U;
+#pragma unroll
+  for (int m = SL / 2; m >= 1; m >>= 1) {
+    left >>= 1;
+    const bool upper = sl & m;
+#pragma unroll
+    for (int i = 0; i < U / 2; ++i) {
+      if (i < left) {
+        const float send = upper ? v[i] : v[i + left];
+        v[i] = (upper ? v[i + left] : v[i]) + __shfl_xor_sync(0xffffffffu, send, m);
+      }
+    }
+  }
+}
+
+// FULL: the state has exactly NS * SL rows (the strides of B and C in shared memory are then constants).
+template <typename T, int NS, int P, bool FULL>
 __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams prm, const int tile) {
   constexpr int SL = kThreads / P;  // lanes sharing one state column
   constexpr int NS4 = NS / 4;
   extern __shared__ __align__(16) float smem[];
-  const int n = prm.n;
+  const int n = FULL ? NS * SL : prm.n;
   float* Xs = smem;                  // [tile][P]   x_t * dt_t
   float* Bs = Xs + tile * P;         // [tile][n]
   float* Cs = Bs + tile * n;         // [tile][n]
@@ -154,6 +182,7 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
       araw[tid] = a;
       dec[tid] = expf(a);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (Dg) {  // x~ = x * dt (model_ref.py:144)
       for (int i = tid; i < rows * P; i += kThreads) {
@@ -162,57 +191,70 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
       }
       __syncthreads();
     }
-    // (several tokens in line: only the state's fma chain links them, the shared-memory reads and the shuffles of one token
-    //  run under those of the others)
-    if (prm.compute_y) {
-#pragma unroll 4
-      for (int t = 0; t < rows; ++t) {
-        const float x = Xs[t * P + j];
-        const float d = dec[t];
-        const float4* B4 = reinterpret_cast<const float4*>(Bs + t * n);
-        const float4* C4 = reinterpret_cast<const float4*>(Cs + t * n);
-        float y = 0.f;
+    // U tokens in line: only the state's fma chain links them, so the shared-memory reads, the sums over the row groups and the
+    // stores of one token run under those of the others (kept apart by hand: the compiler may not move a read of X, B or C
+    // over a store of Y).
+    auto tokens = [&](int t, auto ucount, auto want_y) {
+      constexpr int U = decltype(ucount)::value;
+      constexpr bool kY = decltype(want_y)::value;   // (a branch inside would end what the compiler may interleave)
+      float x[U], d[U], y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        x[u] = Xs[(t + u) * P + j];
+        d[u] = dec[t + u];
+        y[u] = 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float4* B4 = reinterpret_cast<const float4*>(Bs + (t + u) * n);
+        const float4* C4 = reinterpret_cast<const float4*>(Cs + (t + u) * n);
 #pragma unroll
         for (int k = 0; k < NS4; ++k) {
           if ((k * SL) * 4 < n) {
             const float4 bv = B4[k * SL + sl];
-            const float4 cv = C4[k * SL + sl];
-            h[k * 4 + 0] = fmaf(h[k * 4 + 0], d, bv.x * x);
-            h[k * 4 + 1] = fmaf(h[k * 4 + 1], d, bv.y * x);
-            h[k * 4 + 2] = fmaf(h[k * 4 + 2], d, bv.z * x);
-            h[k * 4 + 3] = fmaf(h[k * 4 + 3], d, bv.w * x);
-            y = fmaf(cv.x, h[k * 4 + 0], y);
-            y = fmaf(cv.y, h[k * 4 + 1], y);
-            y = fmaf(cv.z, h[k * 4 + 2], y);
-            y = fmaf(cv.w, h[k * 4 + 3], y);
-          }
-        }
-#pragma unroll
-        for (int m = 1; m < SL; m <<= 1) y += __shfl_xor_sync(0xffffffffu, y, m);
-        if (sl == 0) Ys[t * P + j] = y;
-      }
-    } else {
-#pragma unroll 4
-      for (int t = 0; t < rows; ++t) {
-        const float x = Xs[t * P + j];
-        const float d = dec[t];
-        const float4* B4 = reinterpret_cast<const float4*>(Bs + t * n);
-#pragma unroll
-        for (int k = 0; k < NS4; ++k) {
-          if ((k * SL) * 4 < n) {
-            const float4 bv = B4[k * SL + sl];
-            h[k * 4 + 0] = fmaf(h[k * 4 + 0], d, bv.x * x);
-            h[k * 4 + 1] = fmaf(h[k * 4 + 1], d, bv.y * x);
-            h[k * 4 + 2] = fmaf(h[k * 4 + 2], d, bv.z * x);
-            h[k * 4 + 3] = fmaf(h[k * 4 + 3], d, bv.w * x);
+            h[k * 4 + 0] = fmaf(h[k * 4 + 0], d[u], bv.x * x[u]);
+            h[k * 4 + 1] = fmaf(h[k * 4 + 1], d[u], bv.y * x[u]);
+            h[k * 4 + 2] = fmaf(h[k * 4 + 2], d[u], bv.z * x[u]);
+            h[k * 4 + 3] = fmaf(h[k * 4 + 3], d[u], bv.w * x[u]);
+            if constexpr (kY) {
+              const float4 cv = C4[k * SL + sl];
+              y[u] = fmaf(cv.x, h[k * 4 + 0], y[u]);
+              y[u] = fmaf(cv.y, h[k * 4 + 1], y[u]);
+              y[u] = fmaf(cv.z, h[k * 4 + 2], y[u]);
+              y[u] = fmaf(cv.w, h[k * 4 + 3], y[u]);
+            }
           }
         }
       }
-    }
+      if constexpr (kY && U > 1) {
+        reduce_scatter<U, SL>(y, sl);
+#pragma unroll
+        for (int i = 0; i < U / SL; ++i) {
+          const int u = sl * (U / SL) + i;
+          if constexpr (sizeof(T) == 4) Yg[(int64_t)(t0 + t + u) * prm.ys[1] + j] = y[i];   // (whole sectors: no staging)
+          else Ys[(t + u) * P + j] = y[i];
+        }
+      } else if constexpr (kY) {
+#pragma unroll
+        for (int m = 1; m < SL; m <<= 1) y[0] += __shfl_xor_sync(0xffffffffu, y[0], m);
+        if (sl == 0) {
+          if constexpr (sizeof(T) == 4) Yg[(int64_t)(t0 + t) * prm.ys[1] + j] = y[0];
+          else Ys[t * P + j] = y[0];
+        }
+      }
+    };
+    constexpr int kInLine = NS >= 16 && SL <= 4 ? 4 : 8;   // (at least SL; fewer where the state fills the registers)
+    auto all = [&](auto want_y) {
+      int t = 0;
+      for (; t + kInLine <= rows; t += kInLine) tokens(t, std::integral_constant<int, kInLine>{}, want_y);
+      for (; t < rows; ++t) tokens(t, std::integral_constant<int, 1>{}, want_y);
+    };
+    if (prm.compute_y) all(std::true_type{});
+    else all(std::false_type{});
     if (tid == 0 && prm.fin_ld) {
       for (int t = 0; t < rows; ++t) asum += (double)araw[t];
     }
-    if (prm.compute_y) {
+    if (sizeof(T) < 4 && prm.compute_y) {
       __syncthreads();
       T* Yt = Yg + (int64_t)t0 * prm.ys[1];
       if (vec_ok) {
@@ -287,7 +329,7 @@ template <typename T, int NS, int P>
 int launch_one(const ScanParams& prm, cudaStream_t stream) {
   const int tile = tile_tokens(prm, P);
   const size_t smem = smem_bytes(tile, P, prm.n);
-  auto kern = ssd_scan_f32_kernel<T, NS, P>;
+  auto kern = prm.n == NS * (kThreads / P) ? ssd_scan_f32_kernel<T, NS, P, true> : ssd_scan_f32_kernel<T, NS, P, false>;
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SSD_ERR_CUDA;
