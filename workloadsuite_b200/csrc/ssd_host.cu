@@ -34,8 +34,9 @@ struct Plan {
   int tokens;      // tokens per chunk (the last chunk of a sequence may be shorter)
   int nchunks;     // chunks per batch entry
   int group;       // batch entries per chunk (> 1 only when a whole entry is much smaller than a chunk)
-  size_t x_bytes, a_bytes, dt_bytes, bc_bytes, ws_bytes, ld_bytes, st_bytes;   // a, dt, bc: one whole batch entry
-  size_t slot_bytes, entry_bytes, ldall_bytes, total_bytes;
+  int set_entries; // batch entries whose B, C, A, dt (and entering state) travel together
+  size_t x_bytes, a_bytes, dt_bytes, bc_bytes, ws_bytes, st_bytes, enter_bytes;   // a, dt, bc, enter: one set
+  size_t slot_bytes, set_bytes, ldall_bytes, total_bytes;
   int nslices;
 };
 
@@ -68,44 +69,86 @@ void chunk_args(const SsdArgs* a, int tokens, int entries, SsdArgs* s) {
   }
 }
 
-struct Slice { int bi, nb, ci, t0, tokens; bool first, last; };   // nb batch entries from bi on
+struct Slice {
+  int bi, nb, ci, t0, tokens;   // nb batch entries from bi on
+  bool first, last;
+  int set, set_bi, set_nb;      // ordinal of the set that the entries belong to, and its entries
+};
 
-// The chunks of all batch entries in order.  The first entry opens and the last one closes with a ramp of smaller
-// chunks (1/8, 1/8, 1/4, 1/2 of the regular length), so that the device->host stream starts early and the
-// host->device stream ends late: the two directions then overlap for all but a fraction of a chunk.
-std::vector<Slice> make_slices(const SsdArgs* host, int tokens_per_chunk, int group) {
+// A copy costs some 20 us beside one in the other direction, whatever its size: what is small next to X goes in few
+// copies, several batch entries at a time, only the first set being as small as the first chunk.
+void make_sets(std::vector<Slice>& slices, int set_entries) {
+  int set = -1, begin = 0, end = 0;
+  for (size_t i = 0; i < slices.size(); ++i) {
+    if (slices[i].bi + slices[i].nb > end) {
+      ++set;
+      begin = slices[i].bi;
+      end = begin + slices[i].nb;
+      for (size_t k = i + 1; set > 0 && k < slices.size() && slices[k].bi + slices[k].nb - begin <= set_entries; ++k)
+        end = slices[k].bi + slices[k].nb;
+    }
+    slices[i].set = set;
+    slices[i].set_bi = begin;
+    slices[i].set_nb = end - begin;
+  }
+}
+
+// Pieces of 1/4, 1/4, 1/2 of `regular` (multiples of `unit`), as far as they fit into `left` with `keep` to spare and
+// are worth a copy of their own (at least `least`).
+std::vector<int> ramp(int regular, int unit, int least, int keep, int* left) {
+  std::vector<int> pieces;
+  const int div[] = {4, 4, 2};
+  for (int d : div) {
+    const int len = regular / d / unit * unit;
+    if (len >= std::max(1, least) && *left - len >= keep) {
+      pieces.push_back(len);
+      *left -= len;
+    }
+  }
+  return pieces;
+}
+
+// The chunks of all batch entries in order.  They open and close with a ramp of smaller ones, so that the device->host
+// stream starts early and the host->device stream ends late: the two directions then overlap for all but a fraction of a
+// chunk (also where a chunk is a whole batch entry, or several).
+std::vector<Slice> make_slices(const SsdArgs* host, int tokens_per_chunk, int group, int set_entries) {
   std::vector<Slice> slices;
   const int b = host->batch, s = host->seqlen;
+  const int64_t row = (int64_t)host->nheads * host->headdim * esize(host->dtype);
+  constexpr int64_t kLeastBytes = 384 << 10;   // of X in a piece: a copy, a launch and two event waits cost some 10 us
   int unit = host->chunk / gcd_int(host->chunk, 128) * 128;
   if (s % unit != 0) unit = host->chunk;
-  for (int bi = 0; bi < b && group > 1; bi += group)
-    slices.push_back({bi, std::min(group, b - bi), 0, 0, s, true, true});
-  for (int bi = 0; bi < b && group == 1; ++bi) {
-    std::vector<int> lens;
+  if (group > 1) {
+    const int least = (int)std::min<int64_t>(b, (kLeastBytes + row * s - 1) / (row * s));
+    int left = b;
+    const std::vector<int> head = ramp(group, 1, least, std::min(b, 2 * group) / 2, &left);
+    std::vector<int> tail = ramp(group, 1, least, 0, &left);
+    std::vector<int> sizes = head;
+    for (; left > 0; left -= std::min(group, left)) sizes.push_back(std::min(group, left));
+    sizes.insert(sizes.end(), tail.rbegin(), tail.rend());
+    int bi = 0;
+    for (int nb : sizes) {
+      slices.push_back({bi, nb, 0, 0, s, true, true, 0, 0, 0});
+      bi += nb;
+    }
+    make_sets(slices, set_entries);
+    return slices;
+  }
+  const int least = (int)std::min<int64_t>(s, (kLeastBytes + row - 1) / row);
+  for (int bi = 0; bi < b; ++bi) {
     int left = s;
-    const int ramp[4] = {tokens_per_chunk / 8, tokens_per_chunk / 8, tokens_per_chunk / 4, tokens_per_chunk / 2};
-    std::vector<int> head, tail;
-    if (bi == 0)
-      for (int k = 0; k < 4; ++k) {
-        const int len = ramp[k] / unit * unit;
-        if (len > 0 && left - len >= tokens_per_chunk) { head.push_back(len); left -= len; }
-      }
-    if (bi == b - 1)
-      for (int k = 0; k < 4; ++k) {
-        const int len = ramp[k] / unit * unit;
-        if (len > 0 && left - len >= tokens_per_chunk) { tail.insert(tail.begin(), len); left -= len; }
-      }
-    lens = head;
+    std::vector<int> lens, tail;
+    if (bi == 0) lens = ramp(tokens_per_chunk, unit, least, b == 1 ? std::min(s, 2 * tokens_per_chunk) / 2 : 0, &left);
+    if (bi == b - 1) tail = ramp(tokens_per_chunk, unit, least, 0, &left);
     while (left > 0) { const int len = std::min(tokens_per_chunk, left); lens.push_back(len); left -= len; }
-    // (ramp-down pieces are listed largest first, so that the last copies are the small ones)
-    std::sort(tail.begin(), tail.end(), [](int a, int c) { return a > c; });
-    lens.insert(lens.end(), tail.begin(), tail.end());
+    lens.insert(lens.end(), tail.rbegin(), tail.rend());   // the smallest last
     int t0 = 0;
     for (size_t k = 0; k < lens.size(); ++k) {
-      slices.push_back({bi, 1, (int)k, t0, lens[k], k == 0, k + 1 == lens.size()});
+      slices.push_back({bi, 1, (int)k, t0, lens[k], k == 0, k + 1 == lens.size(), 0, 0, 0});
       t0 += lens[k];
     }
   }
+  make_sets(slices, set_entries);
   return slices;
 }
 
@@ -115,12 +158,14 @@ Plan make_plan(const SsdArgs* a) {
   // chunk length: a multiple of the caller's chunk and of the tensor-core tile (128) when the sequence allows,
   // sized so that the X chunk is at most 48 MiB (measured on the 2.7B layer shape, 84 MB of X per batch entry: two chunks
   // of 42 MB per entry 8.5 ms, chunks of 24 / 28 / 56 / 84 MB 8.9 / 9.0 / 9.1 / 9.0 ms; with 8 MiB chunks the copies
-  // in both directions together reach 78 GB/s, with 24 MiB and more 82-86 GB/s)
+  // in both directions together reach 78 GB/s, with 24 MiB and more 82-86 GB/s), and a quarter of the whole where that is less:
+  // beside copies in the other direction every copy costs some 20 us of its own (50 MB each way take 1.05 ms in one piece,
+  // 1.2 in 8, 1.4 in 16, 1.65 in 32)
   int unit = a->chunk / gcd_int(a->chunk, 128) * 128;
   if (a->seqlen % unit != 0) unit = a->chunk;
   const size_t per_token = (size_t)a->nheads * a->headdim * e;
   const size_t total = per_token * a->seqlen * a->batch;
-  const size_t cap = std::max<size_t>((size_t)1 << 20, std::min<size_t>((size_t)48 << 20, total / 8));
+  const size_t cap = std::max<size_t>((size_t)1 << 20, std::min<size_t>((size_t)48 << 20, total / 4));
   // ... and a batch entry is cut into equal chunks (no short remainder chunk at the end of every entry)
   long long tokens = (long long)(cap / per_token) / unit * unit;
   tokens = std::max<long long>(unit, std::min<long long>(tokens, a->seqlen));
@@ -138,13 +183,19 @@ Plan make_plan(const SsdArgs* a) {
     pl.group = (int)std::min<size_t>((size_t)a->batch, cap / per_entry);
   const size_t k = (size_t)pl.group;
   pl.x_bytes = align_up(per_token * pl.tokens * k, 256);
-  pl.a_bytes = align_up(k * a->seqlen * a->nheads * 4, 256);
-  pl.dt_bytes = a->dt ? align_up(k * a->seqlen * a->nheads * e, 256) : 0;
-  pl.bc_bytes = align_up(k * a->seqlen * a->ngroups * a->dstate * e, 256);
-  pl.ld_bytes = align_up(k * a->nheads * 4, 256);
-  pl.st_bytes = align_up(k * a->nheads * a->dstate * a->headdim * 4, 256);
+  const size_t entry_a = (size_t)a->seqlen * a->nheads * 4, entry_dt = a->dt ? (size_t)a->seqlen * a->nheads * e : 0;
+  const size_t entry_bc = (size_t)a->seqlen * a->ngroups * a->dstate * e;
+  const size_t entry_st = (size_t)a->nheads * a->dstate * a->headdim * 4;
+  const size_t per_set = entry_a + entry_dt + 2 * entry_bc + entry_st;
+  const size_t q = std::max(k, std::min<size_t>((size_t)a->batch, ((size_t)16 << 20) / per_set));
+  pl.set_entries = (int)q;
+  pl.a_bytes = align_up(q * entry_a, 256);
+  pl.dt_bytes = align_up(q * entry_dt, 256);
+  pl.bc_bytes = align_up(q * entry_bc, 256);
+  pl.enter_bytes = align_up(q * entry_st, 256);
+  pl.st_bytes = align_up(k * entry_st, 256);
   // scratch of the forward: the largest need over every (entries, tokens) shape the pipeline will launch
-  const std::vector<Slice> slices = make_slices(a, pl.tokens, pl.group);
+  const std::vector<Slice> slices = make_slices(a, pl.tokens, pl.group, pl.set_entries);
   pl.nslices = (int)slices.size();
   pl.ws_bytes = 0;
   int seen_nb = -1, seen_tokens = -1;
@@ -158,11 +209,11 @@ Plan make_plan(const SsdArgs* a) {
   // per-slice log-decay sums stay on the device until the end (one copy back)
   pl.ldall_bytes = a->final_logdecay ? align_up((size_t)pl.nslices * k * a->nheads * 4, 256) : 0;
   pl.slot_bytes = 2 * pl.x_bytes + pl.ws_bytes;
-  // B, C, A, dt travel once per batch entry (small copies cost a fixed ~10 us each), double-buffered
-  pl.entry_bytes = 2 * pl.bc_bytes + pl.a_bytes + pl.dt_bytes;
-  // + the carried state (ping-pong), the entering state and the leaving state of a batch entry (two each)
+  // B, C, A, dt and the entering states travel per set, double-buffered
+  pl.set_bytes = 2 * pl.bc_bytes + pl.a_bytes + pl.dt_bytes + pl.enter_bytes;
+  // + the carried state (ping-pong) and the leaving state of a batch entry (two)
   // + every slice's log-decay sums + the status word of the kernels
-  pl.total_bytes = kSlots * pl.slot_bytes + 2 * pl.entry_bytes + 6 * pl.st_bytes + pl.ldall_bytes + 256;
+  pl.total_bytes = kSlots * pl.slot_bytes + 2 * pl.set_bytes + 4 * pl.st_bytes + pl.ldall_bytes + 256;
   return pl;
 }
 
@@ -194,12 +245,12 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
 
   const int e = esize(host->dtype);
   const int b = host->batch, s = host->seqlen, h = host->nheads, p = host->headdim, n = host->dstate, g = host->ngroups;
-  const std::vector<Slice> slices = make_slices(host, pl.tokens, pl.group);
+  const std::vector<Slice> slices = make_slices(host, pl.tokens, pl.group, pl.set_entries);
   const int nslices = (int)slices.size();
-  // The per-entry buffers (B, C, A, dt, entering and leaving state) exist twice; `set` alternates per entry (group).
+  // The buffers of a set (B, C, A, dt, entering state) exist twice, and so does the leaving state of an entry (group).
   int last_run_user[2] = {-1, -1};     // last slice whose kernels read buffer set 0 / 1
   int last_leave_user[2] = {-1, -1};   // last slice whose final-state copy read the leaving-state buffer 0 / 1
-  int nsets_used = 0;
+  int nentries = 0, nsets = 0;
   const size_t np = (size_t)n * p;
 
   int rc = SSD_OK;
@@ -226,13 +277,12 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
   cudaEvent_t* ev_out = ev_run + nslices;
 
   char* base = static_cast<char*>(dev_scratch);
-  char* entry_base = base + kSlots * pl.slot_bytes;
-  char* st_base = entry_base + 2 * pl.entry_bytes;
+  char* set_base = base + kSlots * pl.slot_bytes;
+  char* st_base = set_base + 2 * pl.set_bytes;
   float* carry[2] = {reinterpret_cast<float*>(st_base), reinterpret_cast<float*>(st_base + pl.st_bytes)};
-  float* enter[2] = {reinterpret_cast<float*>(st_base + 2 * pl.st_bytes), reinterpret_cast<float*>(st_base + 3 * pl.st_bytes)};
-  float* leave[2] = {reinterpret_cast<float*>(st_base + 4 * pl.st_bytes), reinterpret_cast<float*>(st_base + 5 * pl.st_bytes)};
-  float* ld_all = reinterpret_cast<float*>(st_base + 6 * pl.st_bytes);   // [slice][entry of the group][head]
-  int32_t* dev_status = reinterpret_cast<int32_t*>(st_base + 6 * pl.st_bytes + pl.ldall_bytes);
+  float* leave[2] = {reinterpret_cast<float*>(st_base + 2 * pl.st_bytes), reinterpret_cast<float*>(st_base + 3 * pl.st_bytes)};
+  float* ld_all = reinterpret_cast<float*>(st_base + 4 * pl.st_bytes);   // [slice][entry of the group][head]
+  int32_t* dev_status = reinterpret_cast<int32_t*>(st_base + 4 * pl.st_bytes + pl.ldall_bytes);
   // every kernel of the pipeline reports a wait that ran out to this word (the kernels run on st_run, in order)
   ck(cudaMemsetAsync(dev_status, 0, sizeof(int32_t), st_run));
   const char* hX = static_cast<const char*>(host->X);
@@ -245,37 +295,38 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
   for (int i = 0; i < nslices && rc == SSD_OK; ++i) {
     const int bi = slices[i].bi, nb = slices[i].nb, ci = slices[i].ci, t0 = slices[i].t0, tokens = slices[i].tokens;
     const bool first = slices[i].first, last = slices[i].last;
-    if (first) ++nsets_used;
-    const int set = (nsets_used - 1) & 1;
+    if (first) ++nentries;
+    const int set = slices[i].set & 1, out = (nentries - 1) & 1;
     char* slot = base + (size_t)(i % kSlots) * pl.slot_bytes;
     char* dX = slot;
     char* dY = dX + pl.x_bytes;
     char* dW = dY + pl.x_bytes;
     float* dL = ld_all + (size_t)i * pl.group * h;
-    char* eB = entry_base + (size_t)set * pl.entry_bytes;   // whole batch entries: B, C, A, dt
+    char* eB = set_base + (size_t)set * pl.set_bytes;   // whole batch entries of the set: B, C, A, dt, entering state
     char* eC = eB + pl.bc_bytes;
     char* eA = eC + pl.bc_bytes;
     char* eD = eA + pl.a_bytes;
-    char* dB = eB + (size_t)t0 * g * n * e;
-    char* dC = eC + (size_t)t0 * g * n * e;
-    char* dA = eA + (size_t)t0 * h * 4;
-    char* dD = eD + (size_t)t0 * h * e;
+    float* enter = reinterpret_cast<float*>(eD + pl.dt_bytes);
+    const size_t row = (size_t)(bi - slices[i].set_bi) * s + t0;   // first token of the chunk within the set
+    char* dB = eB + row * g * n * e;
+    char* dC = eC + row * g * n * e;
+    char* dA = eA + row * h * 4;
+    char* dD = eD + row * h * e;
     const size_t tok0 = (size_t)bi * s + t0;   // first token of the chunk in the [b*s] token axis
 
     // stage 1: copies in (the slot is free once the chunk that used it has left); every block is contiguous
     if (i >= kSlots) ck(cudaStreamWaitEvent(st_in, ev_out[i - kSlots], 0));
-    if (first) {
-      // B, C, A, dt (and the entering state) of the whole batch entry; their buffers were last read by the kernels
-      // of batch entry bi-2
+    if (slices[i].set == nsets) {
+      // a new set; its buffers were last read by the kernels of the set before the last
+      ++nsets;
       if (last_run_user[set] >= 0) ck(cudaStreamWaitEvent(st_in, ev_run[last_run_user[set]], 0));
-      const size_t row0 = (size_t)bi * s, rows = (size_t)nb * s;
+      const size_t bi0 = (size_t)slices[i].set_bi, nb0 = (size_t)slices[i].set_nb, row0 = bi0 * s, rows = nb0 * s;
       ck(cudaMemcpyAsync(eB, hB + row0 * g * n * e, rows * g * n * e, cudaMemcpyHostToDevice, st_in));
       if (hC) ck(cudaMemcpyAsync(eC, hC + row0 * g * n * e, rows * g * n * e, cudaMemcpyHostToDevice, st_in));
       ck(cudaMemcpyAsync(eA, host->A + row0 * h, rows * h * 4, cudaMemcpyHostToDevice, st_in));
       if (hD) ck(cudaMemcpyAsync(eD, hD + row0 * h * e, rows * h * e, cudaMemcpyHostToDevice, st_in));
       if (host->initial_state)
-        ck(cudaMemcpyAsync(enter[set], host->initial_state + (size_t)bi * h * np, (size_t)nb * h * np * 4,
-                           cudaMemcpyHostToDevice, st_in));
+        ck(cudaMemcpyAsync(enter, host->initial_state + bi0 * h * np, nb0 * h * np * 4, cudaMemcpyHostToDevice, st_in));
     }
     ck(cudaMemcpyAsync(dX, hX + tok0 * h * p * e, (size_t)nb * tokens * h * p * e, cudaMemcpyHostToDevice, st_in));
     last_run_user[set] = i;
@@ -283,16 +334,16 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
 
     // stage 2: kernels; the state enters from the previous chunk of the sequence and leaves for the next one
     ck(cudaStreamWaitEvent(st_run, ev_in[i], 0));
-    if (last && want_state && last_leave_user[set] >= 0)
-      ck(cudaStreamWaitEvent(st_run, ev_out[last_leave_user[set]], 0));
+    if (last && want_state && last_leave_user[out] >= 0)
+      ck(cudaStreamWaitEvent(st_run, ev_out[last_leave_user[out]], 0));
     SsdArgs sa;
     chunk_args(host, tokens, nb, &sa);
     sa.X = dX; sa.A = reinterpret_cast<const float*>(dA); sa.B = dB;
     sa.C = hC ? dC : nullptr;
     sa.dt = hD ? dD : nullptr;
     sa.Y = state_only ? nullptr : dY;
-    sa.initial_state = first ? (host->initial_state ? enter[set] : nullptr) : carry[(ci - 1) & 1];
-    sa.final_state = last ? (want_state ? leave[set] : nullptr) : carry[ci & 1];
+    sa.initial_state = first ? (host->initial_state ? enter + (size_t)(bi - slices[i].set_bi) * h * np : nullptr) : carry[(ci - 1) & 1];
+    sa.final_state = last ? (want_state ? leave[out] : nullptr) : carry[ci & 1];
     sa.final_logdecay = host->final_logdecay ? dL : nullptr;
     sa.workspace = pl.ws_bytes ? dW : nullptr;
     sa.workspace_bytes = pl.ws_bytes;
@@ -309,9 +360,9 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
     if (!state_only)
       ck(cudaMemcpyAsync(hY + tok0 * h * p * e, dY, (size_t)nb * tokens * h * p * e, cudaMemcpyDeviceToHost, st_out));
     if (last && want_state) {
-      ck(cudaMemcpyAsync(host->final_state + (size_t)bi * h * np, leave[set], (size_t)nb * h * np * 4,
+      ck(cudaMemcpyAsync(host->final_state + (size_t)bi * h * np, leave[out], (size_t)nb * h * np * 4,
                          cudaMemcpyDeviceToHost, st_out));
-      last_leave_user[set] = i;
+      last_leave_user[out] = i;
     }
     ck(cudaEventRecord(ev_out[i], st_out));
   }
