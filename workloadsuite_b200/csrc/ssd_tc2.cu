@@ -29,6 +29,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <type_traits>
 
 #include "ssd_common.cuh"
@@ -97,8 +98,20 @@ struct alignas(16) Factors {
 
 constexpr int kFactors = 4;   // tiles that the prefix sums may be ahead
 
+// What the MMA issuer does for one kind of product (see there).  `a` and `b` are the low words of the shared-memory
+// descriptors (`a` a tensor-memory address for P.X), advanced by a_in / b_in per k-step and by a_out / b_out per four;
+// the barriers are byte offsets within Misc2 (0: none).
+struct alignas(16) Op {
+  uint32_t a, b, id;
+  uint16_t d, steps;
+  uint16_t a_in, b_in, a_out, b_out;
+  uint16_t wait0, wait1, commit0, commit1;
+};
+enum { kOpS, kOpG, kOpCH, kOpPX0, kOpPX1, kOps };
+
 struct Misc2 {
   Work work;
+  Op ops[2][kOps];                    // [tile parity] (the stage of B and C)
   uint4 causal[17][2];                // the first j of 16 columns kept, as masks of 16-bit pairs
   Factors f[2][kFactors];             // [head][tile ordinal % kFactors]
   uint64_t full_b[2], full_c[2], empty_b[2], empty_c[2];   // [stage]
@@ -225,15 +238,16 @@ struct Cursor {
 // depend on everybody's progress -- holds the clock (guarded_wait).  A role that was released that way runs through
 // its remaining tiles without waiting, on whatever is in the buffers, and leaves.
 // (The phase before a fresh barrier's first counts as over: the parity of "free" in the first round.)
-__device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, const Misc2* m) {
+__device__ __forceinline__ void wait_at(uint32_t bar, uint32_t parity, const Misc2* m) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .u32 a;\n"
       "AGAIN:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra DONE;\n\t"
       "ld.volatile.shared.u32 a, [%2];\n\tsetp.eq.u32 p, a, 0;\n\t@p bra AGAIN;\n"
       "DONE:\n\t}"
-      ::"r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<int*>(&m->abort_flag)))
+      ::"r"(bar), "r"(parity), "r"(smem_u32(const_cast<int*>(&m->abort_flag)))
       : "memory");
 }
+__device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, const Misc2* m) { wait_at(smem_u32(bar), parity, m); }
 // False when the CTA has given up; gives up with `code` when the bound runs out (twice that of the wait for another
 // CTA's hand-over: everything inside the CTA may be waiting behind that one, and the cause should be what reports).
 __device__ __forceinline__ bool guarded_wait(uint64_t* bar, uint32_t parity, Misc2* m, int code) {
@@ -254,21 +268,6 @@ __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
   return r != 0;
-}
-
-// D <- A . B over STEPS k-steps of 16: four MMAs in line (instruction cache), the operands advancing by `ai` / `bi` inside
-// the four and by `ao` / `bo` from one four to the next (descriptor units).
-template <int STEPS>
-__device__ __forceinline__ void issue(uint32_t d, uint64_t a, uint32_t ai, uint32_t ao, uint64_t b, uint32_t bi, uint32_t bo,
-                                      uint32_t id) {
-#pragma unroll 1
-  for (int o = 0; o < STEPS; o += 4) {
-    umma_ss(d, a, b, id, o);
-#pragma unroll
-    for (int i = 1; i < 4; ++i) umma_ss(d, a + i * ai, b + i * bi, id, 1);
-    a += ao;
-    b += bo;
-  }
 }
 
 // Products of fp32 pairs (one instruction for two elements).
@@ -418,75 +417,90 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       }
     } else if (warp == 1) {
       // ---------------------------------------------------------------- MMA issuer (one elected thread issues)
-      constexpr int fmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
-      constexpr uint32_t idKK = umma_idesc(128, 128, fmt, 0, 0);   // G
-      constexpr uint32_t idMM = umma_idesc(128, 128, fmt, 1, 1);   // S
-      constexpr uint32_t idKM = umma_idesc(128, 128, fmt, 0, 1);   // C.H
-      constexpr uint32_t idPX = umma_idesc(128, 64, fmt, 0, 1);    // P.X
-      constexpr uint64_t dK = umma_desc_base(16, 1024);
-      constexpr uint64_t dMN = umma_desc_base(kBlk, 1024);         // B tile; [Xd0|Xd1]; X
-      constexpr uint64_t dMNh = umma_desc_base(N * 128, 1024);     // [H0|H1]
-      constexpr uint32_t kKi = 32 >> 4, kKo = kBlk >> 4, kMi = 2048 >> 4, kMo = 8192 >> 4;   // K-major / MN-major operand steps
-      uint32_t xi = 0;             // X slot of the tile whose P.X is next
-      uint32_t ky = 0;             // Y-producing tiles whose G and C.H have been issued; P.X of the last of them is due
+      // Per tile S <- B^T.Xd, into the columns that P of the tile before was read from; for a tile that produces Y then
+      // G <- C.B^T (both heads have read G of the tile before: their P is done), Yo <- C.H (both heads' Yo and Yd of the
+      // tile before have been read out) and Yd <- P.X per head.  One copy of the code, driven by a table: a copy per kind
+      // is 2 KB more of the instruction cache (the 2.7B layer's shape 272 -> 257 us; with one MMA per step of the loop
+      // instead of four it is slower again).
+      constexpr uint64_t kDescHi = umma_desc_base(0, 1024);
+      constexpr uint32_t kMN = kBlk >> 4;
+      const uint32_t npar = npre & 1, mb = smem_u32(m);
+      if (lane < 2 * kOps) {
+        constexpr int fmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
+        constexpr uint32_t kK = 1, kMNh = N * 128 >> 4;
+        constexpr uint16_t kKi = 32 >> 4, kKo = kBlk >> 4, kMi = 2048 >> 4, kMo = 8192 >> 4;
+        const uint32_t par = lane >= kOps, o = lane - (par ? kOps : 0);
+        const uint32_t sb = par % BC, sc = ((par + npar) & 1) % BC;
+        const uint32_t aB = (sB + sb * (NB * kBlk)) >> 4, aC = (sC + sc * (NB * kBlk)) >> 4;
+        auto at = [&](const void* bar) { return (uint16_t)(smem_u32(bar) - mb); };
+        Op op = {};
+        if (o == kOpS) {
+          op = {kMN << 16 | aB, kMN << 16 | sXd >> 4, umma_idesc(128, 128, fmt, 1, 1), (uint16_t)tSP, KT, kMi, kMi, kMo, kMo,
+                at(&m->bar_xd), at(&m->bar_y[1]), at(&m->bar_s), at(&m->empty_b[sb])};
+        } else if (o == kOpG) {
+          op = {kK << 16 | aC, kK << 16 | aB, umma_idesc(128, 128, fmt, 0, 0), (uint16_t)tG, KN, kKi, kKi, kKo, kKo,
+                at(&m->full_c[sc]), 0, at(&m->bar_g), at(&m->empty_b[sb])};
+        } else if (o == kOpCH) {
+          op = {kK << 16 | aC, kMNh << 16 | sH >> 4, umma_idesc(128, 128, fmt, 0, 1), (uint16_t)tYo, KN, kKi, kMi, kKo, kMo,
+                at(&m->bar_h), at(&m->bar_e), at(&m->bar_ch), at(&m->empty_c[sc])};
+        } else {
+          const uint32_t h = o - kOpPX0;
+          op = {tSP + 64 * h, kMN << 16 | sX >> 4, umma_idesc(128, 64, fmt, 0, 1), (uint16_t)(tYd + 64 * h), KT, 8, kMi, 32, kMo,
+                at(&m->bar_p[h]), 0, at(&m->bar_y[h]), 0};
+        }
+        m->ops[par][o] = op;
+      }
+      __syncwarp();
+      uint32_t xb = 0;                 // X slot of the tile, as a descriptor offset
 #pragma unroll 1
-      for (uint32_t n = 0;; ++n) {
-        if (n > 0) {
+      for (uint32_t n = 0; n < total; ++n) {
+        const uint32_t py = n + npar;  // (its parity is that of the ordinal among the tiles that produce Y)
 #pragma unroll 1
-          for (int h = 0; h < 2; ++h) {
-            if (ky > 0) {
-              wait(&m->bar_p[h], (ky - 1) & 1, m);   // (X is there: Xd was made of it)
-              tc_fence_after();
-              if (elect_one()) {
-                uint32_t pa = tSP + 64 * h;
-                uint64_t xb = umma_desc(dMN, sX + xi * kBlk);
-#pragma unroll 1
-                for (int o = 0; o < KT; o += 4) {
-                  umma_ts(tYd + 64 * h, pa, xb, idPX, o);
-#pragma unroll
-                  for (int i = 1; i < 4; ++i) umma_ts(tYd + 64 * h, pa + 8 * i, xb + i * kMi, idPX, 1);
-                  pa += 32;
-                  xb += kMo;
-                }
-                umma_commit(&m->bar_y[h]);
-              }
+        for (int o = 0; o < kOps; ++o) {
+          const uint4* op = reinterpret_cast<const uint4*>(&m->ops[n & 1][o]);
+          const uint4 lo = op[0], hi = op[1];
+          // S: Xd is there (and B: waited for by the warps that made Xd); P.X of the tile before is done (its commit for
+          // head 1 covers head 0), or S of the state-only tile before has been consumed.
+          // G: C.  C.H: the state copy; the read-out.  P.X: P (X is there: Xd was made of it).
+          uint32_t w1 = hi.z >> 16, c1 = hi.w >> 16, p0 = py, p1 = py + 1;
+          if (o == kOpS) {
+            p0 = n;
+            if (n <= npre) {
+              w1 = n > 0 ? (uint32_t)offsetof(Misc2, bar_u) : 0u;
+              p1 = n + 1;
             }
-            if (++xi == XS) xi = 0;
+            if (n >= npre) c1 = 0;
           }
+          if (o == kOpG) p0 = (n - npre) / BC;
+          wait_at(mb + (hi.z & 0xffffu), p0 & 1, m);
+          if (w1) wait_at(mb + w1, p1 & 1, m);
+          tc_fence_after();
+          const uint32_t x = o >= kOpPX0 ? xb : 0;
+          if (elect_one()) {
+            uint32_t a = lo.x, b = lo.y + x, acc = 0;
+            const uint32_t d = lo.w & 0xffffu, ai = hi.x & 0xffffu, bi = hi.x >> 16, ao = hi.y & 0xffffu, bo = hi.y >> 16;
+            const uint32_t id = lo.z;
+#pragma unroll 1
+            for (uint32_t k = 0; k < lo.w >> 16; k += 4) {
+              if (o < kOpPX0) {
+                umma_ss(d, kDescHi | a, kDescHi | b, id, acc);
+#pragma unroll
+                for (int i = 1; i < 4; ++i) umma_ss(d, kDescHi | (a + i * ai), kDescHi | (b + i * bi), id, 1);
+              } else {
+                umma_ts(d, a, kDescHi | b, id, acc);
+#pragma unroll
+                for (int i = 1; i < 4; ++i) umma_ts(d, a + 8 * i, kDescHi | (b + i * (2048 >> 4)), id, 1);
+              }
+              a += ao; b += bo;
+              acc = 1;
+            }
+            umma_commit_at(mb + (hi.w & 0xffffu));
+            if (c1) umma_commit_at(mb + c1);
+          }
+          if (n < npre) break;
+          if (o >= kOpPX0) xb = xb == (XS - 1) * kMN ? 0 : xb + kMN;
         }
-        if (n == total) break;
-        const uint32_t s = n % BC, sc = ky % BC;
-        const uint32_t sBs = sB + s * (NB * kBlk), sCs = sC + sc * (NB * kBlk);
-        // S <- B^T . Xd, into the columns that P of the tile before was read from; then, for a tile that produces Y,
-        // G <- C . B^T (both heads have read G of the tile before: their P is done) and
-        // Yo <- C . H (both heads' Yo and Yd of the tile before have been read out).
-        wait(&m->full_b[s], (n / BC) & 1, m);
-        wait(&m->bar_xd, n & 1, m);
-        wait(&m->bar_y[1], (ky & 1) ^ 1, m);   // (its commit covers head 0's MMAs too)
-        if (n > 0 && n <= npre) wait(&m->bar_u, (n - 1) & 1, m);
-        tc_fence_after();
-        if (elect_one()) {
-          issue<KT>(tSP, umma_desc(dMN, sBs), kMi, kMo, umma_desc(dMN, sXd), kMi, kMo, idMM);
-          umma_commit(&m->bar_s);
-          if (n < npre) umma_commit(&m->empty_b[s]);
-        }
-        if (n < npre) continue;
-        wait(&m->full_c[sc], (ky / BC) & 1, m);
-        tc_fence_after();
-        if (elect_one()) {
-          issue<KN>(tG, umma_desc(dK, sCs), kKi, kKo, umma_desc(dK, sBs), kKi, kKo, idKK);
-          umma_commit(&m->bar_g);
-          umma_commit(&m->empty_b[s]);
-        }
-        wait(&m->bar_h, ky & 1, m);
-        wait(&m->bar_e, (ky & 1) ^ 1, m);
-        tc_fence_after();
-        if (elect_one()) {
-          issue<KN>(tYo, umma_desc(dK, sCs), kKi, kKo, umma_desc(dMNh, sH), kMi, kMo, idKM);
-          umma_commit(&m->bar_ch);
-          umma_commit(&m->empty_c[sc]);
-        }
-        ++ky;
+        if (n < npre) xb = xb >= (XS - 2) * kMN ? xb - (XS - 2) * kMN : xb + 2 * kMN;
       }
       // Tensor memory is freed at the end of the kernel: the MMAs issued here must have completed by then (bounded).
       if (elect_one()) {
@@ -500,35 +514,38 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       // ---------------------------------------------------------------- prefix sums (warp 2: head 0, warp 3: head 1)
       // Lane i owns tokens 4i .. 4i+3; nothing is fetched for the tile after (this warp is ahead as it is).
       const int h = warp - 2;
+      const int64_t as1 = sp.as[1], ds1 = sp.dts[1], asT = T * as1, dsT = T * ds1;
       const float* Ag = nullptr;
       const T16* Dg = nullptr;
       Cursor c;
 #pragma unroll 1
       for (uint32_t n = 0; n < total; ++n) {
         c.next(prm, wk);
-        const int in = c.live(wk, h) ? sp.seqlen - c.t0 - 4 * lane : 0;   // past the end: decay 1 and x = 0, the state stays as it is
         if (__builtin_expect(c.first_tile(), 0)) {              // (later tiles of the item: where the last one ended)
           const int head = c.head(wk) + h, t = c.t0 + 4 * lane;
           Ag = sp.A + c.b * sp.as[0] + head * sp.as[2] + t * sp.as[1];
           Dg = static_cast<const T16*>(sp.dt) + c.b * sp.dts[0] + head * sp.dts[2] + t * sp.dts[1];
         }
-        float a[4], dt[4];
-        {
-          const float* p = Ag;
-          const T16* q = Dg;
-          T16 d[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e, p += sp.as[1], q += sp.dts[1]) {
-            a[e] = 0.f;
-            d[e] = Cvt<T16>::from_f(1.f);
-            if (e < in) a[e] = *p;
-            if (e < in && sp.dt) d[e] = *q;
+        float a[4], dt[4] = {1.f, 1.f, 1.f, 1.f};
+        if (__builtin_expect(c.t0 + T <= sp.seqlen && c.live(wk, h), 1)) {
+          const float* p1 = Ag + as1;
+          const float* p2 = p1 + as1;
+          a[0] = *Ag; a[1] = *p1; a[2] = *p2; a[3] = p2[as1];
+          if (sp.dt) {
+            const T16* q1 = Dg + ds1;
+            const T16* q2 = q1 + ds1;
+            dt[0] = Cvt<T16>::to_f(*Dg); dt[1] = Cvt<T16>::to_f(*q1); dt[2] = Cvt<T16>::to_f(*q2); dt[3] = Cvt<T16>::to_f(q2[ds1]);
           }
+        } else {
+          const int in = c.live(wk, h) ? sp.seqlen - c.t0 - 4 * lane : 0;   // past the end: decay 1 and x = 0, the state stays as it is
 #pragma unroll
-          for (int e = 0; e < 4; ++e) dt[e] = Cvt<T16>::to_f(d[e]);
+          for (int e = 0; e < 4; ++e) {
+            a[e] = e < in ? Ag[e * as1] : 0.f;
+            if (e < in && sp.dt) dt[e] = Cvt<T16>::to_f(Dg[e * ds1]);
+          }
         }
-        Ag += T * sp.as[1];
-        Dg += T * sp.dts[1];
+        Ag += asT;
+        Dg += dsT;
         float cs = a[0] + a[1] + a[2] + a[3];
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -883,6 +900,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           }
           if (++bi == XS) { bi = 0; bph ^= 1; }
         }
+        wait(&m->full_b[k % BC], (k / BC) & 1, m);   // (for the S MMA, which waits for this group only)
         wait(&m->full_b[k % BC], (k / BC) & 1, m);   // (for the S MMA, which waits for this group only)
         fence_proxy_async();
         warp_arrive(&m->bar_xd);
