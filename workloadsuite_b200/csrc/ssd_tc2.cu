@@ -135,6 +135,7 @@ struct Tc2Params {
   int nitems;   // upairs * nseg
   int upairs;   // batch * head pairs
   int ppg;      // head pairs per B/C group
+  int st32;     // the states that enter and leave start on 32-byte boundaries
 };
 
 // Item `i` of the (segment, batch, group, pair) grid as digits.
@@ -300,6 +301,15 @@ template <typename T16>
 __device__ __forceinline__ uint32_t pack_pair(uint64_t v) {
   const float2 f = unpair(v);
   return pack2<T16>(f.x, f.y);
+}
+
+// 32 bytes per thread (a whole sector: a thread's row of the state would otherwise be moved half a sector at a time, and
+// the load/store unit takes a cycle per sector touched).
+__device__ __forceinline__ void ldg256(const void* p, uint64_t (&v)[4]) {
+  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void stg256(void* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
 }
 
 // EPI: apply the skip and gate of model_ref.py:116-118 to Y on its way out (sp.D / sp.Z; either may be null).
@@ -525,6 +535,11 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           const int head = c.head(wk) + h, t = c.t0 + 4 * lane;
           Ag = sp.A + c.b * sp.as[0] + head * sp.as[2] + t * sp.as[1];
           Dg = static_cast<const T16*>(sp.dt) + c.b * sp.dts[0] + head * sp.dts[2] + t * sp.dts[1];
+          // this warp is the first to know of an item: the state that enters it goes to L2
+          if (sp.init && c.live(wk, h) && c.t_begin == 0) {
+            const float* I = sp.init + ((int64_t)c.b * sp.nheads + head) * sp.init_unit_stride + c.seg * sp.init_seg_stride;
+            for (int e = lane; e < N * P / 32; e += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(I + 32 * e));
+          }
         }
         float a[4], dt[4] = {1.f, 1.f, 1.f, 1.f};
         if (__builtin_expect(c.t0 + T <= sp.seqlen && c.live(wk, h), 1)) {
@@ -697,13 +712,22 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
       fold = sp.chain && c.t_begin > 0 && !from_zero;
       if (sp.init && c.live(wk, h) && !from_zero && !fold && owns_state) {
-        const ulonglong2* I = reinterpret_cast<const ulonglong2*>(
-            sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride + (int64_t)l * P);
+        const float* I = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride +
+                         (int64_t)l * P;
+        if (prm.st32) {
 #pragma unroll
-        for (int e = 0; e < P / 4; ++e) {
-          const ulonglong2 v = I[e];
-          H[2 * e] = v.x;
-          H[2 * e + 1] = v.y;
+          for (int e = 0; e < P / 8; ++e) {
+            uint64_t v[4];
+            ldg256(I + 8 * e, v);
+            H[4 * e] = v[0]; H[4 * e + 1] = v[1]; H[4 * e + 2] = v[2]; H[4 * e + 3] = v[3];
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < P / 4; ++e) {
+            const ulonglong2 v = reinterpret_cast<const ulonglong2*>(I)[e];
+            H[2 * e] = v.x;
+            H[2 * e + 1] = v.y;
+          }
         }
       } else {
 #pragma unroll
@@ -756,9 +780,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       float* ld = publish ? sp.chain_ld + slot
                           : (sp.fin_ld ? sp.fin_ld + unit * sp.finld_unit_stride + seg * sp.finld_seg_stride : nullptr);
       if (to && owns_state) {
-        ulonglong2* F = reinterpret_cast<ulonglong2*>(to + (int64_t)l * P);
+        float* F = to + (int64_t)l * P;
+        if (prm.st32) {
 #pragma unroll
-        for (int e = 0; e < P / 4; ++e) F[e] = make_ulonglong2(H[2 * e], H[2 * e + 1]);
+          for (int e = 0; e < P / 8; ++e) stg256(F + 8 * e, H[4 * e], H[4 * e + 1], H[4 * e + 2], H[4 * e + 3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < P / 4; ++e) reinterpret_cast<ulonglong2*>(F)[e] = make_ulonglong2(H[2 * e], H[2 * e + 1]);
+        }
       }
       if (ld && l == 0) *ld = asum0 + asum;
       if (publish) {
@@ -1131,6 +1160,7 @@ int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
   const int64_t upairs = unit_pairs(a);
   if (upairs * sp.nseg > 0x7fffffffLL || upairs * ((a.seqlen + T - 1) / T) > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
   prm.upairs = (int)upairs;
+  prm.st32 = ((reinterpret_cast<uintptr_t>(sp.init) | reinterpret_cast<uintptr_t>(sp.fin)) & 31) == 0;   // (rows are 256 bytes)
   prm.nitems = prm.upairs * sp.nseg;
   CUtensorMap tx, tb, tc, ty;
   if (!make_map(&tx, a.X, a, P, a.nheads / a.ngroups, a.x_stride, T)) return SSD_ERR_CUDA;
