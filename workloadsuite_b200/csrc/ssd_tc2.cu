@@ -14,7 +14,8 @@
 //     A. P(t)   = G o exp(segsum) o causal  (:139-145)  -> TMEM, the A operand of Yd = P.X
 //     D. 16-bit copy of the state entering tile t+1     -> shared memory -> Yo = C.H   (:160-161)
 //     E. H <- exp(cs_last) H + S(t+1)       (:150,156)  in fp32 registers
-//   warps 12-15   both heads, in this order:
+//   warps 12-15   both heads, in this order (with skip and gate B is a step between A and D of the warps above, which then
+//                 wait for this group):
 //     B. Xd(t+1) = exp(cs_last - cs) x~     (:144,148)  -> shared memory -> S = B^T.Xd
 //     Y(t) = Yd + exp(cs) Yo (:162) [+ skip and gate, :116-118] -> shared memory -> TMA store
 //
@@ -119,7 +120,7 @@ struct Misc2 {
   uint64_t full_f[2][kFactors], empty_f[2][kFactors];
   uint64_t bar_g, bar_s, bar_ch, bar_y[2];   // tcgen05.commit arrivals (S and C.H serve both heads at once)
   uint64_t bar_h, bar_e, bar_u;       // one arrival per warp and head (8); bar_u: S of a state-only tile is consumed
-  uint64_t bar_xd;                    // one arrival per warp of the read-out group (4)
+  uint64_t bar_xd;                    // one arrival per warp that makes Xd (4 of the read-out group; EPI: 8)
   uint64_t bar_p[2];                  // one arrival per warp of the head (4)
   uint64_t bar_drain;                 // all MMAs issued have completed
   uint32_t tmem_base;
@@ -312,6 +313,32 @@ __device__ __forceinline__ void stg256(void* p, uint64_t a, uint64_t b, uint64_t
   asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
 }
 
+// B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148) of rows 32 q .. 32 q + 31, in packed 16-bit arithmetic as the
+// reference does it.  Eight lanes share a row (one 16-byte piece each), a warp moves four rows per instruction.
+template <typename T16>
+__device__ __forceinline__ void make_xd(uint32_t xb, uint32_t xd, const Factors& f, int q, int lane) {
+  uint32_t r = 32 * q + ((uint32_t)lane >> 3);
+  const uint32_t pc = (uint32_t)lane & 7u;
+  const float g = ex2((f.tot * kLog2e) - f.cs2[32 * q + 31]);   // (cf goes as far as the end of the 32-row block)
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i, r += 16) {
+    uint4 a[4];
+    float sc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      a[k] = lds128(xb + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4));
+      sc[k] = f.cf[r + 4 * k] * g;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t d = pack2<T16>(sc[k], sc[k]);
+      uint4 v;
+      v.x = mul2<T16>(a[k].x, d); v.y = mul2<T16>(a[k].y, d); v.z = mul2<T16>(a[k].z, d); v.w = mul2<T16>(a[k].w, d);
+      sts128(xd + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4), v);
+    }
+  }
+}
+
 // EPI: apply the skip and gate of model_ref.py:116-118 to Y on its way out (sp.D / sp.Z; either may be null).
 template <typename T16, int N, bool EPI>
 __global__ void __launch_bounds__(kThreads2, 1)
@@ -346,7 +373,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // an X slot is handed back by four warps: those that read out Y from it, or those that made Xd of a state-only tile
     for (int s = 0; s < XS; ++s) { mbar_init(&m->full_x[s], 1); mbar_init(&m->empty_x[s], 4); }
     mbar_init(&m->bar_g, 1); mbar_init(&m->bar_s, 1); mbar_init(&m->bar_ch, 1);
-    mbar_init(&m->bar_xd, 4); mbar_init(&m->bar_h, 8); mbar_init(&m->bar_e, 8); mbar_init(&m->bar_u, 8);
+    mbar_init(&m->bar_xd, EPI ? 8 : 4); mbar_init(&m->bar_h, 8); mbar_init(&m->bar_e, 8); mbar_init(&m->bar_u, 8);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&m->bar_y[h], 1);
       mbar_init(&m->bar_p[h], 4);
@@ -803,6 +830,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 
     bool cur_y = false;
     uint32_t ky = 0;            // Y-producing tiles prepared
+    uint32_t xi = h, xph = 0;   // (EPI) X slot of the tile being prepared
     if (total > 0) {
       c.next(prm, wk);
       enter_item(npre == 0);
@@ -822,6 +850,18 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       if (n == total) break;
       const bool wy = n >= npre;   // this tile produces Y (a look-back launch starts with a state-only item)
       const uint32_t slot = n % kFactors;
+      if constexpr (EPI) {
+        // B. (the read-out warps have the skip and the gate to do; the S MMA that read the Xd before was waited for in E)
+        wait(&m->full_f[h][slot], (n / kFactors) & 1, m);
+        wait(&m->full_x[xi], xph, m);
+        make_xd<T16>(sX + xi * kBlk, sXd + h * kBlk, m->f[h][slot], q, lane);
+        wait(&m->full_b[n % BC], (n / BC) & 1, m);   // (for the S MMA, which waits for these warps only)
+        fence_proxy_async();
+        warp_arrive(&m->bar_xd);
+        if (!wy && lane == 0) mbar_arrive(&m->empty_x[xi]);
+        xi += 2;
+        if (xi >= XS) { xi -= XS; xph ^= 1; }
+      }
       // D. 16-bit copy of the state for C.H
       if (__builtin_expect(fold, 0)) {
         fold_item();
@@ -875,30 +915,6 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     const int l = lane_base + lane;
     const uint32_t tlane = (uint32_t)lane_base << 16;
     const uint32_t swz = (uint32_t)(l & 7);
-    // B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148), in packed 16-bit arithmetic as the reference does it.
-    // Eight lanes share a row (one 16-byte piece each), a warp moves four rows per instruction.
-    auto make_xd = [&](uint32_t xb, uint32_t xd, const Factors& f) {
-      uint32_t r = 32 * q + ((uint32_t)lane >> 3);
-      const uint32_t pc = (uint32_t)lane & 7u;
-      const float g = ex2((f.tot * kLog2e) - f.cs2[32 * q + 31]);   // (cf goes as far as the end of the 32-row block)
-#pragma unroll 1
-      for (int i = 0; i < 2; ++i, r += 16) {
-        uint4 a[4];
-        float sc[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          a[k] = lds128(xb + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4));
-          sc[k] = f.cf[r + 4 * k] * g;
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t d = pack2<T16>(sc[k], sc[k]);
-          uint4 v;
-          v.x = mul2<T16>(a[k].x, d); v.y = mul2<T16>(a[k].y, d); v.z = mul2<T16>(a[k].z, d); v.w = mul2<T16>(a[k].w, d);
-          sts128(xd + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4), v);
-        }
-      }
-    };
     Cursor c;
     uint32_t bi = 0, bph = 0;   // X slot of the next tile to make Xd of
     uint32_t xi = 0;            // X slot of the tile being read out
@@ -913,13 +929,19 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     };
 #pragma unroll 1
     for (uint32_t k = 0; k <= total; ++k) {   // Xd of tile k, Y of tile k - 1
-      if (k < total) {
+      if (EPI && k < npre) {   // (takes its turn in the factors' ring all the same)
+        for (int h = 0; h < 2; ++h) {
+          wait(&m->full_f[h][k % kFactors], (k / kFactors) & 1, m);
+          warp_arrive(&m->empty_f[h][k % kFactors]);
+        }
+      }
+      if (!EPI && k < total) {
         if (k > 0) wait(&m->bar_s, (k - 1) & 1, m);   // the S MMA has read the Xd before this one
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           wait(&m->full_f[h][k % kFactors], (k / kFactors) & 1, m);
           wait(&m->full_x[bi], bph, m);
-          make_xd(sX + bi * kBlk, sXd + h * kBlk, m->f[h][k % kFactors]);
+          make_xd<T16>(sX + bi * kBlk, sXd + h * kBlk, m->f[h][k % kFactors], q, lane);
           if (k < npre) {   // nothing else reads X and the factors of a state-only tile
             __syncwarp();
             if (lane == 0) {
@@ -965,6 +987,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
               }
             }
           }
+        }
+        if constexpr (EPI) {
+          // the next gate rows, one per lane, as near as they go without registers
+          const int tn = t0 + l + (h ? T : 0);
+          if (sp.Z && tn < sp.seqlen && c.live(wk, h ^ 1))
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] +
+                                                         (c.head(wk) + (h ^ 1)) * sp.zs[2] + (int64_t)tn * sp.zs[1]));
+          wait(&m->full_f[h][slot], (n / kFactors) & 1, m);
         }
         const float el = ex2(m->f[h][slot].cs2[l]);
         warp_arrive(&m->empty_f[h][slot]);
