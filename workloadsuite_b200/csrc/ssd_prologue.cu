@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "ssd_b200.h"
@@ -14,35 +15,80 @@
 namespace ssd {
 namespace {
 
+// The reference adds in the layer's dtype, then takes softplus in that dtype (threshold 20, as torch).
 template <typename T>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ T discretise(T raw, T bias) {
+  const float v = Cvt<T>::to_f(Cvt<T>::from_f(Cvt<T>::to_f(raw) + Cvt<T>::to_f(bias)));
+  return Cvt<T>::from_f(v > 20.f ? v : log1pf(expf(v)));
+}
+
+// V consecutive heads per thread (V = 8: 16-byte pieces of 16-bit rows; V = 1 where rows are not aligned), the same heads
+// in every row of the grid's stride, so that bias and rate are read once and nothing is divided per element.
+template <typename T, int V>
+__global__ void __launch_bounds__(128)
 dt_prologue_kernel(const T* __restrict__ dt_raw, int64_t sb, int64_t sl, const T* __restrict__ dt_bias,
-                   const float* __restrict__ A_log, T* __restrict__ dt_out, float* __restrict__ A_dt, int batch,
+                   const float* __restrict__ A_log, T* __restrict__ dt_out, float* __restrict__ A_dt, int rows,
                    int seqlen, int nheads) {
-  const int64_t total = (int64_t)batch * seqlen * nheads;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int h = (int)(i % nheads);
-    const int64_t r = i / nheads;
-    const int t = (int)(r % seqlen);
-    const int b = (int)(r / seqlen);
-    // the reference adds in the layer's dtype, then softplus in that dtype (threshold 20, as torch)
-    const float v = Cvt<T>::to_f(Cvt<T>::from_f(Cvt<T>::to_f(dt_raw[b * sb + (int64_t)t * sl + h]) +
-                                                  (dt_bias ? Cvt<T>::to_f(dt_bias[h]) : 0.f)));
-    const float sp = v > 20.f ? v : log1pf(expf(v));
-    const T d = Cvt<T>::from_f(sp);
-    dt_out[i] = d;
-    A_dt[i] = -expf(A_log[h]) * Cvt<T>::to_f(d);
+  const int vecs = nheads / V;
+  const int first = blockIdx.x * blockDim.x + threadIdx.x;
+  const int step = (gridDim.x * blockDim.x) / vecs;   // rows per pass; threads past step * vecs have none
+  if (first >= step * vecs) return;
+  const int h0 = (first % vecs) * V;
+  float rate[V];
+  T bias[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    rate[e] = -expf(A_log[h0 + e]);
+    bias[e] = dt_bias ? dt_bias[h0 + e] : Cvt<T>::from_f(0.f);
+  }
+  for (int r = first / vecs; r < rows; r += step) {
+    const int b = r / seqlen;
+    const T* src = dt_raw + b * sb + (int64_t)(r - b * seqlen) * sl + h0;
+    const int64_t o = (int64_t)r * nheads + h0;
+    alignas(16) T in[V], d[V];
+    alignas(16) float a[V];
+    constexpr int kWords = sizeof(T) * V / 16;
+    if constexpr (V > 1) {
+#pragma unroll
+      for (int k = 0; k < kWords; ++k) reinterpret_cast<uint4*>(in)[k] = reinterpret_cast<const uint4*>(src)[k];
+    } else {
+      in[0] = src[0];
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      d[e] = discretise<T>(in[e], bias[e]);
+      a[e] = rate[e] * Cvt<T>::to_f(d[e]);
+    }
+    if constexpr (V > 1) {
+#pragma unroll
+      for (int k = 0; k < kWords; ++k) reinterpret_cast<uint4*>(dt_out + o)[k] = reinterpret_cast<const uint4*>(d)[k];
+#pragma unroll
+      for (int k = 0; k < V / 4; ++k) reinterpret_cast<float4*>(A_dt + o)[k] = reinterpret_cast<const float4*>(a)[k];
+    } else {
+      dt_out[o] = d[0];
+      A_dt[o] = a[0];
+    }
   }
 }
 
 template <typename T>
 int launch_prologue(const void* dt_raw, int64_t sb, int64_t sl, const void* dt_bias, const float* A_log, void* dt_out,
                     float* A_dt, int batch, int seqlen, int nheads, cudaStream_t stream) {
-  const int64_t total = (int64_t)batch * seqlen * nheads;
-  const int grid = (int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
-  dt_prologue_kernel<T><<<grid, 256, 0, stream>>>(static_cast<const T*>(dt_raw), sb, sl, static_cast<const T*>(dt_bias),
-                                                  A_log, static_cast<T*>(dt_out), A_dt, batch, seqlen, nheads);
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  if ((int64_t)batch * seqlen > 0x7fffffffLL || nheads > (1 << 24)) return SSD_ERR_TOO_LARGE;
+  constexpr int V = 8, per16 = 16 / (int)sizeof(T);
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  // (a few rows: one head per thread, so that the functions of the eight do not run one after the other)
+  const bool vec = nheads % V == 0 && (int64_t)batch * seqlen * nheads >= (1 << 17) && al(dt_raw) && al(dt_out) && al(A_dt) && sb % per16 == 0 && sl % per16 == 0;
+  const int rows = batch * seqlen, vecs = vec ? nheads / V : nheads;
+  const int64_t total = (int64_t)rows * vecs;
+  // up to sixteen small CTAs per SM, and at least one pass of whole rows
+  const int64_t ctas = std::max<int64_t>(std::min<int64_t>((total + 127) / 128, 148 * 16), (vecs + 127) / 128);
+  auto go = [&](auto kern) {
+    kern<<<(unsigned)ctas, 128, 0, stream>>>(static_cast<const T*>(dt_raw), sb, sl, static_cast<const T*>(dt_bias), A_log,
+                                             static_cast<T*>(dt_out), A_dt, rows, seqlen, nheads);
+    return cudaGetLastError() == cudaSuccess ? (int)SSD_OK : (int)SSD_ERR_CUDA;
+  };
+  return vec ? go(dt_prologue_kernel<T, V>) : go(dt_prologue_kernel<T, 1>);
 }
 
 }  // namespace
