@@ -972,9 +972,11 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         // (EPI) the gate rows of this warp's 32 tokens, fetched ahead of the wait for the MMA.  Four lanes read half a
         // 128-byte row per load, eight rows per instruction; the rows reach their threads through the staging buffer below.
         uint4 zr[8];
-        float dskip = 0.f;
+        uint32_t dskip = 0;   // D as loaded: a conversion here would hold the warp for the whole memory latency
         if constexpr (EPI) {
-          if (sp.D && live) dskip = load_skip<T16>(sp, c.head(wk) + h);
+          if (sp.D && live)
+            dskip = sp.d_in_dtype ? reinterpret_cast<const uint16_t*>(sp.D)[c.head(wk) + h]
+                                  : reinterpret_cast<const uint32_t*>(sp.D)[c.head(wk) + h];
           if (sp.Z && live) {
             const T16* zbase = static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] + (c.head(wk) + h) * sp.zs[2] + 8 * (lane & 3);
 #pragma unroll
@@ -1022,7 +1024,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             // Y <- (Y + x * D) * silu(z) (model_ref.py:116-118) in fp32; x is this thread's row of the X tile, still in
             // the slot that the Y rows go to; silu(z) = z * (0.5 + 0.5 tanh(z / 2)), the tanh on 16-bit pairs.
             if (sp.D && live) {
-              const uint64_t ds = pair(dskip, dskip);
+              const float dsf = sp.d_in_dtype ? unpack2<T16>(dskip).x : __uint_as_float(dskip);
+              const uint64_t ds = pair(dsf, dsf);
 #pragma unroll
               for (int cc = 0; cc < 4; ++cc) {
                 const uint4 xr = lds128(yrow + (((4 * half + cc) ^ swz) << 4));
