@@ -952,7 +952,6 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           if (++bi == XS) { bi = 0; bph ^= 1; }
         }
         wait(&m->full_b[k % BC], (k / BC) & 1, m);   // (for the S MMA, which waits for this group only)
-        wait(&m->full_b[k % BC], (k / BC) & 1, m);   // (for the S MMA, which waits for this group only)
         fence_proxy_async();
         warp_arrive(&m->bar_xd);
         release();
