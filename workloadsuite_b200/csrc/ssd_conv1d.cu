@@ -16,7 +16,13 @@
 namespace ssd {
 namespace {
 
-constexpr int kTokensPerThread = 32;
+// Tokens per thread: the longest run whose threads still fill the chip (the rows before a run are read once more, so a
+// short run costs (taps - 1) / run of the reads again; but a few hundred threads with long runs leave most SMs idle).
+inline int run_length(int longest, int shortest, int64_t columns, int seqlen, int threads_wanted) {
+  int run = longest;
+  while (run > shortest && columns * ((seqlen + run - 1) / run) < threads_wanted) run /= 2;
+  return run;
+}
 constexpr int kMaxTaps = 8;
 
 // 8 consecutive elements <-> 8 floats, through 16-byte vectors kept in registers when `vec`.
@@ -76,14 +82,14 @@ __device__ __forceinline__ void store8<float>(float* p, const float (&v)[8], boo
   }
 }
 
-// One thread: 8 consecutive channels (one 16-byte vector of a 16-bit row), kTokensPerThread consecutive tokens,
+// One thread: 8 consecutive channels (one 16-byte vector of a 16-bit row), `run` consecutive tokens,
 // the last K-1 rows kept in registers as a sliding window.
 template <typename T, int K>
 __global__ void __launch_bounds__(128, 4)
 conv1d_silu_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
-                   int batch, int seqlen, int channels, int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl, int vec_ok) {
+                   int batch, int seqlen, int channels, int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl, int vec_ok, int run) {
   const int cvecs = channels / 8;
-  const int chunks = (seqlen + kTokensPerThread - 1) / kTokensPerThread;
+  const int chunks = (seqlen + run - 1) / run;
   const int64_t total = (int64_t)batch * chunks * cvecs;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -92,7 +98,7 @@ conv1d_silu_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __
   const int ch = (int)(r % chunks);
   const int b = (int)(r / chunks);
   const int c0 = 8 * cv;
-  const int t_begin = ch * kTokensPerThread, t_end = min(seqlen, t_begin + kTokensPerThread);
+  const int t_begin = ch * run, t_end = min(seqlen, t_begin + run);
 
   float wk[K][8], bs[8];
 #pragma unroll
@@ -171,12 +177,12 @@ conv1d_silu_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __
 
 // ---- 16-bit rows staged through shared memory -----------------------------------------------------------
 // The same arithmetic, arranged for the memory system: a thread streams its 16-byte column (8 channels) of a run of
-// 64 tokens through a private ring of shared-memory slots filled by cp.async (three 8-row pieces in flight per thread,
+// up to 64 tokens through a private ring of shared-memory slots filled by cp.async (three 8-row pieces in flight per thread,
 // up to 147 KB per SM: enough outstanding bytes to cover the DRAM latency, which registers cannot hold); nobody else
 // reads those slots, so cp.async.wait_group is the only synchronisation (no barrier, no spin-wait).  The taps run as
 // packed fp32 pairs (fma.rn.f32x2), and the sliding window lives in a ring of eight register rows whose slots are
 // compile-time constants: no row is ever moved.
-constexpr int kRun = 64, kPiece = 8, kStages = 4, kStagedThreads = 128;
+constexpr int kLongestRun = 64, kPiece = 8, kStages = 4, kStagedThreads = 128;
 constexpr int kStagedSmem = kStages * kPiece * kStagedThreads * 16;
 
 typedef unsigned long long f32x2;   // two packed floats
@@ -205,13 +211,16 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <typename T, int K>
+// RUN: the run length where it is the longest one, 0 where it is an argument.
+template <typename T, int K, int RUN>
 __global__ void __launch_bounds__(kStagedThreads, 3)
 conv1d_silu_staged_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
-                          int batch, int seqlen, int channels, int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl) {
+                          int batch, int seqlen, int channels, int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl,
+                          int run_arg) {
+  const int run_len = RUN ? RUN : run_arg;
   extern __shared__ __align__(16) unsigned char ring_smem[];
   const int cvecs = channels / 8;
-  const int runs = (seqlen + kRun - 1) / kRun;
+  const int runs = (seqlen + run_len - 1) / run_len;
   const int64_t total = (int64_t)batch * runs * cvecs;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -220,7 +229,7 @@ conv1d_silu_staged_kernel(const T* __restrict__ x, const T* __restrict__ w, cons
   const int run = (int)(r % runs);
   const int b = (int)(r / runs);
   const int c0 = 8 * cv;
-  const int t_begin = run * kRun, t_end = min(seqlen, t_begin + kRun);
+  const int t_begin = run * run_len, t_end = min(seqlen, t_begin + run_len);
   const int npieces = (t_end - t_begin + kPiece - 1) / kPiece;
   const T* xcol = x + b * xsb + c0;
   T* ycol = y + b * ysb + c0;
@@ -295,8 +304,9 @@ conv1d_silu_staged_kernel(const T* __restrict__ x, const T* __restrict__ w, cons
 template <typename T>
 int launch_conv(const void* x, const void* w, const void* bias, void* y, int batch, int seqlen, int channels, int taps,
                 int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl, cudaStream_t stream) {
-  const int chunks = (seqlen + kTokensPerThread - 1) / kTokensPerThread;
-  const int64_t total = (int64_t)batch * chunks * (channels / 8);
+  const int64_t columns = (int64_t)batch * (channels / 8);
+  const int run = run_length(32, 4, columns, seqlen, 148 * 192);
+  const int64_t total = columns * ((seqlen + run - 1) / run);
   if ((total + 127) / 128 > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
   const unsigned grid = (unsigned)((total + 127) / 128);
   const int per16 = 16 / (int)sizeof(T);
@@ -308,25 +318,25 @@ int launch_conv(const void* x, const void* w, const void* bias, void* y, int bat
   T* yy = static_cast<T*>(y);
   if constexpr (sizeof(T) == 2) {
     if (al && taps >= 2 && taps <= 4) {
-      const int runs = (seqlen + kRun - 1) / kRun;
-      const int64_t tot = (int64_t)batch * runs * (channels / 8);
+      const int len = run_length(kLongestRun, kPiece, columns, seqlen, 148 * 64);
+      const int64_t tot = columns * ((seqlen + len - 1) / len);
       if ((tot + kStagedThreads - 1) / kStagedThreads > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
       const unsigned g = (unsigned)((tot + kStagedThreads - 1) / kStagedThreads);
       auto go = [&](auto kern) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagedSmem) != cudaSuccess)
           return (int)SSD_ERR_CUDA;
-        kern<<<g, kStagedThreads, kStagedSmem, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl);
+        kern<<<g, kStagedThreads, kStagedSmem, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, len);
         return cudaGetLastError() == cudaSuccess ? (int)SSD_OK : (int)SSD_ERR_CUDA;
       };
-      if (taps == 2) return go(conv1d_silu_staged_kernel<T, 2>);
-      if (taps == 3) return go(conv1d_silu_staged_kernel<T, 3>);
-      return go(conv1d_silu_staged_kernel<T, 4>);
+      if (taps == 2) return len == kLongestRun ? go(conv1d_silu_staged_kernel<T, 2, kLongestRun>) : go(conv1d_silu_staged_kernel<T, 2, 0>);
+      if (taps == 3) return len == kLongestRun ? go(conv1d_silu_staged_kernel<T, 3, kLongestRun>) : go(conv1d_silu_staged_kernel<T, 3, 0>);
+      return len == kLongestRun ? go(conv1d_silu_staged_kernel<T, 4, kLongestRun>) : go(conv1d_silu_staged_kernel<T, 4, 0>);
     }
   }
   switch (taps) {
-    case 2: conv1d_silu_kernel<T, 2><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al); break;
-    case 3: conv1d_silu_kernel<T, 3><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al); break;
-    case 4: conv1d_silu_kernel<T, 4><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al); break;
+    case 2: conv1d_silu_kernel<T, 2><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); break;
+    case 3: conv1d_silu_kernel<T, 3><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); break;
+    case 4: conv1d_silu_kernel<T, 4><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); break;
     default: return SSD_ERR_UNSUPPORTED;
   }
   return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
