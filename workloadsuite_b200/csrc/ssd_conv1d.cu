@@ -162,6 +162,27 @@ conv1d_silu_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __
         }
       }
     }
+  } else if (vec) {
+    // fp32 rows, four at a time: eight 16-byte loads per thread in flight
+    constexpr int kBatch = 4;
+    for (int t0 = t_begin; t0 < t_end; t0 += kBatch) {
+      float rows[kBatch][8];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) load_row(t0 + u < t_end ? t0 + u : -1, rows[u]);
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        if (t0 + u < t_end) {
+#pragma unroll
+          for (int k = 0; k < K - 1; ++k) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) win[k][e] = win[k + 1][e];
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) win[K - 1][e] = rows[u][e];
+          emit(t0 + u, win);
+        }
+      }
+    }
   } else {
     for (int t = t_begin; t < t_end; ++t) {
 #pragma unroll
