@@ -1,0 +1,136 @@
+"""The branches that a call's sizes choose, at the sizes where each can go wrong: tails of tiles, half-empty head pairs,
+cut sequences, short runs, strided operands.  Tolerances as in ``test_ssd_gpu``: 2e-2 for 16-bit types (P and the state
+copy are rounded to 16 bits, 2^-8, and sums of N(0,1) products average that out), 1e-4 for fp32."""
+import pytest
+import torch
+
+from oracle import ssd_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+@pytest.fixture(autouse=True)
+def _no_device_side_timeouts():
+    yield
+    if torch.cuda.is_available():
+        import workloadsuite_b200 as W
+
+        assert W.device_status(DEV) == 0
+
+
+def _check(inp, kernel, tol, dt=None, D=None, z=None, **kw):
+    import workloadsuite_b200 as W
+
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    dev = lambda t: None if t is None else t.to(DEV)
+    Y, H = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, dt=dev(dt), initial_states=d.get("initial_states"),
+                         return_final_state=True, D=dev(D), z=dev(z), kernel=kernel, **kw)
+    torch.cuda.synchronize()
+    Yr, Hr = O.ssd_recurrence(inp["X"], inp["A"], inp["B"], inp["C"], dt=dt, initial_states=inp.get("initial_states"),
+                              return_final_state=True)
+    if D is not None:
+        Yr = Yr + inp["X"].double() * D.double()[None, None, :, None]
+    if z is not None:
+        Yr = Yr * torch.nn.functional.silu(z.double())
+    assert max(O.error_metrics(Y.cpu(), Yr)) < tol
+    assert ((H.cpu().double() - Hr).abs().amax(dim=(2, 3)) / Hr.abs().amax(dim=(2, 3)).clamp_min(1e-30)).max().item() < tol
+
+
+@pytest.mark.parametrize("s", [1, 31, 127, 128, 129, 300])
+@pytest.mark.parametrize("h,g,n", [(3, 1, 128), (4, 2, 64), (5, 5, 64)])
+def test_tensor_core_kernel_takes_any_length_and_odd_heads(s, h, g, n):
+    """Tails that are no whole tile (zero-filled by TMA, clipped on the way out) and groups whose last pair of heads is
+    half empty, with and without skip and gate."""
+    inp = O.make_inputs(b=2, s=s, h=h, p=64, n=n, g=g, dtype=torch.bfloat16, init=True, seed=60 + s, decay_scale=0.1)
+    gen = torch.Generator().manual_seed(s)
+    dt = (0.5 + torch.rand(2, s, h, generator=gen)).bfloat16()
+    _check(inp, "tcgen05", 2e-2, dt=dt)
+    D, z = torch.randn(h, generator=gen).bfloat16(), torch.randn(2, s, h, 64, generator=gen).bfloat16()
+    _check(inp, "tcgen05", 2e-2, dt=dt, D=D, z=z)
+
+
+@pytest.mark.parametrize("shape", [dict(b=50, s=300, h=7, g=1, n=128), dict(b=1, s=1500, h=3, g=1, n=64),
+                                   dict(b=40, s=513, h=8, g=2, n=64)], ids=["chained_odd", "lookback_odd", "chained_n64"])
+def test_cut_sequences_of_no_round_length(shape):
+    """Sequences dealt out over the CTAs (handed on, or folded from what the CTAs before published) whose last tile is
+    ragged; 50 x 7 heads are 200 pairs of which every fourth is half empty."""
+    inp = O.make_inputs(p=64, dtype=torch.float16, init=True, seed=70, decay_scale=0.02, **shape)
+    _check(inp, "tcgen05", 2e-2, nsegments=2)
+    gen = torch.Generator().manual_seed(71)
+    z = torch.randn(shape["b"], shape["s"], shape["h"], 64, generator=gen).half()
+    _check(inp, "tcgen05", 2e-2, nsegments=2, z=z)
+
+
+@pytest.mark.parametrize("s", [3, 8, 37, 130])
+@pytest.mark.parametrize("p,n", [(64, 16), (64, 128), (32, 32), (128, 64)])
+def test_fp32_scan_tokens_in_line_and_the_rest(s, p, n):
+    """Steps of up to 128 tokens, several tokens in line and the remainder one by one, full and partly used states."""
+    inp = O.make_inputs(b=2, s=s, h=2, p=p, n=n, g=1, dtype=torch.float32, init=True, seed=80 + s, decay_scale=0.3)
+    _check(inp, "scan_f32", 1e-4)
+
+
+def test_step_reads_strided_operands_and_d_in_its_own_type():
+    """Columns of a projection's output against the same values copied out: the same arithmetic, so the same bits."""
+    import workloadsuite_b200 as W
+
+    b, h, n, g = 3, 6, 128, 2
+    gen = torch.Generator(DEV).manual_seed(90)
+    proj = torch.randn(b, 2 * h * 64 + 2 * g * n + h + 5, generator=gen, device=DEV).half()
+    x, z, B, C, dt, _ = torch.split(proj, [h * 64, h * 64, g * n, g * n, h, 5], dim=-1)
+    x, z, B, C = x.unflatten(-1, (h, 64)), z.unflatten(-1, (h, 64)), B.unflatten(-1, (g, n)), C.unflatten(-1, (g, n))
+    a = -torch.rand(b, 2 * h, generator=gen, device=DEV)[:, ::2]
+    D = torch.randn(h, generator=gen, device=DEV).half()
+    S1 = torch.randn(b, h, n, 64, generator=gen, device=DEV)
+    S2 = S1.clone()
+    y1 = W.ssd_step(x, a, B, C, S1, dt=dt, D=D, z=z)
+    y2 = W.ssd_step(x.contiguous(), a.contiguous(), B.contiguous(), C.contiguous(), S2, dt=dt.contiguous(), D=D.float(),
+                    z=z.contiguous())
+    assert torch.equal(y1, y2) and torch.equal(S1, S2)
+
+
+@pytest.mark.parametrize("dtype,l,d", [(torch.float16, 1, 64), (torch.float16, 9, 128), (torch.bfloat16, 65, 64),
+                                       (torch.float32, 5, 64), (torch.float32, 67, 192), (torch.bfloat16, 2050, 4096)])
+def test_conv_run_lengths(dtype, l, d):
+    """From a run shorter than a piece to the longest run, against the operator in fp64 (one rounding of the result, and
+    tanh.approx for 16-bit types: 2^-8 of the largest value bounds both)."""
+    import workloadsuite_b200 as W
+
+    gen = torch.Generator().manual_seed(l)
+    x = torch.randn(2, l, d, generator=gen).to(dtype)
+    w, bias = (torch.randn(d, 1, 4, generator=gen) * 0.5).to(dtype), torch.randn(d, generator=gen).to(dtype)
+    y = W.conv1d_silu(x.to(DEV), w.to(DEV), bias.to(DEV)).cpu().double()
+    c = torch.nn.functional.conv1d(x.double().transpose(1, 2), w.double(), bias.double(), padding=3, groups=d)[..., :l]
+    ref = torch.nn.functional.silu(c).transpose(1, 2)
+    assert ((y - ref).abs().max() / ref.abs().max()).item() < (1e-5 if dtype == torch.float32 else 2 ** -8)
+
+
+def test_dt_prologue_eight_heads_per_thread():
+    """More than 2^17 elements take the vector path; the functions are those of the scalar one, so its rows have the same
+    bits as the first rows computed alone."""
+    import workloadsuite_b200 as W
+
+    gen = torch.Generator(DEV).manual_seed(91)
+    raw = (torch.randn(4, 1031, 40 + 8, generator=gen, device=DEV) * 3 - 2).half()[..., 8:]
+    bias, A_log = torch.randn(40, generator=gen, device=DEV).half(), torch.rand(40, generator=gen, device=DEV)
+    dt, A = W.dt_prologue(raw, bias, A_log)
+    dt1, A1 = W.dt_prologue(raw[:, :7], bias, A_log)
+    assert torch.equal(dt[:, :7], dt1) and torch.equal(A[:, :7], A1)
+    ref = torch.nn.functional.softplus((raw + bias).double())
+    assert ((dt.double() - ref).abs() <= 2 ** -10 * ref + 2 ** -24).all()     # half an ulp, or of the smallest step
+
+
+@pytest.mark.parametrize("b,s,h,n", [(3, 2048, 24, 128), (11, 384, 8, 64)], ids=["ramps_in_an_entry", "groups"])
+def test_host_pipeline_chunks_and_sets(b, s, h, n):
+    """Chunks, ramps and sets of batch entries against the device forward over the same tensors (other cuts of the
+    sequence, so other roundings of the carried state's copy)."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=1, dtype=torch.bfloat16, init=True, seed=95, decay_scale=0.05)
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    Y, H = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 128, initial_states=d["initial_states"], return_final_state=True)
+    r = W.HostRunner(b, s, h, 64, n, 1, 128, torch.bfloat16, device=DEV)
+    out, fin = torch.empty_like(inp["X"]), torch.empty(b, h, n, 64)
+    r.run(inp["X"], inp["A"], inp["B"], inp["C"], out, initial_states=inp["initial_states"], final_state=fin)
+    assert max(O.error_metrics(out, Y.cpu())) < 2e-2 and max(O.error_metrics(fin, H.cpu())) < 2e-2
