@@ -413,6 +413,9 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     setmaxnreg_dec<64>();
     if (warp == 0 && lane == 0) {
       // ---------------------------------------------------------------- TMA producer
+      // X is read once; B and C again by every other pair of heads of the group, perhaps much later (where a CTA works on one
+      // pair after the other, or the pairs' CTAs are at different places of the sequence)
+      const uint64_t once = policy_evict_first(), again = policy_evict_last();
       prefetch_tmap(&tmX); prefetch_tmap(&tmB); prefetch_tmap(&tmC); prefetch_tmap(&tmY);
       bool ok = true;
       uint32_t xi = 0, xph = 0;              // next X slot and how often the ring has been walked (parity)
@@ -436,7 +439,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           mbar_expect_tx(full, blocks * kBlk);
 #pragma unroll 1
           for (int kb = 0; kb < blocks; ++kb, dst += kBlk)
-            tma_load_5d(dst, tm, full, 64 * kb, k < 2 ? 2 * c.q + k : 0, c.g, c.t0, c.b);
+            tma_load_5d(dst, tm, full, 64 * kb, k < 2 ? 2 * c.q + k : 0, c.g, c.t0, c.b, k < 2 ? once : again);
           if (k < 2) {
             if (++xi == XS) { xi = 0; xph ^= 1; }
           } else if (k == 2) {
@@ -919,6 +922,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     uint32_t bi = 0, bph = 0;   // X slot of the next tile to make Xd of
     uint32_t xi = 0;            // X slot of the tile being read out
     uint32_t ky = 0;
+    const uint64_t once = policy_evict_first();
     int pending = -1;    // (lane 0) X slot that this warp's last TMA store still reads
     auto release = [&]() {
       if (lane == 0 && pending >= 0) {
@@ -1075,7 +1079,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         if (lane == 0) {
           // each warp hands its own 32 rows to the TMA engine; rows past the end of the sequence are clipped
           if (live && t0 + lane_base < sp.seqlen) {
-            tma_store_5d(&tmY, ystage + lane_base * 128, 0, 2 * c.q + h, c.g, t0 + lane_base, c.b);
+            tma_store_5d(&tmY, ystage + lane_base * 128, 0, 2 * c.q + h, c.g, t0 + lane_base, c.b, once);
             bulk_commit();
           }
           pending = (int)xi;
@@ -1109,8 +1113,14 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return SSD_ERR_CUDA;
   // chained mode: the tiles of all sequences are dealt out evenly, every CTA gets at least one
-  const long long tiles = (long long)prm.upairs * ((prm.sp.seqlen + T - 1) / T);
-  const int grid = prm.sp.chain ? (int)std::min<long long>(tiles, kSms) : std::min(prm.nitems, kSms);
+  const int nt = (prm.sp.seqlen + T - 1) / T;
+  int grid = prm.sp.chain ? (int)std::min<long long>((long long)prm.upairs * nt, kSms) : std::min(prm.nitems, kSms);
+  // Look-back: where it leaves few SMs out, every sequence in the same number of pieces, so that all pairs of heads are at the
+  // same tokens at the same time and find B and C in L2 (one sequence of 131 072 tokens, 16 pairs: 9 pieces each on 144 SMs).
+  if (prm.sp.chain == 2) {
+    const int pieces = std::min(kSms / prm.upairs, nt);
+    if (pieces > 1 && pieces * prm.upairs >= kSms * 93 / 100) grid = pieces * prm.upairs;
+  }
   kern<<<grid, kThreads2, smem, stream>>>(tx, tb, tc, ty, prm);
   return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
