@@ -52,11 +52,12 @@ def test_tensor_core_kernel_takes_any_length_and_odd_heads(s, h, g, n):
 
 
 @pytest.mark.parametrize("shape", [dict(b=50, s=300, h=7, g=1, n=128), dict(b=1, s=1500, h=3, g=1, n=64),
-                                   dict(b=40, s=513, h=8, g=2, n=64)], ids=["chained_odd", "lookback_odd", "chained_n64"])
+                                   dict(b=40, s=513, h=8, g=2, n=64), dict(b=1, s=4500, h=2, g=1, n=128, decay_scale=0.002)],
+                         ids=["chained_odd", "lookback_odd", "chained_n64", "lookback_36_pieces"])
 def test_cut_sequences_of_no_round_length(shape):
     """Sequences dealt out over the CTAs (handed on, or folded from what the CTAs before published) whose last tile is
-    ragged; 50 x 7 heads are 200 pairs of which every fourth is half empty."""
-    inp = O.make_inputs(p=64, dtype=torch.float16, init=True, seed=70, decay_scale=0.02, **shape)
+    ragged; 50 x 7 heads are 200 pairs of which every fourth is half empty; 36 pieces are more than a warp asks for at once."""
+    inp = O.make_inputs(**{"p": 64, "dtype": torch.float16, "init": True, "seed": 70, "decay_scale": 0.02, **shape})
     _check(inp, "tcgen05", 2e-2, nsegments=2)
     gen = torch.Generator().manual_seed(71)
     z = torch.randn(shape["b"], shape["s"], shape["h"], 64, generator=gen).half()

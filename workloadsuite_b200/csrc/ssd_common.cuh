@@ -48,7 +48,7 @@ struct ScanParams {
   // Look-back mode (2): chain_state / chain_ld hold each CTA's state-from-zero and log-decay sum of the last
   // piece of its range; a piece folds those of the CTAs before it.
   int chain;
-  float* chain_state;     // [slot][n*p], slot = 2 * CTA + head of the pair
+  float* chain_state;     // [slot][p/4][n][4], slot = 2 * CTA + head of the pair
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], zeroed before the launch
   // Optional epilogue Y <- (Y + x * D[head]) * silu(z) (model_ref.py:116-118); either pointer may be null.

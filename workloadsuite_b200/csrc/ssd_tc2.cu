@@ -714,20 +714,18 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
       }
     };
-    // (bounded) wait until the four warps of head h of CTAs `from` .. `to` have published.  Every warp asks for itself: a
-    // barrier among the four would hang where one of them has given up.
+    // (bounded) wait until the four warps of head h of CTAs `from` .. `to` have published, a CTA per lane.  Every warp asks for
+    // itself: a barrier among the four would hang where one of them has given up.
     auto wait_published = [&](int to, int from) {
-      if (lane == 0) {
-        const long long c0 = clock64();
-        for (int c = to; c >= from && !m->abort_flag; --c) {
-          while (true) {
-            int f;
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + 2 * c + h) : "memory");
-            if (f >= 4 || m->abort_flag) break;
-            if (clock64() - c0 > m->wait_clocks) {
-              m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
-              break;
-            }
+      const long long c0 = clock64();
+      for (int c = to - lane; c >= from && !m->abort_flag; c -= 32) {
+        while (true) {
+          int f;
+          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + 2 * c + h) : "memory");
+          if (f >= 4 || m->abort_flag) break;
+          if (clock64() - c0 > m->wait_clocks) {
+            m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
+            break;
           }
         }
       }
@@ -767,6 +765,9 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // Chained: what the CTA before this one handed over.  Look-back: fold the pairs (state from zero, log-decay
     // sum) that the CTAs from .. before this one published for their pieces of this sequence, newest first:
     // H_in = sum_c exp(log-decay after c) F_c (+ the same for the caller's initial state).
+    // Latency-bound, a piece after the other, so the flags are asked for by 32 lanes at once and in a slot the threads' 16
+    // bytes stand side by side: rows of 256 bytes, as the caller's states have them, cost 32 cache lines a load.  One sequence
+    // of 64 tiles on 64 SMs: 137 -> 37 us; 16 pairs of 16 tiles 54 -> 27; chained, 250 pairs of 16 tiles 103 -> 99.
     auto fold_item = [&]() {
       const bool look_back = sp.chain == 2;
       const bool init = sp.init && c.live(wk, h) && look_back;
@@ -775,26 +776,26 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       wait_published(p, from);
 #pragma unroll 1
       for (;; --p) {
-        const float* src;
-        if (p >= from) {
-          src = sp.chain_state + (2 * p + h) * (int64_t)(N * P);
-        } else {
-          if (!init) break;
-          src = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride;
-        }
+        const bool piece = p >= from;
+        if (!piece && !init) break;
+        const float* src = piece ? sp.chain_state + (2 * p + h) * (int64_t)(N * P) + l * 4
+                                 : sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride +
+                                       c.seg * sp.init_seg_stride + (int64_t)l * P;
+        const int step = piece ? N : 1;
+        const float ld = piece ? __ldcg(sp.chain_ld + 2 * p + h) : 0.f;
         const float wgt = ex2(asum0 * kLog2e);   // asum0: log-decay between the end of the piece being added and this item
         if (owns_state && wgt != 0.f) {          // (an underflowed piece adds nothing)
-          const float4* I = reinterpret_cast<const float4*>(src + (int64_t)l * P);
+          const ulonglong2* I = reinterpret_cast<const ulonglong2*>(src);
           const uint64_t w2 = pair(wgt, wgt);
 #pragma unroll
           for (int e = 0; e < P / 4; ++e) {
-            const float4 v = __ldcg(I + e);      // (may be written by another SM: bypass L1)
-            H[2 * e] = fma_pair(w2, pair(v.x, v.y), H[2 * e]);
-            H[2 * e + 1] = fma_pair(w2, pair(v.z, v.w), H[2 * e + 1]);
+            const ulonglong2 v = __ldcg(I + e * step);   // (may be written by another SM: bypass L1)
+            H[2 * e] = fma_pair(w2, v.x, H[2 * e]);
+            H[2 * e + 1] = fma_pair(w2, v.y, H[2 * e + 1]);
           }
         }
-        if (p < from) break;
-        asum0 += __ldcg(sp.chain_ld + 2 * p + h);
+        if (!piece) break;
+        asum0 += ld;
       }
     };
     // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
@@ -810,13 +811,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       float* ld = publish ? sp.chain_ld + slot
                           : (sp.fin_ld ? sp.fin_ld + unit * sp.finld_unit_stride + seg * sp.finld_seg_stride : nullptr);
       if (to && owns_state) {
-        float* F = to + (int64_t)l * P;
-        if (prm.st32) {
+        float* F = to + (publish ? l * 4 : l * P);
+        const int step = publish ? N : 1;
+        if (prm.st32 && !publish) {
 #pragma unroll
           for (int e = 0; e < P / 8; ++e) stg256(F + 8 * e, H[4 * e], H[4 * e + 1], H[4 * e + 2], H[4 * e + 3]);
         } else {
 #pragma unroll
-          for (int e = 0; e < P / 4; ++e) reinterpret_cast<ulonglong2*>(F)[e] = make_ulonglong2(H[2 * e], H[2 * e + 1]);
+          for (int e = 0; e < P / 4; ++e) reinterpret_cast<ulonglong2*>(F)[e * step] = make_ulonglong2(H[2 * e], H[2 * e + 1]);
         }
       }
       if (ld && l == 0) *ld = asum0 + asum;
@@ -1142,12 +1144,6 @@ bool tc_supports(const SsdArgs& a) {
   return true;
 }
 
-// Rounds of `items` equal work items over the persistent grid, as a fraction of the ideal.
-static double round_efficiency(int64_t items) {
-  const int64_t rounds = (items + kSms - 1) / kSms;
-  return (double)items / (double)(rounds * kSms);
-}
-
 // How a sequence that is cut (nseg > 1) is scanned by this kernel:
 //   1  with at least one sequence per SM the tiles of all sequences are dealt out evenly over the CTAs inside one
 //      launch; a sequence cut that way hands its state from CTA to CTA through scratch ("chained");
@@ -1166,21 +1162,25 @@ int tc2_chain_mode(const SsdArgs& a, int nseg) {
 int tc2_default_segments(const SsdArgs& a) {
   const int64_t upairs = unit_pairs(a);
   const int tiles = (a.seqlen + T - 1) / T;
-  // whole sequences already fill the rounds of the persistent grid well: no cuts; else the even deal (any count
-  // above one selects it, the cut points follow from the grid)
-  if (upairs >= kSms) return (round_efficiency(upairs) >= 0.97 || tiles < 2) ? 1 : 2;
-  const double whole = (double)tiles + 1.5;   // one CTA per sequence, in tile times
+  // Costs in tile times (2.7 to 3.1 us), fitted to forwards of 1 to 600 pairs and 2 to 64 tiles, each timed whole and cut; the
+  // constants are what a launch takes beside its tiles.  16 pairs of 4, 8 and 64 tiles: whole 17, 28 and 184 us, cut 18, 21
+  // and 49; 250 pairs of 8, 16 and 64 tiles: 53, 104 and 403, cut 56, 99 and 362.
+  const double even = (double)upairs * tiles / kSms;   // tiles per SM under the even deal (any count above one selects it)
+  if (upairs >= kSms) {
+    const double rounds = (double)((upairs + kSms - 1) / kSms);
+    return tiles >= 2 && even * 1.02 + 5.7 < 0.98 * (rounds * tiles + 2.4) ? 2 : 1;
+  }
   if (!(a.flags & (SSD_FLAG_STATE_ONLY | SSD_FLAG_REUSE_SEGMENTS))) {
-    // Look-back: every CTA gets total / SMs tiles plus the state-only scan of its last piece (0.4 of a full
-    // tile, on most of its range) and two item start-ups.
-    const double lookback = (double)upairs * tiles / kSms * 1.3 + 3.5;
-    return (tiles >= 2 && lookback < 0.95 * whole) ? 2 : 1;
+    // Look-back: the state-only scan of the last piece of every range, two start-ups and the round trip through scratch, and
+    // the fold of the pieces before the last one of a sequence.
+    const double pieces = std::min((double)kSms / upairs, (double)tiles);
+    return tiles >= 2 && even * 1.4 + 6 + 0.12 * pieces < 0.98 * (tiles + 2.2) ? 2 : 1;
   }
   if (upairs >= 120) return 1;
   // Two passes: cutting the sequences into concurrently scanned segments costs a second pass
   // (about 0.4 of a full pass) and a per-item start-up (about 1.5 tile times).  Pick the count that
   // minimises the modelled time, in tile times, of the busiest CTA.
-  double best_cost = whole;
+  double best_cost = (double)tiles + 1.5;   // one CTA per sequence
   int best = 1;
   for (int nseg = 2; nseg <= 32 && nseg * 2 <= tiles; ++nseg) {
     const int64_t rounds = (upairs * nseg + kSms - 1) / kSms;
