@@ -1122,6 +1122,10 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
   if (prm.sp.chain == 2) {
     const int pieces = std::min(kSms / prm.upairs, nt);
     if (pieces > 1 && pieces * prm.upairs >= kSms * 93 / 100) grid = pieces * prm.upairs;
+    // With more than half as many pairs as SMs the deal saves little and every tile of a range's last piece is read twice: whole
+    // sequences, unless the saving (at 1.55 of a tile's time for a dealt one) is more than the start-ups of a cut (96 pairs
+    // of 64 tiles: 204 us dealt out, 185 whole; 80 pairs of 64: 174 and 185).
+    if (pieces == 1 && (double)prm.upairs * nt / kSms * 1.55 + 6 > nt + 2.2) grid = prm.upairs;
   }
   kern<<<grid, kThreads2, smem, stream>>>(tx, tb, tc, ty, prm);
   return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
