@@ -133,9 +133,9 @@ const char* ssd_b200_kernel_name(const SsdArgs* args);
 
 /* How ssd_b200_forward() will run these arguments: the resolved SSD_KERNEL_* family, the number of
  * segments each sequence is cut into (2 stands for "cut" where the cut points follow from the grid),
- * and the number of kernel launches it enqueues: 1 for whole sequences; 1 plus a memset where the
- * two-head tensor-core kernel deals the tiles of all sequences out evenly inside one launch (states
- * handed from CTA to CTA, or folded from the pairs each CTA publishes for the last piece of its range);
+ * and the number of kernel launches it enqueues: 1 for whole sequences; 1 plus a clearing of flags
+ * (a block that the launch overlaps) where the two-head tensor-core kernel deals the tiles of all
+ * sequences out evenly inside one launch (states handed from CTA to CTA, or folded from the pairs each CTA publishes for the last piece of its range);
  * 3 for the two-pass segmented scan (2 with SSD_FLAG_STATE_ONLY or SSD_FLAG_REUSE_SEGMENTS).  Any out
  * pointer may be NULL.  Returns SSD_OK or the validation error.  No reference counterpart. */
 int ssd_b200_plan(const SsdArgs* args, int32_t* kernel, int32_t* nsegments, int32_t* launches);

@@ -228,9 +228,7 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
     char* ws = static_cast<char*>(args->workspace);
     float* slot_state = reinterpret_cast<float*>(ws);
     float* slot_ld = reinterpret_cast<float*>(ws + align_up(slots * np * sizeof(float), 256));
-    int32_t* flags = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(slot_ld) + align_up(slots * sizeof(float), 256));
-    // the ready flags must start at zero (the workspace keeps the previous call's contents)
-    if (cudaMemsetAsync(flags, 0, slots * sizeof(int32_t), stream) != cudaSuccess) return SSD_ERR_CUDA;
+    int32_t* flags = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(slot_ld) + align_up(slots * sizeof(float), 256));   // (cleared by the launch)
     ssd::ScanParams pc = prm;
     pc.compute_y = state_only ? 0 : 1;
     pc.chain = chain_mode;

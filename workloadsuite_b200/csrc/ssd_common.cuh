@@ -50,7 +50,7 @@ struct ScanParams {
   int chain;
   float* chain_state;     // [slot][p/4][n][4], slot = 2 * CTA + head of the pair
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
-  int32_t* chain_flag;    // [slot], zeroed before the launch
+  int32_t* chain_flag;    // [slot], cleared by the launch
   // Optional epilogue Y <- (Y + x * D[head]) * silu(z) (model_ref.py:116-118); either pointer may be null.
   const float* D;         // [h], fp32 or (d_in_dtype) elements of the tensors' type
   const void* Z;          // [b,s,h,p], strides zs

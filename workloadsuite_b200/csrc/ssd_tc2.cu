@@ -717,6 +717,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // (bounded) wait until the four warps of head h of CTAs `from` .. `to` have published, a CTA per lane.  Every warp asks for
     // itself: a barrier among the four would hang where one of them has given up.
     auto wait_published = [&](int to, int from) {
+      grid_dependency_wait();
       const long long c0 = clock64();
       for (int c = to - lane; c >= from && !m->abort_flag; c -= 32) {
         while (true) {
@@ -826,6 +827,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         // Each warp publishes its own rows: a release-add by lane 0 after a warp barrier orders the
         // whole warp's stores before the count, and nobody has to wait for the stores to land.
         __syncwarp();
+        grid_dependency_wait();
         if (lane == 0) {
           const int one = 1;
           asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + slot), "r"(one) : "memory");
@@ -1103,8 +1105,17 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   }
   if (warp == 0) {
     __syncwarp();
+    grid_dependency_wait();   // (where no sequence of this CTA was cut)
     tmem_dealloc(m->tmem_base, 512);
   }
+}
+
+// The ready flags of a launch with cut sequences have to start at zero (the workspace keeps the call before's).  The forward
+// starts beside this kernel, which itself starts when all work before it in the stream is done, and asks for its end
+// (grid_dependency_wait) only where a flag is first used; a memset ahead of the forward cost 4 us of every such call.
+__global__ void clear_flags_kernel(int* flags) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  flags[threadIdx.x] = 0;
 }
 
 template <typename T16, int N, bool EPI>
@@ -1125,10 +1136,22 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
     // With more than half as many pairs as SMs the deal saves little and every tile of a range's last piece is read twice: whole
     // sequences, unless the saving (at 1.55 of a tile's time for a dealt one) is more than the start-ups of a cut (96 pairs
     // of 64 tiles: 204 us dealt out, 185 whole; 80 pairs of 64: 174 and 185).
-    if (pieces == 1 && (double)prm.upairs * nt / kSms * 1.55 + 6 > nt + 2.2) grid = prm.upairs;
+    if (pieces == 1 && (double)prm.upairs * nt / kSms * 1.55 + 5 > nt + 2.2) grid = prm.upairs;
   }
-  kern<<<grid, kThreads2, smem, stream>>>(tx, tb, tc, ty, prm);
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = kThreads2;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute early;
+  if (prm.sp.chain) {
+    clear_flags_kernel<<<1, 2 * kSms, 0, stream>>>(prm.sp.chain_flag);
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kern, tx, tb, tc, ty, prm) == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
 
 // Head pairs over the whole batch; a group with an odd number of heads has a half-empty pair.
@@ -1167,18 +1190,18 @@ int tc2_default_segments(const SsdArgs& a) {
   const int64_t upairs = unit_pairs(a);
   const int tiles = (a.seqlen + T - 1) / T;
   // Costs in tile times (2.7 to 3.1 us), fitted to forwards of 1 to 600 pairs and 2 to 64 tiles, each timed whole and cut; the
-  // constants are what a launch takes beside its tiles.  16 pairs of 4, 8 and 64 tiles: whole 17, 28 and 184 us, cut 18, 21
-  // and 49; 250 pairs of 8, 16 and 64 tiles: 53, 104 and 403, cut 56, 99 and 362.
+  // constants are what a launch takes beside its tiles.  16 pairs of 4, 8 and 32 tiles: whole 17, 29 and 95 us, cut 16, 18
+  // and 33; 250 pairs of 4, 8 and 32 tiles: 31, 54 and 199, cut 33, 54 and 181.
   const double even = (double)upairs * tiles / kSms;   // tiles per SM under the even deal (any count above one selects it)
   if (upairs >= kSms) {
     const double rounds = (double)((upairs + kSms - 1) / kSms);
-    return tiles >= 2 && even * 1.02 + 5.7 < 0.98 * (rounds * tiles + 2.4) ? 2 : 1;
+    return tiles >= 2 && even * 1.02 + 4.9 < 0.98 * (rounds * tiles + 2.4) ? 2 : 1;
   }
   if (!(a.flags & (SSD_FLAG_STATE_ONLY | SSD_FLAG_REUSE_SEGMENTS))) {
     // Look-back: the state-only scan of the last piece of every range, two start-ups and the round trip through scratch, and
     // the fold of the pieces before the last one of a sequence.
     const double pieces = std::min((double)kSms / upairs, (double)tiles);
-    return tiles >= 2 && even * 1.4 + 6 + 0.12 * pieces < 0.98 * (tiles + 2.2) ? 2 : 1;
+    return tiles >= 2 && even * 1.4 + 4.9 + 0.12 * pieces < 0.98 * (tiles + 2.2) ? 2 : 1;
   }
   if (upairs >= 120) return 1;
   // Two passes: cutting the sequences into concurrently scanned segments costs a second pass

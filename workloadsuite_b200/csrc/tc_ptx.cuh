@@ -213,6 +213,9 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// Waits for the end of the kernel ahead of a programmatic launch (at once after any other launch).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float lg2(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
