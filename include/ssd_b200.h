@@ -277,7 +277,7 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
  *   - All calls on one device share the array, and it keeps the previous call's
  *     contents.  The two-pass scan writes every segment state before it reads it;
  *     the single-launch (chained) scan needs its ready flags at zero, and the
- *     forward clears them itself with a memset on `stream` ahead of the kernel.
+ *     forward clears them itself on `stream`.
  *     The caller clears nothing.  Two calls whose kernels may overlap on the GPU
  *     (different streams) race on the array: serialise them.
  * ssd_b200_static_scratch_capacity() returns SSD_STATIC_SCRATCH_BYTES. */

@@ -339,7 +339,9 @@ int launch_conv(const void* x, const void* w, const void* bias, void* y, int bat
   T* yy = static_cast<T*>(y);
   if constexpr (sizeof(T) == 2) {
     if (al && taps >= 2 && taps <= 4) {
-      const int len = run_length(kLongestRun, kPiece, columns, seqlen, 148 * 64);
+      // a block per SM (b1 s4096 h32: 13.4 us with half a block's worth, 12.4 so; with two it is 18.0, the rows before the
+      // runs read again and a second round of blocks)
+      const int len = run_length(kLongestRun, kPiece, columns, seqlen, 148 * 128);
       const int64_t tot = columns * ((seqlen + len - 1) / len);
       if ((tot + kStagedThreads - 1) / kStagedThreads > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
       const unsigned g = (unsigned)((tot + kStagedThreads - 1) / kStagedThreads);

@@ -62,7 +62,7 @@ int ssd_b200_forward_static_scratch(const SsdArgs* args, void* stream) {
   }
   // The two-pass forward writes every segment state and log-decay sum before it reads
   // it; the single-launch (chained) forward needs its ready flags at zero and clears
-  // them itself with a memset on `stream`.  So the caller never has to clear the array.
+  // them itself on `stream`.  So the caller never has to clear the array.
   return ssd_b200_forward(&a, stream);
 }
 
