@@ -45,9 +45,11 @@ enum { SSD_DTYPE_F32 = 0, SSD_DTYPE_F16 = 1, SSD_DTYPE_BF16 = 2 };
 
 /* kernel selection */
 enum {
-  SSD_KERNEL_AUTO = 0,    /* tensor-core kernel when the shape allows, else the fp32 scan */
+  SSD_KERNEL_AUTO = 0,    /* tensor-core kernel when the shape allows and the sequence is whole tiles of 128 tokens,
+                             else the fp32 scan */
   SSD_KERNEL_SCAN_F32 = 1,/* fp32 token recurrence on CUDA cores (any dtype in, fp32 math) */
-  SSD_KERNEL_TCGEN05 = 2  /* tcgen05/TMEM chunked kernel (f16/bf16 only) */
+  SSD_KERNEL_TCGEN05 = 2  /* tcgen05/TMEM chunked kernel (f16/bf16 only, any length): many times faster than the scan,
+                             but the masked products, the decayed X and the state's copy are rounded to 16 bits */
 };
 
 /* flags */

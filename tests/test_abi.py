@@ -208,6 +208,17 @@ def test_plan_of_the_benchmark_configurations(lib):
     assert _plan(lib, _shape(2, 512, 3, 64, 128, 3, 128, _lib.DTYPE_F16))[0] == TC
 
 
+def test_lengths_that_are_no_whole_tiles_stay_in_fp32_unless_the_caller_asks(lib):
+    """The tensor-core kernel takes any length, but rounds P and the copy of the state to 16 bits: by itself the library
+    chooses it for whole tiles only."""
+    for s in (20, 127, 129, 300, 3001):
+        a = _shape(2, s, 80, 64, 128, 1, 1, _lib.DTYPE_BF16)
+        assert lib.ssd_b200_kernel_name(C.byref(a)) == b"scan_f32", s
+        a.kernel = _lib.KERNEL_TCGEN05
+        assert lib.ssd_b200_kernel_name(C.byref(a)) == b"tcgen05", s
+    assert lib.ssd_b200_kernel_name(C.byref(_shape(2, 384, 80, 64, 128, 1, 1, _lib.DTYPE_BF16))) == b"tcgen05"
+
+
 def test_host_pipeline_scratch_sizes(lib):
     """The host-buffer entry sizes its device scratch from the shape alone: chunks of at most 24 MiB of X, four slots."""
     big = lib.ssd_b200_host_scratch_bytes(C.byref(_shape(4, 8192, 80, 64, 128, 1, 256, _lib.DTYPE_BF16)))

@@ -51,6 +51,24 @@ def test_tensor_core_kernel_takes_any_length_and_odd_heads(s, h, g, n):
     _check(inp, "tcgen05", 2e-2, dt=dt, D=D, z=z)
 
 
+@pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -11)])
+@pytest.mark.parametrize("s,h,g", [(20, 4, 1), (300, 4, 2), (130, 5, 1)])
+def test_lengths_that_are_no_whole_tiles_are_rounded_once(s, h, g, dtype, eps):
+    """Without a choice of kernel they are computed in fp32: Y is off by its own rounding (half an ulp, eps / 2 of the value
+    and at most eps of it) and the fp32 sums' 1e-5, the fp32 final state by 1e-5."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=2, s=s, h=h, p=64, n=128, g=g, dtype=dtype, init=True, seed=65 + s, decay_scale=0.1)
+    dt = (0.5 + torch.rand(2, s, h, generator=torch.Generator().manual_seed(s))).to(dtype)
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    Y, H = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, dt=dt.to(DEV), initial_states=d["initial_states"],
+                         return_final_state=True)
+    Yr, Hr = O.ssd_recurrence(inp["X"], inp["A"], inp["B"], inp["C"], dt=dt, initial_states=inp["initial_states"],
+                              return_final_state=True)
+    assert ((Y.cpu().double() - Yr).abs() <= eps * Yr.abs() + 1e-5 * Yr.abs().max()).all()
+    assert ((H.cpu().double() - Hr).abs().max() / Hr.abs().max()).item() < 1e-5
+
+
 @pytest.mark.parametrize("shape", [dict(b=50, s=300, h=7, g=1, n=128), dict(b=1, s=1500, h=3, g=1, n=64),
                                    dict(b=40, s=513, h=8, g=2, n=64), dict(b=1, s=4500, h=2, g=1, n=128, decay_scale=0.002)],
                          ids=["chained_odd", "lookback_odd", "chained_n64", "lookback_36_pieces"])

@@ -11,7 +11,7 @@ namespace {
 
 constexpr int kAbiVersion = 3;
 constexpr int kSmCount = 148;  // B200
-constexpr int kShortSequence = 32;   // tokens; one staged piece of the fp32 scan
+constexpr int kTcTile = 128;   // tokens of a tensor-core tile
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -47,11 +47,13 @@ int resolve_kernel(const SsdArgs* a) {
   if (a->kernel == SSD_KERNEL_TCGEN05) return SSD_KERNEL_TCGEN05;
   // (states that are only 4-byte aligned go to the fp32 scan, which moves them element by element)
   const bool st16 = aligned16(a->initial_state) && aligned16(a->final_state);
-  // A tile of the tensor-core kernel takes as long for one token as for 128; a few tokens are quicker in the fp32 scan.
-  return ssd::tc_supports(*a) && st16 && a->seqlen >= kShortSequence ? SSD_KERNEL_TCGEN05 : SSD_KERNEL_SCAN_F32;
+  // Whole tiles only.  The tensor-core kernel takes any length, but rounds P, Xd and the copy of the state to 16 bits; other
+  // lengths stay in fp32 with one rounding of Y unless the caller asks for that kernel.  bf16, 2 x 3001 tokens, against 64
+  // bits: Y 1.66e-3 here (its own rounding) and 2.42e-3 there, final state 1.4e-7 and 2.4e-3.
+  return ssd::tc_supports(*a) && st16 && a->seqlen % kTcTile == 0 ? SSD_KERNEL_TCGEN05 : SSD_KERNEL_SCAN_F32;
 }
 
-int tile_tokens(int kernel) { return kernel == SSD_KERNEL_TCGEN05 ? 128 : ssd::scan_f32_tile_tokens(); }
+int tile_tokens(int kernel) { return kernel == SSD_KERNEL_TCGEN05 ? kTcTile : ssd::scan_f32_tile_tokens(); }
 
 // Number of independently scanned segments per sequence and their length.
 void resolve_segments(const SsdArgs* a, int kernel, int* nseg, int* seg_len) {

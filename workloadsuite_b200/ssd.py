@@ -184,6 +184,12 @@ def ssd_forward(
     reference block's own X, ``model_ref.py:83-89``) is first copied into the row layout.
     All tensors must be on X's device.  No host synchronisation.
 
+    ``kernel``: None lets the library choose.  ``"tcgen05"`` (16-bit tensors, p = 64, n = 64 or 128) runs on the tensor
+    cores and rounds intermediate operands to 16 bits; it is chosen for sequences of whole tiles (multiples of 128 tokens).
+    ``"scan_f32"`` computes in float32 throughout; it is chosen for everything else, and ``kernel="tcgen05"`` takes any
+    length at a fraction of its time where 16-bit intermediates are accurate enough (relative error of Y in bfloat16
+    2.4e-3 instead of 1.7e-3, of the final state 2e-3 instead of 1e-7).
+
     ``nsegments``: None lets the library choose; 1 keeps sequences whole; more cuts them (see ``plan``):
     the tensor-core kernel deals the tiles of all sequences out evenly over the SMs inside one launch, the other
     kernels scan that many segments in two passes joined by a fold.
