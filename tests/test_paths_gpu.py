@@ -51,6 +51,25 @@ def test_tensor_core_kernel_takes_any_length_and_odd_heads(s, h, g, n):
     _check(inp, "tcgen05", 2e-2, dt=dt, D=D, z=z)
 
 
+@pytest.mark.parametrize("dtype,ulp", [(torch.bfloat16, 2 ** -7), (torch.float16, 2 ** -10)])
+@pytest.mark.parametrize("h,g", [(3, 1), (4, 4), (10, 2)])
+def test_groups_with_an_odd_number_of_heads_round_the_decayed_x_once(h, g, dtype, ulp):
+    """A rounding's relative error is ulp / 2 / sqrt(3) * 0.72 in the mean (the 0.72 for mantissas spread over their octave): 0.21
+    ulp.  The final state sums once-rounded products, so that is its error too (0.29 with the scale rounded as well); Y has
+    P, the state's copy and its own rounding, and the gate in fp32 between two roundings (0.38 against 0.48 with a packed gate)."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=2, s=1024, h=h, p=64, n=128, g=g, dtype=dtype, seed=66, decay_scale=1.0)
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    gen = torch.Generator().manual_seed(67)
+    D, z = torch.randn(h, generator=gen).to(dtype), torch.randn(2, 1024, h, 64, generator=gen).to(dtype)
+    Y, H = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 128, D=D.to(DEV), z=z.to(DEV), return_final_state=True)
+    Yr, Hr = O.ssd_recurrence(inp["X"], inp["A"], inp["B"], inp["C"], return_final_state=True)
+    Yr = (Yr + inp["X"].double() * D.double()[:, None]) * torch.nn.functional.silu(z.double())
+    assert ((H.cpu().double() - Hr).norm() / Hr.norm()).item() < 0.24 * ulp
+    assert ((Y.cpu().double() - Yr).norm() / Yr.norm()).item() < 0.42 * ulp
+
+
 @pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -11)])
 @pytest.mark.parametrize("s,h,g", [(20, 4, 1), (300, 4, 2), (130, 5, 1)])
 def test_lengths_that_are_no_whole_tiles_are_rounded_once(s, h, g, dtype, eps):

@@ -295,7 +295,8 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
   if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false);
   // skip and gate of model_ref.py:116-118: fused into the tensor-core kernel, a kernel of their own otherwise
   const int kernel = resolve_kernel(args);
-  const bool fuse = kernel == SSD_KERNEL_TCGEN05 && ssd::tc_supports(*args) && z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
+  const bool fuse = kernel == SSD_KERNEL_TCGEN05 && ssd::tc_supports(*args) && ssd::tc2_fuses_epilogue(*args) &&
+                    z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
   rc = forward_impl(args, stream_v, fuse);
   if (rc != SSD_OK || fuse) return rc;
   ssd::ScanParams ep;

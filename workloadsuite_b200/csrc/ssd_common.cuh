@@ -95,6 +95,7 @@ int launch_fold(const float* states, int64_t st_unit_stride, int64_t st_seg_stri
 
 // tensor-core kernel (ssd_tc2.cu)
 bool tc_supports(const SsdArgs& a);
+bool tc2_fuses_epilogue(const SsdArgs& a);
 int tc2_default_segments(const SsdArgs& a);
 int tc2_chain_mode(const SsdArgs& a, int nseg);   // 1: chained, 2: look-back (one launch each); 0: two passes + fold
 int launch_tc2(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);

@@ -314,8 +314,9 @@ __device__ __forceinline__ void stg256(void* p, uint64_t a, uint64_t b, uint64_t
 }
 
 // B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148) of rows 32 q .. 32 q + 31, in packed 16-bit arithmetic as the
-// reference does it.  Eight lanes share a row (one 16-byte piece each), a warp moves four rows per instruction.
-template <typename T16>
+// reference does it (WIDE: in fp32, rounded once).  Eight lanes share a row (one 16-byte piece each), a warp moves four rows
+// per instruction.
+template <typename T16, bool WIDE>
 __device__ __forceinline__ void make_xd(uint32_t xb, uint32_t xd, const Factors& f, int q, int lane) {
   uint32_t r = 32 * q + ((uint32_t)lane >> 3);
   const uint32_t pc = (uint32_t)lane & 7u;
@@ -331,16 +332,27 @@ __device__ __forceinline__ void make_xd(uint32_t xb, uint32_t xd, const Factors&
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const uint32_t d = pack2<T16>(sc[k], sc[k]);
       uint4 v;
-      v.x = mul2<T16>(a[k].x, d); v.y = mul2<T16>(a[k].y, d); v.z = mul2<T16>(a[k].z, d); v.w = mul2<T16>(a[k].w, d);
+      if constexpr (WIDE) {
+        const uint64_t d = pair(sc[k], sc[k]);
+        auto times = [&](uint32_t x) {
+          const float2 xf = unpack2<T16>(x);
+          return pack_pair<T16>(mul_pair(pair(xf.x, xf.y), d));
+        };
+        v.x = times(a[k].x); v.y = times(a[k].y); v.z = times(a[k].z); v.w = times(a[k].w);
+      } else {
+        const uint32_t d = pack2<T16>(sc[k], sc[k]);
+        v.x = mul2<T16>(a[k].x, d); v.y = mul2<T16>(a[k].y, d); v.z = mul2<T16>(a[k].z, d); v.w = mul2<T16>(a[k].w, d);
+      }
       sts128(xd + (r + 4 * k) * 128 + ((pc ^ ((r + 4 * k) & 7u)) << 4), v);
     }
   }
 }
 
 // EPI: apply the skip and gate of model_ref.py:116-118 to Y on its way out (sp.D / sp.Z; either may be null).
-template <typename T16, int N, bool EPI>
+// WIDE: Xd in fp32 arithmetic.  Groups with an odd number of heads have always had it so (bf16, final state against 64 bits:
+// 1.65e-3, with the packed products 2.23e-3); those with an even number have the reference's packed products.
+template <typename T16, int N, bool EPI, bool WIDE>
 __global__ void __launch_bounds__(kThreads2, 1)
 ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY,
@@ -861,7 +873,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         // B. (the read-out warps have the skip and the gate to do; the S MMA that read the Xd before was waited for in E)
         wait(&m->full_f[h][slot], (n / kFactors) & 1, m);
         wait(&m->full_x[xi], xph, m);
-        make_xd<T16>(sX + xi * kBlk, sXd + h * kBlk, m->f[h][slot], q, lane);
+        make_xd<T16, WIDE>(sX + xi * kBlk, sXd + h * kBlk, m->f[h][slot], q, lane);
         wait(&m->full_b[n % BC], (n / BC) & 1, m);   // (for the S MMA, which waits for these warps only)
         fence_proxy_async();
         warp_arrive(&m->bar_xd);
@@ -949,7 +961,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         for (int h = 0; h < 2; ++h) {
           wait(&m->full_f[h][k % kFactors], (k / kFactors) & 1, m);
           wait(&m->full_x[bi], bph, m);
-          make_xd<T16>(sX + bi * kBlk, sXd + h * kBlk, m->f[h][k % kFactors], q, lane);
+          make_xd<T16, WIDE>(sX + bi * kBlk, sXd + h * kBlk, m->f[h][k % kFactors], q, lane);
           if (k < npre) {   // nothing else reads X and the factors of a state-only tile
             __syncwarp();
             if (lane == 0) {
@@ -1118,10 +1130,10 @@ __global__ void clear_flags_kernel(int* flags) {
   flags[threadIdx.x] = 0;
 }
 
-template <typename T16, int N, bool EPI>
+template <typename T16, int N, bool EPI, bool WIDE>
 int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& ty,
                   const Tc2Params& prm, cudaStream_t stream) {
-  auto kern = ssd_tc2_kernel<T16, N, EPI>;
+  auto kern = ssd_tc2_kernel<T16, N, EPI, WIDE>;
   constexpr int smem = Layout2<N>::kBytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return SSD_ERR_CUDA;
@@ -1154,10 +1166,16 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
   return cudaLaunchKernelEx(&cfg, kern, tx, tb, tc, ty, prm) == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
 
+bool odd_groups(const SsdArgs& a) { return a.nheads / a.ngroups % 2 != 0; }
+
 // Head pairs over the whole batch; a group with an odd number of heads has a half-empty pair.
 int64_t unit_pairs(const SsdArgs& a) { return (int64_t)a.batch * a.ngroups * ((a.nheads / a.ngroups + 1) / 2); }
 
 }  // namespace
+
+// Skip and gate in the kernel: with packed 16-bit gates, which groups with an odd number of heads have never had (bf16, Y
+// against 64 bits: 2.9e-3 with the epilogue kernel's fp32 gate, 3.7e-3 with packed ones).
+bool tc2_fuses_epilogue(const SsdArgs& a) { return !odd_groups(a); }
 
 bool tc_supports(const SsdArgs& a) {
   if (a.dtype != SSD_DTYPE_F16 && a.dtype != SSD_DTYPE_BF16) return false;
@@ -1246,17 +1264,17 @@ int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
     // the gate rows are read with 16-byte loads
     if (sp.Z && ((reinterpret_cast<uintptr_t>(sp.Z) & 15) || sp.zs[0] % 8 || sp.zs[1] % 8 || sp.zs[2] % 8))
       return SSD_ERR_MISALIGNED;
-    if (a.dtype == SSD_DTYPE_BF16)
-      return a.dstate == 128 ? launch_typed2<__nv_bfloat16, 128, true>(tx, tb, tc, ty, prm, stream)
-                             : launch_typed2<__nv_bfloat16, 64, true>(tx, tb, tc, ty, prm, stream);
-    return a.dstate == 128 ? launch_typed2<__half, 128, true>(tx, tb, tc, ty, prm, stream)
-                           : launch_typed2<__half, 64, true>(tx, tb, tc, ty, prm, stream);
   }
-  if (a.dtype == SSD_DTYPE_BF16)
-    return a.dstate == 128 ? launch_typed2<__nv_bfloat16, 128, false>(tx, tb, tc, ty, prm, stream)
-                           : launch_typed2<__nv_bfloat16, 64, false>(tx, tb, tc, ty, prm, stream);
-  return a.dstate == 128 ? launch_typed2<__half, 128, false>(tx, tb, tc, ty, prm, stream)
-                         : launch_typed2<__half, 64, false>(tx, tb, tc, ty, prm, stream);
+  auto go = [&](auto epilogue, auto wide) {
+    constexpr bool E = decltype(epilogue)::value, W = decltype(wide)::value;
+    if (a.dtype == SSD_DTYPE_BF16)
+      return a.dstate == 128 ? launch_typed2<__nv_bfloat16, 128, E, W>(tx, tb, tc, ty, prm, stream)
+                             : launch_typed2<__nv_bfloat16, 64, E, W>(tx, tb, tc, ty, prm, stream);
+    return a.dstate == 128 ? launch_typed2<__half, 128, E, W>(tx, tb, tc, ty, prm, stream)
+                           : launch_typed2<__half, 64, E, W>(tx, tb, tc, ty, prm, stream);
+  };
+  if (epi) return go(std::true_type{}, std::false_type{});
+  return odd_groups(a) ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
 }
 
 }  // namespace ssd
