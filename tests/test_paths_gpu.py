@@ -88,6 +88,46 @@ def test_lengths_that_are_no_whole_tiles_are_rounded_once(s, h, g, dtype, eps):
     assert ((H.cpu().double() - Hr).abs().max() / Hr.abs().max()).item() < 1e-5
 
 
+def _strong_decays(A, dt, case):
+    """Puts decays into A [b,s,h] (and dt) that no run of factors can carry in 32 bits, differently in every head."""
+    b, s, h = A.shape
+    for k in range(h):
+        if case == "every_token":
+            A[:, :, k] = -30.0 - 7 * k
+        elif case == "one_token":
+            A[:, 5 + k::37, k] = -100.0
+        elif case == "reset":
+            A[:, 8 + k::41, k] = -float("inf")
+        elif case == "far":
+            A[:, 3 + k::29, k] = -1e30
+        elif case == "idle_tokens":        # dt = 0, then strong decays
+            A[:, 1::4, k], A[:, 2::4, k], A[:, 3::4, k] = -16.0, -16.0, -16.0
+            dt[:, k % 4::4, k] = 0.0
+        elif case == "steps_of_both_signs":
+            dt[:, k::5, k] *= -1.0
+        elif case == "tiny_steps":
+            dt[:, k::3, k] = 2.0 ** -14
+
+
+@pytest.mark.parametrize("s,h,g", [(128, 4, 1), (384, 4, 2), (300, 4, 1), (256, 5, 1)])
+@pytest.mark.parametrize("case", ["every_token", "one_token", "reset", "far", "idle_tokens", "steps_of_both_signs", "tiny_steps"])
+def test_decays_beyond_the_range_of_a_factor(case, s, h, g):
+    """Factors of P that differ by more than 32-bit numbers can between neighbouring tokens: a strong decay in every token, in
+    single ones at each place of a group of four, resets, dt = 0 and dt < 0.  Weights that survive must be there (the
+    diagonal above all), Y and the states finite, the sum of the log-decays as given."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=2, s=s, h=h, p=64, n=64, g=g, dtype=torch.bfloat16, init=True, seed=72, decay_scale=0.05)
+    dt = (0.5 + torch.rand(2, s, h, generator=torch.Generator().manual_seed(73))).bfloat16()
+    _strong_decays(inp["A"], dt, case)
+    for kernel in ("tcgen05", "scan_f32"):
+        _check(inp, kernel, 2e-2, dt=dt)
+    _check(inp, "tcgen05", 2e-2, dt=dt, nsegments=2)
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    _, ld = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, dt=dt.to(DEV), kernel="tcgen05", return_logdecay=True)
+    assert torch.allclose(ld.cpu().double(), O.total_logdecay(inp["A"]), rtol=1e-5, atol=1e-4)
+
+
 @pytest.mark.parametrize("shape", [dict(b=50, s=300, h=7, g=1, n=128), dict(b=1, s=1500, h=3, g=1, n=64),
                                    dict(b=40, s=513, h=8, g=2, n=64), dict(b=1, s=4500, h=2, g=1, n=128, decay_scale=0.002)],
                          ids=["chained_odd", "lookback_odd", "chained_n64", "lookback_36_pieces"])

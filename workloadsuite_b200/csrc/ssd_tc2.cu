@@ -93,11 +93,22 @@ struct Work {
 struct alignas(16) Factors {
   float cs2[T];       // cs * log2(e)
   float cf[T];        // exp(cs at the end of the row's 32-block - cs of the row) * dt: the row's factor as a column of P
-  float dg[T];        // diagonal blocks: at columns 4i cs * log2(e) - log2(dt), at the three after it the ratio to the column before
+  float dg[T];        // diagonal blocks: at columns 4i cs * log2(e) - log2(dt), at the three after it the ratio to the column before;
+                      // dt in the runs of 16 columns that hold a steep group of four
   float tot;          // cs_last
+  float ld;           // sum of the log-decays as given
+  uint32_t steep;     // groups of four columns in which the factors of P span more than the ratios can carry
 };
 
 constexpr int kFactors = 4;   // tiles that the prefix sums may be ahead
+
+// Log-decays below this count as this in the prefix sums: e^-104 is 2^-150, a factor of zero either way, while -inf (a
+// reset) would make every difference of sums after it NaN, and a very large one would take their digits.
+constexpr float kLowest = -104.f;
+// A group of four columns of a diagonal block is steep if its factors span more than 2^40, or a dt is no ordinary positive
+// number: the ratios start from the group's first column, and where that one underflows (2^-126) the three after it would
+// be lost with it -- the diagonal, of factor dt, too.  So what is lost in the others is below 2^-86.
+constexpr float kSteep = 40.f, kLeastLogDt = -60.f;
 
 // What the MMA issuer does for one kind of product (see there).  `a` and `b` are the low words of the shared-memory
 // descriptors (`a` a tensor-memory address for P.X), advanced by a_in / b_in per k-step and by a_out / b_out per four;
@@ -603,7 +614,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
         Ag += asT;
         Dg += dsT;
-        float cs = a[0] + a[1] + a[2] + a[3];
+        float cs = a[0] + a[1] + a[2] + a[3], ld = cs;
+        const bool low = __any_sync(0xffffffffu, fminf(fminf(a[0], a[1]), fminf(a[2], a[3])) < kLowest) != 0;
+        if (__builtin_expect(low, 0)) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = a[e] < kLowest ? kLowest : a[e];   // (NaN stays NaN)
+          cs = a[0] + a[1] + a[2] + a[3];
+          for (int d = 16; d >= 1; d >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, d);
+        }
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
           const float t = __shfl_up_sync(0xffffffffu, cs, d);
@@ -624,20 +642,29 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         const uint32_t slot = n % kFactors;
         wait(&m->empty_f[h][slot], ((n / kFactors) & 1) ^ 1, m);
         Factors& f = m->f[h][slot];
-        if (lane == 31) f.tot = cs;
         reinterpret_cast<float4*>(f.cs2)[lane] = make_float4(c2[0], c2[1], c2[2], c2[3]);
         float cf[4], cc[4];
+        bool steep = false;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           cf[e] = ex2(ce - c2[e]) * dt[e];
           // dt multiplies the columns of P instead of the rows of X (P.(dt o x) = (P o dt_s).x), so the X tile stays as
-          // loaded (clamped: dt == 0 must not break the chain of ratios; the clamped column then weighs 2^-60, i.e.
-          // nothing).  The ratios are clamped too: one above the diagonal may overflow, it is masked out.
-          cc[e] = c2[e] - fmaxf(lg2(dt[e]), -60.f);        // (lg2(1) is 0)
+          // loaded.  The ratios are clamped: one above the diagonal may overflow, it is masked out.
+          const float lg = lg2(dt[e]);                     // (lg2(1) is 0)
+          steep |= !(lg > kLeastLogDt);
+          cc[e] = c2[e] - lg;
+        }
+        steep |= !(fmaxf(fmaxf(cc[0], cc[1]), fmaxf(cc[2], cc[3])) - fminf(fminf(cc[0], cc[1]), fminf(cc[2], cc[3])) <= kSteep);
+        const uint32_t all_steep = __ballot_sync(0xffffffffu, steep);
+        float4 dg = make_float4(cc[0], ex2(fminf(cc[0] - cc[1], 126.f)), ex2(fminf(cc[1] - cc[2], 126.f)), ex2(fminf(cc[2] - cc[3], 126.f)));
+        if (all_steep >> (lane & 28) & 15u) dg = make_float4(dt[0], dt[1], dt[2], dt[3]);
+        if (lane == 31) {
+          f.tot = cs;
+          f.ld = low ? ld : cs;
+          f.steep = all_steep;
         }
         reinterpret_cast<float4*>(f.cf)[lane] = make_float4(cf[0], cf[1], cf[2], cf[3]);
-        reinterpret_cast<float4*>(f.dg)[lane] =
-            make_float4(cc[0], ex2(fminf(cc[0] - cc[1], 126.f)), ex2(fminf(cc[1] - cc[2], 126.f)), ex2(fminf(cc[2] - cc[3], 126.f)));
+        reinterpret_cast<float4*>(f.dg)[lane] = dg;
         warp_arrive(&m->full_f[h][slot]);
       }
     }
@@ -662,7 +689,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 
     // A. P = (C B^T) o exp(segsum), causal -> TMEM (A operand, 16-bit pairs).  Decay mask per 32-token column block J of
     // this warp's 32 rows (block q is the diagonal one):
-    //   J == q: exp2(cs_l - cs_s), causal, one ex2 per four columns and the ratios between neighbours;
+    //   J == q: exp2(cs_l - cs_s), causal, one ex2 per four columns and the ratios between neighbours (in 16 columns that hold a
+    //           steep group: one ex2 per column);
     //   J <  q: exp(cs_l - cs_s) = rf_J[l] * cf[s] with both factors <= 1 for non-positive log-decays
     //           (rf_J[l] = exp(cs_l - cs_end(J)), cf[s] = exp(cs_end(J) - cs_s)): two multiplies;
     //   J >  q: zero.
@@ -676,14 +704,26 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         const uint4* keep = m->causal[max(0, min(16, lane - 16 * half + 1))];
         tmem_ld_wait();
         uint32_t pk[8];
+        if (__builtin_expect((f.steep >> (8 * q + 4 * half) & 15u) != 0, 0)) {
+          const float4* cv = reinterpret_cast<const float4*>(&f.cs2[32 * q + 16 * half]);
 #pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4) {
-          const float4 d = dv[e4];
-          const float w0 = ex2(cs2 - d.x), w1 = w0 * d.y, w2 = w1 * d.z, w3 = w2 * d.w;
-          const float v0 = __uint_as_float(g[4 * e4]) * w0, v1 = __uint_as_float(g[4 * e4 + 1]) * w1;
-          const float v2 = __uint_as_float(g[4 * e4 + 2]) * w2, v3 = __uint_as_float(g[4 * e4 + 3]) * w3;
-          pk[2 * e4] = pack2<T16>(v0, v1);
-          pk[2 * e4 + 1] = pack2<T16>(v2, v3);
+          for (int e4 = 0; e4 < 4; ++e4) {
+            const float4 d = dv[e4], c = cv[e4];
+            const float v0 = __uint_as_float(g[4 * e4]) * (ex2(cs2 - c.x) * d.x), v1 = __uint_as_float(g[4 * e4 + 1]) * (ex2(cs2 - c.y) * d.y);
+            const float v2 = __uint_as_float(g[4 * e4 + 2]) * (ex2(cs2 - c.z) * d.z), v3 = __uint_as_float(g[4 * e4 + 3]) * (ex2(cs2 - c.w) * d.w);
+            pk[2 * e4] = pack2<T16>(v0, v1);
+            pk[2 * e4 + 1] = pack2<T16>(v2, v3);
+          }
+        } else {
+#pragma unroll
+          for (int e4 = 0; e4 < 4; ++e4) {
+            const float4 d = dv[e4];
+            const float w0 = ex2(cs2 - d.x), w1 = w0 * d.y, w2 = w1 * d.z, w3 = w2 * d.w;
+            const float v0 = __uint_as_float(g[4 * e4]) * w0, v1 = __uint_as_float(g[4 * e4 + 1]) * w1;
+            const float v2 = __uint_as_float(g[4 * e4 + 2]) * w2, v3 = __uint_as_float(g[4 * e4 + 3]) * w3;
+            pk[2 * e4] = pack2<T16>(v0, v1);
+            pk[2 * e4 + 1] = pack2<T16>(v2, v3);
+          }
         }
         const uint4 k0 = keep[0], k1 = keep[1];
         pk[0] &= k0.x; pk[1] &= k0.y; pk[2] &= k0.z; pk[3] &= k0.w;
@@ -895,11 +935,11 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       }
       // E. H <- exp(cs_last) H + S
       wait(&m->full_f[h][slot], (n / kFactors) & 1, m);
-      const float tot = m->f[h][slot].tot;
-      const float gs = ex2(tot * kLog2e);
+      const float gs = ex2(m->f[h][slot].tot * kLog2e);
       {
-        const float yk = tot - acomp, tk = asum + yk;
+        const float yk = m->f[h][slot].ld - acomp, tk = asum + yk;
         acomp = (tk - asum) - yk;
+        if (acomp != acomp) acomp = 0.f;   // (a sum of -inf stays that)
         asum = tk;
       }
       wait(&m->bar_s, n & 1, m);
