@@ -168,6 +168,26 @@ def test_step_reads_strided_operands_and_d_in_its_own_type():
     assert torch.equal(y1, y2) and torch.equal(S1, S2)
 
 
+def test_a_step_after_a_call_that_failed_is_made_once():
+    """A call that ran out of memory leaves a CUDA error behind; the step after it, which updates the state in place, must not
+    take that for its own and be made again."""
+    import ctypes
+
+    import workloadsuite_b200 as W
+    from workloadsuite_b200 import _lib
+
+    b, h, n = 2, 4, 64
+    gen = torch.Generator(DEV).manual_seed(92)
+    x, B, C = (torch.randn(b, k, 64, generator=gen, device=DEV).bfloat16() for k in (h, 1, 1))
+    a = -torch.rand(b, h, generator=gen, device=DEV)
+    S = torch.randn(b, h, n, 64, generator=gen, device=DEV)
+    once, state = S.clone(), S.clone()
+    y = W.ssd_step(x, a, B, C, once)
+    ctx, handle = ctypes.c_void_p(), (ctypes.c_ubyte * _lib.XCHG_HANDLE_BYTES)()
+    assert _lib.load().ssd_b200_xchg_create(1 << 44, 2, ctypes.byref(ctx), handle) == -6     # 32 TiB
+    assert torch.equal(W.ssd_step(x, a, B, C, state), y) and torch.equal(state, once)
+
+
 @pytest.mark.parametrize("dtype,l,d", [(torch.float16, 1, 64), (torch.float16, 9, 128), (torch.bfloat16, 65, 64),
                                        (torch.float32, 5, 64), (torch.float32, 67, 192), (torch.bfloat16, 2050, 4096)])
 def test_conv_run_lengths(dtype, l, d):

@@ -132,13 +132,15 @@ def fast():
     """The binding module ``ssd_b200_torch`` (``csrc/torch_binding.cpp``), bound to the loaded library."""
     global _FAST
     if _FAST is None:
+        from .ssd import _raise
+
         lib = load()
         spec = importlib.util.spec_from_file_location("ssd_b200_torch", str(_build.TORCH_LIB))
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         addr = lambda f: C.cast(f, C.c_void_p).value
         mod.init(addr(lib.ssd_b200_forward), addr(lib.ssd_b200_workspace_bytes), addr(lib.ssd_b200_step_strided),
-                 addr(lib.ssd_b200_conv1d_silu), addr(lib.ssd_b200_dt_prologue))
+                 addr(lib.ssd_b200_conv1d_silu), addr(lib.ssd_b200_dt_prologue), _raise)
         _FAST = mod
     return _FAST
 

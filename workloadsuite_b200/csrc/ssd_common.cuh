@@ -72,6 +72,18 @@ template <> struct Cvt<__nv_bfloat16> {
   static __device__ __forceinline__ __nv_bfloat16 from_f(float v) { return __float2bfloat16_rn(v); }
 };
 
+// Enqueues a kernel and says whether THIS launch failed: cudaGetLastError() behind a launch also reports (once) what an
+// earlier call of the thread left, and a launch that is called failed is made again -- a step would be applied twice.
+template <typename... Params, typename... Args>
+inline int launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+}
+
 // D[head] of the skip term.
 template <typename T>
 __device__ __forceinline__ float load_skip(const ScanParams& p, int head) {

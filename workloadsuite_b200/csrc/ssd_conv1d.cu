@@ -348,21 +348,20 @@ int launch_conv(const void* x, const void* w, const void* bias, void* y, int bat
       auto go = [&](auto kern) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagedSmem) != cudaSuccess)
           return (int)SSD_ERR_CUDA;
-        kern<<<g, kStagedThreads, kStagedSmem, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, len);
-        return cudaGetLastError() == cudaSuccess ? (int)SSD_OK : (int)SSD_ERR_CUDA;
+        return launch(kern, g, kStagedThreads, kStagedSmem, stream, xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, len);
       };
       if (taps == 2) return len == kLongestRun ? go(conv1d_silu_staged_kernel<T, 2, kLongestRun>) : go(conv1d_silu_staged_kernel<T, 2, 0>);
       if (taps == 3) return len == kLongestRun ? go(conv1d_silu_staged_kernel<T, 3, kLongestRun>) : go(conv1d_silu_staged_kernel<T, 3, 0>);
       return len == kLongestRun ? go(conv1d_silu_staged_kernel<T, 4, kLongestRun>) : go(conv1d_silu_staged_kernel<T, 4, 0>);
     }
   }
+  auto go = [&](auto kern) { return launch(kern, grid, 128, 0, stream, xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); };
   switch (taps) {
-    case 2: conv1d_silu_kernel<T, 2><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); break;
-    case 3: conv1d_silu_kernel<T, 3><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); break;
-    case 4: conv1d_silu_kernel<T, 4><<<grid, 128, 0, stream>>>(xx, ww, bb, yy, batch, seqlen, channels, xsb, xsl, ysb, ysl, al, run); break;
+    case 2: return go(conv1d_silu_kernel<T, 2>);
+    case 3: return go(conv1d_silu_kernel<T, 3>);
+    case 4: return go(conv1d_silu_kernel<T, 4>);
     default: return SSD_ERR_UNSUPPORTED;
   }
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
 
 }  // namespace

@@ -84,9 +84,8 @@ int launch_prologue(const void* dt_raw, int64_t sb, int64_t sl, const void* dt_b
   // up to sixteen small CTAs per SM, and at least one pass of whole rows
   const int64_t ctas = std::max<int64_t>(std::min<int64_t>((total + 127) / 128, 148 * 16), (vecs + 127) / 128);
   auto go = [&](auto kern) {
-    kern<<<(unsigned)ctas, 128, 0, stream>>>(static_cast<const T*>(dt_raw), sb, sl, static_cast<const T*>(dt_bias), A_log,
-                                             static_cast<T*>(dt_out), A_dt, rows, seqlen, nheads);
-    return cudaGetLastError() == cudaSuccess ? (int)SSD_OK : (int)SSD_ERR_CUDA;
+    return launch(kern, (unsigned)ctas, 128, 0, stream, static_cast<const T*>(dt_raw), sb, sl, static_cast<const T*>(dt_bias),
+                  A_log, static_cast<T*>(dt_out), A_dt, rows, seqlen, nheads);
   };
   return vec ? go(dt_prologue_kernel<T, V>) : go(dt_prologue_kernel<T, 1>);
 }

@@ -335,8 +335,7 @@ int launch_one(const ScanParams& prm, cudaStream_t stream) {
       return SSD_ERR_CUDA;
   }
   dim3 grid((unsigned)(prm.batch * prm.nheads), (unsigned)prm.nseg);
-  kern<<<grid, kThreads, smem, stream>>>(prm, tile);
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  return launch(kern, grid, kThreads, smem, stream, prm, tile);
 }
 
 template <typename T, int P>
@@ -441,10 +440,9 @@ int launch_epilogue(const ScanParams& p, int dtype, cudaStream_t stream) {
   const int grid = (int)rows;
   const int work = p.nheads * (p.p / 8);
   const int threads = work >= 256 ? 256 : (work >= 128 ? 128 : 64);
-  if (dtype == SSD_DTYPE_F32) ssd_epilogue_kernel<float><<<grid, threads, 0, stream>>>(p);
-  else if (dtype == SSD_DTYPE_F16) ssd_epilogue_kernel<__half><<<grid, threads, 0, stream>>>(p);
-  else ssd_epilogue_kernel<__nv_bfloat16><<<grid, threads, 0, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  if (dtype == SSD_DTYPE_F32) return launch(ssd_epilogue_kernel<float>, grid, threads, 0, stream, p);
+  if (dtype == SSD_DTYPE_F16) return launch(ssd_epilogue_kernel<__half>, grid, threads, 0, stream, p);
+  return launch(ssd_epilogue_kernel<__nv_bfloat16>, grid, threads, 0, stream, p);
 }
 
 int launch_fold(const float* states, int64_t st_unit_stride, int64_t st_seg_stride, const float* ld,
@@ -454,10 +452,8 @@ int launch_fold(const float* states, int64_t st_unit_stride, int64_t st_seg_stri
   if (units <= 0 || np <= 0) return SSD_ERR_BAD_SHAPE;
   if (units > 0x7fffffff || (np + 255) / 256 > 65535) return SSD_ERR_TOO_LARGE;
   dim3 grid((unsigned)units, (unsigned)((np + 255) / 256));
-  ssd_fold_kernel<<<grid, 256, 0, stream>>>(states, st_unit_stride, st_seg_stride, ld, ld_unit_stride,
-                                            ld_seg_stride, init, out_single, out_final, out_ld, upto,
-                                            incoming, np);
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  return launch(ssd_fold_kernel, grid, 256, 0, stream, states, st_unit_stride, st_seg_stride, ld, ld_unit_stride, ld_seg_stride,
+                init, out_single, out_final, out_ld, upto, incoming, np);
 }
 
 }  // namespace ssd

@@ -95,10 +95,7 @@ ssd_step_kernel(const SsdStepArgs p) {
 
 template <typename T>
 int launch_step(const SsdStepArgs& p, cudaStream_t stream) {
-  auto go = [&](auto kern) {
-    kern<<<2 * p.batch * p.nheads, kStepThreads, 0, stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? (int)SSD_OK : (int)SSD_ERR_CUDA;
-  };
+  auto go = [&](auto kern) { return launch(kern, 2 * p.batch * p.nheads, kStepThreads, 0, stream, p); };
   switch (p.dstate / 16) {
     case 1: return go(ssd_step_kernel<T, 1>);
     case 2: return go(ssd_step_kernel<T, 2>);

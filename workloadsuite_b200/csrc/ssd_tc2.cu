@@ -1197,7 +1197,7 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
   cfg.stream = stream;
   cudaLaunchAttribute early;
   if (prm.sp.chain) {
-    clear_flags_kernel<<<1, 2 * kSms, 0, stream>>>(prm.sp.chain_flag);
+    if (launch(clear_flags_kernel, 1, 2 * kSms, 0, stream, prm.sp.chain_flag) != SSD_OK) return SSD_ERR_CUDA;
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &early;

@@ -20,6 +20,7 @@
 #include <new>
 
 #include "ssd_b200.h"
+#include "ssd_common.cuh"
 
 namespace {
 
@@ -163,7 +164,6 @@ int ssd_b200_xchg_connect(void* ctx, const void* handles, int32_t rank) {
     memcpy(&h, static_cast<const unsigned char*>(handles) + (size_t)r * SSD_XCHG_HANDLE_BYTES, sizeof(h));
     void* p = nullptr;
     if (cudaIpcOpenMemHandle(&p, h, cudaIpcMemLazyEnablePeerAccess) != cudaSuccess) {
-      cudaGetLastError();
       for (int q = 0; q < r; ++q)
         if (x->opened[q]) { cudaIpcCloseMemHandle(x->opened[q]); x->opened[q] = nullptr; }
       return SSD_ERR_CUDA;
@@ -192,9 +192,8 @@ int ssd_b200_xchg_all_gather(void* ctx, const void* send, size_t bytes, int32_t*
   XchgDev d = x->d;
   d.wait_clocks = (long long)(wait_limit_ms > 0 ? wait_limit_ms : 2000) * (khz > 0 ? khz : 1965000);
   d.status = status;
-  xchg_all_gather_kernel<<<x->d.world * kChunksPerPeer, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      d, static_cast<const uint4*>(send), bytes);
-  return cudaGetLastError() == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  return ssd::launch(xchg_all_gather_kernel, x->d.world * kChunksPerPeer, kThreads, 0, static_cast<cudaStream_t>(stream), d,
+                     static_cast<const uint4*>(send), bytes);
 }
 
 int ssd_b200_xchg_destroy(void* ctx) {

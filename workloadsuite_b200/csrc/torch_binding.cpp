@@ -2,8 +2,9 @@
 // token, a small layer) is otherwise bound by what Python spends on attribute look-ups, ctypes marshalling and context
 // managers: 15-20 us per call, against 2-3 us here.
 // Every function returns None when the call is not plainly valid for the kernels (other dtypes, shapes that disagree,
-// tensors that have to be copied first, an error code); the Python wrapper then goes its long way, which copies what has
-// to be copied or raises.  Nothing is decided here that the long way would decide otherwise.
+// tensors that have to be copied first, a code that says so); the Python wrapper then goes its long way, which copies what
+// has to be copied or raises.  Nothing is decided here that the long way would decide otherwise.  A CUDA error is raised
+// here: work may have been enqueued by then, and a step made again would advance the state twice.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -23,6 +24,7 @@ decltype(&ssd_b200_workspace_bytes) f_workspace;
 decltype(&ssd_b200_step_strided) f_step;
 decltype(&ssd_b200_conv1d_silu) f_conv;
 decltype(&ssd_b200_dt_prologue) f_dt;
+PyObject* f_raise;   // raises the Python exception of an error code
 
 constexpr int kMaxDevices = 64;
 Tensor* g_workspace[kMaxDevices];   // scratch shared by all calls on a device (never shrinks)
@@ -51,6 +53,13 @@ bool get(PyObject* o, const Tensor** out, bool optional = false) {
 
 bool shaped(const Tensor& t, std::initializer_list<int64_t> s) { return t.sizes() == at::IntArrayRef(s.begin(), s.size()); }
 bool inner(const Tensor& t) { return t.stride(-1) == 1 || t.size(-1) == 1; }
+
+// The result of a call that returned `rc`: None, for the long way, unless that could enqueue work twice.
+PyObject* declined(int rc) {
+  if (rc != SSD_ERR_CUDA) Py_RETURN_NONE;
+  Py_XDECREF(PyObject_CallFunction(f_raise, "i", rc));
+  return nullptr;
+}
 
 struct Where {
   c10::cuda::OptionalCUDAGuard guard;
@@ -127,7 +136,7 @@ PyObject* py_step(PyObject*, PyObject* const* o, Py_ssize_t n) {
     if (dt->defined()) { s.dt = dt->data_ptr(); s.dt_stride[0] = dt->stride(0); s.dt_stride[1] = dt->stride(1); }
     if (z->defined()) { s.z = z->data_ptr(); s.z_stride[0] = z->stride(0); s.z_stride[1] = z->stride(1); }
     if (D->defined()) { s.D = D->data_ptr(); s.d_in_dtype = D->scalar_type() == st && st != at::kFloat; }
-    if (f_step(&s, w.stream()) != SSD_OK) Py_RETURN_NONE;
+    if (const int rc = f_step(&s, w.stream())) return declined(rc);
     return THPVariable_Wrap(std::move(y));
   )
 }
@@ -145,10 +154,10 @@ PyObject* py_dt(PyObject*, PyObject* const* o, Py_ssize_t n) {
     if (!w.here(*bias) || !w.here(*al)) Py_RETURN_NONE;
     Tensor dt = at::empty({b, l, h}, r->options());
     Tensor A = at::empty({b, l, h}, r->options().dtype(at::kFloat));
-    if (f_dt(r->data_ptr(), r->stride(0), r->stride(1), bias->defined() ? bias->data_ptr() : nullptr,
-             static_cast<const float*>(al->data_ptr()), dt.data_ptr(), static_cast<float*>(A.data_ptr()), (int)b, (int)l, (int)h,
-             dtype, w.stream()) != SSD_OK)
-      Py_RETURN_NONE;
+    if (const int rc = f_dt(r->data_ptr(), r->stride(0), r->stride(1), bias->defined() ? bias->data_ptr() : nullptr,
+                            static_cast<const float*>(al->data_ptr()), dt.data_ptr(), static_cast<float*>(A.data_ptr()), (int)b,
+                            (int)l, (int)h, dtype, w.stream()))
+      return declined(rc);
     PyObject* t = PyTuple_New(2);
     if (!t) return nullptr;
     PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(dt)));
@@ -174,9 +183,9 @@ PyObject* py_conv(PyObject*, PyObject* const* o, Py_ssize_t n) {
     Where q(*x);
     if (!q.here(*w) || !q.here(*bias) || !q.here(*out)) Py_RETURN_NONE;
     Tensor y = out->defined() ? *out : at::empty({b, l, d}, x->options());
-    if (f_conv(x->data_ptr(), w->data_ptr(), bias->defined() ? bias->data_ptr() : nullptr, y.data_ptr(), (int)b, (int)l, (int)d,
-               (int)w->size(-1), dtype, x->stride(0), x->stride(1), y.stride(0), y.stride(1), q.stream()) != SSD_OK)
-      Py_RETURN_NONE;
+    if (const int rc = f_conv(x->data_ptr(), w->data_ptr(), bias->defined() ? bias->data_ptr() : nullptr, y.data_ptr(), (int)b,
+                              (int)l, (int)d, (int)w->size(-1), dtype, x->stride(0), x->stride(1), y.stride(0), y.stride(1), q.stream()))
+      return declined(rc);
     return THPVariable_Wrap(std::move(y));
   )
 }
@@ -231,7 +240,7 @@ PyObject* py_forward(PyObject*, PyObject* const* o, Py_ssize_t n) {
       a.workspace = ws.data_ptr();
       a.workspace_bytes = (size_t)ws.numel();
     }
-    if (f_forward(&a, w.stream()) != SSD_OK) Py_RETURN_NONE;
+    if (const int rc = f_forward(&a, w.stream())) return declined(rc);
     if (!want_final) return THPVariable_Wrap(std::move(Y));
     PyObject* t = PyTuple_New(2);
     if (!t) return nullptr;
@@ -256,10 +265,11 @@ PyObject* py_status(PyObject*, PyObject* const* o, Py_ssize_t n) {
   GUARDED(return THPVariable_Wrap(status_word((int)dev));)
 }
 
-// init(forward, workspace_bytes, step_strided, conv1d_silu, dt_prologue): addresses in the loaded library
+// init(forward, workspace_bytes, step_strided, conv1d_silu, dt_prologue, raise): addresses in the loaded library, and the
+// function that raises the exception of an error code
 PyObject* py_init(PyObject*, PyObject* const* o, Py_ssize_t n) {
-  if (n != 5) {
-    PyErr_SetString(PyExc_TypeError, "init takes five addresses");
+  if (n != 6) {
+    PyErr_SetString(PyExc_TypeError, "init takes five addresses and a function");
     return nullptr;
   }
   void* f[5];
@@ -270,6 +280,8 @@ PyObject* py_init(PyObject*, PyObject* const* o, Py_ssize_t n) {
   f_step = reinterpret_cast<decltype(f_step)>(f[2]);
   f_conv = reinterpret_cast<decltype(f_conv)>(f[3]);
   f_dt = reinterpret_cast<decltype(f_dt)>(f[4]);
+  Py_INCREF(o[5]);
+  Py_XSETREF(f_raise, o[5]);
   Py_RETURN_NONE;
 }
 
