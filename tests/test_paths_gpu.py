@@ -188,6 +188,29 @@ def test_a_step_after_a_call_that_failed_is_made_once():
     assert torch.equal(W.ssd_step(x, a, B, C, state), y) and torch.equal(state, once)
 
 
+def test_what_pytorch_throws_in_the_binding_is_raised():
+    """Tensors without sizes, allocations that cannot be made, an output that is refused: Python exceptions, of PyTorch's own
+    kinds."""
+    import workloadsuite_b200 as W
+
+    nested = torch.nested.nested_tensor([torch.ones(4, 64), torch.ones(3, 64)], device=DEV)
+    B, a, S = torch.ones(2, 1, 64, device=DEV), -torch.ones(2, 4, device=DEV), torch.zeros(2, 4, 64, 64, device=DEV)
+    with pytest.raises(RuntimeError):
+        W.ssd_step(nested, a, B, B, S)
+    with pytest.raises(RuntimeError):
+        W.conv1d_silu(nested, torch.ones(64, 1, 4, device=DEV))
+    with pytest.raises(RuntimeError):
+        W.dt_prologue(nested, None, torch.zeros(64, device=DEV))
+    X = torch.ones(1, 128, 4, 64, device=DEV).bfloat16()
+    A, G = -torch.ones(1, 128, 4, device=DEV), torch.ones(1, 128, 1, 64, device=DEV).bfloat16()
+    with pytest.raises(RuntimeError):
+        W.ssd_forward(torch.nested.nested_tensor([torch.ones(128, 4, 64), torch.ones(64, 4, 64)], device=DEV), A, G, G, 64)
+    with pytest.raises(torch.OutOfMemoryError):
+        W.dt_prologue(torch.zeros(1, 1, 64, device=DEV).expand(1 << 20, 1 << 20, 64), None, torch.zeros(64, device=DEV))
+    with pytest.raises(ValueError, match="out_logdecay"):
+        W.ssd_forward(X, A, G, G, 128, out_logdecay=torch.zeros(1, 5, device=DEV))
+
+
 @pytest.mark.parametrize("dtype,l,d", [(torch.float16, 1, 64), (torch.float16, 9, 128), (torch.bfloat16, 65, 64),
                                        (torch.float32, 5, 64), (torch.float32, 67, 192), (torch.bfloat16, 2050, 4096)])
 def test_conv_run_lengths(dtype, l, d):

@@ -10,6 +10,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "ssd_b200.h"
@@ -17,6 +18,10 @@
 namespace {
 
 using at::Tensor;
+
+// The entry points stand between HANDLE_TH_ERRORS and END_HANDLE_TH_ERRORS from their first line on: what PyTorch's C++ throws
+// (a nested tensor has no sizes, an allocation runs out of memory) becomes the Python exception that PyTorch itself raises
+// for it, and would end the process if it left the entry point.
 
 // entry points of the library that the Python side has loaded
 decltype(&ssd_b200_forward) f_forward;
@@ -95,14 +100,9 @@ void strides3(const Tensor& t, int64_t* st) {
   for (int d = 0; d < 3; ++d) st[d] = t.stride(d);
 }
 
-#define GUARDED(...)                                    \
-  try { __VA_ARGS__ } catch (const std::exception& e) { \
-    PyErr_SetString(PyExc_RuntimeError, e.what());      \
-    return nullptr;                                     \
-  }
-
 // step(x, a, B, C, state, dt, D, z, out) -> y
 PyObject* py_step(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   const Tensor *x, *a, *B, *C, *state, *dt, *D, *z, *out;
   if (n != 9 || !get(o[0], &x) || !get(o[1], &a) || !get(o[2], &B) || !get(o[3], &C) || !get(o[4], &state) ||
       !get(o[5], &dt, true) || !get(o[6], &D, true) || !get(o[7], &z, true) || !get(o[8], &out, true) || !x->is_cuda() ||
@@ -121,53 +121,53 @@ PyObject* py_step(PyObject*, PyObject* const* o, Py_ssize_t n) {
   if (D->defined() && (!shaped(*D, {h}) || !D->is_contiguous() || (D->scalar_type() != st && D->scalar_type() != at::kFloat)))
     Py_RETURN_NONE;
   if (out->defined() && (out->scalar_type() != st || !shaped(*out, {b, h, p}) || !out->is_contiguous())) Py_RETURN_NONE;
-  GUARDED(
-    Where w(*x);
-    if (!w.here(*a) || !w.here(*B) || !w.here(*C) || !w.here(*state) || !w.here(*dt) || !w.here(*D) || !w.here(*z) || !w.here(*out))
-      Py_RETURN_NONE;
-    Tensor y = out->defined() ? *out : at::empty({b, h, p}, x->options());
-    SsdStepArgs s = {};
-    s.x = x->data_ptr(); s.a = static_cast<const float*>(a->data_ptr()); s.B = B->data_ptr(); s.C = C->data_ptr();
-    s.state = static_cast<float*>(state->data_ptr()); s.y = y.data_ptr();
-    s.batch = (int)b; s.nheads = (int)h; s.headdim = (int)p; s.dstate = (int)ns; s.ngroups = (int)g; s.dtype = dtype;
-    for (int d = 0; d < 2; ++d) {
-      s.x_stride[d] = x->stride(d); s.a_stride[d] = a->stride(d); s.b_stride[d] = B->stride(d); s.c_stride[d] = C->stride(d);
-    }
-    if (dt->defined()) { s.dt = dt->data_ptr(); s.dt_stride[0] = dt->stride(0); s.dt_stride[1] = dt->stride(1); }
-    if (z->defined()) { s.z = z->data_ptr(); s.z_stride[0] = z->stride(0); s.z_stride[1] = z->stride(1); }
-    if (D->defined()) { s.D = D->data_ptr(); s.d_in_dtype = D->scalar_type() == st && st != at::kFloat; }
-    if (const int rc = f_step(&s, w.stream())) return declined(rc);
-    return THPVariable_Wrap(std::move(y));
-  )
+  Where w(*x);
+  if (!w.here(*a) || !w.here(*B) || !w.here(*C) || !w.here(*state) || !w.here(*dt) || !w.here(*D) || !w.here(*z) || !w.here(*out))
+    Py_RETURN_NONE;
+  Tensor y = out->defined() ? *out : at::empty({b, h, p}, x->options());
+  SsdStepArgs s = {};
+  s.x = x->data_ptr(); s.a = static_cast<const float*>(a->data_ptr()); s.B = B->data_ptr(); s.C = C->data_ptr();
+  s.state = static_cast<float*>(state->data_ptr()); s.y = y.data_ptr();
+  s.batch = (int)b; s.nheads = (int)h; s.headdim = (int)p; s.dstate = (int)ns; s.ngroups = (int)g; s.dtype = dtype;
+  for (int d = 0; d < 2; ++d) {
+    s.x_stride[d] = x->stride(d); s.a_stride[d] = a->stride(d); s.b_stride[d] = B->stride(d); s.c_stride[d] = C->stride(d);
+  }
+  if (dt->defined()) { s.dt = dt->data_ptr(); s.dt_stride[0] = dt->stride(0); s.dt_stride[1] = dt->stride(1); }
+  if (z->defined()) { s.z = z->data_ptr(); s.z_stride[0] = z->stride(0); s.z_stride[1] = z->stride(1); }
+  if (D->defined()) { s.D = D->data_ptr(); s.d_in_dtype = D->scalar_type() == st && st != at::kFloat; }
+  if (const int rc = f_step(&s, w.stream())) return declined(rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
 }
 
 // dt_prologue(dt_raw, dt_bias, A_log) -> (dt, A_dt)
 PyObject* py_dt(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   const Tensor *r, *bias, *al;
   if (n != 3 || !get(o[0], &r) || !get(o[1], &bias, true) || !get(o[2], &al) || !r->is_cuda() || r->dim() != 3) Py_RETURN_NONE;
   const int dtype = dtype_of(*r);
   const int64_t b = r->size(0), l = r->size(1), h = r->size(2);
   if (dtype < 0 || r->stride(2) != 1 || al->scalar_type() != at::kFloat || !shaped(*al, {h}) || !al->is_contiguous()) Py_RETURN_NONE;
   if (bias->defined() && (!shaped(*bias, {h}) || bias->scalar_type() != r->scalar_type() || !bias->is_contiguous())) Py_RETURN_NONE;
-  GUARDED(
-    Where w(*r);
-    if (!w.here(*bias) || !w.here(*al)) Py_RETURN_NONE;
-    Tensor dt = at::empty({b, l, h}, r->options());
-    Tensor A = at::empty({b, l, h}, r->options().dtype(at::kFloat));
-    if (const int rc = f_dt(r->data_ptr(), r->stride(0), r->stride(1), bias->defined() ? bias->data_ptr() : nullptr,
-                            static_cast<const float*>(al->data_ptr()), dt.data_ptr(), static_cast<float*>(A.data_ptr()), (int)b,
-                            (int)l, (int)h, dtype, w.stream()))
-      return declined(rc);
-    PyObject* t = PyTuple_New(2);
-    if (!t) return nullptr;
-    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(dt)));
-    PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(A)));
-    return t;
-  )
+  Where w(*r);
+  if (!w.here(*bias) || !w.here(*al)) Py_RETURN_NONE;
+  Tensor dt = at::empty({b, l, h}, r->options());
+  Tensor A = at::empty({b, l, h}, r->options().dtype(at::kFloat));
+  if (const int rc = f_dt(r->data_ptr(), r->stride(0), r->stride(1), bias->defined() ? bias->data_ptr() : nullptr,
+                          static_cast<const float*>(al->data_ptr()), dt.data_ptr(), static_cast<float*>(A.data_ptr()), (int)b,
+                          (int)l, (int)h, dtype, w.stream()))
+    return declined(rc);
+  PyObject* t = PyTuple_New(2);
+  if (!t) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(dt)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(A)));
+  return t;
+  END_HANDLE_TH_ERRORS
 }
 
 // conv1d_silu(x, weight, bias, out) -> y
 PyObject* py_conv(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   const Tensor *x, *w, *bias, *out;
   if (n != 4 || !get(o[0], &x) || !get(o[1], &w) || !get(o[2], &bias, true) || !get(o[3], &out, true) || !x->is_cuda() || x->dim() != 3)
     Py_RETURN_NONE;
@@ -179,19 +179,19 @@ PyObject* py_conv(PyObject*, PyObject* const* o, Py_ssize_t n) {
     Py_RETURN_NONE;
   if (bias->defined() && (!shaped(*bias, {d}) || bias->scalar_type() != st || !bias->is_contiguous())) Py_RETURN_NONE;
   if (out->defined() && (out->scalar_type() != st || out->sizes() != x->sizes() || !inner(*out))) Py_RETURN_NONE;
-  GUARDED(
-    Where q(*x);
-    if (!q.here(*w) || !q.here(*bias) || !q.here(*out)) Py_RETURN_NONE;
-    Tensor y = out->defined() ? *out : at::empty({b, l, d}, x->options());
-    if (const int rc = f_conv(x->data_ptr(), w->data_ptr(), bias->defined() ? bias->data_ptr() : nullptr, y.data_ptr(), (int)b,
-                              (int)l, (int)d, (int)w->size(-1), dtype, x->stride(0), x->stride(1), y.stride(0), y.stride(1), q.stream()))
-      return declined(rc);
-    return THPVariable_Wrap(std::move(y));
-  )
+  Where q(*x);
+  if (!q.here(*w) || !q.here(*bias) || !q.here(*out)) Py_RETURN_NONE;
+  Tensor y = out->defined() ? *out : at::empty({b, l, d}, x->options());
+  if (const int rc = f_conv(x->data_ptr(), w->data_ptr(), bias->defined() ? bias->data_ptr() : nullptr, y.data_ptr(), (int)b,
+                            (int)l, (int)d, (int)w->size(-1), dtype, x->stride(0), x->stride(1), y.stride(0), y.stride(1), q.stream()))
+    return declined(rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
 }
 
 // forward(X, A, B, C, chunk, dt, initial_states, D, z, out, return_final_state) -> Y or (Y, final_state)
 PyObject* py_forward(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   const Tensor *X, *A, *B, *C, *dt, *init, *D, *z, *out;
   if (n != 11 || !get(o[0], &X) || !get(o[1], &A) || !get(o[2], &B) || !get(o[3], &C) || !PyLong_CheckExact(o[4]) ||
       !get(o[5], &dt, true) || !get(o[6], &init, true) || !get(o[7], &D, true) || !get(o[8], &z, true) ||
@@ -213,56 +213,59 @@ PyObject* py_forward(PyObject*, PyObject* const* o, Py_ssize_t n) {
     Py_RETURN_NONE;
   if (z->defined() && (z->scalar_type() != st || z->sizes() != X->sizes() || !inner(*z))) Py_RETURN_NONE;
   if (out->defined() && (out->scalar_type() != st || out->sizes() != X->sizes() || !inner(*out))) Py_RETURN_NONE;
-  GUARDED(
-    Where w(*X);
-    if (!w.here(*A) || !w.here(*B) || !w.here(*C) || !w.here(*dt) || !w.here(*init) || !w.here(*D) || !w.here(*z) || !w.here(*out))
-      Py_RETURN_NONE;
-    Tensor Y = out->defined() ? *out : at::empty({b, s, h, p}, X->options());
-    Tensor fin;
-    if (want_final) fin = at::empty({b, h, ns, p}, X->options().dtype(at::kFloat));
-    SsdArgs a = {};
-    a.X = X->data_ptr(); a.A = static_cast<const float*>(A->data_ptr()); a.B = B->data_ptr(); a.C = C->data_ptr(); a.Y = Y.data_ptr();
-    if (dt->defined()) { a.dt = dt->data_ptr(); strides3(*dt, a.dt_stride); }
-    if (init->defined()) a.initial_state = static_cast<const float*>(init->data_ptr());
-    if (want_final) a.final_state = static_cast<float*>(fin.data_ptr());
-    if (D->defined()) {
-      a.D = static_cast<const float*>(D->data_ptr());
-      if (D->scalar_type() != at::kFloat) a.flags |= SSD_FLAG_D_IN_DTYPE;
-    }
-    if (z->defined()) { a.Z = z->data_ptr(); strides4(*z, a.z_stride); }
-    a.status = static_cast<int32_t*>(status_word(w.dev.index()).data_ptr());
-    a.batch = (int)b; a.seqlen = (int)s; a.nheads = (int)h; a.headdim = (int)p; a.dstate = (int)ns; a.ngroups = (int)g;
-    a.chunk = (int)chunk; a.dtype = dtype;
-    strides4(*X, a.x_stride); strides3(*A, a.a_stride); strides4(*B, a.b_stride); strides4(*C, a.c_stride); strides4(Y, a.y_stride);
-    const size_t need = f_workspace(&a);
-    if (need) {
-      Tensor& ws = workspace(w.dev.index(), (int64_t)need);
-      a.workspace = ws.data_ptr();
-      a.workspace_bytes = (size_t)ws.numel();
-    }
-    if (const int rc = f_forward(&a, w.stream())) return declined(rc);
-    if (!want_final) return THPVariable_Wrap(std::move(Y));
-    PyObject* t = PyTuple_New(2);
-    if (!t) return nullptr;
-    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(Y)));
-    PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(fin)));
-    return t;
-  )
+  Where w(*X);
+  if (!w.here(*A) || !w.here(*B) || !w.here(*C) || !w.here(*dt) || !w.here(*init) || !w.here(*D) || !w.here(*z) || !w.here(*out))
+    Py_RETURN_NONE;
+  Tensor Y = out->defined() ? *out : at::empty({b, s, h, p}, X->options());
+  Tensor fin;
+  if (want_final) fin = at::empty({b, h, ns, p}, X->options().dtype(at::kFloat));
+  SsdArgs a = {};
+  a.X = X->data_ptr(); a.A = static_cast<const float*>(A->data_ptr()); a.B = B->data_ptr(); a.C = C->data_ptr(); a.Y = Y.data_ptr();
+  if (dt->defined()) { a.dt = dt->data_ptr(); strides3(*dt, a.dt_stride); }
+  if (init->defined()) a.initial_state = static_cast<const float*>(init->data_ptr());
+  if (want_final) a.final_state = static_cast<float*>(fin.data_ptr());
+  if (D->defined()) {
+    a.D = static_cast<const float*>(D->data_ptr());
+    if (D->scalar_type() != at::kFloat) a.flags |= SSD_FLAG_D_IN_DTYPE;
+  }
+  if (z->defined()) { a.Z = z->data_ptr(); strides4(*z, a.z_stride); }
+  a.status = static_cast<int32_t*>(status_word(w.dev.index()).data_ptr());
+  a.batch = (int)b; a.seqlen = (int)s; a.nheads = (int)h; a.headdim = (int)p; a.dstate = (int)ns; a.ngroups = (int)g;
+  a.chunk = (int)chunk; a.dtype = dtype;
+  strides4(*X, a.x_stride); strides3(*A, a.a_stride); strides4(*B, a.b_stride); strides4(*C, a.c_stride); strides4(Y, a.y_stride);
+  const size_t need = f_workspace(&a);
+  if (need) {
+    Tensor& ws = workspace(w.dev.index(), (int64_t)need);
+    a.workspace = ws.data_ptr();
+    a.workspace_bytes = (size_t)ws.numel();
+  }
+  if (const int rc = f_forward(&a, w.stream())) return declined(rc);
+  if (!want_final) return THPVariable_Wrap(std::move(Y));
+  PyObject* t = PyTuple_New(2);
+  if (!t) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(Y)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(fin)));
+  return t;
+  END_HANDLE_TH_ERRORS
 }
 
 // workspace(device_index, bytes), status_word(device_index): the tensors that the long way uses too
 PyObject* py_workspace(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 2) Py_RETURN_NONE;
   const long dev = PyLong_AsLong(o[0]);
   const long long bytes = PyLong_AsLongLong(o[1]);
   if (PyErr_Occurred() || dev < 0 || dev >= kMaxDevices) return PyErr_Occurred() ? nullptr : (Py_INCREF(Py_None), Py_None);
-  GUARDED(return THPVariable_Wrap(workspace((int)dev, bytes));)
+  return THPVariable_Wrap(workspace((int)dev, bytes));
+  END_HANDLE_TH_ERRORS
 }
 PyObject* py_status(PyObject*, PyObject* const* o, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 1) Py_RETURN_NONE;
   const long dev = PyLong_AsLong(o[0]);
   if (PyErr_Occurred() || dev < 0 || dev >= kMaxDevices) return PyErr_Occurred() ? nullptr : (Py_INCREF(Py_None), Py_None);
-  GUARDED(return THPVariable_Wrap(status_word((int)dev));)
+  return THPVariable_Wrap(status_word((int)dev));
+  END_HANDLE_TH_ERRORS
 }
 
 // init(forward, workspace_bytes, step_strided, conv1d_silu, dt_prologue, raise): addresses in the loaded library, and the

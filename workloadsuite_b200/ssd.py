@@ -215,7 +215,7 @@ def ssd_forward(
     that runs into the bound writes a code to the device status word (``device_status``) and returns.
     ``inject_lost_handover`` exists to test that path: see ``SSD_FLAG_INJECT_LOST_HANDOVER``.
     """
-    if (kernel is None and not nsegments and not wait_limit_ms and out_final_state is None
+    if (kernel is None and not nsegments and not wait_limit_ms and out_final_state is None and out_logdecay is None
             and not (state_only or reuse_segments or return_logdecay or separate_epilogue or inject_lost_handover)):
         got = _lib.fast().forward(X, A, B, C_, chunk, dt, initial_states, D, z, out, bool(return_final_state))
         if got is not None:
