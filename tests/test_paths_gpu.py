@@ -242,6 +242,20 @@ def test_dt_prologue_eight_heads_per_thread():
     assert ((dt.double() - ref).abs() <= 2 ** -10 * ref + 2 ** -24).all()     # half an ulp, or of the smallest step
 
 
+@pytest.mark.parametrize("rows", [2 ** 31 - 1024, 2 ** 31 + 1024], ids=["last_pass_past_31_bits", "rows_past_31_bits"])
+def test_dt_prologue_row_counter(rows):
+    """More rows than a 32-bit counter can walk (one head, the same raw value in each: 13 GB of results)."""
+    import workloadsuite_b200 as W
+
+    raw = torch.full((1, 1, 1), -1.5, device=DEV).half().expand(2, rows // 2, 1)
+    A_log = torch.full((1,), 0.5, device=DEV)
+    dt, A = W.dt_prologue(raw, None, A_log)
+    dt1, A1 = W.dt_prologue(raw[:1, :1], None, A_log)
+    assert bool((dt == dt1).all()) and bool((A == A1).all())
+    del dt, A
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("b,s,h,n", [(3, 2048, 24, 128), (11, 384, 8, 64)], ids=["ramps_in_an_entry", "groups"])
 def test_host_pipeline_chunks_and_sets(b, s, h, n):
     """Chunks, ramps and sets of batch entries against the device forward over the same tensors (other cuts of the

@@ -24,16 +24,17 @@ __device__ __forceinline__ T discretise(T raw, T bias) {
 
 // V consecutive heads per thread (V = 8: 16-byte pieces of 16-bit rows; V = 1 where rows are not aligned), the same heads
 // in every row of the grid's stride, so that bias and rate are read once and nothing is divided per element.
-template <typename T, int V>
+// I: int where the row counter stays within it to the end (a division of 64 bits per row is dear), else int64_t.
+template <typename T, int V, typename I>
 __global__ void __launch_bounds__(128)
 dt_prologue_kernel(const T* __restrict__ dt_raw, int64_t sb, int64_t sl, const T* __restrict__ dt_bias,
-                   const float* __restrict__ A_log, T* __restrict__ dt_out, float* __restrict__ A_dt, int rows,
+                   const float* __restrict__ A_log, T* __restrict__ dt_out, float* __restrict__ A_dt, I rows,
                    int seqlen, int nheads) {
-  const int vecs = nheads / V;
-  const int first = blockIdx.x * blockDim.x + threadIdx.x;
-  const int step = (gridDim.x * blockDim.x) / vecs;   // rows per pass; threads past step * vecs have none
+  const I vecs = nheads / V;
+  const I first = (I)blockIdx.x * blockDim.x + threadIdx.x;
+  const I step = (I)gridDim.x * blockDim.x / vecs;   // rows per pass; threads past step * vecs have none
   if (first >= step * vecs) return;
-  const int h0 = (first % vecs) * V;
+  const int h0 = (int)(first % vecs) * V;
   float rate[V];
   T bias[V];
 #pragma unroll
@@ -41,8 +42,8 @@ dt_prologue_kernel(const T* __restrict__ dt_raw, int64_t sb, int64_t sl, const T
     rate[e] = -expf(A_log[h0 + e]);
     bias[e] = dt_bias ? dt_bias[h0 + e] : Cvt<T>::from_f(0.f);
   }
-  for (int r = first / vecs; r < rows; r += step) {
-    const int b = r / seqlen;
+  for (I r = first / vecs; r < rows; r += step) {
+    const I b = r / seqlen;
     const T* src = dt_raw + b * sb + (int64_t)(r - b * seqlen) * sl + h0;
     const int64_t o = (int64_t)r * nheads + h0;
     alignas(16) T in[V], d[V];
@@ -74,20 +75,23 @@ dt_prologue_kernel(const T* __restrict__ dt_raw, int64_t sb, int64_t sl, const T
 template <typename T>
 int launch_prologue(const void* dt_raw, int64_t sb, int64_t sl, const void* dt_bias, const float* A_log, void* dt_out,
                     float* A_dt, int batch, int seqlen, int nheads, cudaStream_t stream) {
-  if ((int64_t)batch * seqlen > 0x7fffffffLL || nheads > (1 << 24)) return SSD_ERR_TOO_LARGE;
   constexpr int V = 8, per16 = 16 / (int)sizeof(T);
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   // (a few rows: one head per thread, so that the functions of the eight do not run one after the other)
-  const bool vec = nheads % V == 0 && (int64_t)batch * seqlen * nheads >= (1 << 17) && al(dt_raw) && al(dt_out) && al(A_dt) && sb % per16 == 0 && sl % per16 == 0;
-  const int rows = batch * seqlen, vecs = vec ? nheads / V : nheads;
-  const int64_t total = (int64_t)rows * vecs;
-  // up to sixteen small CTAs per SM, and at least one pass of whole rows
-  const int64_t ctas = std::max<int64_t>(std::min<int64_t>((total + 127) / 128, 148 * 16), (vecs + 127) / 128);
-  auto go = [&](auto kern) {
+  const int64_t rows = (int64_t)batch * seqlen;
+  const bool vec = nheads % V == 0 && rows >= ((1LL << 17) + nheads - 1) / nheads && al(dt_raw) && al(dt_out) && al(A_dt) &&
+                   sb % per16 == 0 && sl % per16 == 0;
+  const int vecs = vec ? nheads / V : nheads;
+  // up to sixteen small CTAs per SM (as many as there is work for), and at least one pass of whole rows
+  const int64_t most = 148 * 16, wanted = rows >= most * 128 ? most : std::min<int64_t>((rows * vecs + 127) / 128, most);
+  const int64_t ctas = std::max<int64_t>(wanted, (vecs + 127LL) / 128);
+  const bool small = rows + ctas * 128 <= 0x7fffffffLL;   // (a pass is at most ctas * 128 rows)
+  auto go = [&](auto kern, auto nrows) {
     return launch(kern, (unsigned)ctas, 128, 0, stream, static_cast<const T*>(dt_raw), sb, sl, static_cast<const T*>(dt_bias),
-                  A_log, static_cast<T*>(dt_out), A_dt, rows, seqlen, nheads);
+                  A_log, static_cast<T*>(dt_out), A_dt, nrows, seqlen, nheads);
   };
-  return vec ? go(dt_prologue_kernel<T, V>) : go(dt_prologue_kernel<T, 1>);
+  if (small) return vec ? go(dt_prologue_kernel<T, V, int>, (int)rows) : go(dt_prologue_kernel<T, 1, int>, (int)rows);
+  return vec ? go(dt_prologue_kernel<T, V, int64_t>, rows) : go(dt_prologue_kernel<T, 1, int64_t>, rows);
 }
 
 }  // namespace
