@@ -199,7 +199,13 @@ def test_plan_of_the_benchmark_configurations(lib):
     assert _plan(lib, so) == (TC, nseg, 2)
     # 96 pairs of only 16 tiles (config 1): the state-only scans and the start-ups would eat the gain: whole sequences
     assert _plan(lib, _shape(8, 2048, 24, 64, 128, 1, 256, _lib.DTYPE_BF16))[1:] == (1, 1)
-    assert _plan(lib, _shape(8, 8192, 24, 64, 128, 1, 256, _lib.DTYPE_BF16))[1:] == (2, 1)
+    # ... and of 64 tiles: the deal would save less than it costs, so the call is planned whole, as it is launched, and asks for
+    # no scratch; a caller's own count is taken as it is
+    long = _shape(8, 8192, 24, 64, 128, 1, 256, _lib.DTYPE_BF16)
+    assert _plan(lib, long)[1:] == (1, 1) and lib.ssd_b200_workspace_bytes(C.byref(long)) == 0
+    long.nsegments = 2
+    assert _plan(lib, long)[1:] == (2, 1) and lib.ssd_b200_workspace_bytes(C.byref(long)) > 0
+    assert _plan(lib, _shape(2, 8192, 80, 64, 128, 1, 256, _lib.DTYPE_BF16))[1:] == (2, 1)      # 80 pairs: cut
     # config 4 (6144 short sequences): whole sequences, one launch
     assert _plan(lib, _shape(256, 512, 48, 64, 64, 8, 128, _lib.DTYPE_BF16)) == (TC, 1, 1)
     # config 0 is fp32: the CUDA-core recurrence

@@ -129,8 +129,9 @@ def test_decays_beyond_the_range_of_a_factor(case, s, h, g):
 
 
 @pytest.mark.parametrize("shape", [dict(b=50, s=300, h=7, g=1, n=128), dict(b=1, s=1500, h=3, g=1, n=64),
-                                   dict(b=40, s=513, h=8, g=2, n=64), dict(b=1, s=4500, h=2, g=1, n=128, decay_scale=0.002)],
-                         ids=["chained_odd", "lookback_odd", "chained_n64", "lookback_36_pieces"])
+                                   dict(b=40, s=513, h=8, g=2, n=64), dict(b=1, s=4500, h=2, g=1, n=128, decay_scale=0.002),
+                                   dict(b=19, s=500, h=8, g=1, n=64), dict(b=49, s=300, h=6, g=1, n=64)],
+                         ids=["chained_odd", "lookback_odd", "chained_n64", "lookback_36_pieces", "lookback_76_pairs", "lookback_147_pairs"])
 def test_cut_sequences_of_no_round_length(shape):
     """Sequences dealt out over the CTAs (handed on, or folded from what the CTAs before published) whose last tile is
     ragged; 50 x 7 heads are 200 pairs of which every fourth is half empty; 36 pieces are more than a warp asks for at once."""

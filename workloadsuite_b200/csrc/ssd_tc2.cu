@@ -1185,10 +1185,6 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
   if (prm.sp.chain == 2) {
     const int pieces = std::min(kSms / prm.upairs, nt);
     if (pieces > 1 && pieces * prm.upairs >= kSms * 93 / 100) grid = pieces * prm.upairs;
-    // With more than half as many pairs as SMs the deal saves little and every tile of a range's last piece is read twice: whole
-    // sequences, unless the saving (at 1.55 of a tile's time for a dealt one) is more than the start-ups of a cut (96 pairs
-    // of 64 tiles: 204 us dealt out, 185 whole; 80 pairs of 64: 174 and 185).
-    if (pieces == 1 && (double)prm.upairs * nt / kSms * 1.55 + 5 > nt + 2.2) grid = prm.upairs;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -1259,6 +1255,10 @@ int tc2_default_segments(const SsdArgs& a) {
     // Look-back: the state-only scan of the last piece of every range, two start-ups and the round trip through scratch, and
     // the fold of the pieces before the last one of a sequence.
     const double pieces = std::min((double)kSms / upairs, (double)tiles);
+    // With more than half as many pairs as SMs the deal saves little and every tile of a range's last piece is read twice: whole
+    // sequences, unless the saving (at 1.55 of a tile's time for a dealt one) is more than the start-ups of a cut (96 pairs
+    // of 64 tiles: 204 us dealt out, 185 whole; 80 pairs of 64: 174 and 185).
+    if (pieces < 2 && even * 1.55 + 5 > tiles + 2.2) return 1;
     return tiles >= 2 && even * 1.4 + 4.9 + 0.12 * pieces < 0.98 * (tiles + 2.2) ? 2 : 1;
   }
   if (upairs >= 120) return 1;
