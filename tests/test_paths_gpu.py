@@ -228,6 +228,22 @@ def test_conv_run_lengths(dtype, l, d):
     assert ((y - ref).abs().max() / ref.abs().max()).item() < (1e-5 if dtype == torch.float32 else 2 ** -8)
 
 
+@pytest.mark.parametrize("dtype,l", [(torch.float16, 64), (torch.bfloat16, 33), (torch.float32, 32)])
+def test_conv_in_place_up_to_the_longest_run(dtype, l):
+    """A column of up to 64 tokens (fp32: 32) is one thread's, so a call that writes over its input has the bits of one that does
+    not; many calls, since a race need not show in one."""
+    import workloadsuite_b200 as W
+
+    gen = torch.Generator(DEV).manual_seed(l)
+    x = torch.randn(1, l, 2048, generator=gen, device=DEV).to(dtype)
+    w, bias = torch.randn(2048, 1, 4, generator=gen, device=DEV).to(dtype), torch.randn(2048, generator=gen, device=DEV).to(dtype)
+    want = W.conv1d_silu(x, w, bias)
+    for _ in range(100):
+        y = x.clone()
+        W.conv1d_silu(y, w, bias, out=y)
+        assert torch.equal(y, want)
+
+
 def test_dt_prologue_eight_heads_per_thread():
     """More than 2^17 elements take the vector path; the functions are those of the scalar one, so its rows have the same
     bits as the first rows computed alone."""

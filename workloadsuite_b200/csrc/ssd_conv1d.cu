@@ -326,7 +326,12 @@ template <typename T>
 int launch_conv(const void* x, const void* w, const void* bias, void* y, int batch, int seqlen, int channels, int taps,
                 int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl, cudaStream_t stream) {
   const int64_t columns = (int64_t)batch * (channels / 8);
-  const int run = run_length(32, 4, columns, seqlen, 148 * 192);
+  // Threads of one column read the rows before their runs.  Where y lies over x (a call in place), columns are not cut below the
+  // longest run, so that up to its length each is one thread's, which reads a row before it writes it.
+  const char *x0 = static_cast<const char*>(x), *y0 = static_cast<const char*>(y);
+  const bool in_place = x0 < y0 + ((batch - 1) * ysb + (seqlen - 1) * ysl + channels) * (int64_t)sizeof(T) &&
+                        y0 < x0 + ((batch - 1) * xsb + (seqlen - 1) * xsl + channels) * (int64_t)sizeof(T);
+  const int run = in_place ? 32 : run_length(32, 4, columns, seqlen, 148 * 192);
   const int64_t total = columns * ((seqlen + run - 1) / run);
   if ((total + 127) / 128 > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
   const unsigned grid = (unsigned)((total + 127) / 128);
@@ -341,7 +346,7 @@ int launch_conv(const void* x, const void* w, const void* bias, void* y, int bat
     if (al && taps >= 2 && taps <= 4) {
       // a block per SM (b1 s4096 h32: 13.4 us with half a block's worth, 12.4 so; with two it is 18.0, the rows before the
       // runs read again and a second round of blocks)
-      const int len = run_length(kLongestRun, kPiece, columns, seqlen, 148 * 128);
+      const int len = in_place ? kLongestRun : run_length(kLongestRun, kPiece, columns, seqlen, 148 * 128);
       const int64_t tot = columns * ((seqlen + len - 1) / len);
       if ((tot + kStagedThreads - 1) / kStagedThreads > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
       const unsigned g = (unsigned)((tot + kStagedThreads - 1) / kStagedThreads);
