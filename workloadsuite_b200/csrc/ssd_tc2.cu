@@ -94,7 +94,7 @@ struct alignas(16) Factors {
   float cs2[T];       // cs * log2(e)
   float cf[T];        // exp(cs at the end of the row's 32-block - cs of the row) * dt: the row's factor as a column of P
   float dg[T];        // diagonal blocks: at columns 4i cs * log2(e) - log2(dt), at the three after it the ratio to the column before;
-                      // dt in the runs of 16 columns that hold a steep group of four
+                      // dt in steep groups of four
   float tot;          // cs_last
   float ld;           // sum of the log-decays as given
   uint32_t steep;     // groups of four columns in which the factors of P span more than the ratios can carry
@@ -105,7 +105,7 @@ constexpr int kFactors = 4;   // tiles that the prefix sums may be ahead
 // Log-decays below this count as this in the prefix sums: e^-104 is 2^-150, a factor of zero either way, while -inf (a
 // reset) would make every difference of sums after it NaN, and a very large one would take their digits.
 constexpr float kLowest = -104.f;
-// A group of four columns of a diagonal block is steep if its factors span more than 2^40, or a dt is no ordinary positive
+// A group of four columns of a diagonal block is steep if its ratios go through more than 2^40, or a dt is no ordinary positive
 // number: the ratios start from the group's first column, and where that one underflows (2^-126) the three after it would
 // be lost with it -- the diagonal, of factor dt, too.  So what is lost in the others is below 2^-86.
 constexpr float kSteep = 40.f, kLeastLogDt = -60.f;
@@ -620,6 +620,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll
           for (int e = 0; e < 4; ++e) a[e] = a[e] < kLowest ? kLowest : a[e];   // (NaN stays NaN)
           cs = a[0] + a[1] + a[2] + a[3];
+#pragma unroll 1
           for (int d = 16; d >= 1; d >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, d);
         }
 #pragma unroll
@@ -644,20 +645,21 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         Factors& f = m->f[h][slot];
         reinterpret_cast<float4*>(f.cs2)[lane] = make_float4(c2[0], c2[1], c2[2], c2[3]);
         float cf[4], cc[4];
-        bool steep = false;
+        float least = 0.f;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           cf[e] = ex2(ce - c2[e]) * dt[e];
           // dt multiplies the columns of P instead of the rows of X (P.(dt o x) = (P o dt_s).x), so the X tile stays as
           // loaded.  The ratios are clamped: one above the diagonal may overflow, it is masked out.
           const float lg = lg2(dt[e]);                     // (lg2(1) is 0)
-          steep |= !(lg > kLeastLogDt);
+          least = fminf(least, lg);
           cc[e] = c2[e] - lg;
         }
-        steep |= !(fmaxf(fmaxf(cc[0], cc[1]), fmaxf(cc[2], cc[3])) - fminf(fminf(cc[0], cc[1]), fminf(cc[2], cc[3])) <= kSteep);
+        const float r0 = cc[0] - cc[1], r1 = cc[1] - cc[2], r2 = cc[2] - cc[3];
+        const bool steep = !(fabsf(r0) + fabsf(r1) + fabsf(r2) <= kSteep && least > kLeastLogDt);   // (NaN: dt < 0, or dt = 0 throughout)
         const uint32_t all_steep = __ballot_sync(0xffffffffu, steep);
-        float4 dg = make_float4(cc[0], ex2(fminf(cc[0] - cc[1], 126.f)), ex2(fminf(cc[1] - cc[2], 126.f)), ex2(fminf(cc[2] - cc[3], 126.f)));
-        if (all_steep >> (lane & 28) & 15u) dg = make_float4(dt[0], dt[1], dt[2], dt[3]);
+        float4 dg = make_float4(cc[0], ex2(fminf(r0, 126.f)), ex2(fminf(r1, 126.f)), ex2(fminf(r2, 126.f)));
+        if (steep) dg = make_float4(dt[0], dt[1], dt[2], dt[3]);
         if (lane == 31) {
           f.tot = cs;
           f.ld = low ? ld : cs;
@@ -689,8 +691,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 
     // A. P = (C B^T) o exp(segsum), causal -> TMEM (A operand, 16-bit pairs).  Decay mask per 32-token column block J of
     // this warp's 32 rows (block q is the diagonal one):
-    //   J == q: exp2(cs_l - cs_s), causal, one ex2 per four columns and the ratios between neighbours (in 16 columns that hold a
-    //           steep group: one ex2 per column);
+    //   J == q: exp2(cs_l - cs_s), causal, one ex2 per four columns and the ratios between neighbours (steep groups: one ex2 per
+    //           column, in a second pass);
     //   J <  q: exp(cs_l - cs_s) = rf_J[l] * cf[s] with both factors <= 1 for non-positive log-decays
     //           (rf_J[l] = exp(cs_l - cs_end(J)), cf[s] = exp(cs_end(J) - cs_s)): two multiplies;
     //   J >  q: zero.
@@ -704,26 +706,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         const uint4* keep = m->causal[max(0, min(16, lane - 16 * half + 1))];
         tmem_ld_wait();
         uint32_t pk[8];
-        if (__builtin_expect((f.steep >> (8 * q + 4 * half) & 15u) != 0, 0)) {
-          const float4* cv = reinterpret_cast<const float4*>(&f.cs2[32 * q + 16 * half]);
 #pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {
-            const float4 d = dv[e4], c = cv[e4];
-            const float v0 = __uint_as_float(g[4 * e4]) * (ex2(cs2 - c.x) * d.x), v1 = __uint_as_float(g[4 * e4 + 1]) * (ex2(cs2 - c.y) * d.y);
-            const float v2 = __uint_as_float(g[4 * e4 + 2]) * (ex2(cs2 - c.z) * d.z), v3 = __uint_as_float(g[4 * e4 + 3]) * (ex2(cs2 - c.w) * d.w);
-            pk[2 * e4] = pack2<T16>(v0, v1);
-            pk[2 * e4 + 1] = pack2<T16>(v2, v3);
-          }
-        } else {
-#pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {
-            const float4 d = dv[e4];
-            const float w0 = ex2(cs2 - d.x), w1 = w0 * d.y, w2 = w1 * d.z, w3 = w2 * d.w;
-            const float v0 = __uint_as_float(g[4 * e4]) * w0, v1 = __uint_as_float(g[4 * e4 + 1]) * w1;
-            const float v2 = __uint_as_float(g[4 * e4 + 2]) * w2, v3 = __uint_as_float(g[4 * e4 + 3]) * w3;
-            pk[2 * e4] = pack2<T16>(v0, v1);
-            pk[2 * e4 + 1] = pack2<T16>(v2, v3);
-          }
+        for (int e4 = 0; e4 < 4; ++e4) {
+          const float4 d = dv[e4];
+          const float w0 = ex2(cs2 - d.x), w1 = w0 * d.y, w2 = w1 * d.z, w3 = w2 * d.w;
+          const float v0 = __uint_as_float(g[4 * e4]) * w0, v1 = __uint_as_float(g[4 * e4 + 1]) * w1;
+          const float v2 = __uint_as_float(g[4 * e4 + 2]) * w2, v3 = __uint_as_float(g[4 * e4 + 3]) * w3;
+          pk[2 * e4] = pack2<T16>(v0, v1);
+          pk[2 * e4 + 1] = pack2<T16>(v2, v3);
         }
         const uint4 k0 = keep[0], k1 = keep[1];
         pk[0] &= k0.x; pk[1] &= k0.y; pk[2] &= k0.z; pk[3] &= k0.w;
@@ -746,6 +736,23 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           pk[2 * e4 + 1] = pack_pair<T16>(mul_pair(pair(g[4 * e4 + 2], g[4 * e4 + 3]), mul_pair(rf2, c.y)));
         }
         tmem_st16(tP + tlane + 16 * J, pk);
+      }
+      const uint32_t steep = f.steep >> (8 * q) & 255u;
+      if (__builtin_expect(steep != 0, 0)) {   // steep groups of the diagonal block, over what the ratios made of them
+        tmem_st_wait();
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i) {
+          if (!(steep >> i & 1)) continue;
+          uint32_t g[4];
+          tmem_ld4(tG + tlane + 32 * q + 4 * i, g);
+          const float4 d = reinterpret_cast<const float4*>(f.dg)[8 * q + i], c = reinterpret_cast<const float4*>(f.cs2)[8 * q + i];
+          const float w[4] = {ex2(cs2 - c.x) * d.x, ex2(cs2 - c.y) * d.y, ex2(cs2 - c.z) * d.z, ex2(cs2 - c.w) * d.w};
+          tmem_ld_wait();
+          float v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = 4 * i + e <= lane ? __uint_as_float(g[e]) * w[e] : 0.f;
+          tmem_st2(tP + tlane + 16 * q + 2 * i, pack2<T16>(v[0], v[1]), pack2<T16>(v[2], v[3]));
+        }
       }
       if (q < 3) {
         uint32_t pz[16];
