@@ -227,6 +227,8 @@ def test_lengths_that_are_no_whole_tiles_stay_in_fp32_unless_the_caller_asks(lib
 
 def test_host_pipeline_scratch_sizes(lib):
     """The host-buffer entry sizes its device scratch from the shape alone: chunks of at most 24 MiB of X, four slots."""
+    # 16 entries of 10.5 MB: chunks of two of them (X and Y, four slots), not of four
+    assert lib.ssd_b200_host_scratch_bytes(C.byref(_shape(16, 1024, 80, 64, 128, 1, 128, _lib.DTYPE_BF16))) < 12 * (21 << 20)
     big = lib.ssd_b200_host_scratch_bytes(C.byref(_shape(4, 8192, 80, 64, 128, 1, 256, _lib.DTYPE_BF16)))
     small = lib.ssd_b200_host_scratch_bytes(C.byref(_shape(2, 512, 8, 64, 64, 2, 128, _lib.DTYPE_BF16)))
     assert 0 < small < big < (1 << 30)

@@ -273,7 +273,8 @@ def test_dt_prologue_row_counter(rows):
     torch.cuda.empty_cache()
 
 
-@pytest.mark.parametrize("b,s,h,n", [(3, 2048, 24, 128), (11, 384, 8, 64)], ids=["ramps_in_an_entry", "groups"])
+@pytest.mark.parametrize("b,s,h,n", [(3, 2048, 24, 128), (11, 384, 8, 64), (35, 512, 32, 64), (2, 4096, 80, 128)],
+                         ids=["ramps_in_an_entry", "groups", "groups_of_a_large_whole", "ramps_in_an_entry_of_a_large_whole"])
 def test_host_pipeline_chunks_and_sets(b, s, h, n):
     """Chunks, ramps and sets of batch entries against the device forward over the same tensors (other cuts of the
     sequence, so other roundings of the carried state's copy)."""

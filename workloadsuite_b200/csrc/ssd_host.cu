@@ -93,11 +93,19 @@ void make_sets(std::vector<Slice>& slices, int set_entries) {
   }
 }
 
-// Pieces of 1/4, 1/4, 1/2 of `regular` (multiples of `unit`), as far as they fit into `left` with `keep` to spare and
-// are worth a copy of their own (at least `least`).
-std::vector<int> ramp(int regular, int unit, int least, int keep, int* left) {
+// From 64 MiB of X on the link is busy for long enough that what a copy costs of its own (some 20 us) matters less than how much
+// of the last chunk is still to come back when the last input is in: chunks of an eighth of the whole, and what is small next to
+// X with its own chunk.  Below, fewer and larger ones.  16 entries of 10.5 MB: 4.14 ms so, 4.46 in quarters with sets of four
+// entries; 16 of 12.6 MB: 5.25 and 5.54; but 4 entries of 6.3 MB: 0.99 and 0.86, 64 of 0.13 MB: 0.49 and 0.40.
+bool is_large(const SsdArgs* a) {
+  return (int64_t)a->nheads * a->headdim * esize(a->dtype) * a->seqlen >= (((int64_t)64 << 20) + a->batch - 1) / a->batch;
+}
+
+// Pieces of 1/4, 1/4, 1/2 of `regular` (`fine`: 1/8, 1/8, 1/4, 1/2; multiples of `unit`), as far as they fit into `left` with
+// `keep` to spare and are worth a copy of their own (at least `least`).
+std::vector<int> ramp(int regular, int unit, int least, int keep, int* left, bool fine) {
   std::vector<int> pieces;
-  const int div[] = {4, 4, 2};
+  const std::vector<int> div = fine ? std::vector<int>{8, 8, 4, 2} : std::vector<int>{4, 4, 2};
   for (int d : div) {
     const int len = regular / d / unit * unit;
     if (len >= std::max(1, least) && *left - len >= keep) {
@@ -110,20 +118,23 @@ std::vector<int> ramp(int regular, int unit, int least, int keep, int* left) {
 
 // The chunks of all batch entries in order.  They open and close with a ramp of smaller ones, so that the device->host
 // stream starts early and the host->device stream ends late: the two directions then overlap for all but a fraction of a
-// chunk (also where a chunk is a whole batch entry, or several).
+// chunk (also where a chunk is a whole batch entry; or several, where the whole is not large).
 std::vector<Slice> make_slices(const SsdArgs* host, int tokens_per_chunk, int group, int set_entries) {
   std::vector<Slice> slices;
   const int b = host->batch, s = host->seqlen;
   const int64_t row = (int64_t)host->nheads * host->headdim * esize(host->dtype);
+  const bool large = is_large(host);
   constexpr int64_t kLeastBytes = 384 << 10;   // of X in a piece: a copy, a launch and two event waits cost some 10 us
   int unit = host->chunk / gcd_int(host->chunk, 128) * 128;
   if (s % unit != 0) unit = host->chunk;
   if (group > 1) {
     const int least = (int)std::min<int64_t>(b, (kLeastBytes + row * s - 1) / (row * s));
     int left = b;
-    const std::vector<int> head = ramp(group, 1, least, std::min(b, 2 * group) / 2, &left);
-    std::vector<int> tail = ramp(group, 1, least, 0, &left);
-    std::vector<int> sizes = head;
+    std::vector<int> sizes, tail;
+    if (!large) {
+      sizes = ramp(group, 1, least, std::min(b, 2 * group) / 2, &left, false);
+      tail = ramp(group, 1, least, 0, &left, false);
+    }
     for (; left > 0; left -= std::min(group, left)) sizes.push_back(std::min(group, left));
     sizes.insert(sizes.end(), tail.rbegin(), tail.rend());
     int bi = 0;
@@ -138,8 +149,9 @@ std::vector<Slice> make_slices(const SsdArgs* host, int tokens_per_chunk, int gr
   for (int bi = 0; bi < b; ++bi) {
     int left = s;
     std::vector<int> lens, tail;
-    if (bi == 0) lens = ramp(tokens_per_chunk, unit, least, b == 1 ? std::min(s, 2 * tokens_per_chunk) / 2 : 0, &left);
-    if (bi == b - 1) tail = ramp(tokens_per_chunk, unit, least, 0, &left);
+    const int keep = large ? tokens_per_chunk : b == 1 ? std::min(s, 2 * tokens_per_chunk) / 2 : 0;
+    if (bi == 0) lens = ramp(tokens_per_chunk, unit, least, keep, &left, large);
+    if (bi == b - 1) tail = ramp(tokens_per_chunk, unit, least, large ? tokens_per_chunk : 0, &left, large);
     while (left > 0) { const int len = std::min(tokens_per_chunk, left); lens.push_back(len); left -= len; }
     lens.insert(lens.end(), tail.rbegin(), tail.rend());   // the smallest last
     int t0 = 0;
@@ -158,14 +170,15 @@ Plan make_plan(const SsdArgs* a) {
   // chunk length: a multiple of the caller's chunk and of the tensor-core tile (128) when the sequence allows,
   // sized so that the X chunk is at most 48 MiB (measured on the 2.7B layer shape, 84 MB of X per batch entry: two chunks
   // of 42 MB per entry 8.5 ms, chunks of 24 / 28 / 56 / 84 MB 8.9 / 9.0 / 9.1 / 9.0 ms; with 8 MiB chunks the copies
-  // in both directions together reach 78 GB/s, with 24 MiB and more 82-86 GB/s), and a quarter of the whole where that is less:
-  // beside copies in the other direction every copy costs some 20 us of its own (50 MB each way take 1.05 ms in one piece,
-  // 1.2 in 8, 1.4 in 16, 1.65 in 32)
+  // in both directions together reach 78 GB/s, with 24 MiB and more 82-86 GB/s), and an eighth of the whole, or a quarter, where
+  // that is less (is_large): beside copies in the other direction every copy costs some 20 us of its own (50 MB each way take
+  // 1.05 ms in one piece, 1.2 in 8, 1.4 in 16, 1.65 in 32)
   int unit = a->chunk / gcd_int(a->chunk, 128) * 128;
   if (a->seqlen % unit != 0) unit = a->chunk;
   const size_t per_token = (size_t)a->nheads * a->headdim * e;
   const size_t total = per_token * a->seqlen * a->batch;
-  const size_t cap = std::max<size_t>((size_t)1 << 20, std::min<size_t>((size_t)48 << 20, total / 4));
+  const bool large = is_large(a);
+  const size_t cap = std::max<size_t>((size_t)1 << 20, std::min<size_t>((size_t)48 << 20, total / (large ? 8 : 4)));
   // ... and a batch entry is cut into equal chunks (no short remainder chunk at the end of every entry)
   long long tokens = (long long)(cap / per_token) / unit * unit;
   tokens = std::max<long long>(unit, std::min<long long>(tokens, a->seqlen));
@@ -187,7 +200,7 @@ Plan make_plan(const SsdArgs* a) {
   const size_t entry_bc = (size_t)a->seqlen * a->ngroups * a->dstate * e;
   const size_t entry_st = (size_t)a->nheads * a->dstate * a->headdim * 4;
   const size_t per_set = entry_a + entry_dt + 2 * entry_bc + entry_st;
-  const size_t q = std::max(k, std::min<size_t>((size_t)a->batch, ((size_t)16 << 20) / per_set));
+  const size_t q = large ? k : std::max(k, std::min<size_t>((size_t)a->batch, ((size_t)16 << 20) / per_set));
   pl.set_entries = (int)q;
   pl.a_bytes = align_up(q * entry_a, 256);
   pl.dt_bytes = align_up(q * entry_dt, 256);
