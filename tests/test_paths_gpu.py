@@ -150,6 +150,15 @@ def test_fp32_scan_tokens_in_line_and_the_rest(s, p, n):
     _check(inp, "scan_f32", 1e-4)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("units,s", [(8, 3), (8, 11), (304, 3), (304, 11), (304, 21), (640, 21)])
+@pytest.mark.parametrize("n", [32, 64, 128])
+def test_fp32_scan_with_registers_for_more_ctas(n, units, s, dtype):
+    """Tokens in line or one after the other, registers for two to five CTAs of an SM: chosen by the sequences and their tokens."""
+    inp = O.make_inputs(b=units // 8, s=s, h=8, p=64, n=n, g=2, dtype=dtype, init=True, seed=83 + s, decay_scale=0.3)
+    _check(inp, "scan_f32", 1e-4 if dtype == torch.float32 else 2e-2, nsegments=1)
+
+
 def test_step_reads_strided_operands_and_d_in_its_own_type():
     """Columns of a projection's output against the same values copied out: the same arithmetic, so the same bits."""
     import workloadsuite_b200 as W

@@ -79,7 +79,7 @@ __device__ __forceinline__ void store8<float>(float* dst, const float* src) {
 // Copies `rows` rows of `width` elements (row r at src + r*row_stride) into a
 // dense fp32 [rows][width] shared-memory tile, optionally scaling row r by
 // scale[r].
-template <typename T>
+template <typename T, int UNROLL>
 __device__ __forceinline__ void stage_rows(const T* src, int64_t row_stride, int rows, int width, float* dst,
                                            bool vec_ok, int tid) {
   if (sizeof(T) == 4 && vec_ok) {   // no conversion: asynchronous copies, waited for once all tensors' are under way
@@ -92,7 +92,7 @@ __device__ __forceinline__ void stage_rows(const T* src, int64_t row_stride, int
     }
   } else if (vec_ok) {
     const int per_row = width >> 3;
-#pragma unroll 4
+#pragma unroll UNROLL
     for (int i = tid; i < rows * per_row; i += kThreads) {
       const int r = i / per_row, c = (i - r * per_row) << 3;
       load8<T>(src + r * row_stride + c, dst + r * width + c);
@@ -124,8 +124,10 @@ __device__ __forceinline__ void reduce_scatter(float (&v)[U], int sl) {
 }
 
 // FULL: the state has exactly NS * SL rows (the strides of B and C in shared memory are then constants).
-template <typename T, int NS, int P, bool FULL>
-__global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams prm, const int tile) {
+// LINE: tokens worked on in line (1: one after the other).  CTAS: as many of an SM the registers have to leave room for (0: as
+// it comes).  Tokens in line take 64 to 126 registers, one after the other 32 to 80; see launch_one().
+template <typename T, int NS, int P, bool FULL, int LINE, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const ScanParams prm, const int tile) {
   constexpr int SL = kThreads / P;  // lanes sharing one state column
   constexpr int NS4 = NS / 4;
   extern __shared__ __align__(16) float smem[];
@@ -174,9 +176,10 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
   for (int t0 = t_begin; t0 < t_end; t0 += tile) {
     const int rows = min(tile, t_end - t0);
     __syncthreads();  // previous tile fully consumed (Ys stored, Xs/Bs/Cs read)
-    stage_rows<T>(Xg + (int64_t)t0 * prm.xs[1], prm.xs[1], rows, P, Xs, vec_ok, tid);
-    stage_rows<T>(Bg + (int64_t)t0 * prm.bs[1], prm.bs[1], rows, n, Bs, vec_ok, tid);
-    if (prm.compute_y) stage_rows<T>(Cg + (int64_t)t0 * prm.cs[1], prm.cs[1], rows, n, Cs, vec_ok, tid);
+    constexpr int kAhead = LINE == 1 ? 1 : 4;
+    stage_rows<T, kAhead>(Xg + (int64_t)t0 * prm.xs[1], prm.xs[1], rows, P, Xs, vec_ok, tid);
+    stage_rows<T, kAhead>(Bg + (int64_t)t0 * prm.bs[1], prm.bs[1], rows, n, Bs, vec_ok, tid);
+    if (prm.compute_y) stage_rows<T, kAhead>(Cg + (int64_t)t0 * prm.cs[1], prm.cs[1], rows, n, Cs, vec_ok, tid);
     if (tid < rows) {
       const float a = Ag[(int64_t)(t0 + tid) * prm.as[1]];
       araw[tid] = a;
@@ -243,10 +246,10 @@ __global__ void __launch_bounds__(kThreads) ssd_scan_f32_kernel(const ScanParams
         }
       }
     };
-    constexpr int kInLine = NS >= 16 && SL <= 4 ? 4 : 8;   // (at least SL; fewer where the state fills the registers)
     auto all = [&](auto want_y) {
       int t = 0;
-      for (; t + kInLine <= rows; t += kInLine) tokens(t, std::integral_constant<int, kInLine>{}, want_y);
+      if constexpr (LINE > 1)
+        for (; t + LINE <= rows; t += LINE) tokens(t, std::integral_constant<int, LINE>{}, want_y);
       for (; t < rows; ++t) tokens(t, std::integral_constant<int, 1>{}, want_y);
     };
     if (prm.compute_y) all(std::true_type{});
@@ -329,7 +332,27 @@ template <typename T, int NS, int P>
 int launch_one(const ScanParams& prm, cudaStream_t stream) {
   const int tile = tile_tokens(prm, P);
   const size_t smem = smem_bytes(tile, P, prm.n);
-  auto kern = prm.n == NS * (kThreads / P) ? ssd_scan_f32_kernel<T, NS, P, true> : ssd_scan_f32_kernel<T, NS, P, false>;
+  // Tokens in line hide what links one to the next, but their registers leave an SM two CTAs (16-bit inputs, whose staging takes
+  // them too, and any with 32 rows a thread).  Where more CTAs than that are waiting, they hide it as well:
+  //  - fewer tokens than go in line: one after the other, in registers for one CTA more than the 64 or 80 that this takes leave
+  //    room for where there are as many (bf16, 5120 sequences of one token, n 64: 43 us with the registers of the others, 22 so);
+  //  - fp32 with 32 rows a thread, up to four CTAs per SM: one after the other (384 sequences of 200 tokens, n 128: 230 us in
+  //    line, 178 so);
+  //  - 16-bit, up to 16 rows a thread: in line in registers for four CTAs (444 sequences of 200 tokens, n 32: 88 us with two, 67
+  //    so); 32 rows a thread and few tokens: for three.
+  constexpr int SL = kThreads / P, kLine = NS >= 16 && SL <= 4 ? 4 : 8;   // (at least SL; fewer where the state fills the registers)
+  constexpr bool k16 = sizeof(T) == 2;
+  constexpr int kMany = !k16 ? 0 : NS >= 32 ? 3 : 4, kMost = !k16 || NS == 4 ? 0 : (NS >= 32 ? 4 : 5) - (P == 128 ? 1 : 0);
+  const int64_t ctas = (int64_t)prm.batch * prm.nheads * prm.nseg;
+  const int tokens = std::min(prm.seqlen, prm.seg_len);
+  const bool many = ctas > 2 * 148, full = prm.n == NS * SL;
+  auto kern = full ? ssd_scan_f32_kernel<T, NS, P, true, kLine, 0> : ssd_scan_f32_kernel<T, NS, P, false, kLine, 0>;
+  if (k16 && full && tokens < kLine && ctas > kMany * 148)
+    kern = ssd_scan_f32_kernel<T, NS, P, true, 1, kMost>;
+  else if (tokens < kLine || (!k16 && NS == 32 && many && ctas <= 4 * 148))
+    kern = full ? ssd_scan_f32_kernel<T, NS, P, true, 1, 0> : ssd_scan_f32_kernel<T, NS, P, false, 1, 0>;
+  else if (k16 && many && (NS <= 16 || tokens < 16))
+    kern = full ? ssd_scan_f32_kernel<T, NS, P, true, kLine, kMany> : ssd_scan_f32_kernel<T, NS, P, false, kLine, kMany>;
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SSD_ERR_CUDA;
