@@ -159,11 +159,12 @@ def test_fp32_scan_with_registers_for_more_ctas(n, units, s, dtype):
     _check(inp, "scan_f32", 1e-4 if dtype == torch.float32 else 2e-2, nsegments=1)
 
 
-def test_step_reads_strided_operands_and_d_in_its_own_type():
-    """Columns of a projection's output against the same values copied out: the same arithmetic, so the same bits."""
+@pytest.mark.parametrize("b,h,n,g", [(3, 6, 128, 2), (1, 4, 256, 1), (40, 6, 16, 3), (40, 6, 32, 2), (40, 6, 256, 6), (2, 1, 64, 1)])
+def test_step_reads_strided_operands_and_d_in_its_own_type(b, h, n, g):
+    """Columns of a projection's output against the same values copied out: the same arithmetic, so the same bits.  CTAs of half
+    and of all columns."""
     import workloadsuite_b200 as W
 
-    b, h, n, g = 3, 6, 128, 2
     gen = torch.Generator(DEV).manual_seed(90)
     proj = torch.randn(b, 2 * h * 64 + 2 * g * n + h + 5, generator=gen, device=DEV).half()
     x, z, B, C, dt, _ = torch.split(proj, [h * 64, h * 64, g * n, g * n, h, 5], dim=-1)

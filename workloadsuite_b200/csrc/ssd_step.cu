@@ -3,11 +3,11 @@
 //   H[b,h] <- exp(a[b,h]) * H[b,h] + B[b,g] (x) (dt[b,h] * x[b,h])        H is [n, p] fp32
 //   y[b,h] <- C[b,g] . H[b,h]   (+ x * D[h], then * silu(z), as model_ref.py:116-118, when given)
 // HBM-bound: the fp32 state is read and written once (2 * n * p * 4 bytes per (b, h)); everything else is small.
-// One CTA of 128 threads per (batch, head) and half of the columns (columns are independent, rows are what y sums over):
-// thread (r, c) owns four state columns of the rows r, r + 16, ...; all of its state loads are issued before the first
-// use (n / 16 sixteen-byte loads in flight per thread), y is reduced over the sixteen row groups through shared memory.
-// Half-size CTAs because the whole grid is a few waves at most: the tail is shorter, and a small model's heads reach
-// twice the SMs.
+// One CTA of 128 threads per (batch, head) and half of the columns, or of 256 threads and all of them (columns are independent,
+// rows are what y sums over): thread (r, c) owns four state columns of the rows r, r + 16, ...; all of its state loads are
+// issued before the first use (n / 16 sixteen-byte loads in flight per thread), y is reduced over the sixteen row groups
+// through shared memory.  Contiguous operands have an instance of their own, whose offsets follow from the unit: with few state
+// rows the 64-bit products of the strides are a third of a CTA's time (5120 heads, n 16: 11.7 us with them, 8.2 without).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -21,19 +21,18 @@ namespace ssd {
 namespace {
 
 constexpr int kHeadDim = 64;
-constexpr int kCols = 32;                       // columns of a CTA
-constexpr int kLanes = kCols / 4;               // threads per state row
-constexpr int kStepThreads = 16 * kLanes;
 constexpr int kMaxRowsPerThread = 16;           // dstate <= 256
 
-template <typename T, int ROWS>   // ROWS = dstate / 16
-__global__ void __launch_bounds__(kStepThreads)
+// ROWS = dstate / 16; COLS: columns of a CTA; DENSE: every operand contiguous.
+template <typename T, int ROWS, int COLS, bool DENSE>
+__global__ void __launch_bounds__(4 * COLS)
 ssd_step_kernel(const SsdStepArgs p) {
+  constexpr int kCols = COLS, kLanes = COLS / 4, kStepThreads = 16 * kLanes, kParts = kHeadDim / COLS;
   __shared__ float ypart[16][kCols];
   __shared__ float bs[16 * ROWS], cs[16 * ROWS];
   constexpr int n = 16 * ROWS;
-  const int unit = blockIdx.x >> 1;          // b * nheads + h
-  const int col0 = (blockIdx.x & 1) * kCols;
+  const int unit = blockIdx.x / kParts;      // b * nheads + h
+  const int col0 = (blockIdx.x % kParts) * kCols;
   const int b = unit / p.nheads, h = unit - b * p.nheads;
   const int g = h / (p.nheads / p.ngroups);
   const int tid = threadIdx.x, r = tid / kLanes, c = tid % kLanes;
@@ -41,16 +40,17 @@ ssd_step_kernel(const SsdStepArgs p) {
   float4 hv[ROWS];
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) hv[i] = S[(int64_t)(i * 16 + r) * (kHeadDim / 4)];   // all loads first
-  const T* Bg = static_cast<const T*>(p.B) + b * p.b_stride[0] + g * p.b_stride[1];
-  const T* Cg = static_cast<const T*>(p.C) + b * p.c_stride[0] + g * p.c_stride[1];
+  const int64_t row_bc = (int64_t)(b * p.ngroups + g) * n;
+  const T* Bg = static_cast<const T*>(p.B) + (DENSE ? row_bc : b * p.b_stride[0] + g * p.b_stride[1]);
+  const T* Cg = static_cast<const T*>(p.C) + (DENSE ? row_bc : b * p.c_stride[0] + g * p.c_stride[1]);
   for (int i = tid; i < n; i += kStepThreads) {
     bs[i] = Cvt<T>::to_f(Bg[i]);
     cs[i] = Cvt<T>::to_f(Cg[i]);
   }
-  const T* xr = static_cast<const T*>(p.x) + b * p.x_stride[0] + h * p.x_stride[1] + col0;
+  const T* xr = static_cast<const T*>(p.x) + (DENSE ? (int64_t)unit * kHeadDim : b * p.x_stride[0] + h * p.x_stride[1]) + col0;
   const bool has_dt = p.dt != nullptr;
-  const float dtv = has_dt ? Cvt<T>::to_f(static_cast<const T*>(p.dt)[b * p.dt_stride[0] + h * p.dt_stride[1]]) : 1.f;
-  const float av = p.a[b * p.a_stride[0] + h * p.a_stride[1]];
+  const float dtv = has_dt ? Cvt<T>::to_f(static_cast<const T*>(p.dt)[DENSE ? unit : b * p.dt_stride[0] + h * p.dt_stride[1]]) : 1.f;
+  const float av = p.a[DENSE ? unit : b * p.a_stride[0] + h * p.a_stride[1]];
   // x * dt in the layer's precision, as the reference forms it (model_ref.py:144)
   float xd[4];
 #pragma unroll
@@ -65,7 +65,7 @@ ssd_step_kernel(const SsdStepArgs p) {
       xs = Cvt<T>::to_f(xr[tid]);
       ds = p.d_in_dtype ? Cvt<T>::to_f(static_cast<const T*>(p.D)[h]) : static_cast<const float*>(p.D)[h];
     }
-    if (p.z) zs = Cvt<T>::to_f(static_cast<const T*>(p.z)[b * p.z_stride[0] + h * p.z_stride[1] + col0 + tid]);
+    if (p.z) zs = Cvt<T>::to_f(static_cast<const T*>(p.z)[(DENSE ? (int64_t)unit * kHeadDim : b * p.z_stride[0] + h * p.z_stride[1]) + col0 + tid]);
   }
   const float decay = __expf(av);
   __syncthreads();
@@ -93,15 +93,38 @@ ssd_step_kernel(const SsdStepArgs p) {
   }
 }
 
-template <typename T>
+bool dense(const SsdStepArgs& p) {
+  const int64_t h = p.nheads, g = p.ngroups, n = p.dstate;
+  auto is = [&](const int64_t* st, int64_t heads, int64_t inner) {
+    return (p.batch == 1 || st[0] == heads * inner) && (heads == 1 || st[1] == inner);
+  };
+  return is(p.x_stride, h, kHeadDim) && is(p.a_stride, h, 1) && is(p.b_stride, g, n) && is(p.c_stride, g, n) &&
+         (!p.dt || is(p.dt_stride, h, 1)) && (!p.z || is(p.z_stride, h, kHeadDim));
+}
+
+template <typename T, int ROWS>
 int launch_step(const SsdStepArgs& p, cudaStream_t stream) {
-  auto go = [&](auto kern) { return launch(kern, 2 * p.batch * p.nheads, kStepThreads, 0, stream, p); };
+  // Half of the columns per CTA where that reaches more SMs, and for n = 64 and 128 (1024 heads, n 128, states in L2: 7.1 us, 7.6
+  // with all columns; from memory 12.7 and 12.4).  With fewer rows a CTA has too little to do (5120 heads, n 16: 9.8 and 8.2;
+  // n 32: 10.7 and 10.0, but strided 14.4 and 15.3), with more the loads of half the columns are enough in flight (20480
+  // heads, n 256: 393 and 388).
+  const int units = p.batch * p.nheads;
+  const bool d = dense(p), half = ROWS == 4 || ROWS == 8 || (ROWS == 2 && !d) || 2 * units <= 148;
+  if (d)
+    return half ? launch(ssd_step_kernel<T, ROWS, 32, true>, 2 * units, 128, 0, stream, p)
+                : launch(ssd_step_kernel<T, ROWS, 64, true>, units, 256, 0, stream, p);
+  return half ? launch(ssd_step_kernel<T, ROWS, 32, false>, 2 * units, 128, 0, stream, p)
+              : launch(ssd_step_kernel<T, ROWS, 64, false>, units, 256, 0, stream, p);
+}
+
+template <typename T>
+int launch_rows(const SsdStepArgs& p, cudaStream_t stream) {
   switch (p.dstate / 16) {
-    case 1: return go(ssd_step_kernel<T, 1>);
-    case 2: return go(ssd_step_kernel<T, 2>);
-    case 4: return go(ssd_step_kernel<T, 4>);
-    case 8: return go(ssd_step_kernel<T, 8>);
-    case 16: return go(ssd_step_kernel<T, 16>);
+    case 1: return launch_step<T, 1>(p, stream);
+    case 2: return launch_step<T, 2>(p, stream);
+    case 4: return launch_step<T, 4>(p, stream);
+    case 8: return launch_step<T, 8>(p, stream);
+    case 16: return launch_step<T, 16>(p, stream);
     default: return SSD_ERR_UNSUPPORTED;
   }
 }
@@ -119,9 +142,9 @@ extern "C" int ssd_b200_step_strided(const SsdStepArgs* p, void* stream) {
   if (reinterpret_cast<uintptr_t>(p->state) & 15) return SSD_ERR_MISALIGNED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (p->dtype) {
-    case SSD_DTYPE_F32: return ssd::launch_step<float>(*p, s);
-    case SSD_DTYPE_F16: return ssd::launch_step<__half>(*p, s);
-    case SSD_DTYPE_BF16: return ssd::launch_step<__nv_bfloat16>(*p, s);
+    case SSD_DTYPE_F32: return ssd::launch_rows<float>(*p, s);
+    case SSD_DTYPE_F16: return ssd::launch_rows<__half>(*p, s);
+    case SSD_DTYPE_BF16: return ssd::launch_rows<__nv_bfloat16>(*p, s);
     default: return SSD_ERR_UNSUPPORTED;
   }
 }
