@@ -210,7 +210,7 @@ def test_plan_of_the_benchmark_configurations(lib):
     assert _plan(lib, _shape(256, 512, 48, 64, 64, 8, 128, _lib.DTYPE_BF16)) == (TC, 1, 1)
     # config 0 is fp32: the CUDA-core recurrence
     assert _plan(lib, _shape(16, 128, 8, 64, 16, 8, 64, _lib.DTYPE_F32))[0] == SCAN
-    # odd heads per group cannot pair up: still the tensor-core family (one head per CTA)
+    # odd heads per group: the last pair of a group is half empty
     assert _plan(lib, _shape(2, 512, 3, 64, 128, 3, 128, _lib.DTYPE_F16))[0] == TC
 
 

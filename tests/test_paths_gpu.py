@@ -224,16 +224,17 @@ def test_what_pytorch_throws_in_the_binding_is_raised():
 
 @pytest.mark.parametrize("dtype,l,d", [(torch.float16, 1, 64), (torch.float16, 9, 128), (torch.bfloat16, 65, 64),
                                        (torch.float32, 5, 64), (torch.float32, 67, 192), (torch.bfloat16, 2050, 4096)])
-def test_conv_run_lengths(dtype, l, d):
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_conv_run_lengths(dtype, l, d, taps):
     """From a run shorter than a piece to the longest run, against the operator in fp64 (one rounding of the result, and
     tanh.approx for 16-bit types: 2^-8 of the largest value bounds both)."""
     import workloadsuite_b200 as W
 
     gen = torch.Generator().manual_seed(l)
     x = torch.randn(2, l, d, generator=gen).to(dtype)
-    w, bias = (torch.randn(d, 1, 4, generator=gen) * 0.5).to(dtype), torch.randn(d, generator=gen).to(dtype)
+    w, bias = (torch.randn(d, 1, taps, generator=gen) * 0.5).to(dtype), torch.randn(d, generator=gen).to(dtype)
     y = W.conv1d_silu(x.to(DEV), w.to(DEV), bias.to(DEV)).cpu().double()
-    c = torch.nn.functional.conv1d(x.double().transpose(1, 2), w.double(), bias.double(), padding=3, groups=d)[..., :l]
+    c = torch.nn.functional.conv1d(x.double().transpose(1, 2), w.double(), bias.double(), padding=taps - 1, groups=d)[..., :l]
     ref = torch.nn.functional.silu(c).transpose(1, 2)
     assert ((y - ref).abs().max() / ref.abs().max()).item() < (1e-5 if dtype == torch.float32 else 2 ** -8)
 

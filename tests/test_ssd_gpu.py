@@ -228,8 +228,8 @@ def test_chained_segments_tensor_core():
     assert torch.allclose(D.cpu().double(), O.total_logdecay(inp["A"]), rtol=1e-5, atol=1e-5)
 
 
-def test_one_head_per_cta_variant_when_groups_are_single_heads():
-    """Heads that do not pair up inside a B/C group (one head per group) take the single-head kernel."""
+def test_groups_of_single_heads():
+    """Heads that do not pair up inside a B/C group (one head per group): every pair is half empty."""
     if not _tc_available():
         pytest.skip("tensor-core kernel not available")
     inp = O.make_inputs(b=2, s=512, h=3, p=64, n=128, g=3, dtype=torch.float16, init=True, seed=22, decay_scale=0.05)

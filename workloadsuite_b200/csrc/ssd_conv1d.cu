@@ -344,7 +344,7 @@ int launch_conv(const void* x, const void* w, const void* bias, void* y, int bat
   T* yy = static_cast<T*>(y);
   if constexpr (sizeof(T) == 2) {
     if (al && taps >= 2 && taps <= 4) {
-      // a block per SM (b1 s4096 h32: 13.4 us with half a block's worth, 12.4 so; with two it is 18.0, the rows before the
+      // a block per SM (b1 s4096 h32 bf16: 12.8 us with half a block's worth, 11.8 so; with two it is 18.0, the rows before the
       // runs read again and a second round of blocks)
       const int len = in_place ? kLongestRun : run_length(kLongestRun, kPiece, columns, seqlen, 148 * 128);
       const int64_t tot = columns * ((seqlen + len - 1) / len);

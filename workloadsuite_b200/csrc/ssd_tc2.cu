@@ -22,7 +22,7 @@
 // What bounds it.  A 128xNx16 tcgen05.mma takes 62 cycles at N = 128 and 55 at N = 64 (any operand layout), so the
 // four contractions of a tile pair need 2 430 tensor-pipe cycles; HBM needs 2 800 cycles per SM for its 64 KB of X
 // and Y.  The loop that sets the period is A -> P.X -> S -> E -> A, which is
-// why Xd has other warps than P (with B in the warps of A, D and E a tile took 5 400 cycles).  Tensor memory (512 columns) is what limits overlap: G 128,
+// why Xd has other warps than P (a tile takes 5 200 to 5 500 cycles).  Tensor memory (512 columns) is what limits overlap: G 128,
 // Yo 128, Yd 128 and 128 columns that S and P take turns in -- S(t+1) is consumed (step E) before P(t+1) is written
 // (step A), and S(t+1) is issued once P.X(t) has read P(t).  Keeping Yo and Yd apart means that nothing has to be
 // scaled in place between C.H and P.X, and that C.H(t+1) and the reloads of B and C run under steps A, B and D.
@@ -1171,7 +1171,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 
 // The ready flags of a launch with cut sequences have to start at zero (the workspace keeps the call before's).  The forward
 // starts beside this kernel, which itself starts when all work before it in the stream is done, and asks for its end
-// (grid_dependency_wait) only where a flag is first used; a memset ahead of the forward cost 4 us of every such call.
+// (grid_dependency_wait) only where a flag is first used; a memset ahead of the forward cost 2.5 to 3.5 us of every such call.
 __global__ void clear_flags_kernel(int* flags) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   flags[threadIdx.x] = 0;
