@@ -46,9 +46,10 @@ enum { SSD_DTYPE_F32 = 0, SSD_DTYPE_F16 = 1, SSD_DTYPE_BF16 = 2 };
 /* kernel selection */
 enum {
   SSD_KERNEL_AUTO = 0,    /* tensor-core kernel when the shape allows and the sequence is whole tiles of 128 tokens,
-                             else the fp32 scan */
+                             else the fp32 scan, on the tensor cores (products of 16-bit pieces that hold fp32
+                             numbers) where the shape allows that */
   SSD_KERNEL_SCAN_F32 = 1,/* fp32 token recurrence on CUDA cores (any dtype in, fp32 math) */
-  SSD_KERNEL_TCGEN05 = 2  /* tcgen05/TMEM chunked kernel (f16/bf16 only, any length): many times faster than the scan,
+  SSD_KERNEL_TCGEN05 = 2  /* tcgen05/TMEM chunked kernel (f16/bf16 only, any length): faster than the scan,
                              but the masked products, the decayed X and the state's copy are rounded to 16 bits */
 };
 
@@ -138,7 +139,9 @@ const char* ssd_b200_kernel_name(const SsdArgs* args);
  * and the number of kernel launches it enqueues: 1 for whole sequences; 1 plus a clearing of flags
  * (a block that the launch overlaps) where the two-head tensor-core kernel deals the tiles of all
  * sequences out evenly inside one launch (states handed from CTA to CTA, or folded from the pairs each CTA publishes for the last piece of its range);
- * 3 for the two-pass segmented scan (2 with SSD_FLAG_STATE_ONLY or SSD_FLAG_REUSE_SEGMENTS).  Any out
+ * 1 more where the fp32 scan runs on the tensor cores (the recurrence behind it, which ends at once unless a number was
+ * not finite or a log-decay far above zero); 3 for the two-pass segmented scan (2 with SSD_FLAG_STATE_ONLY or
+ * SSD_FLAG_REUSE_SEGMENTS).  Any out
  * pointer may be NULL.  Returns SSD_OK or the validation error.  No reference counterpart. */
 int ssd_b200_plan(const SsdArgs* args, int32_t* kernel, int32_t* nsegments, int32_t* launches);
 

@@ -234,3 +234,55 @@ def test_host_pipeline_scratch_sizes(lib):
     assert 0 < small < big < (1 << 30)
     assert big >= 4 * 2 * (24 << 20) * 0.9            # X and Y of four 24 MiB chunks
     assert lib.ssd_b200_host_scratch_bytes(C.byref(_shape(2, 500, 8, 64, 64, 2, 128, _lib.DTYPE_BF16))) == 0   # ragged
+
+
+def test_route_of_the_fp32_scan(lib):
+    """Which calls of the fp32 scan run on the tensor cores (a word of scratch per SM and one more launch): 16-bit tensors whose
+    kernel and cuts the caller leaves open, of some length, that write nowhere near their inputs."""
+    redo, slots = 768, 2 * 148
+    chain = slots * 128 * 64 * 4 + 2 * 1280
+    need = lambda a: lib.ssd_b200_workspace_bytes(C.byref(a))
+
+    def shape(s=300, h=4, n=128, b=2, dtype=_lib.DTYPE_BF16, g=1):
+        return _shape(b, s, h, 64, n, g, 1, dtype)
+
+    for dtype in (_lib.DTYPE_BF16, _lib.DTYPE_F16):
+        assert need(shape(dtype=dtype)) == redo and _plan(lib, shape(dtype=dtype)) == (1, 1, 2)
+        assert need(shape(s=3001, h=80, dtype=dtype)) == chain + redo        # 160 heads: dealt out over the SMs
+    assert _plan(lib, shape(s=3001, h=80)) == (1, 2, 2)
+    assert [need(shape(s=s)) for s in (31, 32)] == [0, redo] and [need(shape(s=s, n=64)) for s in (63, 65)] == [0, redo]
+    assert [need(shape(s=s, h=80)) for s in (19, 20)] == [0, redo]              # more heads than SMs
+    assert need(shape(dtype=_lib.DTYPE_F32)) == _lib_two_pass(lib, shape(dtype=_lib.DTYPE_F32))
+    asked = shape()
+    asked.kernel = _lib.KERNEL_SCAN_F32
+    assert need(asked) == _lib_two_pass(lib, asked)
+    for field, value in (("nsegments", 2), ("flags", _lib.FLAG_STATE_ONLY), ("flags", _lib.FLAG_REUSE_SEGMENTS)):
+        a = shape()
+        setattr(a, field, value)
+        assert _plan(lib, a)[2] != 2 or a.flags, field
+        k = shape()
+        k.kernel = _lib.KERNEL_SCAN_F32
+        setattr(k, field, value)
+        assert (need(a), _plan(lib, a)) == (need(k), _plan(lib, k)), field
+    a = shape(h=160)      # whole sequences in the recurrence: no scratch
+    a.X, a.B, a.C, a.A, a.Y = 1 << 20, 1 << 30, 1 << 31, 1 << 32, 1 << 33
+    a.y_stride = a.x_stride
+    assert need(a) > 0
+    for where in (a.X, a.X + 2 * 300 * 160 * 64, a.B + 64, a.C - 64, a.A + 4096):
+        a.Y = where
+        assert need(a) == 0
+    a.Y = 1 << 33
+    a.initial_state, a.final_state = 1 << 34, 1 << 35
+    assert need(a) > 0
+    a.final_state = a.initial_state
+    assert need(a) == 0
+    a.final_state = (1 << 35) + 4            # the recurrence takes states that are not 16-byte aligned
+    assert need(a) == 0
+
+
+def _lib_two_pass(lib, a):
+    _, nseg, launches = _plan(lib, a)
+    assert launches == (3 if nseg > 1 else 1)
+    units = a.batch * a.nheads
+    up = lambda v: (v + 255) // 256 * 256
+    return 0 if nseg == 1 else 2 * up(units * nseg * a.dstate * a.headdim * 4) + up(units * nseg * 4)

@@ -298,3 +298,86 @@ def test_host_pipeline_chunks_and_sets(b, s, h, n):
     out, fin = torch.empty_like(inp["X"]), torch.empty(b, h, n, 64)
     r.run(inp["X"], inp["A"], inp["B"], inp["C"], out, initial_states=inp["initial_states"], final_state=fin)
     assert max(O.error_metrics(out, Y.cpu())) < 2e-2 and max(O.error_metrics(fin, H.cpu())) < 2e-2
+
+
+@pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -11)])
+@pytest.mark.parametrize("b,s,h,g,n,nsegments", [(2, 33, 3, 1, 128, 1), (2, 127, 4, 2, 64, 1), (1, 129, 4, 1, 128, 1), (3, 500, 4, 4, 64, 1),
+                                                 (50, 300, 6, 2, 128, None), (1, 3001, 5, 1, 64, None), (1, 4700, 2, 1, 128, None)],
+                         ids=["one_tile", "tile_less_one", "tile_plus_one", "whole", "chained", "lookback", "lookback_37_tiles"])
+def test_fp32_scan_on_the_tensor_cores(b, s, h, g, n, nsegments, dtype, eps):
+    """Products of 16-bit pieces that hold fp32 numbers: Y is off by its own rounding (eps of the value at most) and the fp32
+    sums' 1e-5, as with the recurrence; the state, a sum over the tokens that decay leaves (tens), by four units of 2^-24.
+    Columns of a wider tensor, as a projection's output has them, and every output of the call."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=g, dtype=dtype, init=True, seed=80 + s, decay_scale=0.1)
+    inp["A"].neg_().abs_().neg_()
+    dt = (0.01 + 0.2 * torch.rand(b, s, h, generator=torch.Generator().manual_seed(s))).to(dtype)
+    wide = torch.cat([inp["B"].flatten(2), inp["X"].flatten(2), inp["C"].flatten(2)], dim=-1).to(DEV)
+    B, X, C = torch.split(wide, [g * n, h * 64, g * n], dim=-1)
+    X, B, C = X.unflatten(-1, (h, 64)), B.unflatten(-1, (g, n)), C.unflatten(-1, (g, n))
+    plan = W.plan(X, inp["A"].to(DEV), B, C, 1, nsegments=nsegments)
+    assert plan["kernel"] == "scan_f32" and plan["launches"] == 2
+    Y, H, ld = W.ssd_forward(X, inp["A"].to(DEV), B, C, 1, dt=dt.to(DEV), initial_states=inp["initial_states"].to(DEV),
+                             return_final_state=True, return_logdecay=True, nsegments=nsegments)
+    Yr, Hr = O.ssd_recurrence(inp["X"], inp["A"], inp["B"], inp["C"], dt=dt, initial_states=inp["initial_states"],
+                              return_final_state=True)
+    assert ((Y.cpu().double() - Yr).abs() <= eps * Yr.abs() + 1e-5 * Yr.abs().max()).all()
+    assert ((H.cpu().double() - Hr).norm() / Hr.norm()).item() < 4 * 2 ** -24
+    total = inp["A"].double().sum(1)
+    assert ((ld.cpu().double() - total).abs() <= 2 ** -24 * total.abs()).all()      # summed in 64 bits, rounded once
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("b,s,h,n", [(2, 300, 4, 128), (1, 3001, 8, 64), (50, 300, 6, 128)], ids=["whole", "lookback", "chained"])
+@pytest.mark.parametrize("what", ["x_nan", "x_inf", "b_inf", "c_nan", "a_nan", "growth", "state_inf", "overflow"])
+def test_what_the_tensor_cores_cannot_do_at_fp32_is_the_recurrence_s(what, b, s, h, n, dtype):
+    """Numbers that are not finite (which must not reach tokens before their own), log-decays above zero, and what overflows
+    in fp16 pieces: bit by bit what the recurrence gives."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=1, dtype=dtype, init=True, seed=81, decay_scale=0.1)
+    X, A, B, C, init = (inp[k] for k in ("X", "A", "B", "C", "initial_states"))
+    if what == "x_nan":
+        X[0, 150, 1, 3] = float("nan")
+    elif what == "x_inf":
+        X[0, 150, 1, 3] = float("inf")
+    elif what == "b_inf":
+        B[0, 150, 0, 3] = -float("inf")
+    elif what == "c_nan":
+        C[0, 150, 0, 3] = float("nan")
+    elif what == "a_nan":
+        A[0, 150, 1] = float("nan")
+    elif what == "growth":
+        A[0, 100:130, 1] = 1.5
+    elif what == "state_inf":
+        init[0, 1, 5, 5] = float("inf")
+    elif what == "overflow":
+        if dtype == torch.bfloat16:
+            pytest.skip("bf16 has the range of fp32")
+        X.mul_(8000)
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    run = lambda **kw: W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, initial_states=d["initial_states"],
+                                     return_final_state=True, **kw)
+    for got, want in zip(run(), run(kernel="scan_f32", nsegments=1)):
+        assert torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)) and torch.equal(got.isnan(), want.isnan())
+
+
+def test_scratch_of_calls_on_two_streams_is_their_own():
+    import workloadsuite_b200 as W
+
+    sets = [{k: v.to(DEV) for k, v in O.make_inputs(b=2, s=3001, h=80, p=64, n=128, g=1, dtype=torch.bfloat16, seed=83 + i,
+                                                    decay_scale=0.1).items()} for i in range(2)]
+    run = lambda d: W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, return_final_state=True)
+    want = [run(d) for d in sets]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(8):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[i].append(run(sets[i]))
+    torch.cuda.synchronize()
+    for i in range(2):
+        for Y, H in got[i]:
+            assert torch.equal(Y, want[i][0]) and torch.equal(H, want[i][1])

@@ -86,7 +86,7 @@ def source_fingerprint() -> str:
     the compiler flags: what an ncu summary of that kernel must have been captured from to describe the kernel that
     runs now."""
     h = hashlib.sha256()
-    for name in ("ssd_tc2.cu", "tc_common.cuh", "tc_ptx.cuh", "ssd_common.cuh"):
+    for name in ("ssd_tc2.cu", "tile_walk.cuh", "tc_common.cuh", "tc_ptx.cuh", "ssd_common.cuh"):
         h.update(name.encode())
         h.update((CSRC / name).read_bytes())
     h.update(" ".join(NVCC_FLAGS).encode())

@@ -53,15 +53,55 @@ int resolve_kernel(const SsdArgs* a) {
   return ssd::tc_supports(*a) && st16 && a->seqlen % kTcTile == 0 ? SSD_KERNEL_TCGEN05 : SSD_KERNEL_SCAN_F32;
 }
 
-int tile_tokens(int kernel) { return kernel == SSD_KERNEL_TCGEN05 ? kTcTile : ssd::scan_f32_tile_tokens(); }
+// First and one past the last byte of a tensor's elements.
+void extent(const void* p, const int64_t* st, int n0, int n1, int n2, int inner, int size, uintptr_t* lo, uintptr_t* hi) {
+  *lo = reinterpret_cast<uintptr_t>(p);
+  *hi = *lo + (uintptr_t)(((n0 - 1) * st[0] + (n1 - 1) * st[1] + (n2 - 1) * st[2] + inner) * size);
+}
+
+// Whether an output may share memory with an input: a call that is done again (below) needs its inputs as they were.
+bool outputs_on_inputs(const SsdArgs* a) {
+  if (a->initial_state && a->final_state) {
+    const int64_t bytes = (int64_t)a->batch * a->nheads * a->dstate * a->headdim * 4;
+    const intptr_t d = reinterpret_cast<intptr_t>(a->final_state) - reinterpret_cast<intptr_t>(a->initial_state);
+    if (d < bytes && -d < bytes) return true;
+  }
+  if (!a->Y) return false;
+  uintptr_t y0, y1, x0, x1;
+  extent(a->Y, a->y_stride, a->batch, a->seqlen, a->nheads, a->headdim, 2, &y0, &y1);
+  auto on = [&](const void* p, const int64_t* st, int groups, int inner, int size) {
+    if (!p) return false;
+    extent(p, st, a->batch, a->seqlen, groups, inner, size, &x0, &x1);
+    return x0 < y1 && y0 < x1;
+  };
+  return on(a->X, a->x_stride, a->nheads, a->headdim, 2) || on(a->B, a->b_stride, a->ngroups, a->dstate, 2) ||
+         on(a->C, a->c_stride, a->ngroups, a->dstate, 2) || on(a->dt, a->dt_stride, a->nheads, 1, 2) ||
+         on(a->A, a->a_stride, a->nheads, 1, 4);
+}
+
+// The fp32 scan of a call whose kernel is not chosen by the caller: on the tensor cores at fp32 precision where they can
+// (ssd_split.cu), unless the sequences are so short that the recurrence is through before the other kernel's pipeline has
+// filled.  Its time goes with tokens x state, bf16: 8 heads of 17, 33 and 100 tokens, n 128: 8.5, 13.6 and 33 us, there 9.3, 9.4
+// and 9.7; n 64: 5.8, 8.9 and 19, there 8.5, 8.5 and 8.8.  With more heads than SMs it falls behind earlier: 1 280 of 17 and 33,
+// n 128: 54 and 99 us, there 38 and 39; n 64: 29 and 54, there 35 and 36.
+bool use_split(const SsdArgs* a, int kernel) {
+  const int64_t least = (int64_t)a->batch * a->nheads > kSmCount ? 2560 : 4096;
+  return kernel == SSD_KERNEL_SCAN_F32 && (int64_t)a->seqlen * a->dstate >= least && a->kernel == SSD_KERNEL_AUTO && a->nsegments <= 1 &&
+         !(a->flags & (SSD_FLAG_STATE_ONLY | SSD_FLAG_REUSE_SEGMENTS)) && aligned16(a->initial_state) && aligned16(a->final_state) &&
+         ssd::split_supports(*a) && !outputs_on_inputs(a);
+}
+
+// What the kernels that run these arguments work on: pairs of heads, or heads.
+int64_t tc_units(const SsdArgs* a, bool split) { return split ? (int64_t)a->batch * a->nheads : ssd::tc2_units(*a); }
 
 // Number of independently scanned segments per sequence and their length.
-void resolve_segments(const SsdArgs* a, int kernel, int* nseg, int* seg_len) {
-  const int tile = tile_tokens(kernel);
+void resolve_segments(const SsdArgs* a, int kernel, bool split, int* nseg, int* seg_len) {
+  const bool tensor = split || kernel == SSD_KERNEL_TCGEN05;
+  const int tile = tensor ? kTcTile : ssd::scan_f32_tile_tokens();
   int want = a->nsegments;
   if (want <= 0) {
-    if (kernel == SSD_KERNEL_TCGEN05) {
-      want = ssd::tc2_default_segments(*a);
+    if (tensor) {
+      want = ssd::tc_default_segments(*a, tc_units(a, split));
     } else {
       const int64_t units = (int64_t)a->batch * a->nheads;
       // Two passes cost about 1.5x the work of one, so split only when the
@@ -77,6 +117,14 @@ void resolve_segments(const SsdArgs* a, int kernel, int* nseg, int* seg_len) {
   *seg_len = len;
   *nseg = (a->seqlen + len - 1) / len;
 }
+
+int chain_mode(const SsdArgs* a, int kernel, bool split, int nseg) {
+  return split || kernel == SSD_KERNEL_TCGEN05 ? ssd::tc_chain_mode(*a, nseg, tc_units(a, split)) : 0;
+}
+
+// Scratch of a launch that hands states from CTA to CTA: one slot per CTA and head of the pair -- state, log-decay sum, ready flag.
+constexpr size_t kSlots = 2 * (size_t)kSmCount;
+size_t chain_bytes(size_t np) { return align_up(kSlots * np * sizeof(float), 256) + 2 * align_up(kSlots * sizeof(float), 256); }
 
 bool strides_mult(const int64_t* s, int m) { return s[0] % m == 0 && s[1] % m == 0 && s[2] % m == 0; }
 
@@ -151,15 +199,17 @@ int ssd_b200_plan(const SsdArgs* args, int32_t* kernel_out, int32_t* nsegments_o
   const int rc = validate(args);
   if (rc != SSD_OK) return rc;
   const int kernel = resolve_kernel(args);
+  const bool split = use_split(args, kernel);
   int nseg, seg_len;
-  resolve_segments(args, kernel, &nseg, &seg_len);
+  resolve_segments(args, kernel, split, &nseg, &seg_len);
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
   int launches = 1;
   if (nseg > 1) {
-    const bool chained = kernel == SSD_KERNEL_TCGEN05 && ssd::tc2_chain_mode(*args, nseg) != 0;
+    const bool chained = chain_mode(args, kernel, split, nseg) != 0;
     launches = chained ? 1 : (state_only ? 2 : 3);
     if (!chained && (args->flags & SSD_FLAG_REUSE_SEGMENTS)) launches -= 1;
   }
+  if (split) launches += 1;   // (the scan that does the call again where it has to)
   if (kernel_out) *kernel_out = kernel;
   if (nsegments_out) *nsegments_out = nseg;
   if (launches_out) *launches_out = launches;
@@ -169,16 +219,14 @@ int ssd_b200_plan(const SsdArgs* args, int32_t* kernel_out, int32_t* nsegments_o
 size_t ssd_b200_workspace_bytes(const SsdArgs* args) {
   if (validate(args) != SSD_OK) return 0;
   const int kernel = resolve_kernel(args);
+  const bool split = use_split(args, kernel);
   int nseg, seg_len;
-  resolve_segments(args, kernel, &nseg, &seg_len);
-  if (nseg <= 1) return 0;
+  resolve_segments(args, kernel, split, &nseg, &seg_len);
+  const size_t redo = split ? align_up(kSmCount * sizeof(int32_t), 256) : 0;   // a word per CTA
+  if (nseg <= 1) return redo;
   const size_t units = (size_t)args->batch * args->nheads;
   const size_t np = (size_t)args->dstate * args->headdim;
-  if (kernel == SSD_KERNEL_TCGEN05 && ssd::tc2_chain_mode(*args, nseg) != 0) {
-    // chained / look-back mode: one slot per CTA and head of the pair -- state, log-decay sum, ready flag
-    const size_t slots = 2 * (size_t)kSmCount;
-    return align_up(slots * np * sizeof(float), 256) + 2 * align_up(slots * sizeof(float), 256);
-  }
+  if (chain_mode(args, kernel, split, nseg) != 0) return chain_bytes(np) + redo;
   // two passes: zero-start segment states, states entering the segments, segment log-decay sums
   return 2 * align_up(units * nseg * np * sizeof(float), 256) + align_up(units * nseg * sizeof(float), 256);
 }
@@ -197,8 +245,9 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
   if (kernel == SSD_KERNEL_SCAN_F32 && !ssd::scan_f32_supports(args->headdim, args->dstate))
     return SSD_ERR_UNSUPPORTED;
 
+  const bool split = use_split(args, kernel);
   int nseg, seg_len;
-  resolve_segments(args, kernel, &nseg, &seg_len);
+  resolve_segments(args, kernel, split, &nseg, &seg_len);
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
   const int64_t units = (int64_t)args->batch * args->nheads;
   const int64_t np = (int64_t)args->dstate * args->headdim;
@@ -208,45 +257,44 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
   prm.seg_len = seg_len;
   prm.nseg = nseg;
   if (!fuse_epilogue || state_only) prm.D = nullptr, prm.Z = nullptr;
-
-  if (nseg <= 1) {
-    prm.compute_y = state_only ? 0 : 1;
-    prm.init = args->initial_state;
-    prm.init_unit_stride = np;
-    prm.fin = args->final_state;
-    prm.fin_unit_stride = np;
-    prm.fin_ld = args->final_logdecay;
-    prm.finld_unit_stride = 1;
-    return launch_kernel(kernel, args, prm, stream);
-  }
+  // whole sequences, or pieces of them within one launch: the caller's states and sums directly
+  ssd::ScanParams whole = prm;
+  whole.compute_y = state_only ? 0 : 1;
+  whole.init = args->initial_state;
+  whole.init_unit_stride = np;
+  whole.fin = args->final_state;
+  whole.fin_unit_stride = np;
+  whole.fin_ld = args->final_logdecay;
+  whole.finld_unit_stride = 1;
+  if (nseg <= 1 && !split) return launch_kernel(kernel, args, whole, stream);
 
   const size_t need = ssd_b200_workspace_bytes(args);
   if (!args->workspace || args->workspace_bytes < need) return SSD_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(args->workspace) & 255) return SSD_ERR_MISALIGNED;
-  const int chain_mode = kernel == SSD_KERNEL_TCGEN05 ? ssd::tc2_chain_mode(*args, nseg) : 0;
-  if (chain_mode != 0) {
-    // one launch: the pieces of a sequence pass their state through the workspace, one slot per CTA and head
-    const size_t slots = 2 * (size_t)kSmCount;
+  const int chain = chain_mode(args, kernel, split, nseg);
+  if (chain != 0 || split) {
+    // one launch: the pieces of a sequence pass their state through the workspace (see chain_bytes())
     char* ws = static_cast<char*>(args->workspace);
-    float* slot_state = reinterpret_cast<float*>(ws);
-    float* slot_ld = reinterpret_cast<float*>(ws + align_up(slots * np * sizeof(float), 256));
-    int32_t* flags = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(slot_ld) + align_up(slots * sizeof(float), 256));   // (cleared by the launch)
-    ssd::ScanParams pc = prm;
-    pc.compute_y = state_only ? 0 : 1;
-    pc.chain = chain_mode;
-    pc.chain_state = slot_state;
-    pc.chain_ld = slot_ld;
-    pc.chain_flag = flags;
-    pc.init = args->initial_state;   // only read by the first segment
-    pc.init_unit_stride = np;
-    pc.init_seg_stride = 0;
-    pc.fin = args->final_state;      // only written by the last segment
-    pc.fin_unit_stride = np;
-    pc.fin_seg_stride = 0;
-    pc.fin_ld = args->final_logdecay;
-    pc.finld_unit_stride = 1;
-    pc.finld_seg_stride = 0;
-    return launch_kernel(kernel, args, pc, stream);
+    ssd::ScanParams pc = whole;
+    if (chain != 0) {
+      pc.chain = chain;
+      pc.chain_state = reinterpret_cast<float*>(ws);
+      pc.chain_ld = reinterpret_cast<float*>(ws + align_up(kSlots * np * sizeof(float), 256));
+      pc.chain_flag = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(pc.chain_ld) + align_up(kSlots * sizeof(float), 256));   // (cleared by the launch)
+      ws += chain_bytes(np);
+    }
+    if (!split) return launch_kernel(kernel, args, pc, stream);
+    pc.redo = reinterpret_cast<int32_t*>(ws);
+    rc = ssd::launch_split(*args, pc, stream);
+    whole.nseg = 1;
+    whole.seg_len = (int)align_up(args->seqlen, ssd::scan_f32_tile_tokens());
+    if (rc == SSD_OK) {
+      whole.redo = pc.redo;
+      whole.redo_n = ssd::split_grid(*args, chain);
+    } else if (rc != SSD_ERR_UNSUPPORTED) {
+      return rc;
+    }
+    return ssd::launch_scan_f32(whole, args->dtype, stream);
   }
 
   float* seg_states = static_cast<float*>(args->workspace);

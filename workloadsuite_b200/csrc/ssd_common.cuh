@@ -51,6 +51,10 @@ struct ScanParams {
   float* chain_state;     // [slot][p/4][n][4], slot = 2 * CTA + head of the pair
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], cleared by the launch
+  // The tensor-core kernel at fp32 precision writes a word per CTA: not 0 if the fp32 scan has to do the call again.  The scan, when
+  // given them (redo_n of them), starts beside that kernel's end and leaves at once if all are 0.
+  int32_t* redo;
+  int redo_n;
   // Optional epilogue Y <- (Y + x * D[head]) * silu(z) (model_ref.py:116-118); either pointer may be null.
   const float* D;         // [h], fp32 or (d_in_dtype) elements of the tensors' type
   const void* Z;          // [b,s,h,p], strides zs
@@ -84,6 +88,22 @@ inline int launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
 }
 
+// The same for a kernel that may start beside the end of the one ahead, and waits for that end itself.
+template <typename... Params, typename... Args>
+inline int launch_early(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+}
+
 // D[head] of the skip term.
 template <typename T>
 __device__ __forceinline__ float load_skip(const ScanParams& p, int head) {
@@ -108,9 +128,16 @@ int launch_fold(const float* states, int64_t st_unit_stride, int64_t st_seg_stri
 // tensor-core kernel (ssd_tc2.cu)
 bool tc_supports(const SsdArgs& a);
 bool tc2_fuses_epilogue(const SsdArgs& a);
-int tc2_default_segments(const SsdArgs& a);
-int tc2_chain_mode(const SsdArgs& a, int nseg);   // 1: chained, 2: look-back (one launch each); 0: two passes + fold
+int64_t tc2_units(const SsdArgs& a);   // pairs of heads
+int tc_default_segments(const SsdArgs& a, int64_t units);
+int tc_chain_mode(const SsdArgs& a, int nseg, int64_t units);   // 1: chained, 2: look-back (one launch each); 0: two passes + fold
 int launch_tc2(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);
+int launch_clear_flags(int32_t* flags, int count, cudaStream_t stream);   // to zero, beside what is launched next
+
+// tensor-core kernel at fp32 precision (ssd_split.cu)
+bool split_supports(const SsdArgs& a);
+int split_grid(const SsdArgs& a, int chain);   // CTAs, each of which writes its word of ScanParams::redo
+int launch_split(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);   // SSD_ERR_UNSUPPORTED: nothing was enqueued
 
 
 }  // namespace ssd

@@ -139,6 +139,26 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
   float* dec = Ys + tile * P;        // [tile]  exp(a_t)
   float* araw = dec + tile;          // [tile]  a_t
 
+  if (prm.redo) {   // only if the kernel ahead says so
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int any = 0;
+    for (int i = threadIdx.x; i < prm.redo_n; i += kThreads) any |= __ldcg(prm.redo + i);
+    if (!__syncthreads_or(any)) {   // (that kernel leaves the sum of the log-decays to this one: in 64 bits, as below)
+      if (!prm.fin_ld) return;
+      const float* A = prm.A + (int64_t)(blockIdx.x / prm.nheads) * prm.as[0] + (int64_t)(blockIdx.x % prm.nheads) * prm.as[2];
+      double sum = 0.0;
+      for (int t = threadIdx.x; t < prm.seqlen; t += kThreads) sum += (double)A[(int64_t)t * prm.as[1]];
+      for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      double* part = reinterpret_cast<double*>(smem);
+      if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < kThreads / 32; ++w) sum += part[w];
+        prm.fin_ld[(int64_t)blockIdx.x * prm.finld_unit_stride] = (float)sum;
+      }
+      return;
+    }
+  }
   const int unit = blockIdx.x;
   const int seg = blockIdx.y;
   const int bi = unit / prm.nheads, hi = unit - bi * prm.nheads;
@@ -358,7 +378,7 @@ int launch_one(const ScanParams& prm, cudaStream_t stream) {
       return SSD_ERR_CUDA;
   }
   dim3 grid((unsigned)(prm.batch * prm.nheads), (unsigned)prm.nseg);
-  return launch(kern, grid, kThreads, smem, stream, prm, tile);
+  return prm.redo ? launch_early(kern, grid, kThreads, smem, stream, prm, tile) : launch(kern, grid, kThreads, smem, stream, prm, tile);
 }
 
 template <typename T, int P>

@@ -36,6 +36,7 @@
 #include "ssd_common.cuh"
 #include "tc_common.cuh"
 #include "tc_ptx.cuh"
+#include "tile_walk.cuh"
 
 namespace ssd {
 namespace {
@@ -44,7 +45,7 @@ using namespace ptx;
 using namespace tc;
 
 constexpr int kThreads2 = 512;
-constexpr int kSms = 148;
+using Cursor = CursorOf<2>;
 
 template <int N>
 struct Layout2 {
@@ -61,32 +62,6 @@ struct Layout2 {
   static constexpr int oMisc = oH + 2 * N * 128;
   static constexpr int kMiscBytes = 16384;
   static constexpr int kBytes = oMisc + kMiscBytes;   // no slack: the dynamic segment must start 1024-byte aligned
-};
-
-// Work list of this CTA.
-//  - Regular mode: items blockIdx.x, blockIdx.x + gridDim.x, ... of the (segment, sequence) grid.
-//  - Chained mode (sp.chain == 1): all tiles of all sequences, laid end to end, are cut into gridDim.x equal
-//    ranges, so every CTA gets the same number of tiles (+-1) whatever the number of sequences.  A range holds
-//    the tail of one sequence, whole sequences and the head of another; they are walked in reverse, head first:
-//    the head's state is what the next CTA's tail piece waits for, and a tail piece (walked last) then finds
-//    the state it needs already there when there is at least one sequence per CTA.
-//  - Look-back mode (sp.chain == 2), for fewer sequences than CTAs: the same even cut, but a piece cannot wait
-//    for the full scan of the piece before it (the pieces of one sequence would run one after the other).
-//    Instead every CTA first scans the LAST piece of its range from a zero state, state and log-decay sum only
-//    (item 0, skipped when that piece ends its sequence), and publishes the pair.  Then it walks its pieces like
-//    the chained mode; a piece that starts inside a sequence folds the published pairs of the CTAs before it, back
-//    to the one that holds the sequence's first tile (the recurrence is linear: H_in = sum_c exp(sum of the
-//    log-decays after c) F_c), skipping those whose decay factor has underflowed.
-// Computed once per CTA (thread 0, into shared memory): the 64-bit divisions are bulky code.
-struct Work {
-  int total;            // tiles of all items
-  int npre;             // the first npre of them produce a state only
-  int lo, hi, nt, first;   // chained modes: global tile range, tiles per sequence, first tile of item 0's sequence
-  int from;             // look-back mode: the CTA that holds the first tile of the range's first sequence
-  int hpg, ppg;         // heads per B/C group, head pairs per group
-  // item 0 as (pair of the group, group, batch entry, segment), and the step from one item to the next in the same
-  // mixed-radix digits: the walk needs no division
-  int d0[4], step[4];
 };
 
 // Factors of one tile of one head, written by the prefix-sum warp.
@@ -142,188 +117,6 @@ struct Misc2 {
 static_assert(sizeof(Misc2) <= Layout2<128>::kMiscBytes, "Misc2 outgrew its shared-memory slot");
 static_assert(Layout2<128>::kBytes <= 232448 && Layout2<64>::kBytes <= 232448, "shared memory budget of one SM exceeded");
 
-struct Tc2Params {
-  ScanParams sp;
-  int nitems;   // upairs * nseg
-  int upairs;   // batch * head pairs
-  int ppg;      // head pairs per B/C group
-  int st32;     // the states that enter and leave start on 32-byte boundaries
-};
-
-// Item `i` of the (segment, batch, group, pair) grid as digits.
-__device__ __forceinline__ void digits(int i, const Tc2Params& prm, int (&d)[4]) {
-  d[0] = i % prm.ppg; i /= prm.ppg;
-  d[1] = i % prm.sp.ngroups; i /= prm.sp.ngroups;
-  d[2] = i % prm.sp.batch; d[3] = i / prm.sp.batch;
-}
-
-__device__ __forceinline__ void work_list(const Tc2Params& prm, Work& wk) {
-  const ScanParams& sp = prm.sp;
-  wk.nt = (sp.seqlen + T - 1) / T;
-  wk.hpg = sp.nheads / sp.ngroups;
-  wk.ppg = prm.ppg;
-  wk.npre = sp.compute_y ? 0 : 0x7fffffff;
-  wk.lo = wk.hi = wk.first = wk.from = 0;
-  if (sp.chain) {
-    const long long total = (long long)prm.upairs * wk.nt;
-    wk.lo = (int)((long long)blockIdx.x * total / gridDim.x);
-    wk.hi = (int)((long long)(blockIdx.x + 1) * total / gridDim.x);
-    wk.total = wk.hi - wk.lo;
-    const int last = (wk.hi - 1) / wk.nt;     // (every CTA has at least one tile)
-    wk.first = last * wk.nt;
-    if (sp.chain == 2 && wk.hi % wk.nt != 0) {
-      wk.npre = wk.hi - max(wk.lo, wk.first);
-      wk.total += wk.npre;
-    }
-    // the largest c with lo(c) <= first tile of the range's first sequence
-    const int first = wk.lo / wk.nt * wk.nt;
-    int c = (int)((((long long)first + 1) * gridDim.x - 1) / total);
-    while (c > 0 && (long long)c * total / gridDim.x > first) --c;
-    while ((long long)(c + 1) * total / gridDim.x <= first) ++c;
-    wk.from = c;
-    digits(last, prm, wk.d0);
-    wk.step[0] = -1;
-    wk.step[1] = wk.step[2] = wk.step[3] = 0;
-  } else {
-    wk.total = 0;
-    for (int i = blockIdx.x; i < prm.nitems; i += gridDim.x) {
-      const int t = i / prm.upairs * sp.seg_len;
-      wk.total += (min(sp.seqlen, t + sp.seg_len) - t + T - 1) / T;
-    }
-    digits(blockIdx.x, prm, wk.d0);
-    digits(gridDim.x, prm, wk.step);
-  }
-}
-
-// Walks the tiles of all items of this CTA, in order.  An item is a run of `ntiles` tiles of one (batch, head pair)
-// sequence from token t_begin on.
-struct Cursor {
-  int t0, left;           // first token of the current tile, tiles of the item after it
-  int t_begin, ntiles;
-  int q, g, b, seg;       // pair of the group, group, batch entry, segment
-  int first;              // chained modes: first tile of the sequence in the laid-out order
-  int item;
-  __device__ __forceinline__ Cursor() : left(0), item(-1) {}
-  __device__ __forceinline__ void next(const Tc2Params& prm, const Work& wk) {
-    if (__builtin_expect(left > 0, 1)) {
-      --left;
-      t0 += T;
-      return;
-    }
-    const ScanParams& sp = prm.sp;
-    if (++item == 0) {
-      q = wk.d0[0]; g = wk.d0[1]; b = wk.d0[2]; seg = wk.d0[3];
-      first = wk.first;
-    } else if (!(item == 1 && sp.chain == 2 && wk.npre > 0)) {   // (after the state-only scan: the same piece again)
-      first -= wk.nt;
-      int c = 0;
-      q += wk.step[0];
-      if (q >= prm.ppg) { q -= prm.ppg; c = 1; }
-      if (q < 0) { q += prm.ppg; c = -1; }
-      g += wk.step[1] + c;
-      c = 0;
-      if (g >= sp.ngroups) { g -= sp.ngroups; c = 1; }
-      if (g < 0) { g += sp.ngroups; c = -1; }
-      b += wk.step[2] + c;
-      c = 0;
-      if (b >= sp.batch) { b -= sp.batch; c = 1; }
-      seg += wk.step[3] + c;
-    }
-    if (sp.chain) {
-      const int start = max(wk.lo, first), end = min(wk.hi, first + wk.nt);
-      t_begin = (start - first) * T;
-      ntiles = end - start;
-    } else {
-      t_begin = seg * sp.seg_len;
-      ntiles = (min(sp.seqlen, t_begin + sp.seg_len) - t_begin + T - 1) / T;
-    }
-    t0 = t_begin;
-    left = ntiles - 1;
-  }
-  __device__ __forceinline__ bool first_tile() const { return left == ntiles - 1; }
-  __device__ __forceinline__ int head(const Work& wk) const { return g * wk.hpg + 2 * q; }   // first of the pair
-  __device__ __forceinline__ bool live(const Work& wk, int h) const { return 2 * q + h < wk.hpg; }
-};
-
-// Waits.  Instructions are what this kernel is short of: a scheduler's own instruction cache holds a few KB, and code
-// that streams past it from the SM's (about 24 KB) arrives at 2.7 cycles per instruction, past that one at five to ten.
-// So a wait is only "until the phase is over, or the CTA has given up", and one thread -- the TMA producer, whose waits
-// depend on everybody's progress -- holds the clock (guarded_wait).  A role that was released that way runs through
-// its remaining tiles without waiting, on whatever is in the buffers, and leaves.
-// (The phase before a fresh barrier's first counts as over: the parity of "free" in the first round.)
-__device__ __forceinline__ void wait_at(uint32_t bar, uint32_t parity, const Misc2* m) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .u32 a;\n"
-      "AGAIN:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra DONE;\n\t"
-      "ld.volatile.shared.u32 a, [%2];\n\tsetp.eq.u32 p, a, 0;\n\t@p bra AGAIN;\n"
-      "DONE:\n\t}"
-      ::"r"(bar), "r"(parity), "r"(smem_u32(const_cast<int*>(&m->abort_flag)))
-      : "memory");
-}
-__device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, const Misc2* m) { wait_at(smem_u32(bar), parity, m); }
-// False when the CTA has given up; gives up with `code` when the bound runs out (twice that of the wait for another
-// CTA's hand-over: everything inside the CTA may be waiting behind that one, and the cause should be what reports).
-__device__ __forceinline__ bool guarded_wait(uint64_t* bar, uint32_t parity, Misc2* m, int code) {
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (m->abort_flag) return false;
-    if (clock64() - t0 > 2 * m->wait_clocks) {
-      m->abort_flag = code;   // reported to the caller's status word at kernel end
-      return false;
-    }
-  }
-  return m->abort_flag == 0;
-}
-// (the same for all lanes of the warp)
-__device__ __forceinline__ bool given_up(const Misc2* m) { return __any_sync(0xffffffffu, m->abort_flag != 0) != 0; }
-
-__device__ __forceinline__ bool elect_one() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
-  return r != 0;
-}
-
-// Products of fp32 pairs (one instruction for two elements).
-__device__ __forceinline__ uint64_t pair(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t pair(uint32_t a, uint32_t b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpair(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-template <typename T16>
-__device__ __forceinline__ uint32_t pack_pair(uint64_t v) {
-  const float2 f = unpair(v);
-  return pack2<T16>(f.x, f.y);
-}
-
-// 32 bytes per thread (a whole sector: a thread's row of the state would otherwise be moved half a sector at a time, and
-// the load/store unit takes a cycle per sector touched).
-__device__ __forceinline__ void ldg256(const void* p, uint64_t (&v)[4]) {
-  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
-}
-__device__ __forceinline__ void stg256(void* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
-  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
-}
-
 // B. Xd = exp(cs_last - cs_l) * dt * x (model_ref.py:144,148) of rows 32 q .. 32 q + 31, in packed 16-bit arithmetic as the
 // reference does it (WIDE: in fp32, rounded once).  Eight lanes share a row (one 16-byte piece each), a warp moves four rows
 // per instruction.
@@ -367,7 +160,7 @@ template <typename T16, int N, bool EPI, bool WIDE>
 __global__ void __launch_bounds__(kThreads2, 1)
 ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY,
-               const Tc2Params prm) {
+               const TileParams prm) {
   using L = Layout2<N>;
   constexpr int NB = L::NB;
   constexpr int KN = N / 16;
@@ -1179,34 +972,14 @@ __global__ void clear_flags_kernel(int* flags) {
 
 template <typename T16, int N, bool EPI, bool WIDE>
 int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& ty,
-                  const Tc2Params& prm, cudaStream_t stream) {
+                  const TileParams& prm, cudaStream_t stream) {
   auto kern = ssd_tc2_kernel<T16, N, EPI, WIDE>;
   constexpr int smem = Layout2<N>::kBytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return SSD_ERR_CUDA;
-  // chained mode: the tiles of all sequences are dealt out evenly, every CTA gets at least one
   const int nt = (prm.sp.seqlen + T - 1) / T;
-  int grid = prm.sp.chain ? (int)std::min<long long>((long long)prm.upairs * nt, kSms) : std::min(prm.nitems, kSms);
-  // Look-back: where it leaves few SMs out, every sequence in the same number of pieces, so that all pairs of heads are at the
-  // same tokens at the same time and find B and C in L2 (one sequence of 131 072 tokens, 16 pairs: 9 pieces each on 144 SMs).
-  if (prm.sp.chain == 2) {
-    const int pieces = std::min(kSms / prm.upairs, nt);
-    if (pieces > 1 && pieces * prm.upairs >= kSms * 93 / 100) grid = pieces * prm.upairs;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = kThreads2;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute early;
-  if (prm.sp.chain) {
-    if (launch(clear_flags_kernel, 1, 2 * kSms, 0, stream, prm.sp.chain_flag) != SSD_OK) return SSD_ERR_CUDA;
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-  }
-  return cudaLaunchKernelEx(&cfg, kern, tx, tb, tc, ty, prm) == cudaSuccess ? SSD_OK : SSD_ERR_CUDA;
+  const int grid = prm.sp.chain ? dealt_grid(prm.upairs, nt, prm.sp.chain) : std::min(prm.nitems, kSms);
+  return launch_tiles(kern, grid, kThreads2, smem, prm.sp, stream, tx, tb, tc, ty, prm);
 }
 
 bool odd_groups(const SsdArgs& a) { return a.nheads / a.ngroups % 2 != 0; }
@@ -1215,6 +988,12 @@ bool odd_groups(const SsdArgs& a) { return a.nheads / a.ngroups % 2 != 0; }
 int64_t unit_pairs(const SsdArgs& a) { return (int64_t)a.batch * a.ngroups * ((a.nheads / a.ngroups + 1) / 2); }
 
 }  // namespace
+
+int64_t tc2_units(const SsdArgs& a) { return unit_pairs(a); }
+
+int launch_clear_flags(int32_t* flags, int count, cudaStream_t stream) {
+  return launch(clear_flags_kernel, 1, count, 0, stream, flags);
+}
 
 // Skip and gate in the kernel: with packed 16-bit gates, which groups with an odd number of heads have never had (bf16, Y
 // against 64 bits: 2.9e-3 with the epilogue kernel's fp32 gate, 3.7e-3 with packed ones).
@@ -1240,15 +1019,13 @@ bool tc_supports(const SsdArgs& a) {
 //      ("look-back"), still one launch;
 //   0  two passes and a fold (three launches): kept for the state-only run and the run that reuses its segment
 //      states, which a sequence-sharded forward makes around its exchange.
-int tc2_chain_mode(const SsdArgs& a, int nseg) {
+int tc_chain_mode(const SsdArgs& a, int nseg, int64_t upairs) {
   if (nseg <= 1) return 0;
-  const int64_t upairs = unit_pairs(a);
   if (upairs >= kSms) return 1;
   return (a.flags & (SSD_FLAG_STATE_ONLY | SSD_FLAG_REUSE_SEGMENTS)) ? 0 : 2;
 }
 
-int tc2_default_segments(const SsdArgs& a) {
-  const int64_t upairs = unit_pairs(a);
+int tc_default_segments(const SsdArgs& a, int64_t upairs) {
   const int tiles = (a.seqlen + T - 1) / T;
   // Costs in tile times (2.7 to 3.1 us), fitted to forwards of 1 to 600 pairs and 2 to 64 tiles, each timed whole and cut; the
   // constants are what a launch takes beside its tiles.  16 pairs of 4, 8 and 32 tiles: whole 17, 29 and 95 us, cut 16, 18
@@ -1288,7 +1065,7 @@ int tc2_default_segments(const SsdArgs& a) {
 
 int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
   if (sp.seg_len % T != 0) return SSD_ERR_UNSUPPORTED;
-  Tc2Params prm;
+  TileParams prm;
   prm.sp = sp;
   prm.ppg = (a.nheads / a.ngroups + 1) / 2;
   const int64_t upairs = unit_pairs(a);

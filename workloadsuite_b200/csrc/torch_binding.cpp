@@ -32,7 +32,7 @@ decltype(&ssd_b200_dt_prologue) f_dt;
 PyObject* f_raise;   // raises the Python exception of an error code
 
 constexpr int kMaxDevices = 64;
-Tensor* g_workspace[kMaxDevices];   // scratch shared by all calls on a device (never shrinks)
+Tensor* g_workspace[kMaxDevices];   // scratch of the runs that leave results for a later one (never shrinks)
 Tensor* g_status[kMaxDevices];      // the kernels' status word
 
 int dtype_of(const Tensor& t) {
@@ -234,10 +234,11 @@ PyObject* py_forward(PyObject*, PyObject* const* o, Py_ssize_t n) {
   a.chunk = (int)chunk; a.dtype = dtype;
   strides4(*X, a.x_stride); strides3(*A, a.a_stride); strides4(*B, a.b_stride); strides4(*C, a.c_stride); strides4(Y, a.y_stride);
   const size_t need = f_workspace(&a);
+  Tensor ws;   // from the current stream's memory: calls on other streams have their own
   if (need) {
-    Tensor& ws = workspace(w.dev.index(), (int64_t)need);
+    ws = at::empty({(int64_t)need}, X->options().dtype(at::kByte));
     a.workspace = ws.data_ptr();
-    a.workspace_bytes = (size_t)ws.numel();
+    a.workspace_bytes = need;
   }
   if (const int rc = f_forward(&a, w.stream())) return declined(rc);
   if (!want_final) return THPVariable_Wrap(std::move(Y));

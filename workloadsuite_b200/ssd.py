@@ -186,18 +186,18 @@ def ssd_forward(
 
     ``kernel``: None lets the library choose.  ``"tcgen05"`` (16-bit tensors, p = 64, n = 64 or 128) runs on the tensor
     cores and rounds intermediate operands to 16 bits; it is chosen for sequences of whole tiles (multiples of 128 tokens).
-    ``"scan_f32"`` computes in float32 throughout; it is chosen for everything else, and ``kernel="tcgen05"`` takes any
-    length at a fraction of its time where 16-bit intermediates are accurate enough (relative error of Y in bfloat16
-    2.4e-3 instead of 1.7e-3, of the final state 2e-3 instead of 1e-7).
+    ``"scan_f32"`` computes in float32 throughout; it is chosen for everything else, where it runs on the tensor cores too
+    if the shape allows (asked for by name, it is the token-by-token recurrence).  ``kernel="tcgen05"`` takes any length where
+    16-bit intermediates are accurate enough (relative error of Y in bfloat16 2.4e-3 instead of 1.7e-3, of the final
+    state 2e-3 instead of 1e-7) at three quarters of the time.
 
     ``nsegments``: None lets the library choose; 1 keeps sequences whole; more cuts them (see ``plan``):
     the tensor-core kernel deals the tiles of all sequences out evenly over the SMs inside one launch, the other
     kernels scan that many segments in two passes joined by a fold.
 
-    A sequence that is cut into segments uses one scratch buffer per device, kept between
-    calls and shared by all of them: calls that may overlap on the GPU (different streams)
-    must be serialised by the caller, and ``reuse_segments`` relies on no other segmented
-    call on that device coming between the two runs.
+    Scratch comes from the current stream's memory, but ``state_only`` and ``reuse_segments`` runs share one buffer per
+    device, kept between calls: those that may overlap on the GPU (different streams) must be serialised by the caller,
+    and ``reuse_segments`` relies on no other ``state_only`` run on that device coming between the two.
 
     ``D`` [h] and ``z`` [b,s,h,p] (dtype of X) add the layer's skip and gate to the kernel's epilogue:
     ``Y <- (Y + X * D[head]) * silu(z)`` (``model_ref.py:116-118``), evaluated in float32 and rounded once;
@@ -271,7 +271,11 @@ def ssd_forward(
         args.z_stride = _strides3(z, "z")
     with torch.cuda.device(dev):
         need = lib.ssd_b200_workspace_bytes(C.byref(args))
-        ws = _workspace(dev, need)
+        # what a state-only run leaves for the run that reuses it stays; other scratch is the current stream's
+        if state_only or reuse_segments:
+            ws = _workspace(dev, need)
+        else:
+            ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
         if ws is not None:
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
         rc = lib.ssd_b200_forward(C.byref(args), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
