@@ -26,10 +26,10 @@
 //   warps 20-23   Xd = exp(cs_last - cs) x~ of the next tile, in pieces -> shared memory -> S
 //     Y = P.X + exp(cs) C.H -> shared memory -> TMA store
 //
-// What bounds it (bf16): the MMAs of a tile take 3 800 tensor-pipe cycles (G 8, S and C.H 16 each at 62, P.X 24 at 55) and
-// shared memory moves 590 KB, 4 600 cycles; a tile takes 5 500 to 6 000.  On the way round P -> P.X -> G -> P the tensor pipe
-// has S and C.H to do while P is made.  P on eight warps instead of sixteen: 104 us instead of 98.7 (2 x 3001 tokens, 80 heads;
-// the recurrence takes 1 895); the pieces unpacked by integer instructions: 98.7 instead of 97.2.
+// What bounds it (bf16, n = 128): a 128 x N x 16 MMA takes 55 cycles at N = 64, 62 at 128, some 90 at 192, a tile 3 900 (G 8 of 128, S 8 of
+// 192, C.H and P.X 24 of 64 each); G, S and C.H read both operands from shared memory, which moves 560 KB a tile, 4 400
+// cycles.  The MMA issuer goes round in some 5 000.  P on eight warps instead of sixteen: 104 us instead of 98.7 (2 x 3001
+// tokens, 80 heads; the recurrence takes 1 895); the pieces unpacked by integer instructions: 98.7 instead of 97.2.
 #include <cuda.h>
 
 #include <algorithm>
@@ -65,7 +65,7 @@ struct LayoutS {
 // 32 tokens take the same 32 columns and 16 more behind G, so that a thread writes over nothing that another one reads.
 template <int kPieces>
 struct Columns {
-  static constexpr uint32_t G = 0, Yo = kPieces == 3 ? 192 : 128, S = Yo + 128, Yd = S + 128;
+  static constexpr uint32_t G = 0, S = kPieces == 3 ? 192 : 128, Yo = S + 64 * kPieces, Yd = kPieces == 3 ? 448 : 384;
   // the first piece of k-step ks (16 tokens), and the second (the third is 8 columns behind it)
   static __device__ __forceinline__ uint32_t first(uint32_t ks) { return kPieces == 3 ? 16 * ks + 8 * (ks & 1) : 16 * ks; }
   static __device__ __forceinline__ uint32_t second(uint32_t ks) { return kPieces == 3 && (ks & 1) ? 128 + 8 * (ks - 1) : 16 * ks + 8; }
@@ -110,8 +110,8 @@ constexpr float kLowestS = -104.f;   // as in ssd_tc2.cu: a factor of zero eithe
 constexpr float kGrowth = 1.f / 32.f;
 
 // Two fp32 numbers as sums of 16-bit ones, packed.
-// bf16: high, low, middle, eight bits at a time from the top, so all subtractions are exact; HALF: the low one halved.  (The
-// multiply-add that takes 16-bit factors spares the unpacking, which is the integer pipe's, of half the rate.)
+// bf16: high, middle, low, eight bits at a time from the top, so all subtractions are exact.  (The multiply-add that takes
+// 16-bit factors spares the unpacking, which is the integer pipe's, of half the rate.)
 // fp16: high (11 bits, rounded) and UP times the rest (rounded to 11 bits; the factor keeps it out of the subnormal numbers).
 __device__ __forceinline__ uint32_t top_pair(uint64_t v) {
   const float2 f = unpair(v);
@@ -133,14 +133,13 @@ __device__ __forceinline__ uint64_t less(uint64_t v, uint32_t packed) {
         : "r"(packed), "f"(f.x), "f"(f.y));
   return pair(x, y);
 }
-template <typename T16, bool HALF, int UP>
+template <typename T16, int UP>
 __device__ __forceinline__ void split(uint64_t v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
   if constexpr (std::is_same<T16, __nv_bfloat16>::value) {
     p0 = top_pair(v);
     const uint64_t r = less<T16>(v, p0);
-    p2 = top_pair(r);
-    const uint64_t rest = less<T16>(r, p2);
-    p1 = top_pair(HALF ? mul_pair(rest, pair(0.5f, 0.5f)) : rest);
+    p1 = top_pair(r);
+    p2 = top_pair(less<T16>(r, p1));
   } else {
     p0 = pack_pair<T16>(v);
     p1 = pack_pair<T16>(mul_pair(less<T16>(v, p0), pair((float)UP, (float)UP)));
@@ -151,11 +150,10 @@ __device__ __forceinline__ void split(uint64_t v, uint32_t& p0, uint32_t& p1, ui
 // 2^-16 are held to 2^-24 of them: x, which is given in fp16, in weights of up to 2.
 constexpr int kUp = 1 << 11, kUpX = 1 << 14;
 
-// What the accumulators of the pieces hold together (fp16: times `unit`).
-template <bool kF16, int UP>
-__device__ __forceinline__ uint64_t both(uint64_t a0, uint64_t a1, float unit) {
-  if constexpr (kF16) return mul_pair(fma_pair(a1, pair(1.f / UP, 1.f / UP), a0), pair(unit, unit));
-  return add_pair(a0, a1);
+// (fp16) What the accumulators of the pieces hold together, times `unit`.
+template <int UP>
+__device__ __forceinline__ uint64_t low_and_high(uint64_t low, uint64_t high, float unit) {
+  return mul_pair(fma_pair(low, pair(1.f / UP, 1.f / UP), high), pair(unit, unit));
 }
 
 // The power of two at or below x >= 0, but 2^-100 at least, and 1 for what is too large to have a unit (2^127 and more, infinity,
@@ -266,14 +264,15 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // bf16: S and C.H are two products of 128 columns onto the same two accumulators: (low / 2 | middle), then (high | low / 2).
-    // Products onto one accumulator have one shape, so they run in the order they are issued in.  An accumulator cuts off what
-    // it cannot hold, so the small pieces go first (the other way round, the final state is off by 2.1e-7 instead of 8e-8).
+    // S has an accumulator for each piece, one product of 192 (128) columns.  bf16: C.H and P.X have one, products of 64 columns,
+    // the low pieces first: an accumulator cuts off what it cannot hold (small ones last, the final state was off by 2.1e-7
+    // instead of 8e-8).  (Shared memory is what the first three are short of: S as two products of 128 columns reads the B tile
+    // twice.  2 x 3001 tokens, 80 heads: S and C.H that way 93.1 us, this way 86.0.)  fp16: two accumulators each.
     constexpr int fmt = kF16 ? 0 : 1;
     constexpr uint64_t kHi = umma_desc_base(0, 1024);
     constexpr uint32_t kMN = kBlk >> 4, kMNh = N * 128 >> 4, kRow16 = 2048 >> 4, kCol16 = 32 >> 4;
-    constexpr uint32_t idG = umma_idesc(128, 128, fmt, 0, 0), idS = umma_idesc(128, 128, fmt, 1, 1);
-    constexpr uint32_t idCH = umma_idesc(128, 128, fmt, 0, 1), idPX = umma_idesc(128, 64, fmt, 0, 1);
+    constexpr uint32_t idG = umma_idesc(128, 128, fmt, 0, 0), idS = umma_idesc(128, 64 * kPieces, fmt, 1, 1);
+    constexpr uint32_t idCH = umma_idesc(128, kF16 ? 128 : 64, fmt, 0, 1), idPX = umma_idesc(128, 64, fmt, 0, 1);
     uint32_t xb = 0;   // X slot of the tile, as a descriptor offset
 #pragma unroll 1
     for (uint32_t n = 0; n < total; ++n) {
@@ -302,13 +301,9 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       if (n > 0) wait(&m->bar_u, (n - 1) & 1, m);
       tc_fence_after();
       if (elect_one()) {
-#pragma unroll 1
-        for (uint32_t v = 0; v < kPieces - 1; ++v) {
-          const uint32_t bx = (sXd >> 4) + (kPieces - 2 - v) * kMN;
 #pragma unroll
-          for (uint32_t k = 0; k < KT; ++k)
-            umma_ss(tS, kHi | (kMN << 16 | (aB + k * kRow16)), kHi | (kMN << 16 | (bx + k * kRow16)), idS, v + k);
-        }
+        for (uint32_t k = 0; k < KT; ++k)
+          umma_ss(tS, kHi | (kMN << 16 | (aB + k * kRow16)), kHi | (kMN << 16 | ((sXd >> 4) + k * kRow16)), idS, k);
         umma_commit(&m->bar_s);
         umma_commit(&m->empty_b[sb]);
       }
@@ -319,8 +314,8 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll 1
-          for (uint32_t v = 0; v < kPieces - 1; ++v) {
-            const uint32_t bh = (sH >> 4) + (kPieces - 2 - v) * kMNh;
+          for (uint32_t v = 0; v < (kF16 ? 1 : 3); ++v) {   // (low, middle, high)
+            const uint32_t bh = (sH >> 4) + (kF16 ? 0 : 2 - v) * kMNh;
 #pragma unroll
             for (uint32_t k = 0; k < KN; ++k)
               umma_ss(tYo, kHi | (1u << 16 | (aC + (k >> 2) * kMN + (k & 3) * kCol16)), kHi | (kMNh << 16 | (bh + k * kRow16)),
@@ -511,15 +506,11 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                           2 * e + 1 <= last ? __uint_as_float(g[2 * e + 1]) * w[2 * e + 1] : 0.f);
           }
 #pragma unroll
-          for (int e = 0; e < 8; ++e) split<T16, false, kUp>(v[e], p0[e], p1[e], p2[e]);
+          for (int e = 0; e < 8; ++e) split<T16, kUp>(v[e], p0[e], p1[e], p2[e]);
         }
         tmem_st8(tlane + Col::first(ks), p0);
-        if constexpr (kF16) {
-          tmem_st8(tlane + Col::second(ks), p1);
-        } else {
-          tmem_st8(tlane + Col::second(ks), p2);
-          tmem_st8(tlane + Col::second(ks) + 8, p1);
-        }
+        tmem_st8(tlane + Col::second(ks), p1);
+        if constexpr (!kF16) tmem_st8(tlane + Col::second(ks) + 8, p2);
       }
     };
     // The state's pieces, in shared memory; fp16 in units of h_unit / 2^14, which keeps the largest below 2^15.
@@ -531,7 +522,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       for (int k = 0; k < 2; ++k) {
         uint32_t p0[4], p1[4], p2[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) split<T16, true, kUp>(kF16 ? mul_pair(H[4 * k + e], pair(inv, inv)) : H[4 * k + e], p0[e], p1[e], p2[e]);
+        for (int e = 0; e < 4; ++e) split<T16, kUp>(kF16 ? mul_pair(H[4 * k + e], pair(inv, inv)) : H[4 * k + e], p0[e], p1[e], p2[e]);
         const uint32_t at = sH + l * 128 + (((2 * J + k) ^ swz) << 4);
         sts128(at, make_uint4(p0[0], p0[1], p0[2], p0[3]));
         sts128(at + N * 128, make_uint4(p1[0], p1[1], p1[2], p1[3]));
@@ -704,12 +695,21 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       if (owns_state) {
         const uint64_t g2 = pair(gs, gs);
         uint32_t s0[16], s1[16];
-        tmem_ld16(tS + tlane + 16 * J, s0);
-        tmem_ld16(tS + tlane + 64 + 16 * J, s1);
+        tmem_ld16(tS + tlane + 64 + 16 * J, s0);
+        tmem_ld16(tS + tlane + (kF16 ? 0 : 128) + 16 * J, s1);
         tmem_ld_wait();
+        if constexpr (kF16) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          H[e] = fma_pair(H[e], g2, both<kF16, kUpX>(pair(s0[2 * e], s0[2 * e + 1]), pair(s1[2 * e], s1[2 * e + 1]), su));
+          for (int e = 0; e < 8; ++e) H[e] = fma_pair(H[e], g2, low_and_high<kUpX>(pair(s0[2 * e], s0[2 * e + 1]), pair(s1[2 * e], s1[2 * e + 1]), su));
+        } else {   // (middle and low pieces, then the high ones: for the registers)
+          uint64_t ml[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) ml[e] = add_pair(pair(s0[2 * e], s0[2 * e + 1]), pair(s1[2 * e], s1[2 * e + 1]));
+          tmem_ld16(tS + tlane + 16 * J, s0);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 8; ++e) H[e] = fma_pair(H[e], g2, add_pair(pair(s0[2 * e], s0[2 * e + 1]), ml[e]));
+        }
       }
       tc_fence_before();
       warp_arrive(&m->bar_u);
@@ -762,7 +762,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float2 x = unpack2<T16>(aw[e]);
-            split<T16, true, kUpX>(mul_pair(pair(x.x, x.y), w2), p0[e], p1[e], p2[e]);
+            split<T16, kUpX>(mul_pair(pair(x.x, x.y), w2), p0[e], p1[e], p2[e]);
           }
           sts128(sXd + at, make_uint4(p0[0], p0[1], p0[2], p0[3]));
           sts128(sXd + kBlk + at, make_uint4(p1[0], p1[1], p1[2], p1[3]));
@@ -808,11 +808,13 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       };
 #pragma unroll 1
       for (int i = 0; i < P / W; ++i) {
-        uint32_t o0[W], o1[W], d[W], d1[W];
-        load(tYo + tlane + W * i, o0);
-        load(tYo + 64 + tlane + W * i, o1);
+        uint32_t o[W], o1[W], d[W], d1[W];
+        load(tYo + tlane + W * i, o);
         load(tYd + tlane + W * i, d);
-        if constexpr (kF16) load(tYd + 64 + tlane + W * i, d1);
+        if constexpr (kF16) {
+          load(tYo + 64 + tlane + W * i, o1);
+          load(tYd + 64 + tlane + W * i, d1);
+        }
         tmem_ld_wait();
         if (i == P / W - 1) {
           tc_fence_before();
@@ -821,9 +823,11 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         uint32_t w[W / 2];
 #pragma unroll
         for (int e = 0; e < W / 2; ++e) {
-          const uint64_t yo = both<kF16, kUp>(pair(o0[2 * e], o0[2 * e + 1]), pair(o1[2 * e], o1[2 * e + 1]), 1.f);
-          uint64_t yd = pair(d[2 * e], d[2 * e + 1]);
-          if constexpr (kF16) yd = both<kF16, kUp>(yd, pair(d1[2 * e], d1[2 * e + 1]), unit);
+          uint64_t yo = pair(o[2 * e], o[2 * e + 1]), yd = pair(d[2 * e], d[2 * e + 1]);
+          if constexpr (kF16) {
+            yo = low_and_high<kUp>(pair(o1[2 * e], o1[2 * e + 1]), yo, 1.f);
+            yd = low_and_high<kUp>(pair(d1[2 * e], d1[2 * e + 1]), yd, unit);
+          }
           const uint64_t y = fma_pair(yo, el2, yd);
           odd = fma_pair(y, zero2, odd);
           w[e] = pack_pair<T16>(y);
