@@ -250,8 +250,9 @@ def test_route_of_the_fp32_scan(lib):
         assert need(shape(dtype=dtype)) == redo and _plan(lib, shape(dtype=dtype)) == (1, 1, 2)
         assert need(shape(s=3001, h=80, dtype=dtype)) == chain + redo        # 160 heads: dealt out over the SMs
     assert _plan(lib, shape(s=3001, h=80)) == (1, 2, 2)
-    assert [need(shape(s=s)) for s in (31, 32)] == [0, redo] and [need(shape(s=s, n=64)) for s in (63, 65)] == [0, redo]
-    assert [need(shape(s=s, h=80)) for s in (19, 20)] == [0, redo]              # more heads than SMs
+    assert [need(shape(s=s)) for s in (23, 24)] == [0, redo] and [need(shape(s=s, n=64)) for s in (47, 48)] == [0, redo]
+    assert [need(shape(s=s, h=80)) for s in (16, 17)] == [0, redo]              # more heads than SMs
+    assert [need(shape(s=s, h=80, b=8)) for s in (11, 12)] == [0, redo]
     assert need(shape(dtype=_lib.DTYPE_F32)) == _lib_two_pass(lib, shape(dtype=_lib.DTYPE_F32))
     asked = shape()
     asked.kernel = _lib.KERNEL_SCAN_F32

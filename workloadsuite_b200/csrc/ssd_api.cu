@@ -82,10 +82,11 @@ bool outputs_on_inputs(const SsdArgs* a) {
 // The fp32 scan of a call whose kernel is not chosen by the caller: on the tensor cores at fp32 precision where they can
 // (ssd_split.cu), unless the sequences are so short that the recurrence is through before the other kernel's pipeline has
 // filled.  Its time goes with tokens x state, bf16: 8 heads of 17, 33 and 100 tokens, n 128: 8.5, 13.6 and 33 us, there 9.3, 9.4
-// and 9.7; n 64: 5.8, 8.9 and 19, there 8.5, 8.5 and 8.8.  With more heads than SMs it falls behind earlier: 1 280 of 17 and 33,
-// n 128: 54 and 99 us, there 38 and 39; n 64: 29 and 54, there 35 and 36.
+// and 9.5; n 64: 5.8, 8.9 and 19, there 8.5, 8.5 and 8.8.  With more heads than SMs it falls behind earlier: 296 heads of 17 tokens,
+// n 128, and of 33, n 64: 13.4 and 14.0 us, there 13.8 and 13.2; 1 280 of 17 tokens, n 128 and 64: 54 and 29 us, there 35 and 33.
 bool use_split(const SsdArgs* a, int kernel) {
-  const int64_t least = (int64_t)a->batch * a->nheads > kSmCount ? 2560 : 4096;
+  const int64_t heads = (int64_t)a->batch * a->nheads;
+  const int64_t least = heads <= kSmCount ? 3072 : heads <= 4 * kSmCount ? 2112 : 1536;
   return kernel == SSD_KERNEL_SCAN_F32 && (int64_t)a->seqlen * a->dstate >= least && a->kernel == SSD_KERNEL_AUTO && a->nsegments <= 1 &&
          !(a->flags & (SSD_FLAG_STATE_ONLY | SSD_FLAG_REUSE_SEGMENTS)) && aligned16(a->initial_state) && aligned16(a->final_state) &&
          ssd::split_supports(*a) && !outputs_on_inputs(a);

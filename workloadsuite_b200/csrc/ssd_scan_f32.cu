@@ -126,7 +126,9 @@ __device__ __forceinline__ void reduce_scatter(float (&v)[U], int sl) {
 // FULL: the state has exactly NS * SL rows (the strides of B and C in shared memory are then constants).
 // LINE: tokens worked on in line (1: one after the other).  CTAS: as many of an SM the registers have to leave room for (0: as
 // it comes).  Tokens in line take 64 to 126 registers, one after the other 32 to 80; see launch_one().
-template <typename T, int NS, int P, bool FULL, int LINE, int CTAS>
+// REDO: behind the tensor-core kernel at fp32 precision (ssd_split.cu), all heads in as many CTAs as the chip holds, and only if that
+// kernel says so.
+template <typename T, int NS, int P, bool FULL, int LINE, int CTAS, bool REDO>
 __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const ScanParams prm, const int tile) {
   constexpr int SL = kThreads / P;  // lanes sharing one state column
   constexpr int NS4 = NS / 4;
@@ -139,28 +141,32 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
   float* dec = Ys + tile * P;        // [tile]  exp(a_t)
   float* araw = dec + tile;          // [tile]  a_t
 
-  if (prm.redo) {   // only if the kernel ahead says so
+  int unit = blockIdx.x;
+  if constexpr (REDO) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int any = 0;
     for (int i = threadIdx.x; i < prm.redo_n; i += kThreads) any |= __ldcg(prm.redo + i);
     if (!__syncthreads_or(any)) {   // (that kernel leaves the sum of the log-decays to this one: in 64 bits, as below)
       if (!prm.fin_ld) return;
-      const float* A = prm.A + (int64_t)(blockIdx.x / prm.nheads) * prm.as[0] + (int64_t)(blockIdx.x % prm.nheads) * prm.as[2];
-      double sum = 0.0;
-      for (int t = threadIdx.x; t < prm.seqlen; t += kThreads) sum += (double)A[(int64_t)t * prm.as[1]];
-      for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
       double* part = reinterpret_cast<double*>(smem);
-      if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        for (int w = 1; w < kThreads / 32; ++w) sum += part[w];
-        prm.fin_ld[(int64_t)blockIdx.x * prm.finld_unit_stride] = (float)sum;
+      for (; unit < prm.batch * prm.nheads; unit += gridDim.x) {
+        const float* A = prm.A + (int64_t)(unit / prm.nheads) * prm.as[0] + (int64_t)(unit % prm.nheads) * prm.as[2];
+        double sum = 0.0;
+        for (int t = threadIdx.x; t < prm.seqlen; t += kThreads) sum += (double)A[(int64_t)t * prm.as[1]];
+        for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          for (int w = 1; w < kThreads / 32; ++w) sum += part[w];
+          prm.fin_ld[(int64_t)unit * prm.finld_unit_stride] = (float)sum;
+        }
+        __syncthreads();
       }
       return;
     }
   }
-  const int unit = blockIdx.x;
-  const int seg = blockIdx.y;
+  const int seg = REDO ? 0 : blockIdx.y;
+  do {
   const int bi = unit / prm.nheads, hi = unit - bi * prm.nheads;
   const int gi = hi / (prm.nheads / prm.ngroups);
   const int tid = threadIdx.x;
@@ -307,6 +313,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
   }
   if (prm.fin_ld && tid == 0)
     prm.fin_ld[unit * prm.finld_unit_stride + seg * prm.finld_seg_stride] = (float)asum;
+  } while (REDO && (unit += gridDim.x) < prm.batch * prm.nheads);
 }
 
 // H_in(seg) for every segment of every unit, from the zero-start final states:
@@ -366,19 +373,30 @@ int launch_one(const ScanParams& prm, cudaStream_t stream) {
   const int64_t ctas = (int64_t)prm.batch * prm.nheads * prm.nseg;
   const int tokens = std::min(prm.seqlen, prm.seg_len);
   const bool many = ctas > 2 * 148, full = prm.n == NS * SL;
-  auto kern = full ? ssd_scan_f32_kernel<T, NS, P, true, kLine, 0> : ssd_scan_f32_kernel<T, NS, P, false, kLine, 0>;
+  auto kern = full ? ssd_scan_f32_kernel<T, NS, P, true, kLine, 0, false> : ssd_scan_f32_kernel<T, NS, P, false, kLine, 0, false>;
   if (k16 && full && tokens < kLine && ctas > kMany * 148)
-    kern = ssd_scan_f32_kernel<T, NS, P, true, 1, kMost>;
+    kern = ssd_scan_f32_kernel<T, NS, P, true, 1, kMost, false>;
   else if (tokens < kLine || (!k16 && NS == 32 && many && ctas <= 4 * 148))
-    kern = full ? ssd_scan_f32_kernel<T, NS, P, true, 1, 0> : ssd_scan_f32_kernel<T, NS, P, false, 1, 0>;
+    kern = full ? ssd_scan_f32_kernel<T, NS, P, true, 1, 0, false> : ssd_scan_f32_kernel<T, NS, P, false, 1, 0, false>;
   else if (k16 && many && (NS <= 16 || tokens < 16))
-    kern = full ? ssd_scan_f32_kernel<T, NS, P, true, kLine, kMany> : ssd_scan_f32_kernel<T, NS, P, false, kLine, kMany>;
+    kern = full ? ssd_scan_f32_kernel<T, NS, P, true, kLine, kMany, false> : ssd_scan_f32_kernel<T, NS, P, false, kLine, kMany, false>;
+  bool early = false;
+  if constexpr (k16 && P == 64 && NS >= 16) {
+    if (prm.redo) {
+      if (!full || prm.nseg != 1) return SSD_ERR_UNSUPPORTED;
+      kern = ssd_scan_f32_kernel<T, NS, P, true, kLine, 0, true>;
+      early = true;
+    }
+  }
+  if (prm.redo && !early) return SSD_ERR_UNSUPPORTED;
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SSD_ERR_CUDA;
   }
+  // (As many CTAs as the chip holds: one for each of 5 120 heads that only look whether there is work take 20 us, these 1.)
+  if (early) return launch_early(kern, (unsigned)std::min<int64_t>(ctas, 4 * 148), kThreads, smem, stream, prm, tile);
   dim3 grid((unsigned)(prm.batch * prm.nheads), (unsigned)prm.nseg);
-  return prm.redo ? launch_early(kern, grid, kThreads, smem, stream, prm, tile) : launch(kern, grid, kThreads, smem, stream, prm, tile);
+  return launch(kern, grid, kThreads, smem, stream, prm, tile);
 }
 
 template <typename T, int P>

@@ -215,6 +215,8 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // The recurrence's CTAs may come once all of these are on their SMs: they wait for the end of this kernel, but not to be launched.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t sB = smem_u32(smem + L::oB), sC = smem_u32(smem + L::oC), sX = smem_u32(smem + L::oX);
   const uint32_t sXd = smem_u32(smem + L::oXd), sH = smem_u32(smem + L::oH);
   const Work& wk = m->work;
@@ -858,7 +860,6 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   // ---------------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     if (status) {
       if (m->tmem_base != 0) atomicCAS(status, 0, (int)STATUS_TMEM_ALLOC);
