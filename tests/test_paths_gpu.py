@@ -381,3 +381,48 @@ def test_scratch_of_calls_on_two_streams_is_their_own():
     for i in range(2):
         for Y, H in got[i]:
             assert torch.equal(Y, want[i][0]) and torch.equal(H, want[i][1])
+
+
+@pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -11)])
+@pytest.mark.parametrize("b,s,h,g,n", [(2, 65, 4, 2, 128), (1, 300, 3, 1, 64), (1, 2001, 18, 1, 128), (40, 300, 5, 1, 128)],
+                         ids=["one_tile", "three", "lookback", "too_many_to_fuse"])
+@pytest.mark.parametrize("which", ["D", "z", "both", "z_rows_apart"])
+def test_skip_and_gate_of_the_fp32_scan(which, b, s, h, g, n, dtype, eps):
+    """(Y + x D) silu(z) in fp32 ahead of the one rounding: off by that (eps of the value at most), the sums' 1e-5 and the gate's
+    (exp and a division, some 2^-21 each), against the gate's size; many tiles, which are not fused; and what the recurrence has
+    to do again, with both."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=g, dtype=dtype, init=True, seed=90 + s, decay_scale=0.1)
+    gen = torch.Generator().manual_seed(s)
+    D = torch.randn(h, generator=gen).to(dtype) if which in ("D", "both") else None
+    z = 3 * torch.randn(b, s, h, 64, generator=gen)
+    z = z.to(dtype) if which != "D" else None
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    zd = None if z is None else z.to(DEV)
+    if which == "z_rows_apart":       # columns of a wider tensor
+        wide = torch.zeros(b, s, h * 64 + 24, dtype=dtype, device=DEV)
+        wide[..., 8:8 + h * 64] = zd.flatten(2)
+        zd = wide[..., 8:8 + h * 64].unflatten(-1, (h, 64))
+    run = lambda **kw: W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, initial_states=d["initial_states"], z=zd,
+                                     D=None if D is None else D.to(DEV), **kw)
+    Yr = O.ssd_recurrence(inp["X"], inp["A"], inp["B"], inp["C"], initial_states=inp["initial_states"])
+    size = Yr.abs().max()
+    gate = torch.ones(()) if z is None else torch.nn.functional.silu(z.double())
+    if D is not None:
+        Yr = Yr + inp["X"].double() * D.double()[:, None]
+    Yr = Yr * gate
+    got, apart = run().cpu().double(), run(separate_epilogue=True).cpu().double()
+    # in a kernel of their own Y has a rounding ahead of them as well
+    twice = 2.1 * eps * (Yr.abs() + size * eps) + 1e-5 * size * (1 + gate.abs()) + eps * size * gate.abs()
+    assert ((apart - Yr).abs() <= twice).all()
+    if b * h * ((s + 127) // 128) <= 2 * 148:
+        assert ((got - Yr).abs() <= eps * Yr.abs() + (1e-5 * size + 2 ** -20 * Yr.abs()) * (1 + gate.abs())).all()
+    else:                                    # more tiles than that: not in the kernel
+        assert torch.equal(got, apart)
+    # growth (above 1/32): done again by the recurrence, where Y has a rounding before the skip and the gate; e^1.2 in all, or
+    # Y times the gate overflows fp16 in both
+    d["A"][0, 10:40, 0] = 0.04
+    again, want = run().double(), run(kernel="scan_f32", nsegments=1).double()
+    assert ((again - want).abs() <= 2.1 * eps * want.abs() + 2 * eps * want.abs().max()).all()
+    assert torch.equal(run(separate_epilogue=True).double(), want)

@@ -295,7 +295,11 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
     } else if (rc != SSD_ERR_UNSUPPORTED) {
       return rc;
     }
-    return ssd::launch_scan_f32(whole, args->dtype, stream);
+    if (whole.redo || (!whole.D && !whole.Z)) return ssd::launch_scan_f32(whole, args->dtype, stream);
+    ssd::ScanParams ep = whole;
+    whole.D = nullptr, whole.Z = nullptr;
+    rc = ssd::launch_scan_f32(whole, args->dtype, stream);
+    return rc != SSD_OK ? rc : ssd::launch_epilogue(ep, args->dtype, stream);
   }
 
   float* seg_states = static_cast<float*>(args->workspace);
@@ -342,10 +346,11 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
   if (rc != SSD_OK) return rc;
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
   if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false);
-  // skip and gate of model_ref.py:116-118: fused into the tensor-core kernel, a kernel of their own otherwise
+  // skip and gate of model_ref.py:116-118: fused into the tensor-core kernels, a kernel of their own otherwise
   const int kernel = resolve_kernel(args);
-  const bool fuse = kernel == SSD_KERNEL_TCGEN05 && ssd::tc_supports(*args) && ssd::tc2_fuses_epilogue(*args) &&
-                    z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
+  const bool can = kernel == SSD_KERNEL_TCGEN05 ? ssd::tc_supports(*args) && ssd::tc2_fuses_epilogue(*args)
+                                                  : use_split(args, kernel) && ssd::split_fuses_epilogue(*args);
+  const bool fuse = can && z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
   rc = forward_impl(args, stream_v, fuse);
   if (rc != SSD_OK || fuse) return rc;
   ssd::ScanParams ep;

@@ -136,6 +136,7 @@ int launch_clear_flags(int32_t* flags, int count, cudaStream_t stream);   // to 
 
 // tensor-core kernel at fp32 precision (ssd_split.cu)
 bool split_supports(const SsdArgs& a);
+bool split_fuses_epilogue(const SsdArgs& a);
 int split_grid(const SsdArgs& a, int chain);   // CTAs, each of which writes its word of ScanParams::redo
 int launch_split(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);   // SSD_ERR_UNSUPPORTED: nothing was enqueued
 

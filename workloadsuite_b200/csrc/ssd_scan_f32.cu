@@ -286,6 +286,20 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
     if (sizeof(T) < 4 && prm.compute_y) {
       __syncthreads();
       T* Yt = Yg + (int64_t)t0 * prm.ys[1];
+      if constexpr (REDO) {   // with the skip and the gate, which that kernel applies too
+        const T* Zg = prm.Z ? static_cast<const T*>(prm.Z) + bi * prm.zs[0] + hi * prm.zs[2] + (int64_t)t0 * prm.zs[1] : nullptr;
+        for (int i = tid; (prm.D || Zg) && i < rows * P; i += kThreads) {
+          const int r = i / P, c = i - r * P;
+          float v = Ys[i];
+          if (prm.D) v = fmaf(Cvt<T>::to_f(Xg[(int64_t)(t0 + r) * prm.xs[1] + c]), load_skip<T>(prm, hi), v);
+          if (Zg) {
+            const float z = Cvt<T>::to_f(Zg[(int64_t)r * prm.zs[1] + c]);
+            v *= z / (1.f + __expf(-z));
+          }
+          Ys[i] = v;
+        }
+        __syncthreads();
+      }
       if (vec_ok) {
         constexpr int per_row = P >> 3;
         for (int i = tid; i < rows * per_row; i += kThreads) {

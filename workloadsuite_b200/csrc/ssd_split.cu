@@ -24,7 +24,7 @@
 //     P = G o exp(segsum) o causal, in pieces -> TMEM (into the columns that G is read from) -> P.X
 //     H <- exp(cs_last) H + S
 //   warps 20-23   Xd = exp(cs_last - cs) x~ of the next tile, in pieces -> shared memory -> S
-//     Y = P.X + exp(cs) C.H -> shared memory -> TMA store
+//     Y = P.X + exp(cs) C.H [+ skip and gate] -> shared memory -> TMA store
 //
 // What bounds it (bf16, n = 128): a 128 x N x 16 MMA takes 55 cycles at N = 64, 62 at 128, some 90 at 192, a tile 3 900 (G 8 of 128, S 8 of
 // 192, C.H and P.X 24 of 64 each); G, S and C.H read both operands from shared memory, which moves 560 KB a tile, 4 400
@@ -164,7 +164,8 @@ __device__ __forceinline__ float power_below(float x) {
 }
 __device__ __forceinline__ float inverse_power(float x) { return __uint_as_float(0x7f000000u - __float_as_uint(x)); }
 
-template <typename T16, int N>
+// EPI: skip and gate of model_ref.py:116-118 (sp.D / sp.Z; either may be null) applied to Y in fp32 ahead of its one rounding.
+template <typename T16, int N, bool EPI>
 __global__ void __launch_bounds__(kThreadsS, 1)
 ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY, const TileParams prm) {
@@ -797,13 +798,29 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         wait(&m->full_h[ky % 4], (ky / 4) & 1, m);
         el *= m->h_unit[ky % 4] * (1.f / 16384.f);
       }
+      // (EPI) this thread's gate row, fetched some columns ahead
+      constexpr int W = kF16 || EPI ? 8 : 16;   // columns at a time
+      const int64_t tok = c.t0 + l;
+      const bool gated = EPI && sp.Z && tok < sp.seqlen;
+      const T16* zrow = static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] + tok * sp.zs[1] + c.head(wk) * sp.zs[2];
+      uint4 zn[W / 8];
+      auto gate = [&](int i) {
+        if (gated) {
+#pragma unroll
+          for (int k = 0; k < W / 8; ++k) zn[k] = __ldg(reinterpret_cast<const uint4*>(zrow + W * i) + k);
+        }
+      };
+      float skip = 0.f;
+      if constexpr (EPI) {
+        gate(0);
+        if (sp.D) skip = load_skip<T16>(sp, c.head(wk));
+      }
       wait(&m->bar_y, ky & 1, m);
       tc_fence_after();
       release();
       const uint64_t el2 = pair(el, el);
       // X is consumed (its P.X MMAs are complete): the 16-bit Y rows are staged in its slot
       const uint32_t ystage = sX + xi * kBlk, yrow = ystage + l * 128;
-      constexpr int W = kF16 ? 8 : 16;   // columns at a time
       auto load = [](uint32_t at, uint32_t (&v)[W]) {
         if constexpr (W == 8) tmem_ld8(at, v);
         else tmem_ld16(at, v);
@@ -823,6 +840,16 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           warp_arrive(&m->bar_e);
         }
         uint32_t w[W / 2];
+        uint32_t xw[W / 2], zw[W / 2];
+        if constexpr (EPI) {
+#pragma unroll
+          for (int k = 0; k < W / 8; ++k) {
+            const uint4 x = lds128(yrow + (((W / 8 * i + k) ^ swz) << 4));   // (X's row, still in the slot)
+            xw[4 * k] = x.x; xw[4 * k + 1] = x.y; xw[4 * k + 2] = x.z; xw[4 * k + 3] = x.w;
+            zw[4 * k] = zn[k].x; zw[4 * k + 1] = zn[k].y; zw[4 * k + 2] = zn[k].z; zw[4 * k + 3] = zn[k].w;
+          }
+          if (i + 1 < P / W) gate(i + 1);
+        }
 #pragma unroll
         for (int e = 0; e < W / 2; ++e) {
           uint64_t yo = pair(o[2 * e], o[2 * e + 1]), yd = pair(d[2 * e], d[2 * e + 1]);
@@ -830,8 +857,16 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             yo = low_and_high<kUp>(pair(o1[2 * e], o1[2 * e + 1]), yo, 1.f);
             yd = low_and_high<kUp>(pair(d1[2 * e], d1[2 * e + 1]), yd, unit);
           }
-          const uint64_t y = fma_pair(yo, el2, yd);
+          uint64_t y = fma_pair(yo, el2, yd);
           odd = fma_pair(y, zero2, odd);
+          if constexpr (EPI) {
+            const float2 x = unpack2<T16>(xw[e]);
+            if (sp.D) y = fma_pair(pair(x.x, x.y), pair(skip, skip), y);
+            if (gated) {
+              const float2 z = unpack2<T16>(zw[e]);
+              y = mul_pair(y, pair(__fdividef(z.x, 1.f + __expf(-z.x)), __fdividef(z.y, 1.f + __expf(-z.y))));
+            }
+          }
           w[e] = pack_pair<T16>(y);
         }
 #pragma unroll
@@ -874,10 +909,10 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   }
 }
 
-template <typename T16, int N>
+template <typename T16, int N, bool EPI>
 int launch_typed(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& ty, const TileParams& prm,
                  int grid, cudaStream_t stream) {
-  auto kern = ssd_split_kernel<T16, N>;
+  auto kern = ssd_split_kernel<T16, N, EPI>;
   constexpr int smem = LayoutS<N, std::is_same<T16, __half>::value ? 2 : 3>::kBytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return SSD_ERR_CUDA;
   return launch_tiles(kern, grid, kThreadsS, smem, prm.sp, stream, tx, tb, tc, ty, prm);
@@ -888,6 +923,13 @@ int launch_typed(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap
 bool split_supports(const SsdArgs& a) {
   const int64_t units = (int64_t)a.batch * a.nheads;
   return tc_supports(a) && units * ((a.seqlen + T - 1) / T) <= 0x7fffffffLL;
+}
+
+// Skip and gate in the kernel: where that saves a launch of some 3 us (and its 4 us of host time) and costs less.  A tile takes
+// 3.2 us longer with them (its four read-out warps have no time to spare), the epilogue kernel 1.7 us per tile and SM:
+// 256 tiles 20.1 us with them and 21.0 without, 24 of them 12.1 and 13.7; 640 64 and 55; 16 384 706 and 543.
+bool split_fuses_epilogue(const SsdArgs& a) {
+  return (int64_t)a.batch * a.nheads * ((a.seqlen + T - 1) / T) <= 2 * kSms;
 }
 
 int split_grid(const SsdArgs& a, int chain) {
@@ -907,11 +949,15 @@ int launch_split(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
       !make_map(&tc, a.C, a, a.dstate, 1, a.c_stride, T) || !make_map(&ty, a.Y, a, P, hpg, a.y_stride, 32))
     return SSD_ERR_UNSUPPORTED;
   const int grid = split_grid(a, sp.chain);
-  if (a.dtype == SSD_DTYPE_F16)
-    return a.dstate == 128 ? launch_typed<__half, 128>(tx, tb, tc, ty, prm, grid, stream)
-                           : launch_typed<__half, 64>(tx, tb, tc, ty, prm, grid, stream);
-  return a.dstate == 128 ? launch_typed<__nv_bfloat16, 128>(tx, tb, tc, ty, prm, grid, stream)
-                         : launch_typed<__nv_bfloat16, 64>(tx, tb, tc, ty, prm, grid, stream);
+  auto go = [&](auto epilogue) {
+    constexpr bool E = decltype(epilogue)::value;
+    if (a.dtype == SSD_DTYPE_F16)
+      return a.dstate == 128 ? launch_typed<__half, 128, E>(tx, tb, tc, ty, prm, grid, stream)
+                             : launch_typed<__half, 64, E>(tx, tb, tc, ty, prm, grid, stream);
+    return a.dstate == 128 ? launch_typed<__nv_bfloat16, 128, E>(tx, tb, tc, ty, prm, grid, stream)
+                           : launch_typed<__nv_bfloat16, 64, E>(tx, tb, tc, ty, prm, grid, stream);
+  };
+  return sp.D || sp.Z ? go(std::true_type{}) : go(std::false_type{});
 }
 
 }  // namespace ssd
