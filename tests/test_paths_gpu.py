@@ -128,6 +128,57 @@ def test_decays_beyond_the_range_of_a_factor(case, s, h, g):
     assert torch.allclose(ld.cpu().double(), O.total_logdecay(inp["A"]), rtol=1e-5, atol=1e-4)
 
 
+@pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -11)])
+@pytest.mark.parametrize("b,s,h,n", [(2, 300, 4, 64), (1, 3001, 4, 128)], ids=["whole", "lookback"])
+@pytest.mark.parametrize("case", ["every_token", "one_token", "reset", "far", "idle_tokens", "steps_of_both_signs", "tiny_steps"])
+def test_strong_decays_at_fp32_precision(case, b, s, h, n, dtype, eps):
+    """The same where the library chooses and the length is no whole tiles: Y off by its own rounding and the fp32 sums' 1e-5, the
+    state by 1e-6 (a sum over the few tokens that such decays leave), the sum of the log-decays rounded once."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=1, dtype=dtype, init=True, seed=74, decay_scale=0.05)
+    inp["A"].abs_().neg_()
+    dt = (0.5 + torch.rand(b, s, h, generator=torch.Generator().manual_seed(75))).to(dtype)
+    _strong_decays(inp["A"], dt, case)
+    d = {k: v.to(DEV) for k, v in inp.items()}
+    plan = W.plan(d["X"], d["A"], d["B"], d["C"], 1)
+    assert plan["kernel"] == "scan_f32" and plan["launches"] == 2      # on the tensor cores, and the recurrence behind them
+    Y, H, ld = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, dt=dt.to(DEV), initial_states=d["initial_states"],
+                             return_final_state=True, return_logdecay=True)
+    Yr, Hr = O.ssd_recurrence(inp["X"], inp["A"], inp["B"], inp["C"], dt=dt, initial_states=inp["initial_states"],
+                              return_final_state=True)
+    assert ((Y.cpu().double() - Yr).abs() <= eps * Yr.abs() + 1e-5 * Yr.abs().max()).all()
+    assert ((H.cpu().double() - Hr).norm() / Hr.norm()).item() < 1e-6
+    assert torch.allclose(ld.cpu().double(), inp["A"].double().sum(1), rtol=2 ** -23, atol=0)
+
+
+@pytest.mark.parametrize("resets", [1, 8, 20])
+@pytest.mark.parametrize("decay", [-float("inf"), -100.0, -20.0])
+def test_weights_behind_strong_decays_are_those_of_their_own_exponents(decay, resets):
+    """One token with an x right behind tokens of strong decay: Y of the tokens after it is x (C.B) exp(mild decays), whatever
+    came before.  What the 32 768 elements of a token are off by in the mean, from the exact value rounded to fp16, is the error
+    of the weight (an approximate exponential's 2^-22 and four products' 2^-24: 5e-7) and of C.B (64 products in four accumulations,
+    each of which cuts off up to 2^-23: 5e-7; one more in P.X), 1.1e-6, and what the elements add that it rounds the other way: a step
+    of 7e-4 in 1.1e-6 / 7e-4 of them, 51, whose spread leaves 1.5e-7; three times that."""
+    import workloadsuite_b200 as W
+
+    b, s, h = 16, 290, 32
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=64, g=1, dtype=torch.float16, seed=76)
+    B, C = inp["B"].abs(), inp["C"].abs()      # (no cancellation in C.B)
+    at = [32 * k + resets + 1 for k in range(s // 32)]
+    X = torch.zeros_like(inp["X"])
+    X[:, at] = inp["X"][:, at]
+    A = torch.full_like(inp["A"], -0.01) * (1 + torch.rand(s, generator=torch.Generator().manual_seed(77)))[:, None]
+    for k in range(s // 32):
+        A[:, 32 * k:32 * k + resets] = decay
+    Y = W.ssd_forward(X.to(DEV), A.to(DEV), B.to(DEV), C.to(DEV), 1).cpu().double()
+    Yr = O.ssd_recurrence(X, A, B, C)
+    rows = [l for t in at for l in range(t, (t // 32 + 1) * 32)]
+    normal = Yr.abs() > 2 ** -14
+    off = torch.where(normal, (Y - Yr.half().double()) / Yr, 0).sum(dim=(0, 2, 3)) / normal.sum(dim=(0, 2, 3))
+    assert off[rows].abs().max().item() < 1.6e-6
+
+
 @pytest.mark.parametrize("shape", [dict(b=50, s=300, h=7, g=1, n=128), dict(b=1, s=1500, h=3, g=1, n=64),
                                    dict(b=40, s=513, h=8, g=2, n=64), dict(b=1, s=4500, h=2, g=1, n=128, decay_scale=0.002),
                                    dict(b=19, s=500, h=8, g=1, n=64), dict(b=49, s=300, h=6, g=1, n=64)],

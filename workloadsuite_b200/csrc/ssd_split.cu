@@ -6,9 +6,9 @@
 // fp16 numbers, which are off by 2^-24 of it, as fp32 itself is.  So P.X is three (two) products with X, and S = B^T.Xd and
 // C.H take the pieces side by side as columns; all products are exact, the sums fp32, the state is carried in fp32
 // registers, and Y is rounded once.  Log-decays are summed from the place they count from (the end of the tile for the
-// state's weights, the start of a row's 32-token block for P's), so a weight's error is that of its own exponent, however
-// much has decayed before.  Against 64 bits (2 x 3001 tokens, 80 heads, n 128, bf16): Y 1.66e-3, its own rounding, here and in
-// the recurrence; final state 8.0e-8 here, 1.24e-7 there.
+// state's weights, the borders of 32-token blocks for P's, and see kStrong), so a weight's error is that of its own exponent,
+// however much has decayed before.  Against 64 bits (2 x 3001 tokens, 80 heads, n 128, bf16): Y 1.66e-3, its own rounding,
+// here and in the recurrence; final state 8.0e-8 here, 1.24e-7 there.
 //
 // What cannot be done this way is left to the recurrence: a CTA that meets a number that is not finite (0 * inf in a masked
 // place would reach tokens before its own; an fp16 piece overflows at 65 504) or a log-decay above zero that a tile's factors
@@ -73,14 +73,16 @@ struct Columns {
 
 // Factors of one tile.
 struct alignas(16) FactorsS {
-  float p2[T];     // log-decay from the start of the token's 32-token block to the token, * log2(e)
+  float n2[T];     // minus the log-decay from the start of the token's 32-token block to the token, * log2(e)
   float cf[T];     // exp(log-decay from the token to the end of its block) * dt
   float xw[T];     // exp(log-decay from the token to the end of the tile) * dt
-  float dt[T];
+  float dt[T];     // (of a tile with strong decays / exp(what the sum in n2 lacks))
+  float row[T];    // of a tile with strong decays: exp(what the sum in n2 lacks)
   float blk2[4];   // log-decay of each block, * log2(e)
   float g;         // exp(log-decay of the tile)
   float unit;      // cf, xw and dt are in units of this (a power of two)
   float ld;        // its log-decay as given
+  int strong;      // a block decays by more than kStrong
 };
 
 struct MiscS {
@@ -108,6 +110,10 @@ static_assert(LayoutS<128, 2>::kBytes <= 232448 && LayoutS<64, 2>::kBytes <= 232
 constexpr float kLowestS = -104.f;   // as in ssd_tc2.cu: a factor of zero either way
 // Log-decays above zero: up to this in each token (4 in a tile) the product of two factors loses nothing that matters.
 constexpr float kGrowth = 1.f / 32.f;
+// On the diagonal a weight is 2^(difference of two sums from the start of the block), and what both hold from before takes bits of it:
+// 150 behind one reset 2e-5 of it, 3 600 behind 24 of them 5e-4.  Where a block decays by more than this much (up to which they take
+// 2e-6 of it), the sums are taken in 64 bits too, and the factors of a row and a column carry what their 32 bits lack.
+constexpr float kStrong = 16.f;
 
 // Two fp32 numbers as sums of 16-bit ones, packed.
 // bf16: high, middle, low, eight bits at a time from the top, so all subtractions are exact.  (The multiply-add that takes
@@ -412,7 +418,8 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       const int blk = lane >> 3;
       const float rest = blk == 0 ? D[3] + D[2] + D[1] : blk == 1 ? D[3] + D[2] : blk == 2 ? D[3] : 0.f;   // blocks after this one
       const float fr = expf(rest);
-      const float p[4] = {before + a[0], before + s01, before + (s01 + a[2]), up};
+      const float n2[4] = {(before + a[0]) * -kLog2e, (before + s01) * -kLog2e, (before + (s01 + a[2])) * -kLog2e, up * -kLog2e};
+      const bool strong = __any_sync(0xffffffffu, up < -kStrong);
       const float x[4] = {after + (s23 + a[1]), after + s23, after + a[3], after};
       float unit = 1.f;
       if constexpr (kF16) {   // weights of up to 2: what fp16 has to hold is then x, and G, and not their products with small steps
@@ -429,12 +436,32 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       float cf[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) cf[e] = expf(x[e]) * dt[e];
-      reinterpret_cast<float4*>(f.p2)[lane] = make_float4(p[0] * kLog2e, p[1] * kLog2e, p[2] * kLog2e, p[3] * kLog2e);
+      reinterpret_cast<float4*>(f.n2)[lane] = make_float4(n2[0], n2[1], n2[2], n2[3]);
+      if (strong) {
+        double from = 0.0, to = ((double)a[0] + (double)a[1]) + ((double)a[2] + (double)a[3]);
+#pragma unroll 1
+        for (int d = 1; d < 8; d <<= 1) {
+          const double u = __shfl_up_sync(0xffffffffu, to, d, 8);
+          if ((lane & 7) >= d) to += u;
+        }
+        from = __shfl_up_sync(0xffffffffu, to, 1, 8);
+        if ((lane & 7) == 0) from = 0.0;
+        float row[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          from += (double)a[e];
+          const float lacks = (float)(from - (double)n2[e] * -0.6931471805599453);   // (2e-3 at most: exp by its series)
+          row[e] = fmaf(lacks, fmaf(lacks, 0.5f, 1.f), 1.f);
+          dt[e] *= fmaf(-lacks, fmaf(-lacks, 0.5f, 1.f), 1.f);
+        }
+        reinterpret_cast<float4*>(f.row)[lane] = make_float4(row[0], row[1], row[2], row[3]);
+      }
       reinterpret_cast<float4*>(f.cf)[lane] = make_float4(cf[0], cf[1], cf[2], cf[3]);
       reinterpret_cast<float4*>(f.xw)[lane] = make_float4(cf[0] * fr, cf[1] * fr, cf[2] * fr, cf[3] * fr);
       reinterpret_cast<float4*>(f.dt)[lane] = make_float4(dt[0], dt[1], dt[2], dt[3]);
       if (lane < 4) f.blk2[lane] = (lane == 0 ? D[0] : lane == 1 ? D[1] : lane == 2 ? D[2] : D[3]) * kLog2e;
       if (lane == 4) {
+        f.strong = strong;
         f.g = expf(((D[3] + D[2]) + D[1]) + D[0]);
         f.ld = ld;
         f.unit = unit;
@@ -462,8 +489,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     // P of this thread's row, 32 columns.  The block is below the diagonal (weight = decay from the block's end to the row * decay
     // to the block's end, both in one product), on it (an exponential per column), or above (zero).
     auto make_p = [&](const FactorsS& f) {
-      const float row2 = f.p2[l];
-      float r = row2;
+      float r = -f.n2[l];
 #pragma unroll 1
       for (int b = J + 1; b < q; ++b) r += f.blk2[b];
       const float rf = ex2(r);
@@ -491,22 +517,31 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             for (int e = 0; e < 8; ++e) v[e] = mul_pair(pair(g[2 * e], g[2 * e + 1]), v[e]);
           } else {
             const int last = lane - 16 * (ks & 1);   // columns up to this one are not after the row
-            const float4* pp = reinterpret_cast<const float4*>(f.p2 + 16 * ks);
-            const float4* dd = reinterpret_cast<const float4*>(f.dt + 16 * ks);
-            float w[16];
+            const ulonglong2* nn = reinterpret_cast<const ulonglong2*>(f.n2 + 16 * ks);
+            const ulonglong2* dd = reinterpret_cast<const ulonglong2*>(f.dt + 16 * ks);
+            const float row2 = -f.n2[l];
+            const uint64_t rows2 = pair(row2, row2);
+            auto weight = [&](uint64_t n2, uint64_t d) {
+              const float2 x = unpair(add_pair(rows2, n2));
+              return mul_pair(pair(ex2(x.x), ex2(x.y)), d);
+            };
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float4 s = pp[e], d = dd[e];
-              w[4 * e] = ex2(row2 - s.x) * d.x;
-              w[4 * e + 1] = ex2(row2 - s.y) * d.y;
-              w[4 * e + 2] = ex2(row2 - s.z) * d.z;
-              w[4 * e + 3] = ex2(row2 - s.w) * d.w;
+              const ulonglong2 n2 = nn[e], d = dd[e];
+              v[2 * e] = weight(n2.x, d.x);
+              v[2 * e + 1] = weight(n2.y, d.y);
             }
             tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-              v[e] = pair(2 * e <= last ? __uint_as_float(g[2 * e]) * w[2 * e] : 0.f,
-                          2 * e + 1 <= last ? __uint_as_float(g[2 * e + 1]) * w[2 * e + 1] : 0.f);
+            for (int e = 0; e < 8; ++e) {
+              const float2 x = unpair(mul_pair(pair(g[2 * e], g[2 * e + 1]), v[e]));
+              v[e] = pair(2 * e <= last ? x.x : 0.f, 2 * e + 1 <= last ? x.y : 0.f);
+            }
+            if (__builtin_expect(f.strong, 0)) {
+              const float r = f.row[l];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[e] = mul_pair(v[e], pair(r, r));
+            }
           }
 #pragma unroll
           for (int e = 0; e < 8; ++e) split<T16, kUp>(v[e], p0[e], p1[e], p2[e]);
@@ -788,7 +823,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         continue;
       }
       const FactorsS& f = m->f[slot];
-      float r = f.p2[l];
+      float r = -f.n2[l];
 #pragma unroll 1
       for (int b = 0; b < q; ++b) r += f.blk2[b];
       float el = ex2(r);
