@@ -379,6 +379,33 @@ def test_fp32_scan_on_the_tensor_cores(b, s, h, g, n, nsegments, dtype, eps):
     assert ((ld.cpu().double() - total).abs() <= 2 ** -24 * total.abs()).all()      # summed in 64 bits, rounded once
 
 
+def _state_of_small_numbers(s, x, dt, A=None, rows=slice(None), n=128):
+    """The worst relative error (2-norm) of a head's final state, fp16, X of size x in some rows, and the same of the recurrence."""
+    import workloadsuite_b200 as W
+
+    b, h = 2, 4
+    inp = O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=1, dtype=torch.float16, seed=85 + s, decay_scale=0.02)
+    X = torch.zeros_like(inp["X"])
+    X[:, rows] = (inp["X"][:, rows].float() * x).half()
+    A = -inp["A"].abs() if A is None else torch.full_like(inp["A"], A)
+    step = dt * (0.5 + torch.rand(b, s, h, generator=torch.Generator().manual_seed(s)))
+    step = step.half()
+    run = lambda **kw: W.ssd_forward(X.to(DEV), A.to(DEV), inp["B"].to(DEV), inp["C"].to(DEV), 1, dt=step.to(DEV),
+                                     return_final_state=True, **kw)[1].cpu().double()
+    Hr = O.ssd_recurrence(X, A, inp["B"], inp["C"], dt=step, return_final_state=True)[1]
+    off = lambda H: ((H - Hr).norm(dim=(2, 3)) / Hr.norm(dim=(2, 3))).max().item()
+    return off(run()), off(run(kernel="scan_f32"))
+
+
+@pytest.mark.parametrize("dt", [0.5, 1e-2, 1e-3, 1e-4])
+@pytest.mark.parametrize("s", [33, 129, 300])
+def test_fp16_small_steps_in_a_last_tile(s, dt):
+    """The steps' unit comes from the tokens that are there: the last tile's state is as close as the others'.  A sum of up to 128
+    products of 22 to 23 bits in random directions, cut off in eight accumulations (up to 2^-23 each, all downwards: four units of
+    2^-24 in the mean), and the tiles' sum: five units."""
+    assert _state_of_small_numbers(s, 1e-3, dt)[0] < 5 * 2 ** -24
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("b,s,h,n", [(2, 300, 4, 128), (1, 3001, 8, 64), (50, 300, 6, 128)], ids=["whole", "lookback", "chained"])
 @pytest.mark.parametrize("what", ["x_nan", "x_inf", "b_inf", "c_nan", "a_nan", "growth", "state_inf", "overflow"])

@@ -383,12 +383,12 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           for (int e = lane; e < N * P / 32; e += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(I + 32 * e));
         }
       }
-      float a[4], dt[4] = {1.f, 1.f, 1.f, 1.f};
-      const int in = sp.seqlen - c.t0 - 4 * lane;   // past the end: decay 1 and x = 0, the state stays as it is
+      float a[4], dt[4];
+      const int in = sp.seqlen - c.t0 - 4 * lane;   // past the end: decay 1 and x = 0, the state stays as it is (a step of 0: no unit of its own)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         a[e] = e < in ? Ag[e * as1] : 0.f;
-        if (e < in && sp.dt) dt[e] = Cvt<T16>::to_f(Dg[e * ds1]);
+        dt[e] = e >= in ? 0.f : sp.dt ? Cvt<T16>::to_f(Dg[e * ds1]) : 1.f;
       }
       Ag += asT;
       Dg += dsT;
