@@ -406,6 +406,19 @@ def test_fp16_small_steps_in_a_last_tile(s, dt):
     assert _state_of_small_numbers(s, 1e-3, dt)[0] < 5 * 2 ** -24
 
 
+@pytest.mark.parametrize("n", [64, 128])
+@pytest.mark.parametrize("s,x,dt,A,rows", [(33, 1e-5, 1e-2, None, slice(None)), (129, 1e-4, 1e-4, None, slice(None)), (300, 1e-6, 0.5, None, slice(None)),
+                                           (300, 1e-6, 1e-3, None, slice(None)), (3001, 1e-5, 1e-3, None, slice(None)), (300, 1.0, 0.5, -0.4, slice(130, 160)),
+                                           (300, 1000.0, 0.5, -0.4, slice(130, 160)), (300, 1000.0, 1e-4, None, slice(None))],
+                         ids=["one_tile", "last_token", "smallest", "smallest_steps", "lookback", "decayed", "decayed_large", "large"])
+def test_fp16_numbers_of_any_size_keep_their_bits(s, x, dt, A, rows, n):
+    """Small x, small steps, and x that 96 tokens of the tile have decayed to 1e-17 of it: six units of 2^-24 (of the eight
+    accumulations' cut-offs, 16 units at most and four in the mean; the worst of eight heads), and where the decay itself is most of
+    the error (38 nats in a tile, summed in fp32), no more than the recurrence."""
+    here, recurrence = _state_of_small_numbers(s, x, dt, A, rows, n)
+    assert here < max(6 * 2 ** -24, recurrence if A else 0)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("b,s,h,n", [(2, 300, 4, 128), (1, 3001, 8, 64), (50, 300, 6, 128)], ids=["whole", "lookback", "chained"])
 @pytest.mark.parametrize("what", ["x_nan", "x_inf", "b_inf", "c_nan", "a_nan", "growth", "state_inf", "overflow"])

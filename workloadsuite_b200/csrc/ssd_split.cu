@@ -3,9 +3,11 @@
 //
 // Of each product one operand is a caller's tensor, exact in 16 bits; the other (the masked products P, the decayed X, the
 // state) is an fp32 number, taken as the sum of 16-bit ones (split below): three bf16 numbers, which hold it exactly, or two
-// fp16 numbers, which are off by 2^-24 of it, as fp32 itself is.  So P.X is three (two) products with X, and S = B^T.Xd and
-// C.H take the pieces side by side as columns; all products are exact, the sums fp32, the state is carried in fp32
-// registers, and Y is rounded once.  Log-decays are summed from the place they count from (the end of the tile for the
+// fp16 numbers, which are off by up to 2^-23 of it (fp32 by 2^-24).  Those of Xd and of the state are in units from the largest of
+// the tile, those of P in units of the tile's largest step, so that P below 2^-13 is off by up to 2^-36 instead; Y, which is all
+// that comes of P, is rounded to 2^-11 of it or 2^-25.  So P.X is three (two) products with X, and S = B^T.Xd and C.H take the
+// pieces side by side as columns; all products are exact, the sums fp32, the state is carried in fp32 registers, and Y is
+// rounded once.  Log-decays are summed from the place they count from (the end of the tile for the
 // state's weights, the borders of 32-token blocks for P's, and see kStrong), so a weight's error is that of its own exponent,
 // however much has decayed before.  Against 64 bits (2 x 3001 tokens, 80 heads, n 128, bf16): Y 1.66e-3, its own rounding,
 // here and in the recurrence; final state 8.0e-8 here, 1.24e-7 there.
@@ -19,6 +21,7 @@
 //   warp 0        TMA producer
 //   warp 1        MMA issuer: G = C.B^T, S = B^T.Xd, C.H, P.X of a tile, in this order
 //   warp 2        sums of the log-decay and every factor derived from them, up to four tiles ahead
+//   warp 3        (fp16) units of Xd's pieces
 //   warps 4-19    thread = tile row = TMEM lane; every four warps have 32 tokens as columns of P and 16 columns of the state:
 //     state entering the tile, in pieces -> shared memory -> C.H
 //     P = G o exp(segsum) o causal, in pieces -> TMEM (into the columns that G is read from) -> P.X
@@ -81,6 +84,7 @@ struct alignas(16) FactorsS {
   float blk2[4];   // log-decay of each block, * log2(e)
   float g;         // exp(log-decay of the tile)
   float unit;      // cf, xw and dt are in units of this (a power of two)
+  float x_scale, x_unit;   // (fp16) Xd * x_scale is taken to pieces, which are in units of x_unit
   float ld;        // its log-decay as given
   int strong;      // a block decays by more than kStrong
 };
@@ -90,7 +94,7 @@ struct MiscS {
   FactorsS f[kFactorsS];
   uint64_t full_b[2], full_c[2], empty_b[2], empty_c[2];   // [stage]
   uint64_t full_x[4], empty_x[4];
-  uint64_t full_f[kFactorsS], empty_f[kFactorsS];
+  uint64_t full_f[kFactorsS], empty_f[kFactorsS], full_u[kFactorsS];   // (full_u, fp16: with the unit of Xd's pieces)
   uint64_t bar_g, bar_s, bar_ch, bar_y;   // tcgen05.commit arrivals
   uint64_t bar_h, bar_p, bar_u;           // the state's pieces, P's pieces are stored; S has been read (16 warps)
   uint64_t bar_xd, bar_e;                 // Xd's pieces are stored; C.H and P.X have been read (4 warps)
@@ -152,9 +156,16 @@ __device__ __forceinline__ void split(uint64_t v, uint32_t& p0, uint32_t& p1, ui
     p2 = 0;
   }
 }
-// With 2^11 the low piece does not overflow where the high one does not; with 2^14 it does from 4 096 on, and numbers down to
-// 2^-16 are held to 2^-24 of them: x, which is given in fp16, in weights of up to 2.
+// With 2^11 the low piece does not overflow where the high one does not.  With 2^14 it does from 4 096 on, and a number in units that make
+// the largest 2^11 to 2^12 is held to 2^-23 of it, or to 2^-50 of the largest.
 constexpr int kUp = 1 << 11, kUpX = 1 << 14;
+
+// The larger magnitudes of two pairs of fp16 numbers (of a NaN the other's), with some sign.
+__device__ __forceinline__ uint32_t max_abs2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 
 // (fp16) What the accumulators of the pieces hold together, times `unit`.
 template <int UP>
@@ -203,7 +214,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       mbar_init(&m->empty_b[s], 1); mbar_init(&m->empty_c[s], 1);
     }
     for (int s = 0; s < XS; ++s) { mbar_init(&m->full_x[s], 1); mbar_init(&m->empty_x[s], 4); }
-    for (int s = 0; s < kFactorsS; ++s) { mbar_init(&m->full_f[s], 1); mbar_init(&m->empty_f[s], 20); }
+    for (int s = 0; s < kFactorsS; ++s) { mbar_init(&m->full_f[s], 1); mbar_init(&m->empty_f[s], 20); mbar_init(&m->full_u[s], 1); }
     mbar_init(&m->bar_g, 1); mbar_init(&m->bar_s, 1); mbar_init(&m->bar_ch, 1); mbar_init(&m->bar_y, 1);
     mbar_init(&m->bar_h, 16); mbar_init(&m->bar_p, 16); mbar_init(&m->bar_u, 16);
     mbar_init(&m->bar_xd, 4); mbar_init(&m->bar_e, 4);
@@ -469,6 +480,40 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       warp_arrive(&m->full_f[slot]);
     }
     if (growth) m->bad = 1;
+  } else if (kF16 && warp == 3) {
+    // ------------------------------------------------------------------ (fp16) units of Xd's pieces
+    // A power of two from the tile's largest |Xd| (up to 2^11: larger ones stay as they are), so that small numbers keep their
+    // bits, and those that decay by far within the tile.  (2 x 3001 tokens, 80 heads: 92.8 us without units; 101.3 with them found by the
+    // warps that make Xd; here 99.9 with eight lanes to a row, 94.9 with a row to a lane, which takes a third of the instructions.)
+    uint32_t xi = 0, xph = 0;
+#pragma unroll 1
+    for (uint32_t n = 0; n < total; ++n) {
+      const uint32_t slot = n % kFactorsS;
+      wait(&m->full_f[slot], (n / kFactorsS) & 1, m);
+      wait(&m->full_x[xi], xph, m);
+      FactorsS& f = m->f[slot];
+      float most = 0.f;
+      const uint32_t at = sX + xi * kBlk + lane * 128 + ((lane & 7) << 4);   // (rows lane, lane + 32, ..., their pieces in an order without conflicts)
+#pragma unroll 1
+      for (int r = 0; r < T; r += 32) {
+        uint32_t x2 = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+          const uint4 a = lds128((at + 128 * r) ^ (k << 4));
+          x2 = max_abs2(x2, max_abs2(max_abs2(a.x, a.y), max_abs2(a.z, a.w)));
+        }
+        const float2 x = unpack2<T16>(x2);
+        most = fmaxf(most, fmaxf(fabsf(x.x), fabsf(x.y)) * fabsf(f.xw[lane + r]));
+      }
+      most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most)));
+      if (lane == 0) {
+        const float unit = fminf(power_below(most), 2048.f);
+        f.x_scale = inverse_power(unit) * 2048.f;
+        f.x_unit = unit * (1.f / 2048.f) * f.unit;
+        mbar_arrive(&m->full_u[slot]);
+      }
+      if (++xi == XS) { xi = 0; xph ^= 1; }
+    }
   } else if (warp >= 4 && warp < 20) {
     // ------------------------------------------------------------------ warps 4-19: P and the state
     const int J = (warp - 4) >> 2;       // tokens 32 J .. 32 J + 31 as columns of P, columns 16 J .. 16 J + 15 of the state
@@ -727,7 +772,12 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (acomp != acomp) acomp = 0.f;   // (a sum of -inf stays that)
         asum = tk;
       }
-      const float gs = f.g, su = f.unit;
+      const float gs = f.g;
+      float su = 1.f;
+      if constexpr (kF16) {
+        wait(&m->full_u[slot], (n / kFactorsS) & 1, m);
+        su = f.x_unit;
+      }
       wait(&m->bar_s, n & 1, m);
       tc_fence_after();
       if (owns_state) {
@@ -783,17 +833,18 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     for (uint32_t k = 0; k <= total; ++k) {   // Xd of tile k, Y of tile k - 1
       if (k < total) {
         const uint32_t slot = k % kFactorsS;
-        wait(&m->full_f[slot], (k / kFactorsS) & 1, m);
+        wait(kF16 ? &m->full_u[slot] : &m->full_f[slot], (k / kFactorsS) & 1, m);   // (warp 3 has waited for the others)
         wait(&m->full_x[bi], bph, m);
         if (k > 0) wait(&m->bar_s, (k - 1) & 1, m);   // the S MMAs have read the Xd before this one
         // eight lanes share a row (one 16-byte piece each), a warp moves four rows per instruction
         const uint32_t xb = sX + bi * kBlk, pc = (uint32_t)lane & 7u;
         const FactorsS& f = m->f[slot];
+        const float scale = kF16 ? f.x_scale : 1.f;
 #pragma unroll 2
         for (int i = 0; i < 8; ++i) {
           const uint32_t r = 32 * q + 4 * i + ((uint32_t)lane >> 3), at = r * 128 + ((pc ^ (r & 7u)) << 4);
           const uint4 a = lds128(xb + at);
-          const float w = f.xw[r];
+          const float w = f.xw[r] * scale;
           const uint64_t w2 = pair(w, w);
           const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
           uint32_t p0[4], p1[4], p2[4];
