@@ -119,6 +119,15 @@ void resolve_segments(const SsdArgs* a, int kernel, bool split, int* nseg, int* 
   *nseg = (a->seqlen + len - 1) / len;
 }
 
+// The segments of the recurrence behind the tensor-core kernel at fp32 precision: its own, up to a head for every other SM.  Beyond,
+// whole sequences take less (n 128, 3001 tokens: 24, 48 and 64 heads 353, 685 and 839 us cut, 950, 1 019 and 1 037 whole; 80, 120 and
+// 160: 1 156, 1 623 and 2 264 cut, 1 046, 1 057 and 1 946 whole; n 64, 20 001 tokens: 64 heads 3 551 and 3 940, 80 4 760 and 4 006).
+void redo_segments(const SsdArgs* a, int* nseg, int* seg_len) {
+  *nseg = 1;
+  if (2 * (int64_t)a->batch * a->nheads <= kSmCount) resolve_segments(a, SSD_KERNEL_SCAN_F32, false, nseg, seg_len);
+  if (*nseg == 1) *seg_len = (int)align_up(a->seqlen, ssd::scan_f32_tile_tokens());
+}
+
 int chain_mode(const SsdArgs* a, int kernel, bool split, int nseg) {
   return split || kernel == SSD_KERNEL_TCGEN05 ? ssd::tc_chain_mode(*a, nseg, tc_units(a, split)) : 0;
 }
@@ -126,6 +135,20 @@ int chain_mode(const SsdArgs* a, int kernel, bool split, int nseg) {
 // Scratch of a launch that hands states from CTA to CTA: one slot per CTA and head of the pair -- state, log-decay sum, ready flag.
 constexpr size_t kSlots = 2 * (size_t)kSmCount;
 size_t chain_bytes(size_t np) { return align_up(kSlots * np * sizeof(float), 256) + 2 * align_up(kSlots * sizeof(float), 256); }
+
+// Scratch of the two passes over cut sequences: segment states and log-decay sums, and the states entering the segments (`keep`) or
+// those written over the former.
+size_t two_pass_bytes(const SsdArgs* a, int nseg, bool keep) {
+  const size_t units = (size_t)a->batch * a->nheads, np = (size_t)a->dstate * a->headdim;
+  return (keep ? 2 : 1) * align_up(units * nseg * np * sizeof(float), 256) + align_up(units * nseg * sizeof(float), 256);
+}
+
+// Scratch of the tensor-core kernel at fp32 precision and the recurrence behind it, which do not need theirs at the same time.
+size_t split_bytes(const SsdArgs* a, int chain, int redo_nseg) {
+  const size_t np = (size_t)a->dstate * a->headdim;
+  return ssd::RedoWords::kBytes +
+         std::max(chain != 0 ? chain_bytes(np) : 0, redo_nseg > 1 ? two_pass_bytes(a, redo_nseg, false) : 0);
+}
 
 bool strides_mult(const int64_t* s, int m) { return s[0] % m == 0 && s[1] % m == 0 && s[2] % m == 0; }
 
@@ -223,13 +246,14 @@ size_t ssd_b200_workspace_bytes(const SsdArgs* args) {
   const bool split = use_split(args, kernel);
   int nseg, seg_len;
   resolve_segments(args, kernel, split, &nseg, &seg_len);
-  const size_t redo = split ? align_up(kSmCount * sizeof(int32_t), 256) : 0;   // a word per CTA
-  if (nseg <= 1) return redo;
-  const size_t units = (size_t)args->batch * args->nheads;
-  const size_t np = (size_t)args->dstate * args->headdim;
-  if (chain_mode(args, kernel, split, nseg) != 0) return chain_bytes(np) + redo;
-  // two passes: zero-start segment states, states entering the segments, segment log-decay sums
-  return 2 * align_up(units * nseg * np * sizeof(float), 256) + align_up(units * nseg * sizeof(float), 256);
+  const int chain = chain_mode(args, kernel, split, nseg);
+  if (split) {
+    int redo_nseg, redo_len;
+    redo_segments(args, &redo_nseg, &redo_len);
+    return split_bytes(args, chain, redo_nseg);
+  }
+  if (nseg <= 1) return 0;
+  return chain != 0 ? chain_bytes((size_t)args->dstate * args->headdim) : two_pass_bytes(args, nseg, true);
 }
 
 // The forward proper.  `fuse_epilogue`: the selected kernel applies D / Z itself; otherwise they are dropped here
@@ -269,41 +293,47 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
   whole.finld_unit_stride = 1;
   if (nseg <= 1 && !split) return launch_kernel(kernel, args, whole, stream);
 
-  const size_t need = ssd_b200_workspace_bytes(args);
-  if (!args->workspace || args->workspace_bytes < need) return SSD_ERR_WORKSPACE;
+  if (!args->workspace || args->workspace_bytes < ssd::least_workspace(args)) return SSD_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(args->workspace) & 255) return SSD_ERR_MISALIGNED;
   const int chain = chain_mode(args, kernel, split, nseg);
   if (chain != 0 || split) {
     // one launch: the pieces of a sequence pass their state through the workspace (see chain_bytes())
     char* ws = static_cast<char*>(args->workspace);
     ssd::ScanParams pc = whole;
+    if (split) {
+      pc.redo = reinterpret_cast<int32_t*>(ws);
+      ws += ssd::RedoWords::kBytes;
+    }
     if (chain != 0) {
       pc.chain = chain;
       pc.chain_state = reinterpret_cast<float*>(ws);
       pc.chain_ld = reinterpret_cast<float*>(ws + align_up(kSlots * np * sizeof(float), 256));
       pc.chain_flag = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(pc.chain_ld) + align_up(kSlots * sizeof(float), 256));   // (cleared by the launch)
-      ws += chain_bytes(np);
     }
     if (!split) return launch_kernel(kernel, args, pc, stream);
-    pc.redo = reinterpret_cast<int32_t*>(ws);
     rc = ssd::launch_split(*args, pc, stream);
-    whole.nseg = 1;
-    whole.seg_len = (int)align_up(args->seqlen, ssd::scan_f32_tile_tokens());
     if (rc == SSD_OK) {
+      // the recurrence, where the call has to be done again: in segments, if there is scratch for them
+      redo_segments(args, &nseg, &seg_len);
+      if (args->workspace_bytes < split_bytes(args, chain, nseg)) nseg = 1, seg_len = (int)align_up(args->seqlen, ssd::scan_f32_tile_tokens());
+      whole.nseg = nseg;
+      whole.seg_len = seg_len;
       whole.redo = pc.redo;
       whole.redo_n = ssd::split_grid(*args, chain);
-    } else if (rc != SSD_ERR_UNSUPPORTED) {
-      return rc;
+      whole.chain_state = reinterpret_cast<float*>(ws);
+      whole.chain_ld = reinterpret_cast<float*>(ws + align_up((size_t)units * nseg * np * sizeof(float), 256));
+      return ssd::launch_scan_f32(whole, args->dtype, stream);
     }
-    if (whole.redo || (!whole.D && !whole.Z)) return ssd::launch_scan_f32(whole, args->dtype, stream);
-    ssd::ScanParams ep = whole;
-    whole.D = nullptr, whole.Z = nullptr;
-    rc = ssd::launch_scan_f32(whole, args->dtype, stream);
-    return rc != SSD_OK ? rc : ssd::launch_epilogue(ep, args->dtype, stream);
+    if (rc != SSD_ERR_UNSUPPORTED) return rc;
+    SsdArgs scan = *args;   // (strides that a tensor map cannot have)
+    scan.kernel = SSD_KERNEL_SCAN_F32;
+    if (args->workspace_bytes < ssd_b200_workspace_bytes(&scan)) scan.nsegments = 1;
+    if (!whole.D && !whole.Z) scan.D = nullptr, scan.Z = nullptr;   // (the caller of this applies them)
+    return ssd_b200_forward(&scan, stream);
   }
 
   float* seg_states = static_cast<float*>(args->workspace);
-  const size_t st_bytes = align_up((size_t)units * nseg * np * sizeof(float), 256);
+  const size_t st_bytes = align_up((size_t)units * nseg * np * sizeof(float), 256);   // (see two_pass_bytes())
   float* seg_in = reinterpret_cast<float*>(static_cast<char*>(args->workspace) + st_bytes);
   float* seg_ld = reinterpret_cast<float*>(static_cast<char*>(args->workspace) + 2 * st_bytes);
 
@@ -368,3 +398,13 @@ int ssd_b200_fold_states(const float* states, int64_t states_shard_stride, const
 }
 
 }  // extern "C"
+
+size_t ssd::least_workspace(const SsdArgs* args) {
+  const size_t need = ssd_b200_workspace_bytes(args);
+  if (need == 0) return 0;
+  const int kernel = resolve_kernel(args);
+  if (!use_split(args, kernel)) return need;
+  int nseg, seg_len;
+  resolve_segments(args, kernel, true, &nseg, &seg_len);
+  return split_bytes(args, chain_mode(args, kernel, true, nseg), 1);
+}

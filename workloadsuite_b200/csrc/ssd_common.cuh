@@ -21,6 +21,11 @@ enum : int {
   STATUS_WAIT_TIMEOUT_CHAIN = 6  // a bounded wait for the previous segment of a chained sequence ran out
 };
 
+// Words of ScanParams::redo: one per CTA of the tensor-core kernel at fp32 precision, and the counters of the scan behind it.
+struct RedoWords {
+  static constexpr int kNext = 148, kScanned = 149, kFolded = 150, kBytes = 768;
+};
+
 // One launch of a scan over [seg_begin, seg_end) of every (batch, head) unit.
 // Strides are in elements.  "unit" = batch * nheads + head.
 struct ScanParams {
@@ -52,7 +57,8 @@ struct ScanParams {
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], cleared by the launch
   // The tensor-core kernel at fp32 precision writes a word per CTA: not 0 if the fp32 scan has to do the call again.  The scan, when
-  // given them (redo_n of them), starts beside that kernel's end and leaves at once if all are 0.
+  // given them (redo_n of them), starts beside that kernel's end and leaves at once if all are 0; cut sequences' segment states and
+  // log-decay sums are then in chain_state and chain_ld, [unit][segment].
   int32_t* redo;
   int redo_n;
   // Optional epilogue Y <- (Y + x * D[head]) * silu(z) (model_ref.py:116-118); either pointer may be null.
@@ -140,5 +146,6 @@ bool split_fuses_epilogue(const SsdArgs& a);
 int split_grid(const SsdArgs& a, int chain);   // CTAs, each of which writes its word of ScanParams::redo
 int launch_split(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);   // SSD_ERR_UNSUPPORTED: nothing was enqueued
 
+size_t least_workspace(const SsdArgs* a);   // what the call can do with (ssd_b200_workspace_bytes(): what it asks for)
 
 }  // namespace ssd

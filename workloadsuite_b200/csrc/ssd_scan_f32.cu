@@ -126,8 +126,113 @@ __device__ __forceinline__ void reduce_scatter(float (&v)[U], int sl) {
 // FULL: the state has exactly NS * SL rows (the strides of B and C in shared memory are then constants).
 // LINE: tokens worked on in line (1: one after the other).  CTAS: as many of an SM the registers have to leave room for (0: as
 // it comes).  Tokens in line take 64 to 126 registers, one after the other 32 to 80; see launch_one().
-// REDO: behind the tensor-core kernel at fp32 precision (ssd_split.cu), all heads in as many CTAs as the chip holds, and only if that
-// kernel says so.
+// REDO: behind the tensor-core kernel at fp32 precision (ssd_split.cu), and only if that kernel says so; see Jobs.
+// A piece of a scan.
+struct Job {
+  int unit, seg;
+  bool compute_y;
+  const float* init;   // or null
+  float* fin;          // or null
+  float* fin_ld;       // or null
+};
+
+// What the two passes and the fold of cut sequences do (or whole sequences one after the other), in one launch of as many CTAs as
+// the chip holds, which take numbers from a counter: first every segment from a zero state, then the states entering the
+// segments (256 elements a time, written over what they are made of), then every segment again.  What a number waits for has
+// lower ones, which CTAs that run already have taken, so no wait needs a CTA that is still to come.  The counters are behind the
+// words that say whether there is anything to do (RedoWords), cleared by the kernel ahead.
+struct Jobs {
+  const ScanParams& p;
+  unsigned* number;   // of the present job, in shared memory: what a job is is worked out again at its end, for the registers
+
+  __device__ __forceinline__ bool cut() const { return p.nseg > 1; }
+  __device__ __forceinline__ int64_t np() const { return (int64_t)p.n * p.p; }
+  __device__ __forceinline__ unsigned units() const { return (unsigned)(p.batch * p.nheads); }
+  __device__ __forceinline__ unsigned segs() const { return units() * (unsigned)p.nseg; }
+  __device__ __forceinline__ unsigned parts() const { return (unsigned)((np() + kThreads - 1) / kThreads); }
+  __device__ __forceinline__ unsigned first() const { return cut() ? segs() : 0; }             // number of the first fold,
+  __device__ __forceinline__ unsigned second() const { return cut() ? segs() + units() * parts() : 0; }   // of the second pass
+  // To the next one, or false.  All threads of the CTA.
+  __device__ __forceinline__ bool next() const {
+    while (true) {
+      if (threadIdx.x == 0) {
+        unsigned t = atomicAdd(reinterpret_cast<unsigned*>(p.redo + RedoWords::kNext), 1u);
+        if (t >= second() + segs()) t = ~0u;
+        else if (cut() && t >= second()) t = finished(RedoWords::kFolded, second() - first()) ? t : ~0u;
+        else if (cut() && t >= first()) t = finished(RedoWords::kScanned, first()) ? t : ~0u;
+        *number = t;
+      }
+      __syncthreads();
+      const unsigned t = *number;
+      if (t == ~0u) return false;
+      if (t < first() || t >= second()) return true;
+      fold((t - first()) / parts(), (t - first()) % parts());
+      done(RedoWords::kFolded);
+    }
+  }
+  __device__ __forceinline__ Job job() const {
+    const unsigned t = *static_cast<volatile unsigned*>(number);
+    const bool again = t >= second();
+    const unsigned i = again ? t - second() : t, seg = i / units(), unit = i - seg * units();   // (the units of a segment share B and C)
+    Job j = {(int)unit, (int)seg, again, nullptr, nullptr, nullptr};
+    const int64_t at = (int64_t)unit * p.nseg + seg;
+    if (!again) {
+      j.fin = p.chain_state + at * np();
+      j.fin_ld = p.chain_ld + at;
+    } else if (cut()) {
+      j.init = p.chain_state + at * np();
+    } else {
+      if (p.init) j.init = p.init + unit * np();
+      if (p.fin) j.fin = p.fin + unit * np();
+      if (p.fin_ld) j.fin_ld = p.fin_ld + unit;
+    }
+    return j;
+  }
+  // Behind the last write of a job.  All threads of the CTA.
+  __device__ __forceinline__ void scanned() const {
+    if (*number < first()) done(RedoWords::kScanned);
+  }
+  __device__ __forceinline__ void done(int word) const {
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.redo + word) : "memory");
+  }
+  // (bounded: by what a wait may take, and ten microseconds for each token of a segment)
+  __device__ __forceinline__ bool finished(int word, unsigned count) const {
+    const long long t0 = clock64(), limit = p.wait_clocks + 20000LL * p.seg_len;
+    while (true) {
+      unsigned n;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(p.redo + word) : "memory");
+      if (n >= count) return true;
+      __nanosleep(100);
+      if (clock64() - t0 > limit) {
+        if (p.status) atomicCAS(p.status, 0, (int)STATUS_WAIT_TIMEOUT_CHAIN);
+        return false;
+      }
+    }
+  }
+  // As ssd_fold_kernel below.
+  __device__ __forceinline__ void fold(unsigned unit, unsigned part) const {
+    const int64_t e = (int64_t)part * kThreads + threadIdx.x;
+    const float* D = p.chain_ld + (int64_t)unit * p.nseg;
+    const int64_t np = this->np();
+    if (e < np) {
+      float run = p.init ? p.init[unit * np + e] : 0.f;
+      float* F = p.chain_state + (int64_t)unit * p.nseg * np + e;
+      for (int s = 0; s < p.nseg; ++s) {
+        const float f = __ldcg(F + s * np);
+        F[s * np] = run;
+        run = fmaf(run, expf(__ldcg(D + s)), f);
+      }
+      if (p.fin) p.fin[unit * np + e] = run;
+    }
+    if (p.fin_ld && part == 0 && threadIdx.x == 0) {
+      double tot = 0.0;
+      for (int s = 0; s < p.nseg; ++s) tot += (double)__ldcg(D + s);
+      p.fin_ld[unit] = (float)tot;
+    }
+  }
+};
+
 template <typename T, int NS, int P, bool FULL, int LINE, int CTAS, bool REDO>
 __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const ScanParams prm, const int tile) {
   constexpr int SL = kThreads / P;  // lanes sharing one state column
@@ -141,7 +246,6 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
   float* dec = Ys + tile * P;        // [tile]  exp(a_t)
   float* araw = dec + tile;          // [tile]  a_t
 
-  int unit = blockIdx.x;
   if constexpr (REDO) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int any = 0;
@@ -149,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
     if (!__syncthreads_or(any)) {   // (that kernel leaves the sum of the log-decays to this one: in 64 bits, as below)
       if (!prm.fin_ld) return;
       double* part = reinterpret_cast<double*>(smem);
-      for (; unit < prm.batch * prm.nheads; unit += gridDim.x) {
+      for (int unit = blockIdx.x; unit < prm.batch * prm.nheads; unit += gridDim.x) {
         const float* A = prm.A + (int64_t)(unit / prm.nheads) * prm.as[0] + (int64_t)(unit % prm.nheads) * prm.as[2];
         double sum = 0.0;
         for (int t = threadIdx.x; t < prm.seqlen; t += kThreads) sum += (double)A[(int64_t)t * prm.as[1]];
@@ -165,8 +269,17 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
       return;
     }
   }
-  const int seg = REDO ? 0 : blockIdx.y;
+  __shared__ unsigned number;
+  const Jobs jobs = {prm, &number};
+  Job job = {};
+  int unit = blockIdx.x, seg = blockIdx.y;
+  if (REDO && !jobs.next()) return;
   do {
+  if constexpr (REDO) {
+    job = jobs.job();
+    unit = job.unit;
+    seg = job.seg;
+  }
   const int bi = unit / prm.nheads, hi = unit - bi * prm.nheads;
   const int gi = hi / (prm.nheads / prm.ngroups);
   const int tid = threadIdx.x;
@@ -184,14 +297,14 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
   T* Yg = prm.Y ? static_cast<T*>(prm.Y) + bi * prm.ys[0] + hi * prm.ys[2] : nullptr;
 
   float h[NS];
-  if (prm.init) {
-    const float* I = prm.init + unit * prm.init_unit_stride + seg * prm.init_seg_stride;
+  if (REDO ? job.init != nullptr : prm.init != nullptr) {
+    const float* I = REDO ? job.init : prm.init + unit * prm.init_unit_stride + seg * prm.init_seg_stride;
 #pragma unroll
     for (int k = 0; k < NS4; ++k)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int ni = (k * SL + sl) * 4 + q;
-        h[k * 4 + q] = (ni < n) ? I[(int64_t)ni * P + j] : 0.f;
+        h[k * 4 + q] = (ni < n) ? (REDO ? __ldcg(I + (int64_t)ni * P + j) : I[(int64_t)ni * P + j]) : 0.f;
       }
   } else {
 #pragma unroll
@@ -205,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
     constexpr int kAhead = LINE == 1 ? 1 : 4;
     stage_rows<T, kAhead>(Xg + (int64_t)t0 * prm.xs[1], prm.xs[1], rows, P, Xs, vec_ok, tid);
     stage_rows<T, kAhead>(Bg + (int64_t)t0 * prm.bs[1], prm.bs[1], rows, n, Bs, vec_ok, tid);
-    if (prm.compute_y) stage_rows<T, kAhead>(Cg + (int64_t)t0 * prm.cs[1], prm.cs[1], rows, n, Cs, vec_ok, tid);
+    if (REDO ? job.compute_y : prm.compute_y) stage_rows<T, kAhead>(Cg + (int64_t)t0 * prm.cs[1], prm.cs[1], rows, n, Cs, vec_ok, tid);
     if (tid < rows) {
       const float a = Ag[(int64_t)(t0 + tid) * prm.as[1]];
       araw[tid] = a;
@@ -278,27 +391,29 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
         for (; t + LINE <= rows; t += LINE) tokens(t, std::integral_constant<int, LINE>{}, want_y);
       for (; t < rows; ++t) tokens(t, std::integral_constant<int, 1>{}, want_y);
     };
-    if (prm.compute_y) all(std::true_type{});
+    if (REDO ? job.compute_y : prm.compute_y) all(std::true_type{});
     else all(std::false_type{});
-    if (tid == 0 && prm.fin_ld) {
+    if (tid == 0 && (REDO && prm.nseg > 1 ? !job.compute_y : prm.fin_ld != nullptr)) {
       for (int t = 0; t < rows; ++t) asum += (double)araw[t];
     }
-    if (sizeof(T) < 4 && prm.compute_y) {
+    if (sizeof(T) < 4 && (REDO ? job.compute_y : prm.compute_y)) {
       __syncthreads();
       T* Yt = Yg + (int64_t)t0 * prm.ys[1];
       if constexpr (REDO) {   // with the skip and the gate, which that kernel applies too
         const T* Zg = prm.Z ? static_cast<const T*>(prm.Z) + bi * prm.zs[0] + hi * prm.zs[2] + (int64_t)t0 * prm.zs[1] : nullptr;
-        for (int i = tid; (prm.D || Zg) && i < rows * P; i += kThreads) {
-          const int r = i / P, c = i - r * P;
-          float v = Ys[i];
-          if (prm.D) v = fmaf(Cvt<T>::to_f(Xg[(int64_t)(t0 + r) * prm.xs[1] + c]), load_skip<T>(prm, hi), v);
-          if (Zg) {
-            const float z = Cvt<T>::to_f(Zg[(int64_t)r * prm.zs[1] + c]);
-            v *= z / (1.f + __expf(-z));
+        if (prm.D || Zg) {
+          for (int i = tid; i < rows * P; i += kThreads) {
+            const int r = i / P, c = i - r * P;
+            float v = Ys[i];
+            if (prm.D) v = fmaf(Cvt<T>::to_f(Xg[(int64_t)(t0 + r) * prm.xs[1] + c]), load_skip<T>(prm, hi), v);
+            if (Zg) {
+              const float z = Cvt<T>::to_f(Zg[(int64_t)r * prm.zs[1] + c]);
+              v *= z / (1.f + __expf(-z));
+            }
+            Ys[i] = v;
           }
-          Ys[i] = v;
+          __syncthreads();
         }
-        __syncthreads();
       }
       if (vec_ok) {
         constexpr int per_row = P >> 3;
@@ -315,8 +430,9 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
     }
   }
 
-  if (prm.fin) {
-    float* F = prm.fin + unit * prm.fin_unit_stride + seg * prm.fin_seg_stride;
+  if constexpr (REDO) job = jobs.job();
+  if (REDO ? job.fin != nullptr : prm.fin != nullptr) {
+    float* F = REDO ? job.fin : prm.fin + unit * prm.fin_unit_stride + seg * prm.fin_seg_stride;
 #pragma unroll
     for (int k = 0; k < NS4; ++k)
 #pragma unroll
@@ -325,9 +441,10 @@ __global__ void __launch_bounds__(kThreads, CTAS) ssd_scan_f32_kernel(const Scan
         if (ni < n) F[(int64_t)ni * P + j] = h[k * 4 + q];
       }
   }
-  if (prm.fin_ld && tid == 0)
-    prm.fin_ld[unit * prm.finld_unit_stride + seg * prm.finld_seg_stride] = (float)asum;
-  } while (REDO && (unit += gridDim.x) < prm.batch * prm.nheads);
+  if ((REDO ? job.fin_ld : prm.fin_ld) && tid == 0)
+    *(REDO ? job.fin_ld : prm.fin_ld + unit * prm.finld_unit_stride + seg * prm.finld_seg_stride) = (float)asum;
+  if constexpr (REDO) jobs.scanned();
+  } while (REDO && jobs.next());
 }
 
 // H_in(seg) for every segment of every unit, from the zero-start final states:
@@ -397,8 +514,9 @@ int launch_one(const ScanParams& prm, cudaStream_t stream) {
   bool early = false;
   if constexpr (k16 && P == 64 && NS >= 16) {
     if (prm.redo) {
-      if (!full || prm.nseg != 1) return SSD_ERR_UNSUPPORTED;
-      kern = ssd_scan_f32_kernel<T, NS, P, true, kLine, 0, true>;
+      if (!full || tokens < kLine) return SSD_ERR_UNSUPPORTED;
+      kern = many && (NS <= 16 || tokens < 16) ? ssd_scan_f32_kernel<T, NS, P, true, kLine, kMany, true>
+                                               : ssd_scan_f32_kernel<T, NS, P, true, kLine, 0, true>;
       early = true;
     }
   }

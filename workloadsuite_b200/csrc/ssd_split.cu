@@ -15,7 +15,8 @@
 // What cannot be done this way is left to the recurrence: a CTA that meets a number that is not finite (0 * inf in a masked
 // place would reach tokens before its own; an fp16 piece overflows at 65 504) or a log-decay above zero that a tile's factors
 // may not carry says so in `redo`, and the recurrence, launched behind this kernel, does the call again; otherwise that
-// launch ends at once (and sums the log-decays over the sequence where the caller wants that).
+// launch ends at once (and sums the log-decays over the sequence where the caller wants that).  It cuts sequences as it would
+// have by itself.
 //
 // Roles (768 threads), one tile of 128 tokens after the other as one pipeline:
 //   warp 0        TMA producer
@@ -197,6 +198,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   const ScanParams& sp = prm.sp;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int32_t* status = sp.status;
+  if (blockIdx.x == 0 && tid == 0) sp.redo[RedoWords::kNext] = sp.redo[RedoWords::kScanned] = sp.redo[RedoWords::kFolded] = 0;
   if (smem_u32(smem) & 1023u) {
     if (tid == 0) {
       if (status) atomicCAS(status, 0, (int)STATUS_BAD_SMEM_ALIGNMENT);

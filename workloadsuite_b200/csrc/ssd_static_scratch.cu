@@ -51,7 +51,7 @@ int ssd_b200_forward_static_scratch(const SsdArgs* args, void* stream) {
   SsdArgs a = *args;
   a.workspace = nullptr;
   a.workspace_bytes = 0;
-  const size_t need = ssd_b200_workspace_bytes(&a);  // 0 for invalid arguments: the forward reports those
+  const size_t need = ssd::least_workspace(&a);  // 0 for invalid arguments: the forward reports those
   if (need > kStaticScratchBytes) return SSD_ERR_TOO_LARGE;
   if (need > 0) {
     void* scratch = nullptr;
