@@ -520,6 +520,34 @@ def test_a_call_that_is_done_again_takes_what_the_recurrence_takes(b, s, h, n):
     assert ms[0] < 1.4 * ms[1]
 
 
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("b,s,h,n", [(1, 4099, 37, 128), (2, 3001, 80, 64), (1, 700, 1, 128), (2, 300, 4, 64)])
+def test_scratch_asked_for_by_shape_is_enough_for_a_call_of_the_recurrence(b, s, h, n, offset):
+    """A size asked for without pointers, as the sizing of a pipeline's scratch does; the state leaves where it entered, or is only
+    4-byte aligned as well, which makes the call the recurrence's: in segments of its own (37 heads, one) or whole (160)."""
+    import ctypes
+
+    import workloadsuite_b200 as W
+    from workloadsuite_b200 import _lib
+    from workloadsuite_b200.ssd import _fill
+
+    d = {k: v.to(DEV) for k, v in O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=1, dtype=torch.bfloat16, init=True, seed=87,
+                                                decay_scale=0.1).items()}
+    args, lib = _lib.SsdArgs(), _lib.load()
+    _fill(args, d["X"], d["A"], d["B"], d["C"], None, None, None, None, None, 1, None, 0, False)
+    for name in ("X", "A", "B", "C"):
+        setattr(args, name, None)
+    size = int(lib.ssd_b200_workspace_bytes(ctypes.byref(args)))
+    state = torch.empty(b * h * n * 64 + 4, device=DEV)[offset:offset + b * h * n * 64].view(b, h, n, 64).copy_(d["initial_states"])
+    Y, ws = torch.empty_like(d["X"]), torch.empty(max(size, 1), dtype=torch.uint8, device=DEV)
+    _fill(args, d["X"], d["A"], d["B"], d["C"], None, state, Y, state, None, 1, None, 0, False)
+    args.workspace, args.workspace_bytes = ws.data_ptr(), size
+    assert lib.ssd_b200_forward(ctypes.byref(args), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    want = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, initial_states=d["initial_states"], return_final_state=True,
+                         kernel="scan_f32", nsegments=1 if b * h > 74 else None)
+    assert torch.equal(Y, want[0]) and torch.equal(state, want[1])
+
+
 def test_scratch_of_calls_on_two_streams_is_their_own():
     import workloadsuite_b200 as W
 

@@ -92,6 +92,16 @@ bool use_split(const SsdArgs* a, int kernel) {
          ssd::split_supports(*a) && !outputs_on_inputs(a);
 }
 
+// The same as a query without pointers sees it.
+bool split_by_shape(const SsdArgs* a) {
+  SsdArgs s = *a;
+  s.X = s.B = s.C = s.dt = nullptr;
+  s.A = s.initial_state = nullptr;
+  s.Y = nullptr;
+  s.final_state = nullptr;
+  return use_split(&s, resolve_kernel(&s));
+}
+
 // What the kernels that run these arguments work on: pairs of heads, or heads.
 int64_t tc_units(const SsdArgs* a, bool split) { return split ? (int64_t)a->batch * a->nheads : ssd::tc2_units(*a); }
 
@@ -148,6 +158,14 @@ size_t split_bytes(const SsdArgs* a, int chain, int redo_nseg) {
   const size_t np = (size_t)a->dstate * a->headdim;
   return ssd::RedoWords::kBytes +
          std::max(chain != 0 ? chain_bytes(np) : 0, redo_nseg > 1 ? two_pass_bytes(a, redo_nseg, false) : 0);
+}
+
+// What a call of the tensor-core kernel at fp32 precision asks for.
+size_t ask_by_shape(const SsdArgs* a) {
+  int nseg, seg_len, redo_nseg, redo_len;
+  resolve_segments(a, SSD_KERNEL_SCAN_F32, true, &nseg, &seg_len);
+  redo_segments(a, &redo_nseg, &redo_len);
+  return split_bytes(a, chain_mode(a, SSD_KERNEL_SCAN_F32, true, nseg), redo_nseg);
 }
 
 bool strides_mult(const int64_t* s, int m) { return s[0] % m == 0 && s[1] % m == 0 && s[2] % m == 0; }
@@ -246,19 +264,15 @@ size_t ssd_b200_workspace_bytes(const SsdArgs* args) {
   const bool split = use_split(args, kernel);
   int nseg, seg_len;
   resolve_segments(args, kernel, split, &nseg, &seg_len);
-  const int chain = chain_mode(args, kernel, split, nseg);
-  if (split) {
-    int redo_nseg, redo_len;
-    redo_segments(args, &redo_nseg, &redo_len);
-    return split_bytes(args, chain, redo_nseg);
-  }
+  if (split) return ask_by_shape(args);
   if (nseg <= 1) return 0;
-  return chain != 0 ? chain_bytes((size_t)args->dstate * args->headdim) : two_pass_bytes(args, nseg, true);
+  return chain_mode(args, kernel, split, nseg) != 0 ? chain_bytes((size_t)args->dstate * args->headdim) : two_pass_bytes(args, nseg, true);
 }
 
 // The forward proper.  `fuse_epilogue`: the selected kernel applies D / Z itself; otherwise they are dropped here
 // and ssd_b200_forward() runs the stand-alone epilogue kernel afterwards.
-static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue) {
+// `fold_in_place`: the states entering the segments are written over those they are made of, in half the scratch.
+static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue, bool fold_in_place) {
   int rc = validate(args);
   if (rc != SSD_OK) return rc;
   rc = validate_pointers(args);
@@ -293,7 +307,8 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
   whole.finld_unit_stride = 1;
   if (nseg <= 1 && !split) return launch_kernel(kernel, args, whole, stream);
 
-  if (!args->workspace || args->workspace_bytes < ssd::least_workspace(args)) return SSD_ERR_WORKSPACE;
+  if (!args->workspace || args->workspace_bytes < (fold_in_place ? two_pass_bytes(args, nseg, false) : ssd::least_workspace(args)))
+    return SSD_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(args->workspace) & 255) return SSD_ERR_MISALIGNED;
   const int chain = chain_mode(args, kernel, split, nseg);
   if (chain != 0 || split) {
@@ -334,8 +349,8 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue)
 
   float* seg_states = static_cast<float*>(args->workspace);
   const size_t st_bytes = align_up((size_t)units * nseg * np * sizeof(float), 256);   // (see two_pass_bytes())
-  float* seg_in = reinterpret_cast<float*>(static_cast<char*>(args->workspace) + st_bytes);
-  float* seg_ld = reinterpret_cast<float*>(static_cast<char*>(args->workspace) + 2 * st_bytes);
+  float* seg_in = fold_in_place ? seg_states : reinterpret_cast<float*>(static_cast<char*>(args->workspace) + st_bytes);
+  float* seg_ld = reinterpret_cast<float*>(static_cast<char*>(args->workspace) + (fold_in_place ? 1 : 2) * st_bytes);
 
   // pass 1: every segment from a zero state, state and log-decay sum only
   if (!(args->flags & SSD_FLAG_REUSE_SEGMENTS)) {
@@ -375,13 +390,27 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
   int rc = validate(args);
   if (rc != SSD_OK) return rc;
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
-  if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false);
+  // An output on an input, or states that are not 16-byte aligned, make a call the recurrence's that by its shape is the tensor-core
+  // kernel's: it does with the scratch that the shape asked for, in the segments that it would be done again in.
+  SsdArgs scan = *args;
+  bool in_place = false;
+  if (!use_split(args, resolve_kernel(args)) && split_by_shape(args)) {
+    const size_t own = ssd_b200_workspace_bytes(args), given = args->workspace ? args->workspace_bytes : 0;
+    if (given < own && given >= ask_by_shape(args)) {
+      int seg_len;
+      scan.kernel = SSD_KERNEL_SCAN_F32;
+      redo_segments(args, &scan.nsegments, &seg_len);
+      in_place = scan.nsegments > 1;
+      args = &scan;
+    }
+  }
+  if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false, in_place);
   // skip and gate of model_ref.py:116-118: fused into the tensor-core kernels, a kernel of their own otherwise
   const int kernel = resolve_kernel(args);
   const bool can = kernel == SSD_KERNEL_TCGEN05 ? ssd::tc_supports(*args) && ssd::tc2_fuses_epilogue(*args)
                                                   : use_split(args, kernel) && ssd::split_fuses_epilogue(*args);
   const bool fuse = can && z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
-  rc = forward_impl(args, stream_v, fuse);
+  rc = forward_impl(args, stream_v, fuse, in_place);
   if (rc != SSD_OK || fuse) return rc;
   ssd::ScanParams ep;
   fill_params(args, &ep);
