@@ -548,6 +548,20 @@ def test_scratch_asked_for_by_shape_is_enough_for_a_call_of_the_recurrence(b, s,
     assert torch.equal(Y, want[0]) and torch.equal(state, want[1])
 
 
+@pytest.mark.parametrize("b,s,h,n,nsegments", [(2, 300, 4, 64, 0), (50, 300, 6, 128, 0), (1, 3001, 8, 64, 1)])
+@pytest.mark.parametrize("size", [0, 512])
+def test_whole_sequences_need_no_scratch(size, b, s, h, n, nsegments):
+    """Without any, or with less than the tensor-core kernel can do with: the recurrence over whole sequences, which never needed some."""
+    import workloadsuite_b200 as W
+
+    run, d = _redo_args(b, s, h, n, lambda asked: size, nsegments)
+    assert run() == 0
+    want = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, initial_states=d["initial_states"], return_final_state=True,
+                         return_logdecay=True, kernel="scan_f32", nsegments=1)
+    for got, w in zip((d["Y"], d["H"], d["ld"]), want):
+        assert torch.equal(got, w)
+
+
 def test_scratch_of_calls_on_two_streams_is_their_own():
     import workloadsuite_b200 as W
 

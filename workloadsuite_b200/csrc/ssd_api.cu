@@ -404,6 +404,12 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
       args = &scan;
     }
   }
+  // Without scratch that the tensor-core kernel can do with: the recurrence, which needs none for whole sequences.
+  if (use_split(args, resolve_kernel(args)) &&
+      (!args->workspace || args->workspace_bytes < ssd::least_workspace(args) || (reinterpret_cast<uintptr_t>(args->workspace) & 255))) {
+    scan.kernel = SSD_KERNEL_SCAN_F32;
+    args = &scan;
+  }
   if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false, in_place);
   // skip and gate of model_ref.py:116-118: fused into the tensor-core kernels, a kernel of their own otherwise
   const int kernel = resolve_kernel(args);
