@@ -106,3 +106,23 @@ def test_static_scratch_entry_rejects_oversized_problems():
     Y = torch.empty_like(d["X"])
     rc = _call_static(lib, W, d, 256, 16, Y)
     assert rc == -8 and b"limit" in lib.ssd_b200_strerror(rc)
+
+
+@pytest.mark.parametrize("s,h,cut", [(300, 4, False), (3001, 120, False), (3001, 8, True)])
+def test_static_scratch_entry_shares_nothing_between_whole_sequences(s, h, cut):
+    """Calls that the recurrence does not cut need no scratch of it, on any number of streams: they have its bits.  Cut ones (few heads of
+    many tokens) share the array and run on the tensor cores."""
+    import workloadsuite_b200 as W
+    from workloadsuite_b200 import _lib
+
+    lib = _lib.load()
+    d = {k: v.to(DEV) for k, v in O.make_inputs(b=2, s=s, h=h, p=64, n=64, g=1, dtype=torch.bfloat16, init=True, seed=34,
+                                                decay_scale=0.05).items()}
+    kw = dict(initial_states=d["initial_states"])
+    scan = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, kernel="scan_f32", **kw)
+    split = W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, **kw)
+    assert not torch.equal(scan, split)
+    got = torch.empty_like(scan)
+    rc = _call_static(lib, W, d, 1, None, got, kernel=None)
+    assert rc == 0, _lib.strerror(rc)
+    assert torch.equal(got, split if cut else scan)

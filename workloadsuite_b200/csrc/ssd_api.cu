@@ -443,3 +443,11 @@ size_t ssd::least_workspace(const SsdArgs* args) {
   resolve_segments(args, kernel, true, &nseg, &seg_len);
   return split_bytes(args, chain_mode(args, kernel, true, nseg), 1);
 }
+
+bool ssd::whole_without_scratch(const SsdArgs* args) {
+  if (validate(args) != SSD_OK) return false;
+  const int kernel = resolve_kernel(args);
+  int nseg, seg_len;
+  resolve_segments(args, SSD_KERNEL_SCAN_F32, false, &nseg, &seg_len);
+  return use_split(args, kernel) && nseg == 1;
+}

@@ -147,5 +147,6 @@ int split_grid(const SsdArgs& a, int chain);   // CTAs, each of which writes its
 int launch_split(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);   // SSD_ERR_UNSUPPORTED: nothing was enqueued
 
 size_t least_workspace(const SsdArgs* a);   // what the call can do with (ssd_b200_workspace_bytes(): what it asks for)
+bool whole_without_scratch(const SsdArgs* a);   // asks for some, but without it is the recurrence over whole sequences
 
 }  // namespace ssd

@@ -51,7 +51,9 @@ int ssd_b200_forward_static_scratch(const SsdArgs* args, void* stream) {
   SsdArgs a = *args;
   a.workspace = nullptr;
   a.workspace_bytes = 0;
-  const size_t need = ssd::least_workspace(&a);  // 0 for invalid arguments: the forward reports those
+  // 0 for invalid arguments (the forward reports those), and for whole sequences, which share nothing between calls on two streams:
+  // the tensor-core kernel at fp32 precision would share its words of scratch, so they are the recurrence's.
+  const size_t need = ssd::whole_without_scratch(&a) ? 0 : ssd::least_workspace(&a);
   if (need > kStaticScratchBytes) return SSD_ERR_TOO_LARGE;
   if (need > 0) {
     void* scratch = nullptr;
