@@ -279,6 +279,16 @@ def test_route_of_the_fp32_scan(lib):
     assert need(a) == 0
     a.final_state = (1 << 35) + 4            # the recurrence takes states that are not 16-byte aligned
     assert need(a) == 0
+    a.final_state, a.final_logdecay, a.D, a.dt = 1 << 35, 1 << 36, 1 << 37, 1 << 38
+    a.dt_stride = a.a_stride
+    assert need(a) > 0
+    for field, where in (("final_state", a.C), ("final_logdecay", a.D), ("D", a.Y + 64), ("final_logdecay", a.A), ("final_state", a.dt)):
+        kept = getattr(a, field)
+        setattr(a, field, where)
+        assert need(a) == 0, field
+        setattr(a, field, kept)
+    a.Z, a.z_stride = a.Y, a.y_stride        # the gates, which the recurrence reads ahead of what it writes
+    assert need(a) > 0
 
 
 def _lib_two_pass(lib, a):

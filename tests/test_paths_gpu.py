@@ -562,6 +562,27 @@ def test_whole_sequences_need_no_scratch(size, b, s, h, n, nsegments):
         assert torch.equal(got, w)
 
 
+@pytest.mark.parametrize("again", [False, True])
+@pytest.mark.parametrize("b,s,h,n", [(2, 300, 4, 64), (1, 2001, 18, 128), (40, 300, 5, 128)], ids=["whole", "cut", "too_many_to_fuse"])
+def test_y_written_over_the_gates(b, s, h, n, again):
+    """The gates must be read before Y replaces them, also where the call has to be done by the recurrence: the same Y as elsewhere, to
+    its rounding (another kernel's sums) and that of many tiles' separate skip and gate, 2^-8 each."""
+    import workloadsuite_b200 as W
+
+    d = {k: v.to(DEV) for k, v in O.make_inputs(b=b, s=s, h=h, p=64, n=n, g=1, dtype=torch.bfloat16, init=True, seed=88,
+                                                decay_scale=0.1).items()}
+    if again:
+        d["A"][0, 10:40, 0] = 0.04
+    gen = torch.Generator(DEV).manual_seed(s)
+    D, z = torch.randn(h, generator=gen, device=DEV), (3 * torch.randn(b, s, h, 64, generator=gen, device=DEV)).bfloat16()
+    run = lambda z, out: W.ssd_forward(d["X"], d["A"], d["B"], d["C"], 1, initial_states=d["initial_states"], D=D, z=z, out=out)
+    want = run(z, torch.empty_like(z)).double()
+    out = z.clone()
+    assert run(out, out) is out
+    assert ((out.double() - want).abs() <= 2 ** -6 * want.abs() + 2 ** -8 * want.abs().max()).all()
+    assert ((out.double() - want).norm() / want.norm()).item() < 2 ** -7
+
+
 def test_scratch_of_calls_on_two_streams_is_their_own():
     import workloadsuite_b200 as W
 

@@ -54,30 +54,36 @@ int resolve_kernel(const SsdArgs* a) {
 }
 
 // First and one past the last byte of a tensor's elements.
-void extent(const void* p, const int64_t* st, int n0, int n1, int n2, int inner, int size, uintptr_t* lo, uintptr_t* hi) {
-  *lo = reinterpret_cast<uintptr_t>(p);
-  *hi = *lo + (uintptr_t)(((n0 - 1) * st[0] + (n1 - 1) * st[1] + (n2 - 1) * st[2] + inner) * size);
+struct Range {
+  uintptr_t lo, hi;
+  bool on(const Range& o) const { return lo < o.hi && o.lo < hi; }
+};
+Range range(const void* p, int64_t bytes) {
+  const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+  return {lo, p ? lo + (uintptr_t)bytes : lo};
+}
+Range range(const SsdArgs* a, const void* p, const int64_t* st, int heads, int inner, int size) {
+  return range(p, ((a->batch - 1) * st[0] + (a->seqlen - 1) * st[1] + (heads - 1) * st[2] + inner) * size);
+}
+Range output(const SsdArgs* a) { return range(a, a->Y, a->y_stride, a->nheads, a->headdim, elem_size(a->dtype)); }
+
+// Whether an output may share memory with an input (but for Y and Z): a call that is done again (below) needs its inputs as they were.
+bool outputs_on_inputs(const SsdArgs* a) {
+  const int e = elem_size(a->dtype);
+  const int64_t heads = (int64_t)a->batch * a->nheads, state = heads * a->dstate * a->headdim * 4;
+  const Range fin = range(a->final_state, state), ld = range(a->final_logdecay, heads * 4), y = output(a);
+  const Range in[] = {range(a, a->X, a->x_stride, a->nheads, a->headdim, e),  range(a, a->B, a->b_stride, a->ngroups, a->dstate, e),
+                      range(a, a->C, a->c_stride, a->ngroups, a->dstate, e),  range(a, a->dt, a->dt_stride, a->nheads, 1, e),
+                      range(a, a->A, a->a_stride, a->nheads, 1, 4),           range(a->initial_state, state),
+                      range(a->D, a->nheads * (a->flags & SSD_FLAG_D_IN_DTYPE ? e : 4))};
+  for (const Range& r : in)
+    if (r.on(y) || r.on(fin) || r.on(ld)) return true;
+  const Range z = range(a, a->Z, a->z_stride, a->nheads, a->headdim, e);
+  return z.on(fin) || z.on(ld);
 }
 
-// Whether an output may share memory with an input: a call that is done again (below) needs its inputs as they were.
-bool outputs_on_inputs(const SsdArgs* a) {
-  if (a->initial_state && a->final_state) {
-    const int64_t bytes = (int64_t)a->batch * a->nheads * a->dstate * a->headdim * 4;
-    const intptr_t d = reinterpret_cast<intptr_t>(a->final_state) - reinterpret_cast<intptr_t>(a->initial_state);
-    if (d < bytes && -d < bytes) return true;
-  }
-  if (!a->Y) return false;
-  uintptr_t y0, y1, x0, x1;
-  extent(a->Y, a->y_stride, a->batch, a->seqlen, a->nheads, a->headdim, 2, &y0, &y1);
-  auto on = [&](const void* p, const int64_t* st, int groups, int inner, int size) {
-    if (!p) return false;
-    extent(p, st, a->batch, a->seqlen, groups, inner, size, &x0, &x1);
-    return x0 < y1 && y0 < x1;
-  };
-  return on(a->X, a->x_stride, a->nheads, a->headdim, 2) || on(a->B, a->b_stride, a->ngroups, a->dstate, 2) ||
-         on(a->C, a->c_stride, a->ngroups, a->dstate, 2) || on(a->dt, a->dt_stride, a->nheads, 1, 2) ||
-         on(a->A, a->a_stride, a->nheads, 1, 4);
-}
+// Y written over the gates.  A kernel that reads each gate ahead of its place in Y may do that, but not for a second time.
+bool output_on_gate(const SsdArgs* a) { return range(a, a->Z, a->z_stride, a->nheads, a->headdim, elem_size(a->dtype)).on(output(a)); }
 
 // The fp32 scan of a call whose kernel is not chosen by the caller: on the tensor cores at fp32 precision where they can
 // (ssd_split.cu), unless the sequences are so short that the recurrence is through before the other kernel's pipeline has
@@ -326,7 +332,14 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue,
       pc.chain_flag = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(pc.chain_ld) + align_up(kSlots * sizeof(float), 256));   // (cleared by the launch)
     }
     if (!split) return launch_kernel(kernel, args, pc, stream);
-    rc = ssd::launch_split(*args, pc, stream);
+    const bool scan_at_once = fuse_epilogue && output_on_gate(args);   // (by the words that say that it is to be done again)
+    if (scan_at_once) {
+      if (cudaMemsetAsync(pc.redo, 0, ssd::RedoWords::kBytes, stream) != cudaSuccess || cudaMemsetAsync(pc.redo, 1, sizeof(int32_t), stream) != cudaSuccess)
+        return SSD_ERR_CUDA;
+      rc = SSD_OK;
+    } else {
+      rc = ssd::launch_split(*args, pc, stream);
+    }
     if (rc == SSD_OK) {
       // the recurrence, where the call has to be done again: in segments, if there is scratch for them
       redo_segments(args, &nseg, &seg_len);
@@ -334,7 +347,7 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue,
       whole.nseg = nseg;
       whole.seg_len = seg_len;
       whole.redo = pc.redo;
-      whole.redo_n = ssd::split_grid(*args, chain);
+      whole.redo_n = scan_at_once ? 1 : ssd::split_grid(*args, chain);
       whole.chain_state = reinterpret_cast<float*>(ws);
       whole.chain_ld = reinterpret_cast<float*>(ws + align_up((size_t)units * nseg * np * sizeof(float), 256));
       return ssd::launch_scan_f32(whole, args->dtype, stream);
@@ -413,9 +426,10 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
   if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false, in_place);
   // skip and gate of model_ref.py:116-118: fused into the tensor-core kernels, a kernel of their own otherwise
   const int kernel = resolve_kernel(args);
-  const bool can = kernel == SSD_KERNEL_TCGEN05 ? ssd::tc_supports(*args) && ssd::tc2_fuses_epilogue(*args)
-                                                  : use_split(args, kernel) && ssd::split_fuses_epilogue(*args);
-  const bool fuse = can && z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE);
+  const bool split = use_split(args, kernel);
+  const bool can = kernel == SSD_KERNEL_TCGEN05 ? ssd::tc_supports(*args) && ssd::tc2_fuses_epilogue(*args) : split && ssd::split_fuses_epilogue(*args);
+  // (Y over the gates: by the recurrence, with both in it, as a kernel behind it would read its results for gates)
+  const bool fuse = (can && z_vector_friendly(args) && !(args->flags & SSD_FLAG_SEPARATE_EPILOGUE)) || (split && output_on_gate(args));
   rc = forward_impl(args, stream_v, fuse, in_place);
   if (rc != SSD_OK || fuse) return rc;
   ssd::ScanParams ep;
