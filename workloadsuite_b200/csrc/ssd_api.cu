@@ -403,25 +403,28 @@ int ssd_b200_forward(const SsdArgs* args, void* stream_v) {
   int rc = validate(args);
   if (rc != SSD_OK) return rc;
   const bool state_only = (args->flags & SSD_FLAG_STATE_ONLY) != 0;
-  // An output on an input, or states that are not 16-byte aligned, make a call the recurrence's that by its shape is the tensor-core
-  // kernel's: it does with the scratch that the shape asked for, in the segments that it would be done again in.
-  SsdArgs scan = *args;
+  const int chosen = resolve_kernel(args);
+  SsdArgs scan;
   bool in_place = false;
-  if (!use_split(args, resolve_kernel(args)) && split_by_shape(args)) {
-    const size_t own = ssd_b200_workspace_bytes(args), given = args->workspace ? args->workspace_bytes : 0;
-    if (given < own && given >= ask_by_shape(args)) {
+  if (chosen == SSD_KERNEL_SCAN_F32 && args->kernel == SSD_KERNEL_AUTO && args->dtype != SSD_DTYPE_F32) {
+    const size_t given = args->workspace ? args->workspace_bytes : 0;
+    if (use_split(args, chosen)) {
+      // Without scratch that the tensor-core kernel can do with: the recurrence, which needs none for whole sequences.
+      if (given < ssd::least_workspace(args) || (reinterpret_cast<uintptr_t>(args->workspace) & 255)) {
+        scan = *args;
+        scan.kernel = SSD_KERNEL_SCAN_F32;
+        args = &scan;
+      }
+    } else if (split_by_shape(args) && given < ssd_b200_workspace_bytes(args) && given >= ask_by_shape(args)) {
+      // An output on an input, or states that are not 16-byte aligned, make a call the recurrence's that by its shape is the
+      // tensor-core kernel's: it does with the scratch that the shape asked for, in the segments that it would be done again in.
       int seg_len;
+      scan = *args;
       scan.kernel = SSD_KERNEL_SCAN_F32;
       redo_segments(args, &scan.nsegments, &seg_len);
       in_place = scan.nsegments > 1;
       args = &scan;
     }
-  }
-  // Without scratch that the tensor-core kernel can do with: the recurrence, which needs none for whole sequences.
-  if (use_split(args, resolve_kernel(args)) &&
-      (!args->workspace || args->workspace_bytes < ssd::least_workspace(args) || (reinterpret_cast<uintptr_t>(args->workspace) & 255))) {
-    scan.kernel = SSD_KERNEL_SCAN_F32;
-    args = &scan;
   }
   if (state_only || (!args->D && !args->Z)) return forward_impl(args, stream_v, false, in_place);
   // skip and gate of model_ref.py:116-118: fused into the tensor-core kernels, a kernel of their own otherwise
