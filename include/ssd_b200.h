@@ -90,7 +90,8 @@ typedef struct SsdArgs {
   void*        Y;               /* [b,s,h,p]  dtype          :162 (NULL allowed with SSD_FLAG_STATE_ONLY) */
   float*       final_state;     /* [b,h,n,p]  fp32 contiguous, or NULL (the carry after the last chunk, :156) */
   float*       final_logdecay;  /* [b,h]      fp32 sum of A over the sequence, or NULL */
-  void*        workspace;       /* >= ssd_b200_workspace_bytes() bytes, 256-byte aligned; may be NULL if that is 0 */
+  void*        workspace;       /* >= ssd_b200_workspace_bytes() bytes, 256-byte aligned; may be NULL if that is 0, and for
+                                   whole sequences in the fp32 scan (see there) */
   size_t       workspace_bytes;
   int32_t*     status;          /* device int32, or NULL */
   int32_t batch, seqlen, nheads, headdim, dstate, ngroups;
@@ -99,8 +100,8 @@ typedef struct SsdArgs {
   int32_t kernel;               /* SSD_KERNEL_* */
   int32_t flags;                /* SSD_FLAG_* */
   int32_t nsegments;            /* 0 = choose; 1 = whole sequences; >1 = cut each sequence (needs workspace): into
-                                   this many independently scanned segments joined by a state fold, or, for the
-                                   two-head tensor-core kernel's plain forward, at the points an even deal of
+                                   this many independently scanned segments joined by a state fold, or, for a
+                                   tensor-core kernel's plain forward, at the points an even deal of
                                    all tiles over the SMs gives */
   int32_t wait_limit_ms;        /* bound of every device-side wait (a kernel that runs into it writes its code to
                                    `status` and returns); 0 = the default, about one second */
@@ -112,7 +113,8 @@ typedef struct SsdArgs {
   int64_t y_stride[3];          /* b, s, h */
   /* Optional fused epilogue of SSDLayer.forward after the core (model_ref.py:116-118):
    *   Y <- (Y + x * D[head]) * silu(z)
-   * with x the X input, evaluated in fp32 and rounded once.  D == NULL skips the skip term, Z == NULL the gate. */
+   * with x the X input, evaluated in fp32 and rounded once.  D == NULL skips the skip term, Z == NULL the gate.  Where
+   * a kernel of their own applies them, Y must not share memory with Z. */
   const float* D;               /* [h]        fp32 (SSD_FLAG_D_IN_DTYPE: `dtype`), or NULL   model_ref.py:116 */
   const void*  Z;               /* [b,s,h,p]  dtype, or NULL           model_ref.py:118 */
   int64_t z_stride[3];          /* b, s, h */
@@ -124,8 +126,17 @@ int ssd_b200_abi_version(void);
 /* Text for an SSD_ERR_* code (static storage). */
 const char* ssd_b200_strerror(int code);
 
-/* Scratch bytes ssd_b200_forward() needs for these arguments (0 when the
- * sequence is not split).  Returns 0 for invalid arguments; ssd_b200_forward
+/* Scratch bytes ssd_b200_forward() asks for with these arguments: 0 when the
+ * sequence is not split, unless the fp32 scan runs on the tensor cores, which
+ * takes 768 bytes at least.  Asked for without tensor pointers the size is
+ * enough wherever the outputs lie; with them, 16-bit calls of that scan whose
+ * outputs lie on their inputs (a state carried in place) ask for what the
+ * token-by-token recurrence takes.  Without scratch, or with too little,
+ * SSD_ERR_WORKSPACE -- but calls of that scan whose sequences the recurrence
+ * would not cut run as the recurrence, many times slower, and those that it
+ * would cut take as little as the tensor-core kernel needs (9.7 MB at
+ * dstate 128): if numbers that are not finite make it do the call again, it
+ * then does so uncut.  Returns 0 for invalid arguments; ssd_b200_forward
  * reports the error.  No reference counterpart (the reference lets PyTorch
  * allocate its temporaries at model_ref.py:135-161). */
 size_t ssd_b200_workspace_bytes(const SsdArgs* args);
@@ -137,7 +148,7 @@ const char* ssd_b200_kernel_name(const SsdArgs* args);
 /* How ssd_b200_forward() will run these arguments: the resolved SSD_KERNEL_* family, the number of
  * segments each sequence is cut into (2 stands for "cut" where the cut points follow from the grid),
  * and the number of kernel launches it enqueues: 1 for whole sequences; 1 plus a clearing of flags
- * (a block that the launch overlaps) where the two-head tensor-core kernel deals the tiles of all
+ * (a block that the launch overlaps) where a tensor-core kernel deals the tiles of all
  * sequences out evenly inside one launch (states handed from CTA to CTA, or folded from the pairs each CTA publishes for the last piece of its range);
  * 1 more where the fp32 scan runs on the tensor cores (the recurrence behind it, which ends at once unless a number was
  * not finite or a log-decay far above zero); 3 for the two-pass segmented scan (2 with SSD_FLAG_STATE_ONLY or
@@ -270,16 +281,19 @@ int ssd_b200_forward_host(const SsdArgs* host, void* dev_scratch, size_t dev_scr
  * temporaries there, model_ref.py:135-161).
  *
  * Same arguments and results as ssd_b200_forward(); args->workspace and
- * args->workspace_bytes are ignored.  The scratch of the segmented scan comes
+ * args->workspace_bytes are ignored.  The scratch of cut sequences comes
  * from one SSD_STATIC_SCRATCH_BYTES (16 MiB) array that is part of the library
  * image: every GPU that loads the library holds it until the process exits.
- *   - Returns SSD_ERR_TOO_LARGE when ssd_b200_workspace_bytes(args) exceeds
+ *   - Returns SSD_ERR_TOO_LARGE when the least that the call can do with exceeds
  *     that size (reduce args->nsegments, or use ssd_b200_forward()).
+ *   - Whole sequences take none of it: those of 16-bit tensors whose length is no
+ *     multiple of 128 run as the token-by-token recurrence here (the tensor-core
+ *     kernel at fp32 precision, many times faster, needs scratch of its own).
  *   - Calls no cudaMalloc/cudaFree and no allocating library routine.
  *   - The first call on each device looks the array's device address up (with
  *     that device current) and keeps it; make that first call outside any
  *     stream capture.
- *   - All calls on one device share the array, and it keeps the previous call's
+ *   - All calls of cut sequences on one device share the array, and it keeps the previous call's
  *     contents.  The two-pass scan writes every segment state before it reads it;
  *     the single-launch (chained) scan needs its ready flags at zero, and the
  *     forward clears them itself on `stream`.

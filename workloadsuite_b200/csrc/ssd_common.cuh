@@ -48,12 +48,12 @@ struct ScanParams {
   int vec_ok;          // all row starts 16-byte aligned
   long long wait_clocks;   // bound of every device-side wait, in SM clock cycles
   int inject_lost_handover;   // SSD_FLAG_INJECT_LOST_HANDOVER: CTA 0 of a chained launch leaves without working
-  // Chained mode (two-head tensor-core kernel only; 1): a piece of a sequence starts from the state that the
+  // Chained mode (tensor-core kernels; 1): a piece of a sequence starts from the state that the
   // piece before it (on the neighbouring CTA) left in chain_state, once chain_flag says it is there.
   // Look-back mode (2): chain_state / chain_ld hold each CTA's state-from-zero and log-decay sum of the last
   // piece of its range; a piece folds those of the CTAs before it.
   int chain;
-  float* chain_state;     // [slot][p/4][n][4], slot = 2 * CTA + head of the pair
+  float* chain_state;     // [slot][p/4][n][4], slot = 2 * CTA + head of the pair (0 where a kernel works on one head)
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], cleared by the launch
   // The tensor-core kernel at fp32 precision writes a word per CTA: not 0 if the fp32 scan has to do the call again.  The scan, when

@@ -10,7 +10,7 @@
 // rounded once.  Log-decays are summed from the place they count from (the end of the tile for the
 // state's weights, the borders of 32-token blocks for P's, and see kStrong), so a weight's error is that of its own exponent,
 // however much has decayed before.  Against 64 bits (2 x 3001 tokens, 80 heads, n 128, bf16): Y 1.66e-3, its own rounding,
-// here and in the recurrence; final state 8.0e-8 here, 1.24e-7 there.
+// here and in the recurrence; final state 8.4e-8 here, 1.29e-7 there.
 //
 // What cannot be done this way is left to the recurrence: a CTA that meets a number that is not finite (0 * inf in a masked
 // place would reach tokens before its own; an fp16 piece overflows at 65 504) or a log-decay above zero that a tile's factors
@@ -117,7 +117,8 @@ constexpr float kLowestS = -104.f;   // as in ssd_tc2.cu: a factor of zero eithe
 constexpr float kGrowth = 1.f / 32.f;
 // On the diagonal a weight is 2^(difference of two sums from the start of the block), and what both hold from before takes bits of it:
 // 150 behind one reset 2e-5 of it, 3 600 behind 24 of them 5e-4.  Where a block decays by more than this much (up to which they take
-// 2e-6 of it), the sums are taken in 64 bits too, and the factors of a row and a column carry what their 32 bits lack.
+// 2e-6 of it), the sums are taken in 64 bits too, and the factors of a row and a column carry what their 32 bits lack.  (2 x 3001
+// tokens, 80 heads, bf16 and fp16: 85.0 and 90.2 us without, 85.9 and 92.5 so, 88.7 and 92.7 with 64 bits in every tile.)
 constexpr float kStrong = 16.f;
 
 // Two fp32 numbers as sums of 16-bit ones, packed.

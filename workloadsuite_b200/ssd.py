@@ -189,7 +189,10 @@ def ssd_forward(
     ``"scan_f32"`` computes in float32 throughout; it is chosen for everything else, where it runs on the tensor cores too
     if the shape allows (asked for by name, it is the token-by-token recurrence).  ``kernel="tcgen05"`` takes any length where
     16-bit intermediates are accurate enough (relative error of Y in bfloat16 2.4e-3 instead of 1.7e-3, of the final
-    state 2e-3 instead of 1e-7) at five sixths of the time.
+    state 2e-3 instead of 1e-7) at four fifths of the time.  Numbers that are not finite, log-decays above 1/32 and float16
+    numbers beyond some 4 096 make the recurrence do such a call again; outputs on inputs (``out_final_state`` on
+    ``initial_states``, ``out`` on X, or between the columns of a tensor that holds X, or on ``z``) make it the
+    recurrence's at once, some 18 times slower.
 
     ``nsegments``: None lets the library choose; 1 keeps sequences whole; more cuts them (see ``plan``):
     the tensor-core kernel deals the tiles of all sequences out evenly over the SMs inside one launch, the other
