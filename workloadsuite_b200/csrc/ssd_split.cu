@@ -117,8 +117,9 @@ constexpr float kLowestS = -104.f;   // as in ssd_tc2.cu: a factor of zero eithe
 constexpr float kGrowth = 1.f / 32.f;
 // On the diagonal a weight is 2^(difference of two sums from the start of the block), and what both hold from before takes bits of it:
 // 150 behind one reset 2e-5 of it, 3 600 behind 24 of them 5e-4.  Where a block decays by more than this much (up to which they take
-// 3.4e-6 of it at most, 7e-7 in the mean), the sums are taken in 64 bits too, and the factors of a row and a column carry what their 32 bits lack.  (2 x 3001
-// tokens, 80 heads, bf16 and fp16: 85.0 and 90.2 us without, 85.9 and 92.5 so, 88.7 and 92.7 with 64 bits in every tile.)
+// 3.4e-6 of it at most, 7e-7 in the mean), the sums are taken in 64 bits too, and the factors of a row and a column carry what their
+// 32 bits lack.  (2 x 3001 tokens, 80 heads, bf16 and fp16: 85.0 and 90.2 us without, 85.9 and 92.5 so, 88.7 and 92.7 with 64 bits
+// in every tile.)
 constexpr float kStrong = 16.f;
 
 // Two fp32 numbers as sums of 16-bit ones, packed.
