@@ -210,6 +210,56 @@ def test_fp32_scan_with_registers_for_more_ctas(n, units, s, dtype):
     _check(inp, "scan_f32", 1e-4 if dtype == torch.float32 else 2e-2, nsegments=1)
 
 
+@pytest.mark.parametrize("n", [16, 32, 64, 128])
+@pytest.mark.parametrize("s", [64, 65, 79, 128, 129, 200])
+@pytest.mark.parametrize("decays", ["mild", "both_signs", "resets", "strong", "growth", "x_nan", "b_inf", "huge"])
+def test_fp32_tokens_side_by_side(decays, s, n):
+    """Pieces of 16 tokens and tiles of 64 or 128, whole and not, and what sends a tile back to the recurrence: decays that leave the
+    range of a piece, numbers that are not finite or overflow when they are scaled.  A sum of at most 144 products in fp32,
+    2^-24 each, and decays known to as much: some 2e-6 of the largest term, which a result may be a few times smaller than."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=2, s=s, h=4, p=64, n=n, g=2, dtype=torch.float32, init=True, seed=s + n, decay_scale=0.1)
+    gen = torch.Generator().manual_seed(s)
+    dt = 0.2 + torch.rand(2, s, 4, generator=gen)
+    X, A, B, C, init = (inp[k] for k in ("X", "A", "B", "C", "initial_states"))
+    at = s - 17                        # in the last but one piece, or the one before
+    if decays == "both_signs":
+        A = torch.randn(A.shape, generator=gen)
+    elif decays == "resets":
+        A[:, ::23] = -float("inf")
+    elif decays == "strong":
+        A = A - 20.0
+    elif decays == "growth":           # 40 e-folds within a piece, gone again at once; x of nought before
+        X[:, : at + 3] = 0.0
+        init.zero_()
+        A[:, at] = 90.0 - 50.0
+        A[:, at + 2] = -40.0
+    elif decays == "x_nan":
+        X[:, at, 1] = float("nan")
+    elif decays == "b_inf":
+        B[:, at, 0] = float("inf")
+    elif decays == "huge":             # finite results near the top of the range, from a tile whose decays reach e^-35
+        A = torch.full_like(A, -2.2)
+        X, init = X * 1e30, init * 1e30
+    want, Hw = O.ssd_recurrence(X, A, B, C, dt=dt, initial_states=init, return_final_state=True)
+    d = [t.to(DEV) for t in (X, A, B, C, dt, init)]
+    Y, H = W.ssd_forward(d[0], d[1], d[2], d[3], 1, dt=d[4], initial_states=d[5], return_final_state=True)
+    for got, ref in ((Y.cpu().double(), want), (H.cpu().double(), Hw)):
+        assert torch.equal(got.isfinite(), ref.isfinite())
+        ok = ref.isfinite()
+        err, size = ((got - ref).where(ok, 0.0).abs(), ref.where(ok, 0.0).abs())
+        dims = (1, 3) if got.dim() == 4 and got.shape[1] == s else (2, 3)
+        assert (err.amax(dim=dims) / size.amax(dim=dims).clamp_min(1e-30)).max().item() < 1e-5
+    Yc, Hc = W.ssd_forward(d[0], d[1], d[2], d[3], 1, dt=d[4], initial_states=d[5], return_final_state=True, nsegments=2)
+    ok = Y.isfinite()
+    assert torch.equal(ok, Yc.isfinite())
+    if decays in ("mild", "both_signs", "strong", "resets"):
+        assert (Yc - Y).abs().max().item() <= 2e-5 * Y.abs().max().item() and (Hc - H).abs().max().item() <= 2e-5 * H.abs().max().item()
+    again = W.ssd_forward(d[0], d[1], d[2], d[3], 1, dt=d[4], initial_states=d[5], out=d[0])
+    assert torch.equal(again.nan_to_num(), Y.nan_to_num())       # (Y over X)
+
+
 @pytest.mark.parametrize("b,h,n,g", [(3, 6, 128, 2), (1, 4, 256, 1), (40, 6, 16, 3), (40, 6, 32, 2), (40, 6, 256, 6), (2, 1, 64, 1)])
 def test_step_reads_strided_operands_and_d_in_its_own_type(b, h, n, g):
     """Columns of a projection's output against the same values copied out: the same arithmetic, so the same bits.  CTAs of half
