@@ -193,6 +193,52 @@ def test_cut_sequences_of_no_round_length(shape):
     _check(inp, "tcgen05", 2e-2, nsegments=2, z=z)
 
 
+@pytest.mark.parametrize("ragged", [0, 1], ids=["tiles", "ragged"])
+@pytest.mark.parametrize("b,h,n", [(1, 16, 128), (2, 6, 64), (1, 3, 128)])
+@pytest.mark.parametrize("decay", ["fast", "middle", "slow", "one_slow_head", "reset", "impulse", "nan_decay"])
+def test_long_pieces_of_cut_sequences_are_scanned_once(decay, b, h, n, ragged):
+    """Pieces of 30 tiles and more, whose decays leave nothing of the state that enters them after 2, after some 20 or after none of their
+    tiles, against the same sequences uncut: the state entering a piece is a sum in another order (2^-24), of which 16-bit operands and
+    results may round the other way (a few of 2^-8, in a norm 1e-3 at most)."""
+    import workloadsuite_b200 as W
+
+    units = b * h if ragged else b * ((h + 1) // 2)
+    tiles = 44 * (148 // units)
+    s = tiles * 128 + 13 * ragged
+    gen = torch.Generator(DEV).manual_seed(tiles + n)
+    rand = lambda *z: torch.randn(*z, generator=gen, device=DEV)
+    X, B, C = rand(b, s, h, 64).bfloat16(), rand(b, s, 1, n).bfloat16(), rand(b, s, 1, n).bfloat16()
+    init = rand(b, h, n, 64)
+    rate = {"fast": 0.8, "middle": 0.06, "slow": 1e-3, "one_slow_head": 0.3, "reset": 1e-3, "impulse": 2e-3, "nan_decay": 0.3}[decay]
+    A = -rate * torch.rand(b, s, h, generator=gen, device=DEV) * 2.0
+    if decay == "one_slow_head":
+        A[:, :, h - 1] *= 1e-3
+    elif decay == "reset":
+        A[:, 5000::9001] = -float("inf")
+    elif decay == "impulse":           # only what entered earlier is left of most pieces
+        X[:, 1000:-1000] = 0.0
+    elif decay == "nan_decay":
+        A[:, s // 2, 0] = float("nan")
+    kw = dict(initial_states=init, return_final_state=True, return_logdecay=True)
+    whole = W.ssd_forward(X, A, B, C, 1, kernel=None if ragged else "tcgen05", nsegments=1, **kw)
+    got = W.ssd_forward(X, A, B, C, 1, **kw)
+    assert W.plan(X, A, B, C, 1)["nsegments"] > 1
+    assert torch.allclose(got[2], whole[2], rtol=1e-6 * tiles / 32, atol=0, equal_nan=True)
+    for a, c in zip(got[:2], whole[:2]):
+        a, c = a.double(), c.double()
+        if decay == "nan_decay":       # its head from there on: at least to the end of the next piece
+            assert torch.equal(a[..., 1:, :] if a.shape[1] == s else a[:, 1:], a[..., 1:, :] if a.shape[1] == s else a[:, 1:])
+            if a.shape[1] == s:
+                assert a[:, s // 2 : s // 2 + 31 * 128, 0].isnan().all() and not a[:, : s // 2, 0].isnan().any()
+            a, c = (a[:, :, 1:], c[:, :, 1:]) if a.shape[1] == s else (a[:, 1:], c[:, 1:])
+        assert torch.isfinite(a).all()
+        dims = (1, 3) if a.shape[1] == s else (2, 3)
+        assert ((a - c).square().sum(dims) / c.square().sum(dims).clamp_min(1e-60)).sqrt().max().item() < 1e-3
+        if decay == "impulse" and a.shape[1] == s:   # element by element, far below the rest
+            small = (c.abs() < 1e-6 * c.abs().max()) & (c.abs() > 1e-25 * c.abs().max())
+            assert small.any() and ((a - c).abs()[small] / c.abs()[small]).median().item() < 2 ** -6
+
+
 @pytest.mark.parametrize("s", [3, 8, 37, 130])
 @pytest.mark.parametrize("p,n", [(64, 16), (64, 128), (32, 32), (128, 64)])
 def test_fp32_scan_tokens_in_line_and_the_rest(s, p, n):

@@ -106,6 +106,7 @@ struct MiscS {
   uint32_t tmem_base;
   int bad;                   // the recurrence has to do this call again
   long long wait_clocks;
+  float sums[3][kLookTiles][1];   // find_beginning()
   volatile int abort_flag;
 };
 static_assert(sizeof(MiscS) <= LayoutS<128, 3>::kMiscBytes, "MiscS outgrew its shared-memory slot");
@@ -236,6 +237,10 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   if (warp == 0) tmem_alloc(&m->tmem_base, 512);
   tc_fence_before();
   __syncthreads();
+  if (sp.chain == 2) {
+    find_beginning<1>(prm, m->work, m->sums, kThreadsS / 32);
+    __syncthreads();
+  }
   tc_fence_after();
   // The recurrence's CTAs may come once all of these are on their SMs: they wait for the end of this kernel, but not to be launched.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -653,6 +658,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       __syncwarp();
     };
     auto enter_item = [&](bool wy) {
+      if (c.goes_on(wk)) return;
       asum0 = asum = acomp = 0.f;
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
       fold = sp.chain && c.t_begin > 0 && !from_zero;
@@ -685,6 +691,8 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       int p = (int)blockIdx.x - 1;
       const int from = look_back ? wk.from : p;
       wait_published(p, from);
+      float lds = 0.f;   // log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
+      int next = 0;
 #pragma unroll 1
       for (;; --p) {
         const bool piece = p >= from;
@@ -692,7 +700,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const float* src = piece ? sp.chain_state + 2 * p * (int64_t)(N * P) + (4 * J * N + l) * 4
                                  : sp.init + ((int64_t)c.b * sp.nheads + c.head(wk)) * sp.init_unit_stride + (int64_t)l * P + 16 * J;
         const int step = piece ? N : 1;
-        const float ld = piece ? __ldcg(sp.chain_ld + 2 * p) : 0.f;
+        if (next == 0 && p - lane >= from) lds = __ldcg(sp.chain_ld + 2 * (p - lane));
         const float wgt = expf(asum0);           // asum0: log-decay between the end of the piece being added and this item
         if (owns_state && wgt != 0.f) {          // (an underflowed piece adds nothing)
           const ulonglong2* I = reinterpret_cast<const ulonglong2*>(src);
@@ -705,14 +713,15 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           }
         }
         if (!piece) break;
-        asum0 += ld;
+        asum0 += __shfl_sync(0xffffffffu, lds, next);
+        next = (next + 1) & 31;
       }
     };
-    auto leave_item = [&](bool wy) {
+    auto leave_item = [&]() {
 #pragma unroll
       for (int e = 0; e < 8; ++e) odd = fma_pair(H[e], zero2, odd);
       const bool cut_back = sp.chain && c.t_begin / T + c.ntiles < wk.nt;
-      const bool publish = cut_back && !(sp.chain == 2 && wy);   // (look-back: only the state-only scan publishes)
+      const bool publish = cut_back && (sp.chain != 2 || c.scanned(wk));   // (look-back: the scan from zero)
       const int64_t slot = 2 * (int64_t)blockIdx.x;
       const int64_t unit = (int64_t)c.b * sp.nheads + c.head(wk);
       if (publish ? given_up(m) : cut_back) return;
@@ -807,7 +816,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       warp_arrive(&m->bar_u);
       if (lane == 0) mbar_arrive(&m->empty_f[slot]);
       const bool last = c.left == 0;
-      if (__builtin_expect(last, 0)) leave_item(wy);
+      if (__builtin_expect(last, 0)) leave_item();
       if (n + 1 < total) c.next(prm, wk);
       if (__builtin_expect(last && n + 1 < total, 0)) enter_item(n + 1 >= npre);
     }

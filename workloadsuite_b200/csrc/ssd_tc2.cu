@@ -111,6 +111,8 @@ struct Misc2 {
   uint64_t bar_drain;                 // all MMAs issued have completed
   uint32_t tmem_base;
   long long wait_clocks;     // bound of every wait (SM clock cycles)
+  float sums[3][kLookTiles][2];   // find_beginning()
+  float asum1[2];                 // log-decay of the piece that item 1 ended
   volatile int abort_flag;   // 0, or the status code of the first wait that gave up (every role then leaves)
 };
 
@@ -212,6 +214,10 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
+  if (sp.chain == 2) {
+    find_beginning<2>(prm, m->work, m->sums, kThreads2 / 32);
+    __syncthreads();
+  }
   tc_fence_after();
   constexpr uint32_t tG = 0, tSP = 128, tYo = 256, tYd = 384;   // (all 512 columns are ours: the allocation starts at 0)
   const uint32_t sB = smem_u32(smem + L::oB), sC = smem_u32(smem + L::oC), sX = smem_u32(smem + L::oX);
@@ -589,6 +595,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     Cursor c;
     bool fold = false;               // the state entering comes (also) from other CTAs: fold_item() before it is used
     auto enter_item = [&](bool wy) {
+      if (c.goes_on(wk)) return;
       asum0 = asum = acomp = 0.f;
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
       fold = sp.chain && c.t_begin > 0 && !from_zero;
@@ -627,6 +634,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       int p = (int)blockIdx.x - 1;
       const int from = look_back ? wk.from : p;
       wait_published(p, from);
+      float lds = 0.f;   // log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
+      int next = 0;
 #pragma unroll 1
       for (;; --p) {
         const bool piece = p >= from;
@@ -635,7 +644,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
                                  : sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride +
                                        c.seg * sp.init_seg_stride + (int64_t)l * P;
         const int step = piece ? N : 1;
-        const float ld = piece ? __ldcg(sp.chain_ld + 2 * p + h) : 0.f;
+        if (next == 0 && p - lane >= from) lds = __ldcg(sp.chain_ld + 2 * (p - lane) + h);
         const float wgt = ex2(asum0 * kLog2e);   // asum0: log-decay between the end of the piece being added and this item
         if (owns_state && wgt != 0.f) {          // (an underflowed piece adds nothing)
           const ulonglong2* I = reinterpret_cast<const ulonglong2*>(src);
@@ -648,16 +657,22 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           }
         }
         if (!piece) break;
-        asum0 += ld;
+        asum0 += __shfl_sync(0xffffffffu, lds, next);
+        next = (next + 1) & 31;
       }
     };
     // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
-    auto leave_item = [&](bool wy) {
+    auto leave_item = [&]() {
       const bool cut_back = sp.chain && c.t_begin / T + c.ntiles < wk.nt;
-      const bool publish = cut_back && !(sp.chain == 2 && wy);   // (look-back: only the state-only scan publishes)
+      const bool publish = cut_back && (sp.chain != 2 || c.scanned(wk));   // (look-back: the scan from zero)
       const int64_t slot = 2 * (int64_t)blockIdx.x + h;
       const int64_t unit = (int64_t)c.b * sp.nheads + c.head(wk) + h;
       const int seg = sp.chain ? 0 : c.seg;
+      const bool late = wk.again == 2 && !cut_back && c.scanned(wk);   // (what came before is not known yet: item 2 knows)
+      if (wk.again == 2 && c.item <= 2) {
+        if (c.item == 1 && l == 0) m->asum1[h] = asum;
+        if (c.item == 2 && wk.hi % wk.nt == 0 && sp.fin_ld && l == 0 && c.live(wk, h)) sp.fin_ld[unit * sp.finld_unit_stride] = asum0 + m->asum1[h];
+      }
       if (publish ? given_up(m) : (cut_back || !c.live(wk, h))) return;
       float* to = publish ? sp.chain_state + slot * (N * P)
                           : (sp.fin ? sp.fin + unit * sp.fin_unit_stride + seg * sp.fin_seg_stride : nullptr);
@@ -674,7 +689,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           for (int e = 0; e < P / 4; ++e) reinterpret_cast<ulonglong2*>(F)[e * step] = make_ulonglong2(H[2 * e], H[2 * e + 1]);
         }
       }
-      if (ld && l == 0) *ld = asum0 + asum;
+      if (ld && l == 0 && !late) *ld = asum0 + asum;
       if (publish) {
         // Each warp publishes its own rows: a release-add by lane 0 after a warp barrier orders the
         // whole warp's stores before the count, and nobody has to wait for the stores to land.
@@ -761,7 +776,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         if (lane == 0) mbar_arrive(&m->empty_f[h][slot]);
       }
       const bool last = c.left == 0;
-      if (__builtin_expect(last, 0)) leave_item(wy);
+      if (__builtin_expect(last, 0)) leave_item();
       if (n + 1 < total) c.next(prm, wk);
       if (__builtin_expect(last && n + 1 < total, 0)) enter_item(n + 1 >= npre);
       cur_y = wy;

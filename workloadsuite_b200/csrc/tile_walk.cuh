@@ -27,10 +27,15 @@ constexpr int kSms = 148;
 //    the chained mode; a piece that starts inside a sequence folds the published pairs of the CTAs before it, back
 //    to the one that holds the sequence's first tile (the recurrence is linear: H_in = sum_c exp(sum of the
 //    log-decays after c) F_c), skipping those whose decay factor has underflowed.
+//    Of a long piece only a beginning is scanned that way (find_beginning()): from where what enters the piece has decayed to nothing,
+//    the scan from zero is the scan, and writes Y at once (and the sequence's final state, where the piece ends it).  Then the
+//    beginning is done again, from the state that does enter.
 // Computed once per CTA (thread 0, into shared memory): the 64-bit divisions are bulky code.
 struct Work {
   int total;            // tiles of all items
   int npre;             // the first npre of them produce a state only
+  int again;            // look-back mode: items of the range's last piece that follow item 0: 0 or 1 (after its state-only scan), or 2
+                        // where only its beginning is scanned for the state (the rest of the piece, then the beginning again)
   int lo, hi, nt, first;   // chained modes: global tile range, tiles per sequence, first tile of item 0's sequence
   int from;             // look-back mode: the CTA that holds the first tile of the range's first sequence
   int hpg, ppg;         // heads per B/C group, head pairs per group
@@ -60,7 +65,7 @@ __device__ __forceinline__ void work_list(const TileParams& prm, Work& wk) {
   wk.hpg = sp.nheads / sp.ngroups;
   wk.ppg = prm.ppg;
   wk.npre = sp.compute_y ? 0 : 0x7fffffff;
-  wk.lo = wk.hi = wk.first = wk.from = 0;
+  wk.lo = wk.hi = wk.first = wk.from = wk.again = 0;
   if (sp.chain) {
     const long long total = (long long)prm.upairs * wk.nt;
     wk.lo = (int)((long long)blockIdx.x * total / gridDim.x);
@@ -71,6 +76,7 @@ __device__ __forceinline__ void work_list(const TileParams& prm, Work& wk) {
     if (sp.chain == 2 && wk.hi % wk.nt != 0) {
       wk.npre = wk.hi - max(wk.lo, wk.first);
       wk.total += wk.npre;
+      wk.again = 1;
     }
     // the largest c with lo(c) <= first tile of the range's first sequence
     const int first = wk.lo / wk.nt * wk.nt;
@@ -112,7 +118,7 @@ struct CursorOf {
     if (++item == 0) {
       q = wk.d0[0]; g = wk.d0[1]; b = wk.d0[2]; seg = wk.d0[3];
       first = wk.first;
-    } else if (!(item == 1 && sp.chain == 2 && wk.npre > 0)) {   // (after the state-only scan: the same piece again)
+    } else if (item > wk.again) {   // (up to there: the piece scanned first again)
       first -= wk.nt;
       int c = 0;
       q += wk.step[0];
@@ -131,6 +137,10 @@ struct CursorOf {
       const int start = max(wk.lo, first), end = min(wk.hi, first + wk.nt);
       t_begin = (start - first) * T;
       ntiles = end - start;
+      if (wk.again == 2 && item <= 2) {
+        if (item == 1) t_begin += wk.npre * T;
+        ntiles = item == 1 ? ntiles - wk.npre : wk.npre;
+      }
     } else {
       t_begin = seg * sp.seg_len;
       ntiles = (min(sp.seqlen, t_begin + sp.seg_len) - t_begin + T - 1) / T;
@@ -138,10 +148,87 @@ struct CursorOf {
     t0 = t_begin;
     left = ntiles - 1;
   }
+  // Look-back mode: an item that goes on from the state the last one left; one whose end is that of the scan from zero.
+  __device__ __forceinline__ bool goes_on(const Work& wk) const { return wk.again == 2 && item == 1; }
+  __device__ __forceinline__ bool scanned(const Work& wk) const { return wk.again > 0 && item == wk.again - 1; }
   __device__ __forceinline__ bool first_tile() const { return left == ntiles - 1; }
   __device__ __forceinline__ int head(const Work& wk) const { return g * wk.hpg + kHeads * q; }   // first of the item
   __device__ __forceinline__ bool live(const Work& wk, int h) const { return kHeads * q + h < wk.hpg; }
 };
+
+// Look-back mode, all threads of a CTA, behind a barrier after work_list() and ahead of one before the list is used: how much of the
+// range's last piece needs the state that enters it.  Where the log-decays from its first token on sum to less than -150, e^-150 = 2^-216
+// has taken any entering state below 2^67 past the smallest fp32 number (2^-149): it is not there any more.  A layer's slowest heads (rate
+// 1, steps of 0.03) get there after 40 tiles.  1 x 131 072 tokens, 32 heads, 114 tiles a CTA: 530 -> 438 us, bit by bit the same.
+// A piece scanned so is through with its first pass later (n - 0.6 k tile times for a beginning of k tiles) than one scanned for the state
+// only (0.4 n), and what waits for it waits longer.  So the pieces of a sequence all do it or none: if, by the sequence's first tiles, k is
+// at most 0.6 of a piece (32 768 tokens, 64 heads, each piece for itself and up to 1.0: 271 -> 298 us); and only where every range is one
+// piece, as other ranges may begin with one that waits (the same case: 270 -> 305).  A look
+// takes 2 to 3 us; pieces of less than 40 tiles are left alone.
+constexpr int kLookTiles = 16, kLeastBeginning = 40;
+template <int kHeads>   // heads of an item
+__device__ __forceinline__ void find_beginning(const TileParams& prm, Work& wk, float (&sums)[3][kLookTiles][kHeads], int warps) {
+  const ScanParams& sp = prm.sp;
+  const int from = max(wk.lo, wk.first), tiles = wk.hi - from;
+  if (tiles < kLeastBeginning || (int)gridDim.x % prm.upairs != 0 || (wk.again == 0 && from == wk.first)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int head = wk.d0[1] * wk.hpg + kHeads * wk.d0[0], heads = min(kHeads, wk.hpg - kHeads * wk.d0[0]);
+  const float* A = sp.A + wk.d0[2] * sp.as[0] + head * sp.as[2];
+  // sums over tiles of the piece from its `done`-th on, and at first over those that the sequence begins with, all loads ahead
+  auto look = [&](float (&mine)[kLookTiles][kHeads], int done) {
+    constexpr int kMost = 2 * kLookTiles * kHeads / 16;   // (16 warps at least)
+    const int count = (done == 0 ? 2 : 1) * kLookTiles * heads;
+    float s[kMost];
+#pragma unroll
+    for (int k = 0; k < kMost; ++k) {
+      const int i = warp + k * warps, tile = i % kLookTiles, h = i / kLookTiles % heads;
+      const int64_t t = (int64_t)((i < kLookTiles * heads ? from - wk.first + done : 0) + tile) * T + 4 * lane;
+      const float* a = A + t * sp.as[1] + h * sp.as[2];
+      s[k] = 0.f;
+      if (i < count && t + 3 < sp.seqlen) s[k] = (a[0] + a[sp.as[1]]) + (a[2 * sp.as[1]] + a[3 * sp.as[1]]);   // (less at the end: no harm)
+    }
+#pragma unroll
+    for (int k = 0; k < kMost; ++k) {
+      const int i = warp + k * warps;
+      if (i >= count) break;
+      for (int d = 16; d >= 1; d >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], d);
+      if (lane == 0) (i < kLookTiles * heads ? mine : sums[2])[i % kLookTiles][i / kLookTiles % heads] = s[k];
+    }
+  };
+  // every warp for itself: lane 16 h + i has tile i of head h
+  const int i = lane % kLookTiles, h = lane / kLookTiles;
+  const bool mine = h < heads;
+  auto scan = [&](float v) {
+#pragma unroll
+    for (int d = 1; d < kLookTiles; d <<= 1) {
+      const float u = __shfl_up_sync(0xffffffffu, v, d, kLookTiles);
+      if (i >= d) v += u;
+    }
+    return v;
+  };
+  float run = 0.f;
+  int beginning = 0, gone = 0;   // `gone`: tiles after which this lane's head has nothing left
+  for (int done = 0; done < tiles && beginning == 0; done += kLookTiles) {
+    float (&to)[kLookTiles][kHeads] = sums[done / kLookTiles & 1];
+    look(to, done);
+    __syncthreads();
+    if (done == 0) {
+      const float all = __shfl_sync(0xffffffffu, scan(mine ? sums[2][i][h] : 0.f), kLookTiles - 1, kLookTiles);
+      if (__any_sync(0xffffffffu, mine && !(all * (0.6f * ((float)prm.upairs * wk.nt / gridDim.x)) < -150.f * kLookTiles))) break;
+    }
+    const float v = run + scan(mine && done + i < tiles ? to[i][h] : 0.f);
+    const unsigned below = __ballot_sync(0xffffffffu, v < -150.f) >> (kLookTiles * h) & ((1u << kLookTiles) - 1);
+    if (gone == 0 && below) gone = done + __ffs(below);
+    run = __shfl_sync(0xffffffffu, v, kLookTiles - 1, kLookTiles);
+    if (__all_sync(0xffffffffu, gone > 0 || !mine)) beginning = __reduce_max_sync(0xffffffffu, mine ? gone : 0);
+  }
+  __syncthreads();   // (everybody has read the list)
+  if (threadIdx.x == 0 && beginning > 0 && beginning < tiles) {
+    wk.again = 2;
+    wk.npre = beginning;
+    wk.total = wk.hi - wk.lo + beginning;
+  }
+}
 
 // Waits.  Instructions are what this kernel is short of: a scheduler's own instruction cache holds a few KB, and code
 // that streams past it from the SM's (about 24 KB) arrives at 2.7 cycles per instruction, past that one at five to ten.
