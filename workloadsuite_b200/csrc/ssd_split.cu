@@ -48,7 +48,7 @@ using namespace tc;
 
 constexpr int kThreadsS = 768;
 constexpr int kFactorsS = 4;   // tiles that the factors may be ahead
-using Cursor = CursorOf<1>;
+using Cursor = CursorOf<1, true>;
 
 template <int N, int kPieces>
 struct LayoutS {

@@ -45,7 +45,6 @@ using namespace ptx;
 using namespace tc;
 
 constexpr int kThreads2 = 512;
-using Cursor = CursorOf<2>;
 
 template <int N>
 struct Layout2 {
@@ -158,12 +157,16 @@ __device__ __forceinline__ void make_xd(uint32_t xb, uint32_t xd, const Factors&
 // EPI: apply the skip and gate of model_ref.py:116-118 to Y on its way out (sp.D / sp.Z; either may be null).
 // WIDE: Xd in fp32 arithmetic.  Groups with an odd number of heads have always had it so (bf16, final state against 64 bits:
 // 1.65e-3, with the packed products 2.23e-3); those with an even number have the reference's packed products.
-template <typename T16, int N, bool EPI, bool WIDE>
+// LB: an instance for sequences cut in look-back mode (sp.chain == 2), as what a piece's beginning takes costs the walk of the others
+// (see CursorOf).  The others keep their checks of sp.chain == 2, never true there: without them the compiler's registers spill 24 to 60
+// bytes (8 x 2048 tokens of 24 heads 52.1 -> 55.3 us).
+template <typename T16, int N, bool EPI, bool WIDE, bool LB>
 __global__ void __launch_bounds__(kThreads2, 1)
 ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY,
                const TileParams prm) {
   using L = Layout2<N>;
+  using Cursor = CursorOf<2, LB>;
   constexpr int NB = L::NB;
   constexpr int KN = N / 16;
   constexpr int KT = T / 16;
@@ -214,7 +217,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if (sp.chain == 2) {
+  if constexpr (LB) {
     find_beginning<2>(prm, m->work, m->sums, kThreads2 / 32);
     __syncthreads();
   }
@@ -662,14 +665,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       }
     };
     // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
-    auto leave_item = [&]() {
+    auto leave_item = [&](bool wy) {
       const bool cut_back = sp.chain && c.t_begin / T + c.ntiles < wk.nt;
-      const bool publish = cut_back && (sp.chain != 2 || c.scanned(wk));   // (look-back: the scan from zero)
+      const bool publish = cut_back && !(LB ? !c.scanned(wk) : sp.chain == 2 && wy);   // (look-back: the scan from zero)
       const int64_t slot = 2 * (int64_t)blockIdx.x + h;
       const int64_t unit = (int64_t)c.b * sp.nheads + c.head(wk) + h;
       const int seg = sp.chain ? 0 : c.seg;
-      const bool late = wk.again == 2 && !cut_back && c.scanned(wk);   // (what came before is not known yet: item 2 knows)
-      if (wk.again == 2 && c.item <= 2) {
+      const bool late = LB && wk.again == 2 && !cut_back && c.scanned(wk);   // (what came before is not known yet: item 2 knows)
+      if (LB && wk.again == 2 && c.item <= 2) {
         if (c.item == 1 && l == 0) m->asum1[h] = asum;
         if (c.item == 2 && wk.hi % wk.nt == 0 && sp.fin_ld && l == 0 && c.live(wk, h)) sp.fin_ld[unit * sp.finld_unit_stride] = asum0 + m->asum1[h];
       }
@@ -776,7 +779,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         if (lane == 0) mbar_arrive(&m->empty_f[h][slot]);
       }
       const bool last = c.left == 0;
-      if (__builtin_expect(last, 0)) leave_item();
+      if (__builtin_expect(last, 0)) leave_item(wy);
       if (n + 1 < total) c.next(prm, wk);
       if (__builtin_expect(last && n + 1 < total, 0)) enter_item(n + 1 >= npre);
       cur_y = wy;
@@ -985,10 +988,10 @@ __global__ void clear_flags_kernel(int* flags) {
   flags[threadIdx.x] = 0;
 }
 
-template <typename T16, int N, bool EPI, bool WIDE>
+template <typename T16, int N, bool EPI, bool WIDE, bool LB>
 int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& ty,
                   const TileParams& prm, cudaStream_t stream) {
-  auto kern = ssd_tc2_kernel<T16, N, EPI, WIDE>;
+  auto kern = ssd_tc2_kernel<T16, N, EPI, WIDE, LB>;
   constexpr int smem = Layout2<N>::kBytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return SSD_ERR_CUDA;
@@ -1104,16 +1107,19 @@ int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
     if (sp.Z && ((reinterpret_cast<uintptr_t>(sp.Z) & 15) || sp.zs[0] % 8 || sp.zs[1] % 8 || sp.zs[2] % 8))
       return SSD_ERR_MISALIGNED;
   }
-  auto go = [&](auto epilogue, auto wide) {
-    constexpr bool E = decltype(epilogue)::value, W = decltype(wide)::value;
+  auto go = [&](auto epilogue, auto wide, auto look_back) {
+    constexpr bool E = decltype(epilogue)::value, W = decltype(wide)::value, LB = decltype(look_back)::value;
     if (a.dtype == SSD_DTYPE_BF16)
-      return a.dstate == 128 ? launch_typed2<__nv_bfloat16, 128, E, W>(tx, tb, tc, ty, prm, stream)
-                             : launch_typed2<__nv_bfloat16, 64, E, W>(tx, tb, tc, ty, prm, stream);
-    return a.dstate == 128 ? launch_typed2<__half, 128, E, W>(tx, tb, tc, ty, prm, stream)
-                           : launch_typed2<__half, 64, E, W>(tx, tb, tc, ty, prm, stream);
+      return a.dstate == 128 ? launch_typed2<__nv_bfloat16, 128, E, W, LB>(tx, tb, tc, ty, prm, stream)
+                             : launch_typed2<__nv_bfloat16, 64, E, W, LB>(tx, tb, tc, ty, prm, stream);
+    return a.dstate == 128 ? launch_typed2<__half, 128, E, W, LB>(tx, tb, tc, ty, prm, stream)
+                           : launch_typed2<__half, 64, E, W, LB>(tx, tb, tc, ty, prm, stream);
   };
-  if (epi) return go(std::true_type{}, std::false_type{});
-  return odd_groups(a) ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
+  auto one = [&](auto look_back) {
+    if (epi) return go(std::true_type{}, std::false_type{}, look_back);
+    return odd_groups(a) ? go(std::false_type{}, std::true_type{}, look_back) : go(std::false_type{}, std::false_type{}, look_back);
+  };
+  return sp.chain == 2 ? one(std::true_type{}) : one(std::false_type{});
 }
 
 }  // namespace ssd
