@@ -797,6 +797,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     uint32_t xi = 0;            // X slot of the tile being read out
     uint32_t ky = 0;
     const uint64_t once = policy_evict_first();
+    uint32_t skip[2] = {0, 0};       // (EPI) D of both heads as loaded: a conversion there would hold the warp for the memory latency
+    const T16* zp = nullptr;         // (EPI) gate of head 0, row lane / 4 of this warp's, piece lane % 4
     int pending = -1;    // (lane 0) X slot that this warp's last TMA store still reads
     auto release = [&]() {
       if (lane == 0 && pending >= 0) {
@@ -843,26 +845,46 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         continue;
       }
       const int t0 = c.t0;
+      if constexpr (EPI) {
+        // (instructions are what this warp is short of: the gate's addresses are worked out once an item)
+        if (__builtin_expect(c.first_tile(), 0)) {
+          const int head = c.head(wk);
+          if (sp.D) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              if (c.live(wk, h))
+                skip[h] = sp.d_in_dtype ? reinterpret_cast<const uint16_t*>(sp.D)[head + h] : reinterpret_cast<const uint32_t*>(sp.D)[head + h];
+          }
+          zp = static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] + head * sp.zs[2] + (int64_t)(t0 + lane_base + (lane >> 2)) * sp.zs[1] + 8 * (lane & 3);
+        } else {
+          zp += T * sp.zs[1];
+        }
+      }
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         const bool live = c.live(wk, h);
         // (EPI) the gate rows of this warp's 32 tokens, fetched ahead of the wait for the MMA.  Four lanes read half a
         // 128-byte row per load, eight rows per instruction; the rows reach their threads through the staging buffer below.
         uint4 zr[8];
-        uint32_t dskip = 0;   // D as loaded: a conversion here would hold the warp for the whole memory latency
+        const uint32_t dskip = h ? skip[1] : skip[0];
+        const T16* zh = h ? zp + sp.zs[2] : zp;
         if constexpr (EPI) {
-          if (sp.D && live)
-            dskip = sp.d_in_dtype ? reinterpret_cast<const uint16_t*>(sp.D)[c.head(wk) + h]
-                                  : reinterpret_cast<const uint32_t*>(sp.D)[c.head(wk) + h];
           if (sp.Z && live) {
-            const T16* zbase = static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] + (c.head(wk) + h) * sp.zs[2] + 8 * (lane & 3);
+            const int64_t s8 = 8 * sp.zs[1];
+            if (__builtin_expect(t0 + T <= sp.seqlen, 1)) {
+              const T16* r = zh;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int tok = t0 + lane_base + 8 * i + (lane >> 2);
-              if (tok < sp.seqlen) {
-                const uint4* zp = reinterpret_cast<const uint4*>(zbase + (int64_t)tok * sp.zs[1]);
-                zr[i] = __ldg(zp);
-                zr[4 + i] = __ldg(zp + 4);
+              for (int i = 0; i < 4; ++i, r += s8) {
+                zr[i] = __ldg(reinterpret_cast<const uint4*>(r));
+                zr[4 + i] = __ldg(reinterpret_cast<const uint4*>(r) + 4);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (t0 + lane_base + 8 * i + (lane >> 2) < sp.seqlen) {
+                  zr[i] = __ldg(reinterpret_cast<const uint4*>(zh + i * s8));
+                  zr[4 + i] = __ldg(reinterpret_cast<const uint4*>(zh + i * s8) + 4);
+                }
               }
             }
           }
@@ -871,8 +893,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           // the next gate rows, one per lane, as near as they go without registers
           const int tn = t0 + l + (h ? T : 0);
           if (sp.Z && tn < sp.seqlen && c.live(wk, h ^ 1))
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(static_cast<const T16*>(sp.Z) + c.b * sp.zs[0] +
-                                                         (c.head(wk) + (h ^ 1)) * sp.zs[2] + (int64_t)tn * sp.zs[1]));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(zp + (h ? T * sp.zs[1] : sp.zs[2]) + (lane - (lane >> 2)) * sp.zs[1]));
           wait(&m->full_f[h][slot], (n / kFactors) & 1, m);
         }
         const float el = ex2(m->f[h][slot].cs2[l]);
@@ -899,7 +920,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           for (int e = 0; e < 16; ++e) y[e] = fma_pair(pair(o[2 * e], o[2 * e + 1]), el2, pair(d[2 * e], d[2 * e + 1]));
           if constexpr (EPI) {
             // Y <- (Y + x * D) * silu(z) (model_ref.py:116-118) in fp32; x is this thread's row of the X tile, still in
-            // the slot that the Y rows go to; silu(z) = z * (0.5 + 0.5 tanh(z / 2)), the tanh on 16-bit pairs.
+            // the slot that the Y rows go to; silu(z) = z / 2 (1 + tanh(z / 2)), the tanh on 16-bit pairs.
             if (sp.D && live) {
               const float dsf = sp.d_in_dtype ? unpack2<T16>(dskip).x : __uint_as_float(dskip);
               const uint64_t ds = pair(dsf, dsf);
@@ -931,10 +952,10 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
                 const uint32_t zw[4] = {zq.x, zq.y, zq.z, zq.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                  // silu(z) = z * (0.5 + 0.5 tanh(z / 2)) on the packed 16-bit pair, as the reference forms it in
-                  // half precision (model_ref.py:118); the product with Y is taken in fp32
-                  const uint32_t sg = fma2<T16>(tanh2<T16>(mul2<T16>(zw[e], half2)), half2, half2);
-                  const float2 gf = unpack2<T16>(mul2<T16>(zw[e], sg));
+                  // silu(z) = z / 2 + z / 2 tanh(z / 2) on the packed 16-bit pair, rounded once (model_ref.py:118 in half
+                  // precision); the product with Y is taken in fp32
+                  const uint32_t zz = mul2<T16>(zw[e], half2);
+                  const float2 gf = unpack2<T16>(fma2<T16>(zz, tanh2<T16>(zz), zz));
                   y[4 * cc + e] = mul_pair(y[4 * cc + e], pair(gf.x, gf.y));
                 }
               }
