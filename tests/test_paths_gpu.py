@@ -370,10 +370,11 @@ def test_what_pytorch_throws_in_the_binding_is_raised():
 
 
 @pytest.mark.parametrize("dtype,l,d", [(torch.float16, 1, 64), (torch.float16, 9, 128), (torch.bfloat16, 65, 64),
-                                       (torch.float32, 5, 64), (torch.float32, 67, 192), (torch.bfloat16, 2050, 4096)])
+                                       (torch.float32, 5, 64), (torch.float32, 67, 192), (torch.bfloat16, 2050, 4096),
+                                       (torch.float16, 1780, 1024), (torch.bfloat16, 1188, 1024), (torch.float16, 1780, 3072), (torch.bfloat16, 1965, 3072), (torch.float16, 1410, 5120)])
 @pytest.mark.parametrize("taps", [2, 3, 4])
 def test_conv_run_lengths(dtype, l, d, taps):
-    """From a run shorter than a piece to the longest run, against the operator in fp64 (one rounding of the result, and
+    """From a run shorter than a piece to the longest run (64 tokens; the last cases 16 to 56), against the operator in fp64 (one rounding of the result, and
     tanh.approx for 16-bit types: 2^-8 of the largest value bounds both)."""
     import workloadsuite_b200 as W
 

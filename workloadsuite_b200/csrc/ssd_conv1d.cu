@@ -322,6 +322,23 @@ conv1d_silu_staged_kernel(const T* __restrict__ x, const T* __restrict__ w, cons
   cp_async_wait<0>();
 }
 
+// Tokens of a run of the staged kernel.  Where all blocks are on the chip at once, three to an SM at most, a block's time goes with its
+// tokens and some ten for the rows before and the start, and with what it shares the SM with (two 1.4, three 2.0 times that of one alone, from
+// b1 s4096 h32: 64 tokens, one block an SM, 12.8 us, 32 10.0, 24 11.0; b1 s8192 h24: 64 13.6, 32 11.1; b2 s4096 h48: 64 23.8, 56 22.4; b4 s333
+// h80: 32 8.2, 16 7.2).  Otherwise the longest: what is read at a time lies closer together than with longer ones (b4 s8192 h80: 56
+// 115 us, 64 113, 96 114, 192 121, 376, which is a single round, 133).
+int staged_run(int64_t columns, int seqlen) {
+  constexpr int kShare[3] = {5, 7, 10};
+  int best = kLongestRun, cost = 1 << 30;
+  for (int len = kPiece; len <= kLongestRun; len += kPiece) {
+    const int64_t blocks = (columns * ((seqlen + len - 1) / len) + kStagedThreads - 1) / kStagedThreads;
+    if (blocks > 3 * 148) continue;
+    const int c = (std::min(len, (seqlen + kPiece - 1) / kPiece * kPiece) + 10) * kShare[(blocks - 1) / 148];
+    if (c < cost) best = len, cost = c;
+  }
+  return best;
+}
+
 template <typename T>
 int launch_conv(const void* x, const void* w, const void* bias, void* y, int batch, int seqlen, int channels, int taps,
                 int64_t xsb, int64_t xsl, int64_t ysb, int64_t ysl, cudaStream_t stream) {
@@ -344,9 +361,7 @@ int launch_conv(const void* x, const void* w, const void* bias, void* y, int bat
   T* yy = static_cast<T*>(y);
   if constexpr (sizeof(T) == 2) {
     if (al && taps >= 2 && taps <= 4) {
-      // a block per SM (b1 s4096 h32 bf16: 12.8 us with half a block's worth, 11.8 so; with two it is 18.0, the rows before the
-      // runs read again and a second round of blocks)
-      const int len = in_place ? kLongestRun : run_length(kLongestRun, kPiece, columns, seqlen, 148 * 128);
+      const int len = in_place ? kLongestRun : staged_run(columns, seqlen);
       const int64_t tot = columns * ((seqlen + len - 1) / len);
       if ((tot + kStagedThreads - 1) / kStagedThreads > 0x7fffffffLL) return SSD_ERR_TOO_LARGE;
       const unsigned g = (unsigned)((tot + kStagedThreads - 1) / kStagedThreads);
