@@ -48,7 +48,6 @@ using namespace tc;
 
 constexpr int kThreadsS = 768;
 constexpr int kFactorsS = 4;   // tiles that the factors may be ahead
-using Cursor = CursorOf<1, true>;
 
 template <int N, int kPieces>
 struct LayoutS {
@@ -106,8 +105,8 @@ struct MiscS {
   uint32_t tmem_base;
   int bad;                   // the recurrence has to do this call again
   long long wait_clocks;
-  float sums[3][kLookTiles][1];   // find_beginning()
   volatile int abort_flag;
+  float sums[3][kLookTiles][1];   // find_beginning()
 };
 static_assert(sizeof(MiscS) <= LayoutS<128, 3>::kMiscBytes, "MiscS outgrew its shared-memory slot");
 static_assert(LayoutS<128, 3>::kBytes <= 232448 && LayoutS<64, 3>::kBytes <= 232448, "shared memory budget of one SM exceeded");
@@ -186,13 +185,15 @@ __device__ __forceinline__ float power_below(float x) {
 __device__ __forceinline__ float inverse_power(float x) { return __uint_as_float(0x7f000000u - __float_as_uint(x)); }
 
 // EPI: skip and gate of model_ref.py:116-118 (sp.D / sp.Z; either may be null) applied to Y in fp32 ahead of its one rounding.
-template <typename T16, int N, bool EPI>
+// LB: sequences cut in look-back mode, an instance of its own as in ssd_tc2.cu (615 heads of 27 tokens, fp16: 30.6 us without).
+template <typename T16, int N, bool EPI, bool LB>
 __global__ void __launch_bounds__(kThreadsS, 1)
 ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY, const TileParams prm) {
   constexpr bool kF16 = std::is_same<T16, __half>::value;
   constexpr int kPieces = kF16 ? 2 : 3;
   using L = LayoutS<N, kPieces>;
+  using Cursor = CursorOf<1, LB>;
   using Col = Columns<kPieces>;
   constexpr uint32_t tG = Col::G, tYo = Col::Yo, tS = Col::S, tYd = Col::Yd;
   constexpr int NB = L::NB, KN = N / 16, KT = T / 16, BC = L::kBC, XS = L::kXSlots;
@@ -237,7 +238,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   if (warp == 0) tmem_alloc(&m->tmem_base, 512);
   tc_fence_before();
   __syncthreads();
-  if (sp.chain == 2) {
+  if constexpr (LB) {
     find_beginning<1>(prm, m->work, m->sums, kThreadsS / 32);
     __syncthreads();
   }
@@ -691,7 +692,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       int p = (int)blockIdx.x - 1;
       const int from = look_back ? wk.from : p;
       wait_published(p, from);
-      float lds = 0.f;   // log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
+      float lds = 0.f;   // look-back: log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
       int next = 0;
 #pragma unroll 1
       for (;; --p) {
@@ -700,7 +701,9 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const float* src = piece ? sp.chain_state + 2 * p * (int64_t)(N * P) + (4 * J * N + l) * 4
                                  : sp.init + ((int64_t)c.b * sp.nheads + c.head(wk)) * sp.init_unit_stride + (int64_t)l * P + 16 * J;
         const int step = piece ? N : 1;
-        if (next == 0 && p - lane >= from) lds = __ldcg(sp.chain_ld + 2 * (p - lane));
+        float ld = 0.f;
+        if (!LB) ld = piece ? __ldcg(sp.chain_ld + 2 * p) : 0.f;
+        else if (next == 0 && p - lane >= from) lds = __ldcg(sp.chain_ld + 2 * (p - lane));
         const float wgt = expf(asum0);           // asum0: log-decay between the end of the piece being added and this item
         if (owns_state && wgt != 0.f) {          // (an underflowed piece adds nothing)
           const ulonglong2* I = reinterpret_cast<const ulonglong2*>(src);
@@ -713,15 +716,15 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           }
         }
         if (!piece) break;
-        asum0 += __shfl_sync(0xffffffffu, lds, next);
+        asum0 += LB ? __shfl_sync(0xffffffffu, lds, next) : ld;
         next = (next + 1) & 31;
       }
     };
-    auto leave_item = [&]() {
+    auto leave_item = [&](bool wy) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) odd = fma_pair(H[e], zero2, odd);
       const bool cut_back = sp.chain && c.t_begin / T + c.ntiles < wk.nt;
-      const bool publish = cut_back && (sp.chain != 2 || c.scanned(wk));   // (look-back: the scan from zero)
+      const bool publish = cut_back && !(LB ? !c.scanned(wk) : sp.chain == 2 && wy);   // (look-back: the scan from zero)
       const int64_t slot = 2 * (int64_t)blockIdx.x;
       const int64_t unit = (int64_t)c.b * sp.nheads + c.head(wk);
       if (publish ? given_up(m) : cut_back) return;
@@ -816,7 +819,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       warp_arrive(&m->bar_u);
       if (lane == 0) mbar_arrive(&m->empty_f[slot]);
       const bool last = c.left == 0;
-      if (__builtin_expect(last, 0)) leave_item();
+      if (__builtin_expect(last, 0)) leave_item(wy);
       if (n + 1 < total) c.next(prm, wk);
       if (__builtin_expect(last && n + 1 < total, 0)) enter_item(n + 1 >= npre);
     }
@@ -1008,10 +1011,10 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   }
 }
 
-template <typename T16, int N, bool EPI>
+template <typename T16, int N, bool EPI, bool LB>
 int launch_typed(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& ty, const TileParams& prm,
                  int grid, cudaStream_t stream) {
-  auto kern = ssd_split_kernel<T16, N, EPI>;
+  auto kern = ssd_split_kernel<T16, N, EPI, LB>;
   constexpr int smem = LayoutS<N, std::is_same<T16, __half>::value ? 2 : 3>::kBytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return SSD_ERR_CUDA;
   return launch_tiles(kern, grid, kThreadsS, smem, prm.sp, stream, tx, tb, tc, ty, prm);
@@ -1048,15 +1051,17 @@ int launch_split(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
       !make_map(&tc, a.C, a, a.dstate, 1, a.c_stride, T) || !make_map(&ty, a.Y, a, P, hpg, a.y_stride, 32))
     return SSD_ERR_UNSUPPORTED;
   const int grid = split_grid(a, sp.chain);
-  auto go = [&](auto epilogue) {
-    constexpr bool E = decltype(epilogue)::value;
+  auto go = [&](auto epilogue, auto look_back) {
+    constexpr bool E = decltype(epilogue)::value, LB = decltype(look_back)::value;
     if (a.dtype == SSD_DTYPE_F16)
-      return a.dstate == 128 ? launch_typed<__half, 128, E>(tx, tb, tc, ty, prm, grid, stream)
-                             : launch_typed<__half, 64, E>(tx, tb, tc, ty, prm, grid, stream);
-    return a.dstate == 128 ? launch_typed<__nv_bfloat16, 128, E>(tx, tb, tc, ty, prm, grid, stream)
-                           : launch_typed<__nv_bfloat16, 64, E>(tx, tb, tc, ty, prm, grid, stream);
+      return a.dstate == 128 ? launch_typed<__half, 128, E, LB>(tx, tb, tc, ty, prm, grid, stream)
+                             : launch_typed<__half, 64, E, LB>(tx, tb, tc, ty, prm, grid, stream);
+    return a.dstate == 128 ? launch_typed<__nv_bfloat16, 128, E, LB>(tx, tb, tc, ty, prm, grid, stream)
+                           : launch_typed<__nv_bfloat16, 64, E, LB>(tx, tb, tc, ty, prm, grid, stream);
   };
-  return sp.D || sp.Z ? go(std::true_type{}) : go(std::false_type{});
+  const bool epi = sp.D || sp.Z;
+  if (sp.chain == 2) return epi ? go(std::true_type{}, std::true_type{}) : go(std::false_type{}, std::true_type{});
+  return epi ? go(std::true_type{}, std::false_type{}) : go(std::false_type{}, std::false_type{});
 }
 
 }  // namespace ssd

@@ -110,9 +110,9 @@ struct Misc2 {
   uint64_t bar_drain;                 // all MMAs issued have completed
   uint32_t tmem_base;
   long long wait_clocks;     // bound of every wait (SM clock cycles)
+  volatile int abort_flag;   // 0, or the status code of the first wait that gave up (every role then leaves)
   float sums[3][kLookTiles][2];   // find_beginning()
   float asum1[2];                 // log-decay of the piece that item 1 ended
-  volatile int abort_flag;   // 0, or the status code of the first wait that gave up (every role then leaves)
 };
 
 static_assert(sizeof(Misc2) <= Layout2<128>::kMiscBytes, "Misc2 outgrew its shared-memory slot");
@@ -637,7 +637,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       int p = (int)blockIdx.x - 1;
       const int from = look_back ? wk.from : p;
       wait_published(p, from);
-      float lds = 0.f;   // log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
+      float lds = 0.f;   // look-back: log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
       int next = 0;
 #pragma unroll 1
       for (;; --p) {
@@ -647,7 +647,9 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
                                  : sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride +
                                        c.seg * sp.init_seg_stride + (int64_t)l * P;
         const int step = piece ? N : 1;
-        if (next == 0 && p - lane >= from) lds = __ldcg(sp.chain_ld + 2 * (p - lane) + h);
+        float ld = 0.f;
+        if (!LB) ld = piece ? __ldcg(sp.chain_ld + 2 * p + h) : 0.f;
+        else if (next == 0 && p - lane >= from) lds = __ldcg(sp.chain_ld + 2 * (p - lane) + h);
         const float wgt = ex2(asum0 * kLog2e);   // asum0: log-decay between the end of the piece being added and this item
         if (owns_state && wgt != 0.f) {          // (an underflowed piece adds nothing)
           const ulonglong2* I = reinterpret_cast<const ulonglong2*>(src);
@@ -660,7 +662,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           }
         }
         if (!piece) break;
-        asum0 += __shfl_sync(0xffffffffu, lds, next);
+        asum0 += LB ? __shfl_sync(0xffffffffu, lds, next) : ld;
         next = (next + 1) & 31;
       }
     };

@@ -34,14 +34,14 @@ constexpr int kSms = 148;
 struct Work {
   int total;            // tiles of all items
   int npre;             // the first npre of them produce a state only
-  int again;            // look-back mode: items of the range's last piece that follow item 0: 0 or 1 (after its state-only scan), or 2
-                        // where only its beginning is scanned for the state (the rest of the piece, then the beginning again)
   int lo, hi, nt, first;   // chained modes: global tile range, tiles per sequence, first tile of item 0's sequence
   int from;             // look-back mode: the CTA that holds the first tile of the range's first sequence
   int hpg, ppg;         // heads per B/C group, head pairs per group
   // item 0 as (pair of the group, group, batch entry, segment), and the step from one item to the next in the same
   // mixed-radix digits: the walk needs no division
   int d0[4], step[4];
+  int again;            // look-back mode: items of the range's last piece that follow item 0: 0 or 1 (after its state-only scan), or 2
+                        // where only its beginning is scanned for the state (the rest of the piece, then the beginning again)
 };
 
 struct TileParams {
