@@ -172,6 +172,9 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   constexpr int KT = T / 16;
   constexpr int BC = L::kBC;
   constexpr int XS = L::kXSlots;
+  // State-only tiles of the look-back scan: C, the state's copy and their barriers are idle, so every other tile has its B and Xd there.
+  // Nothing then waits for the MMA of the tile before but the accumulator (1 x 32 768 tokens of 24 and 64 heads 116 -> 112.5 and 271 -> 261 us).
+  constexpr bool kTwo = LB && N == 128 && !EPI;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   Misc2* m = reinterpret_cast<Misc2*>(smem + L::oMisc);
@@ -254,10 +257,11 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll 1
         for (int k = 0; k < (n < npre ? 3 : 4); ++k) {
           const CUtensorMap* tm = k < 2 ? &tmX : k == 2 ? &tmB : &tmC;
-          uint64_t* full = k < 2 ? &m->full_x[xi] : k == 2 ? &m->full_b[bs] : &m->full_c[cs];
-          uint64_t* empty = k < 2 ? &m->empty_x[xi] : k == 2 ? &m->empty_b[bs] : &m->empty_c[cs];
-          const uint32_t ph = k < 2 ? xph : k == 2 ? bph : cph;
-          uint32_t dst = k < 2 ? sX + xi * kBlk : k == 2 ? sB + bs * (NB * kBlk) : sC + cs * (NB * kBlk);
+          const bool to_b = k == 2 && !(kTwo && n < npre && (n & 1));
+          uint64_t* full = k < 2 ? &m->full_x[xi] : to_b ? &m->full_b[bs] : &m->full_c[cs];
+          uint64_t* empty = k < 2 ? &m->empty_x[xi] : to_b ? &m->empty_b[bs] : &m->empty_c[cs];
+          const uint32_t ph = k < 2 ? xph : to_b ? bph : cph;
+          uint32_t dst = k < 2 ? sX + xi * kBlk : to_b ? sB + bs * (NB * kBlk) : sC + cs * (NB * kBlk);
           const int blocks = k < 2 ? 1 : NB;
           ok = guarded_wait(empty, ph ^ 1, m, STATUS_WAIT_TIMEOUT_MMA);
           if (!ok) break;
@@ -267,7 +271,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             tma_load_5d(dst, tm, full, 64 * kb, k < 2 ? 2 * c.q + k : 0, c.g, c.t0, c.b, k < 2 ? once : again);
           if (k < 2) {
             if (++xi == XS) { xi = 0; xph ^= 1; }
-          } else if (k == 2) {
+          } else if (to_b) {
             if (++bs == BC) { bs = 0; bph ^= 1; }
           } else {
             if (++cs == BC) { cs = 0; cph ^= 1; }
@@ -323,7 +327,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll 1
         for (int o = 0; o < kOps; ++o) {
           const uint4* op = reinterpret_cast<const uint4*>(&m->ops[n & 1][o]);
-          const uint4 lo = op[0], hi = op[1];
+          uint4 lo = op[0];
+          const uint4 hi = op[1];
           // S: Xd is there (and B: waited for by the warps that made Xd); P.X of the tile before is done (its commit for
           // head 1 covers head 0), or S of the state-only tile before has been consumed.
           // G: C.  C.H: the state copy; the read-out.  P.X: P (X is there: Xd was made of it).
@@ -334,9 +339,15 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
               w1 = n > 0 ? (uint32_t)offsetof(Misc2, bar_u) : 0u;
               p1 = n + 1;
             }
-            if (n >= npre) c1 = 0;
+            if (n >= npre) {
+              c1 = 0;
+            } else if (kTwo && (n & 1)) {
+              lo.x += (sC - sB) >> 4;
+              lo.y += (sH - sXd) >> 4;
+              c1 += (uint32_t)(offsetof(Misc2, empty_c) - offsetof(Misc2, empty_b));
+            }
           }
-          if (o == kOpG) p0 = (n - npre) / BC;
+          if (o == kOpG) p0 = kTwo ? (npre >> 1) + n - npre : (n - npre) / BC;
           wait_at(mb + (hi.z & 0xffffu), p0 & 1, m);
           if (w1) wait_at(mb + w1, p1 & 1, m);
           tc_fence_after();
@@ -818,12 +829,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
       }
       if (!EPI && k < total) {
-        if (k > 0) wait(&m->bar_s, (k - 1) & 1, m);   // the S MMA has read the Xd before this one
+        const bool two = kTwo && k < npre;
+        const uint32_t xd = two && (k & 1) ? sH : sXd;
+        if (k > 0 && !two) wait(&m->bar_s, (k - 1) & 1, m);   // the S MMA has read the Xd before this one
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           wait(&m->full_f[h][k % kFactors], (k / kFactors) & 1, m);
           wait(&m->full_x[bi], bph, m);
-          make_xd<T16, WIDE>(sX + bi * kBlk, sXd + h * kBlk, m->f[h][k % kFactors], q, lane);
+          make_xd<T16, WIDE>(sX + bi * kBlk, xd + h * kBlk, m->f[h][k % kFactors], q, lane);
           if (k < npre) {   // nothing else reads X and the factors of a state-only tile
             __syncwarp();
             if (lane == 0) {
@@ -833,7 +846,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           }
           if (++bi == XS) { bi = 0; bph ^= 1; }
         }
-        wait(&m->full_b[k % BC], (k / BC) & 1, m);   // (for the S MMA, which waits for this group only)
+        // (for the S MMA, which waits for this group only)
+        if constexpr (kTwo) {
+          if (two && k > 0) wait(&m->bar_s, (k - 1) & 1, m);   // (the other Xd is free for the next tile)
+          if (two) wait((k & 1) ? &m->full_c[0] : &m->full_b[0], (k >> 1) & 1, m);
+          else wait(&m->full_b[0], (((npre + 1) >> 1) + k - npre) & 1, m);
+        } else {
+          wait(&m->full_b[k % BC], (k / BC) & 1, m);
+        }
         fence_proxy_async();
         warp_arrive(&m->bar_xd);
         release();
