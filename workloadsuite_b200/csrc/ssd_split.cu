@@ -106,7 +106,7 @@ struct MiscS {
   int bad;                   // the recurrence has to do this call again
   long long wait_clocks;
   volatile int abort_flag;
-  float sums[3][kLookTiles][1];   // find_beginning()
+  Look<1> look;
 };
 static_assert(sizeof(MiscS) <= LayoutS<128, 3>::kMiscBytes, "MiscS outgrew its shared-memory slot");
 static_assert(LayoutS<128, 3>::kBytes <= 232448 && LayoutS<64, 3>::kBytes <= 232448, "shared memory budget of one SM exceeded");
@@ -239,7 +239,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if constexpr (LB) {
-    find_beginning<1>(prm, m->work, m->sums, kThreadsS / 32);
+    find_beginning<1>(prm, m->work, m->look, kThreadsS / 32);
     __syncthreads();
   }
   tc_fence_after();

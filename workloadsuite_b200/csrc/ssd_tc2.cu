@@ -111,7 +111,7 @@ struct Misc2 {
   uint32_t tmem_base;
   long long wait_clocks;     // bound of every wait (SM clock cycles)
   volatile int abort_flag;   // 0, or the status code of the first wait that gave up (every role then leaves)
-  float sums[3][kLookTiles][2];   // find_beginning()
+  Look<2> look;
   float asum1[2];                 // log-decay of the piece that item 1 ended
 };
 
@@ -221,7 +221,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   if constexpr (LB) {
-    find_beginning<2>(prm, m->work, m->sums, kThreads2 / 32);
+    find_beginning<2>(prm, m->work, m->look, kThreads2 / 32);
     __syncthreads();
   }
   tc_fence_after();

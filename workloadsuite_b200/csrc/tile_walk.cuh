@@ -161,68 +161,76 @@ struct CursorOf {
 // Look-back mode, all threads of a CTA, behind a barrier after work_list() and ahead of one before the list is used: how much of the
 // range's last piece needs the state that enters it.  Where the log-decays from its first token on sum to less than -150, e^-150 = 2^-216
 // has taken any entering state below 2^67 past the smallest fp32 number (2^-149): it is not there any more.  A layer's slowest heads (rate
-// 1, steps of 0.03) get there after 40 tiles.  1 x 131 072 tokens, 32 heads, 114 tiles a CTA: 530 -> 438 us, bit by bit the same.
+// 1, steps of 0.03) get there after 40 tiles.  1 x 131 072 tokens, 32 heads, 114 tiles a CTA: 510 -> 432 us, bit by bit the same.
 // A piece scanned so is through with its first pass later (n - 0.6 k tile times for a beginning of k tiles) than one scanned for the state
 // only (0.4 n), and what waits for it waits longer.  So the pieces of a sequence all do it or none: if, by the sequence's first tiles, k is
 // at most 0.6 of a piece (32 768 tokens, 64 heads, each piece for itself and up to 1.0: 271 -> 298 us); and only where every range is one
-// piece, as other ranges may begin with one that waits (the same case: 270 -> 305).  A look
-// takes 2 to 3 us; pieces of less than 40 tiles are left alone.
-constexpr int kLookTiles = 16, kLeastBeginning = 40;
+// piece, as other ranges may begin with one that waits (the same case: 270 -> 305).  A look takes 1.5 us, another where it says yes; pieces
+// of less than 40 tiles are left alone.
+constexpr int kLookTiles = 32, kFirstTiles = 2, kLeastBeginning = 40;
 template <int kHeads>   // heads of an item
-__device__ __forceinline__ void find_beginning(const TileParams& prm, Work& wk, float (&sums)[3][kLookTiles][kHeads], int warps) {
+struct Look {
+  float sums[2][kLookTiles][kHeads], first[kFirstTiles][kHeads];
+};
+template <int kHeads>
+__device__ __forceinline__ void find_beginning(const TileParams& prm, Work& wk, Look<kHeads>& m, int warps) {
   const ScanParams& sp = prm.sp;
   const int from = max(wk.lo, wk.first), tiles = wk.hi - from;
   if (tiles < kLeastBeginning || (int)gridDim.x % prm.upairs != 0 || (wk.again == 0 && from == wk.first)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = wk.d0[1] * wk.hpg + kHeads * wk.d0[0], heads = min(kHeads, wk.hpg - kHeads * wk.d0[0]);
-  const float* A = sp.A + wk.d0[2] * sp.as[0] + head * sp.as[2];
-  // sums over tiles of the piece from its `done`-th on, and at first over those that the sequence begins with, all loads ahead
-  auto look = [&](float (&mine)[kLookTiles][kHeads], int done) {
-    constexpr int kMost = 2 * kLookTiles * kHeads / 16;   // (16 warps at least)
-    const int count = (done == 0 ? 2 : 1) * kLookTiles * heads;
-    float s[kMost];
+  const int heads = min(kHeads, wk.hpg - kHeads * wk.d0[0]);
+  // A tile's sums by one warp, every 32 / kHeads lanes a head.  (A line holds a token's heads: reading it for one at a time, and 16 tiles of
+  // the sequence's beginning, cost 14 to 25 us.)
+  constexpr int kLanes = 32 / kHeads, kTokens = T / kLanes;
+  const int h = lane / kLanes;
+  const float* A = sp.A + wk.d0[2] * sp.as[0] + (wk.d0[1] * wk.hpg + kHeads * wk.d0[0] + min(h, heads - 1)) * sp.as[2];
+  auto sum_of = [&](int tile, float (&to)[kHeads]) {
+    const int64_t t = (int64_t)tile * T + kTokens * (lane % kLanes);
+    float s = 0.f;
+    if (t + kTokens <= sp.seqlen) {   // (less at the end: no harm)
+      const float* a = A + t * sp.as[1];
 #pragma unroll
-    for (int k = 0; k < kMost; ++k) {
-      const int i = warp + k * warps, tile = i % kLookTiles, h = i / kLookTiles % heads;
-      const int64_t t = (int64_t)((i < kLookTiles * heads ? from - wk.first + done : 0) + tile) * T + 4 * lane;
-      const float* a = A + t * sp.as[1] + h * sp.as[2];
-      s[k] = 0.f;
-      if (i < count && t + 3 < sp.seqlen) s[k] = (a[0] + a[sp.as[1]]) + (a[2 * sp.as[1]] + a[3 * sp.as[1]]);   // (less at the end: no harm)
+      for (int e = 0; e < kTokens; ++e, a += sp.as[1]) s += *a;
     }
 #pragma unroll
-    for (int k = 0; k < kMost; ++k) {
-      const int i = warp + k * warps;
-      if (i >= count) break;
-      for (int d = 16; d >= 1; d >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], d);
-      if (lane == 0) (i < kLookTiles * heads ? mine : sums[2])[i % kLookTiles][i / kLookTiles % heads] = s[k];
-    }
+    for (int d = kLanes / 2; d >= 1; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (lane % kLanes == 0) to[h] = s;
   };
-  // every warp for itself: lane 16 h + i has tile i of head h
-  const int i = lane % kLookTiles, h = lane / kLookTiles;
-  const bool mine = h < heads;
-  auto scan = [&](float v) {
-#pragma unroll
-    for (int d = 1; d < kLookTiles; d <<= 1) {
-      const float u = __shfl_up_sync(0xffffffffu, v, d, kLookTiles);
-      if (i >= d) v += u;
-    }
-    return v;
-  };
-  float run = 0.f;
-  int beginning = 0, gone = 0;   // `gone`: tiles after which this lane's head has nothing left
-  for (int done = 0; done < tiles && beginning == 0; done += kLookTiles) {
-    float (&to)[kLookTiles][kHeads] = sums[done / kLookTiles & 1];
-    look(to, done);
+  if (warp < kFirstTiles) sum_of(warp, m.first[warp]);
+  __syncthreads();
+  const float usual = (float)prm.upairs * wk.nt / gridDim.x;
+  bool all = true;
+  for (int k = 0; k < heads; ++k) all = all && (m.first[0][k] + m.first[1][k]) * (0.6f * usual) < -150.f * kFirstTiles;
+  int beginning = 0, gone[kHeads] = {};   // `gone`: tiles after which a head has nothing left
+  float run[kHeads] = {};
+  for (int done = 0; all && done < tiles && beginning == 0; done += kLookTiles) {
+    float (&sums)[kLookTiles][kHeads] = m.sums[done / kLookTiles & 1];
+    for (int i = warp; i < kLookTiles; i += warps) sum_of(from - wk.first + min(done + i, tiles - 1), sums[i]);
     __syncthreads();
-    if (done == 0) {
-      const float all = __shfl_sync(0xffffffffu, scan(mine ? sums[2][i][h] : 0.f), kLookTiles - 1, kLookTiles);
-      if (__any_sync(0xffffffffu, mine && !(all * (0.6f * ((float)prm.upairs * wk.nt / gridDim.x)) < -150.f * kLookTiles))) break;
+    // every warp for itself, a tile to a lane
+#pragma unroll
+    for (int k = 0; k < kHeads; ++k) {
+      if (k >= heads) continue;
+      float v = done + lane < tiles ? sums[lane][k] : 0.f;
+#pragma unroll
+      for (int d = 1; d < kLookTiles; d <<= 1) {
+        const float u = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += u;
+      }
+      v += run[k];
+      const unsigned below = __ballot_sync(0xffffffffu, v < -150.f);
+      if (gone[k] == 0 && below) gone[k] = done + __ffs(below);
+      run[k] = __shfl_sync(0xffffffffu, v, 31);
     }
-    const float v = run + scan(mine && done + i < tiles ? to[i][h] : 0.f);
-    const unsigned below = __ballot_sync(0xffffffffu, v < -150.f) >> (kLookTiles * h) & ((1u << kLookTiles) - 1);
-    if (gone == 0 && below) gone = done + __ffs(below);
-    run = __shfl_sync(0xffffffffu, v, kLookTiles - 1, kLookTiles);
-    if (__all_sync(0xffffffffu, gone > 0 || !mine)) beginning = __reduce_max_sync(0xffffffffu, mine ? gone : 0);
+    beginning = 0;
+    bool both = true;
+#pragma unroll
+    for (int k = 0; k < kHeads; ++k) {
+      if (k >= heads) continue;
+      both = both && gone[k] > 0;
+      beginning = max(beginning, gone[k]);
+    }
+    if (!both) beginning = 0;
   }
   __syncthreads();   // (everybody has read the list)
   if (threadIdx.x == 0 && beginning > 0 && beginning < tiles) {
