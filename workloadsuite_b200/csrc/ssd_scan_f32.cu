@@ -2,7 +2,8 @@
 //   H_t = exp(a_t) H_{t-1} + B_t (x) (x_t dt_t),   y_t = C_t . H_t
 // which the chunked form of the reference (model_ref.py:135-162) is
 // algebraically equal to.  It is the exact-arithmetic path (fp32 inputs, the
-// 1e-4 tolerance) and the fallback for shapes the tensor-core kernel does not
+// 1e-4 tolerance; from 64 tokens on mostly in chunked form, see
+// launch_scan_f32()) and the fallback for shapes the tensor-core kernel does not
 // cover.  One CTA walks one (batch, head[, segment]) with the n x p state held
 // in registers: thread (j, sl) owns column j of the state and the rows
 // n_i = (k*SL + sl)*4 + q, so the B/C rows are read from shared memory as
