@@ -239,6 +239,30 @@ def test_long_pieces_of_cut_sequences_are_scanned_once(decay, b, h, n, ragged):
             assert small.any() and ((a - c).abs()[small] / c.abs()[small]).median().item() < 2 ** -6
 
 
+@pytest.mark.parametrize("gate", [False, True], ids=["plain", "gate"])
+@pytest.mark.parametrize("b,h,n,tiles", [(1, 16, 128, 792), (2, 6, 64, 1056), (1, 16, 128, 90), (25, 4, 128, 16), (1, 3, 128, 300)],
+                         ids=["long", "long_n64", "short_pieces", "two_sequences_a_cta", "odd_heads"])
+def test_cut_sequences_carry_their_state_in_place(b, h, n, tiles, gate):
+    """The final states over the initial ones: the same numbers, bit by bit, as in tensors of their own.  Pieces whose beginnings have different
+    lengths are through with their first pass at different times, the last one ahead of the first or behind it."""
+    import workloadsuite_b200 as W
+
+    s = tiles * 128
+    gen = torch.Generator(DEV).manual_seed(tiles + n)
+    rand = lambda *z: torch.randn(*z, generator=gen, device=DEV)
+    X, B, C, init = rand(b, s, h, 64).bfloat16(), rand(b, s, 1, n).bfloat16(), rand(b, s, 1, n).bfloat16(), 100 * rand(b, h, n, 64)
+    more = {"D": rand(h).bfloat16(), "z": rand(b, s, h, 64).bfloat16()} if gate else {}
+    ramp = torch.linspace(0, 1, s, device=DEV)[None, :, None]
+    for start, end in ((0.5, 0.06), (0.06, 0.5), (0.06, 0.06)):
+        A = -2.0 * (start + (end - start) * ramp) * torch.rand(b, s, h, generator=gen, device=DEV)
+        args = (X, A, B, C, 1)
+        Y, H = W.ssd_forward(*args, initial_states=init, return_final_state=True, nsegments=2, **more)
+        for _ in range(3):
+            state = init.clone()
+            Y2, H2 = W.ssd_forward(*args, initial_states=state, return_final_state=True, out_final_state=state, nsegments=2, **more)
+            assert H2.data_ptr() == state.data_ptr() and torch.equal(Y, Y2) and torch.equal(H, state)
+
+
 @pytest.mark.parametrize("s", [3, 8, 37, 130])
 @pytest.mark.parametrize("p,n", [(64, 16), (64, 128), (32, 32), (128, 64)])
 def test_fp32_scan_tokens_in_line_and_the_rest(s, p, n):

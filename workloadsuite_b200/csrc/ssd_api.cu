@@ -82,6 +82,12 @@ bool outputs_on_inputs(const SsdArgs* a) {
   return z.on(fin) || z.on(ld);
 }
 
+// A state carried in place (or nearly): of cut sequences, the last piece must not write before the others have read.
+bool final_on_initial(const SsdArgs* a) {
+  const int64_t state = (int64_t)a->batch * a->nheads * a->dstate * a->headdim * 4;
+  return range(a->final_state, state).on(range(a->initial_state, state));
+}
+
 // Y written over the gates.  A kernel that reads each gate ahead of its place in Y may do that, but not for a second time.
 bool output_on_gate(const SsdArgs* a) { return range(a, a->Z, a->z_stride, a->nheads, a->headdim, elem_size(a->dtype)).on(output(a)); }
 
@@ -327,6 +333,7 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue,
     }
     if (chain != 0) {
       pc.chain = chain;
+      pc.fin_on_init = chain == 2 && final_on_initial(args) ? 1 : 0;
       pc.chain_state = reinterpret_cast<float*>(ws);
       pc.chain_ld = reinterpret_cast<float*>(ws + align_up(kSlots * np * sizeof(float), 256));
       pc.chain_flag = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(pc.chain_ld) + align_up(kSlots * sizeof(float), 256));   // (cleared by the launch)

@@ -75,6 +75,7 @@ struct alignas(16) Factors {
 };
 
 constexpr int kFactors = 4;   // tiles that the prefix sums may be ahead
+constexpr int kReadBit = 8;   // of a ready flag: from there on it counts the warps that have read what enters their piece
 
 // Log-decays below this count as this in the prefix sums: e^-104 is 2^-150, a factor of zero either way, while -inf (a
 // reset) would make every difference of sums after it NaN, and a very large one would take their digits.
@@ -586,16 +587,16 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
       }
     };
-    // (bounded) wait until the four warps of head h of CTAs `from` .. `to` have published, a CTA per lane.  Every warp asks for
-    // itself: a barrier among the four would hang where one of them has given up.
-    auto wait_published = [&](int to, int from) {
+    // (bounded) wait until the four warps of head h of CTAs `from` .. `to` have published, a CTA per lane (`read`: have read the state
+    // that enters their piece, see settle()).  Every warp asks for itself: a barrier among the four would hang where one of them has given up.
+    auto wait_published = [&](int to, int from, bool read = false) {
       grid_dependency_wait();
       const long long c0 = clock64();
       for (int c = to - lane; c >= from && !m->abort_flag; c -= 32) {
         while (true) {
           int f;
           asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + 2 * c + h) : "memory");
-          if (f >= 4 || m->abort_flag) break;
+          if ((LB && read ? f >> kReadBit : LB ? f & ((1 << kReadBit) - 1) : f) >= 4 || m->abort_flag) break;
           if (clock64() - c0 > m->wait_clocks) {
             m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
             break;
@@ -608,11 +609,13 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // Called as soon as the state of the item before has left, so that the loads are in flight during step A.
     Cursor c;
     bool fold = false;               // the state entering comes (also) from other CTAs: fold_item() before it is used
+    bool entered = false;            // (look-back) settle() behind that
     auto enter_item = [&](bool wy) {
       if (c.goes_on(wk)) return;
       asum0 = asum = acomp = 0.f;
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
       fold = sp.chain && c.t_begin > 0 && !from_zero;
+      entered = LB && !from_zero;
       if (sp.init && c.live(wk, h) && !from_zero && !fold && owns_state) {
         const float* I = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride +
                          (int64_t)l * P;
@@ -677,6 +680,18 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         next = (next + 1) & 31;
       }
     };
+    // Look-back, behind what enters an item that produces Y.  Where the final states lie on the initial ones, the other pieces of the
+    // sequence are told (in the upper bits of the flag: this warp has published by then, if it does) that this one has read.
+    auto settle = [&]() {
+      if (sp.fin_on_init) {
+        __syncwarp();
+        grid_dependency_wait();
+        if (lane == 0) {
+          const int one = 1 << kReadBit;
+          asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + 2 * blockIdx.x + h), "r"(one) : "memory");
+        }
+      }
+    };
     // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
     auto leave_item = [&](bool wy) {
       const bool cut_back = sp.chain && c.t_begin / T + c.ntiles < wk.nt;
@@ -687,17 +702,29 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       const bool late = LB && wk.again == 2 && !cut_back && c.scanned(wk);   // (what came before is not known yet: item 2 knows)
       if (LB && wk.again == 2 && c.item <= 2) {
         if (c.item == 1 && l == 0) m->asum1[h] = asum;
+        if (c.item == 2 && sp.fin_on_init && wk.hi % wk.nt == 0 && c.live(wk, h)) {
+          wait_published((int)blockIdx.x - 1, wk.from, true);
+          if (owns_state) {
+            const ulonglong2* I = reinterpret_cast<const ulonglong2*>(sp.chain_state + slot * (N * P) + l * 4);
+            ulonglong2* F = reinterpret_cast<ulonglong2*>(sp.fin + unit * sp.fin_unit_stride + l * P);
+#pragma unroll 4
+            for (int e = 0; e < P / 4; ++e) F[e] = __ldcg(I + e * N);
+          }
+        }
         if (c.item == 2 && wk.hi % wk.nt == 0 && sp.fin_ld && l == 0 && c.live(wk, h)) sp.fin_ld[unit * sp.finld_unit_stride] = asum0 + m->asum1[h];
       }
       if (publish ? given_up(m) : (cut_back || !c.live(wk, h))) return;
-      float* to = publish ? sp.chain_state + slot * (N * P)
+      // (final states on the initial ones: item 1's waits in the slot, which this CTA has no other use for, until item 2 has ended)
+      const bool to_slot = publish || (late && sp.fin_on_init);
+      if (LB && sp.fin_on_init && !to_slot) wait_published((int)blockIdx.x - 1, wk.from, true);
+      float* to = to_slot ? sp.chain_state + slot * (N * P)
                           : (sp.fin ? sp.fin + unit * sp.fin_unit_stride + seg * sp.fin_seg_stride : nullptr);
       float* ld = publish ? sp.chain_ld + slot
                           : (sp.fin_ld ? sp.fin_ld + unit * sp.finld_unit_stride + seg * sp.finld_seg_stride : nullptr);
       if (to && owns_state) {
-        float* F = to + (publish ? l * 4 : l * P);
-        const int step = publish ? N : 1;
-        if (prm.st32 && !publish) {
+        float* F = to + (to_slot ? l * 4 : l * P);
+        const int step = to_slot ? N : 1;
+        if (prm.st32 && !to_slot) {
 #pragma unroll
           for (int e = 0; e < P / 8; ++e) stg256(F + 8 * e, H[4 * e], H[4 * e + 1], H[4 * e + 2], H[4 * e + 3]);
         } else {
@@ -756,6 +783,10 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       if (__builtin_expect(fold, 0)) {
         fold_item();
         fold = false;
+      }
+      if constexpr (LB) {
+        if (__builtin_expect(entered, 0)) settle();
+        entered = false;
       }
       if (wy) {
         wait(&m->bar_ch, (ky & 1) ^ 1, m);   // the C.H MMA has read the copy before this one
