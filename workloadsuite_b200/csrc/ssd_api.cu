@@ -333,7 +333,8 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue,
     }
     if (chain != 0) {
       pc.chain = chain;
-      pc.fin_on_init = chain == 2 && final_on_initial(args) ? 1 : 0;
+      pc.fin_on_init = chain == 2 && !split && final_on_initial(args) ? 1 : 0;
+      pc.beginnings = chain == 2 && !pc.fin_on_init ? 1 : 0;
       pc.chain_state = reinterpret_cast<float*>(ws);
       pc.chain_ld = reinterpret_cast<float*>(ws + align_up(kSlots * np * sizeof(float), 256));
       pc.chain_flag = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(pc.chain_ld) + align_up(kSlots * sizeof(float), 256));   // (cleared by the launch)

@@ -57,6 +57,7 @@ struct ScanParams {
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], cleared by the launch
   int fin_on_init;        // look-back: `fin` and `init` share memory: a state is written once all pieces of its sequence have read theirs
+  int beginnings;         // look-back: of long pieces only the beginning may be scanned first
   // The tensor-core kernel at fp32 precision writes a word per CTA: not 0 if the fp32 scan has to do the call again.  The scan, when
   // given them (redo_n of them), starts beside that kernel's end and leaves at once if all are 0; cut sequences' segment states and
   // log-decay sums are then in chain_state and chain_ld, [unit][segment].

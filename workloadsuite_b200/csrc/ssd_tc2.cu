@@ -161,13 +161,15 @@ __device__ __forceinline__ void make_xd(uint32_t xb, uint32_t xd, const Factors&
 // LB: an instance for sequences cut in look-back mode (sp.chain == 2), as what a piece's beginning takes costs the walk of the others
 // (see CursorOf).  The others keep their checks of sp.chain == 2, never true there: without them the compiler's registers spill 24 to 60
 // bytes (8 x 2048 tokens of 24 heads 52.1 -> 55.3 us).
-template <typename T16, int N, bool EPI, bool WIDE, bool LB>
+// (2: the final states lie on the initial ones; what that takes costs the others 0.5 us.)
+template <typename T16, int N, bool EPI, bool WIDE, int LB>
 __global__ void __launch_bounds__(kThreads2, 1)
 ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY,
                const TileParams prm) {
   using L = Layout2<N>;
-  using Cursor = CursorOf<2, LB>;
+  using Cursor = CursorOf<2, (LB > 0)>;
+  constexpr bool kCarry = LB == 2;
   constexpr int NB = L::NB;
   constexpr int KN = N / 16;
   constexpr int KT = T / 16;
@@ -221,7 +223,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (LB) {
+  if constexpr (LB == 1) {
     find_beginning<2>(prm, m->work, m->look, kThreads2 / 32);
     __syncthreads();
   }
@@ -596,7 +598,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         while (true) {
           int f;
           asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(sp.chain_flag + 2 * c + h) : "memory");
-          if ((LB && read ? f >> kReadBit : LB ? f & ((1 << kReadBit) - 1) : f) >= 4 || m->abort_flag) break;
+          if ((kCarry && read ? f >> kReadBit : kCarry ? f & ((1 << kReadBit) - 1) : f) >= 4 || m->abort_flag) break;
           if (clock64() - c0 > m->wait_clocks) {
             m->abort_flag = (int)STATUS_WAIT_TIMEOUT_CHAIN;
             break;
@@ -609,13 +611,11 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // Called as soon as the state of the item before has left, so that the loads are in flight during step A.
     Cursor c;
     bool fold = false;               // the state entering comes (also) from other CTAs: fold_item() before it is used
-    bool entered = false;            // (look-back) settle() behind that
     auto enter_item = [&](bool wy) {
       if (c.goes_on(wk)) return;
       asum0 = asum = acomp = 0.f;
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
-      fold = sp.chain && c.t_begin > 0 && !from_zero;
-      entered = LB && !from_zero;
+      fold = sp.chain && !from_zero && (c.t_begin > 0 || kCarry);   // (the latter: settle() is behind it)
       if (sp.init && c.live(wk, h) && !from_zero && !fold && owns_state) {
         const float* I = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride +
                          (int64_t)l * P;
@@ -649,7 +649,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       const bool look_back = sp.chain == 2;
       const bool init = sp.init && c.live(wk, h) && look_back;
       int p = (int)blockIdx.x - 1;
-      const int from = look_back ? wk.from : p;
+      const int from = !look_back ? p : LB && c.t_begin == 0 ? (int)blockIdx.x : wk.from;
       wait_published(p, from);
       float lds = 0.f;   // look-back: log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
       int next = 0;
@@ -680,16 +680,14 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         next = (next + 1) & 31;
       }
     };
-    // Look-back, behind what enters an item that produces Y.  Where the final states lie on the initial ones, the other pieces of the
-    // sequence are told (in the upper bits of the flag: this warp has published by then, if it does) that this one has read.
+    // Where the final states lie on the initial ones, the other pieces of the sequence are told (in the upper bits of the flag: this warp has
+    // published by then, if it does) that this one has read what enters it.
     auto settle = [&]() {
-      if (sp.fin_on_init) {
-        __syncwarp();
-        grid_dependency_wait();
-        if (lane == 0) {
-          const int one = 1 << kReadBit;
-          asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + 2 * blockIdx.x + h), "r"(one) : "memory");
-        }
+      __syncwarp();
+      grid_dependency_wait();
+      if (lane == 0) {
+        const int one = 1 << kReadBit;
+        asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + 2 * blockIdx.x + h), "r"(one) : "memory");
       }
     };
     // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
@@ -699,32 +697,21 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       const int64_t slot = 2 * (int64_t)blockIdx.x + h;
       const int64_t unit = (int64_t)c.b * sp.nheads + c.head(wk) + h;
       const int seg = sp.chain ? 0 : c.seg;
-      const bool late = LB && wk.again == 2 && !cut_back && c.scanned(wk);   // (what came before is not known yet: item 2 knows)
-      if (LB && wk.again == 2 && c.item <= 2) {
+      const bool late = LB == 1 && wk.again == 2 && !cut_back && c.scanned(wk);   // (what came before is not known yet: item 2 knows)
+      if (LB == 1 && wk.again == 2 && c.item <= 2) {
         if (c.item == 1 && l == 0) m->asum1[h] = asum;
-        if (c.item == 2 && sp.fin_on_init && wk.hi % wk.nt == 0 && c.live(wk, h)) {
-          wait_published((int)blockIdx.x - 1, wk.from, true);
-          if (owns_state) {
-            const ulonglong2* I = reinterpret_cast<const ulonglong2*>(sp.chain_state + slot * (N * P) + l * 4);
-            ulonglong2* F = reinterpret_cast<ulonglong2*>(sp.fin + unit * sp.fin_unit_stride + l * P);
-#pragma unroll 4
-            for (int e = 0; e < P / 4; ++e) F[e] = __ldcg(I + e * N);
-          }
-        }
         if (c.item == 2 && wk.hi % wk.nt == 0 && sp.fin_ld && l == 0 && c.live(wk, h)) sp.fin_ld[unit * sp.finld_unit_stride] = asum0 + m->asum1[h];
       }
       if (publish ? given_up(m) : (cut_back || !c.live(wk, h))) return;
-      // (final states on the initial ones: item 1's waits in the slot, which this CTA has no other use for, until item 2 has ended)
-      const bool to_slot = publish || (late && sp.fin_on_init);
-      if (LB && sp.fin_on_init && !to_slot) wait_published((int)blockIdx.x - 1, wk.from, true);
-      float* to = to_slot ? sp.chain_state + slot * (N * P)
+      if (kCarry && !publish) wait_published((int)blockIdx.x - 1, wk.from, true);
+      float* to = publish ? sp.chain_state + slot * (N * P)
                           : (sp.fin ? sp.fin + unit * sp.fin_unit_stride + seg * sp.fin_seg_stride : nullptr);
       float* ld = publish ? sp.chain_ld + slot
                           : (sp.fin_ld ? sp.fin_ld + unit * sp.finld_unit_stride + seg * sp.finld_seg_stride : nullptr);
       if (to && owns_state) {
-        float* F = to + (to_slot ? l * 4 : l * P);
-        const int step = to_slot ? N : 1;
-        if (prm.st32 && !to_slot) {
+        float* F = to + (publish ? l * 4 : l * P);
+        const int step = publish ? N : 1;
+        if (prm.st32 && !publish) {
 #pragma unroll
           for (int e = 0; e < P / 8; ++e) stg256(F + 8 * e, H[4 * e], H[4 * e + 1], H[4 * e + 2], H[4 * e + 3]);
         } else {
@@ -782,11 +769,8 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       // D. 16-bit copy of the state for C.H
       if (__builtin_expect(fold, 0)) {
         fold_item();
+        if constexpr (kCarry) settle();
         fold = false;
-      }
-      if constexpr (LB) {
-        if (__builtin_expect(entered, 0)) settle();
-        entered = false;
       }
       if (wy) {
         wait(&m->bar_ch, (ky & 1) ^ 1, m);   // the C.H MMA has read the copy before this one
@@ -1062,7 +1046,7 @@ __global__ void clear_flags_kernel(int* flags) {
   flags[threadIdx.x] = 0;
 }
 
-template <typename T16, int N, bool EPI, bool WIDE, bool LB>
+template <typename T16, int N, bool EPI, bool WIDE, int LB>
 int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& ty,
                   const TileParams& prm, cudaStream_t stream) {
   auto kern = ssd_tc2_kernel<T16, N, EPI, WIDE, LB>;
@@ -1082,6 +1066,7 @@ int64_t unit_pairs(const SsdArgs& a) { return (int64_t)a.batch * a.ngroups * ((a
 }  // namespace
 
 int64_t tc2_units(const SsdArgs& a) { return unit_pairs(a); }
+
 
 int launch_clear_flags(int32_t* flags, int count, cudaStream_t stream) {
   return launch(clear_flags_kernel, 1, count, 0, stream, flags);
@@ -1182,7 +1167,8 @@ int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
       return SSD_ERR_MISALIGNED;
   }
   auto go = [&](auto epilogue, auto wide, auto look_back) {
-    constexpr bool E = decltype(epilogue)::value, W = decltype(wide)::value, LB = decltype(look_back)::value;
+    constexpr bool E = decltype(epilogue)::value, W = decltype(wide)::value;
+    constexpr int LB = decltype(look_back)::value;
     if (a.dtype == SSD_DTYPE_BF16)
       return a.dstate == 128 ? launch_typed2<__nv_bfloat16, 128, E, W, LB>(tx, tb, tc, ty, prm, stream)
                              : launch_typed2<__nv_bfloat16, 64, E, W, LB>(tx, tb, tc, ty, prm, stream);
@@ -1193,7 +1179,8 @@ int launch_tc2(const SsdArgs& a, const ScanParams& sp, cudaStream_t stream) {
     if (epi) return go(std::true_type{}, std::false_type{}, look_back);
     return odd_groups(a) ? go(std::false_type{}, std::true_type{}, look_back) : go(std::false_type{}, std::false_type{}, look_back);
   };
-  return sp.chain == 2 ? one(std::true_type{}) : one(std::false_type{});
+  if (sp.chain != 2) return one(std::integral_constant<int, 0>{});
+  return sp.fin_on_init ? one(std::integral_constant<int, 2>{}) : one(std::integral_constant<int, 1>{});
 }
 
 }  // namespace ssd

@@ -176,7 +176,7 @@ template <int kHeads>
 __device__ __forceinline__ void find_beginning(const TileParams& prm, Work& wk, Look<kHeads>& m, int warps) {
   const ScanParams& sp = prm.sp;
   const int from = max(wk.lo, wk.first), tiles = wk.hi - from;
-  if (tiles < kLeastBeginning || (int)gridDim.x % prm.upairs != 0 || (wk.again == 0 && from == wk.first)) return;
+  if (!sp.beginnings || tiles < kLeastBeginning || (int)gridDim.x % prm.upairs != 0 || (wk.again == 0 && from == wk.first)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int heads = min(kHeads, wk.hpg - kHeads * wk.d0[0]);
   // A tile's sums by one warp, every 32 / kHeads lanes a head.  (A line holds a token's heads: reading it for one at a time, and 16 tiles of
