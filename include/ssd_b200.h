@@ -150,7 +150,8 @@ const char* ssd_b200_kernel_name(const SsdArgs* args);
  * segments each sequence is cut into (2 stands for "cut" where the cut points follow from the grid),
  * and the number of kernel launches it enqueues: 1 for whole sequences; 1 plus a clearing of flags
  * (a block that the launch overlaps) where a tensor-core kernel deals the tiles of all
- * sequences out evenly inside one launch (states handed from CTA to CTA, or folded from the pairs each CTA publishes for the last piece of its range);
+ * sequences out evenly inside one launch (states handed from CTA to CTA, or folded from the pairs each CTA publishes for the last piece of its range),
+ * and, behind long pieces of 16-bit tensors, another launch that ends at once unless a state was not finite or 2^67 and more;
  * 1 more where the fp32 scan runs on the tensor cores (the recurrence behind it, which ends at once unless a number was
  * not finite or a log-decay far above zero); 3 for the two-pass segmented scan (2 with SSD_FLAG_STATE_ONLY or
  * SSD_FLAG_REUSE_SEGMENTS).  Any out

@@ -195,48 +195,128 @@ def test_cut_sequences_of_no_round_length(shape):
 
 @pytest.mark.parametrize("ragged", [0, 1], ids=["tiles", "ragged"])
 @pytest.mark.parametrize("b,h,n", [(1, 16, 128), (2, 6, 64), (1, 3, 128)])
-@pytest.mark.parametrize("decay", ["fast", "middle", "slow", "one_slow_head", "reset", "impulse", "nan_decay"])
+@pytest.mark.parametrize("decay", ["fast", "middle", "slow", "one_slow_head", "reset", "impulse"])
 def test_long_pieces_of_cut_sequences_are_scanned_once(decay, b, h, n, ragged):
-    """Pieces of 30 tiles and more, whose decays leave nothing of the state that enters them after 2, after some 20 or after none of their
+    """Pieces of 44 tiles, whose decays leave nothing of the state that enters them after 2, after some 20 or after none of their
     tiles, against the same sequences uncut: the state entering a piece is a sum in another order (2^-24), of which 16-bit operands and
     results may round the other way (a few of 2^-8, in a norm 1e-3 at most)."""
     import workloadsuite_b200 as W
 
-    units = b * h if ragged else b * ((h + 1) // 2)
-    tiles = 44 * (148 // units)
-    s = tiles * 128 + 13 * ragged
-    gen = torch.Generator(DEV).manual_seed(tiles + n)
-    rand = lambda *z: torch.randn(*z, generator=gen, device=DEV)
-    X, B, C = rand(b, s, h, 64).bfloat16(), rand(b, s, 1, n).bfloat16(), rand(b, s, 1, n).bfloat16()
-    init = rand(b, h, n, 64)
-    rate = {"fast": 0.8, "middle": 0.06, "slow": 1e-3, "one_slow_head": 0.3, "reset": 1e-3, "impulse": 2e-3, "nan_decay": 0.3}[decay]
-    A = -rate * torch.rand(b, s, h, generator=gen, device=DEV) * 2.0
+    tiles, (X, A, B, C), init = _long_pieces(b, h, n, ragged, decay)
+    s = X.shape[1]
     if decay == "one_slow_head":
         A[:, :, h - 1] *= 1e-3
     elif decay == "reset":
         A[:, 5000::9001] = -float("inf")
     elif decay == "impulse":           # only what entered earlier is left of most pieces
         X[:, 1000:-1000] = 0.0
-    elif decay == "nan_decay":
-        A[:, s // 2, 0] = float("nan")
     kw = dict(initial_states=init, return_final_state=True, return_logdecay=True)
     whole = W.ssd_forward(X, A, B, C, 1, kernel=None if ragged else "tcgen05", nsegments=1, **kw)
     got = W.ssd_forward(X, A, B, C, 1, **kw)
     assert W.plan(X, A, B, C, 1)["nsegments"] > 1
-    assert torch.allclose(got[2], whole[2], rtol=1e-6 * tiles / 32, atol=0, equal_nan=True)
+    assert torch.allclose(got[2], whole[2], rtol=1e-6 * tiles / 32, atol=0)
     for a, c in zip(got[:2], whole[:2]):
-        a, c = a.double(), c.double()
-        if decay == "nan_decay":       # its head from there on: at least to the end of the next piece
-            assert torch.equal(a[..., 1:, :] if a.shape[1] == s else a[:, 1:], a[..., 1:, :] if a.shape[1] == s else a[:, 1:])
-            if a.shape[1] == s:
-                assert a[:, s // 2 : s // 2 + 31 * 128, 0].isnan().all() and not a[:, : s // 2, 0].isnan().any()
-            a, c = (a[:, :, 1:], c[:, :, 1:]) if a.shape[1] == s else (a[:, 1:], c[:, 1:])
-        assert torch.isfinite(a).all()
-        dims = (1, 3) if a.shape[1] == s else (2, 3)
-        assert ((a - c).square().sum(dims) / c.square().sum(dims).clamp_min(1e-60)).sqrt().max().item() < 1e-3
+        _same_but_for_the_order(a, c, s)
         if decay == "impulse" and a.shape[1] == s:   # element by element, far below the rest
+            a, c = a.double(), c.double()
             small = (c.abs() < 1e-6 * c.abs().max()) & (c.abs() > 1e-25 * c.abs().max())
             assert small.any() and ((a - c).abs()[small] / c.abs()[small]).median().item() < 2 ** -6
+
+
+def _long_pieces(b, h, n, ragged, decay, dtype=torch.bfloat16):
+    """Sequences that are cut into one piece of 44 tiles a CTA; their length in tiles, X, A, B, C, and a state to start from."""
+    units = b * h if ragged else b * ((h + 1) // 2)
+    tiles = 44 * (148 // units)
+    s = tiles * 128 + 13 * ragged
+    gen = torch.Generator(DEV).manual_seed(tiles + n)
+    rand = lambda *z: torch.randn(*z, generator=gen, device=DEV)
+    X, B, C = rand(b, s, h, 64).to(dtype), rand(b, s, 1, n).to(dtype), rand(b, s, 1, n).to(dtype)
+    rate = {"fast": 0.8, "middle": 0.06, "slow": 1e-3, "one_slow_head": 0.3, "reset": 1e-3, "impulse": 2e-3}[decay]
+    init = rand(b, h, n, 64)
+    return tiles, (X, -rate * torch.rand(b, s, h, generator=gen, device=DEV) * 2.0, B, C), init
+
+
+def _same_but_for_the_order(a, c, s):
+    """Y or final states of a cut sequence and of the same one uncut, in the norm of each head."""
+    a, c = a.double(), c.double()
+    assert torch.isfinite(a).all()
+    dims = (1, 3) if a.shape[1] == s else (2, 3)
+    assert ((a - c).square().sum(dims) / c.square().sum(dims).clamp_min(1e-60)).sqrt().max().item() < 1e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("decay", ["fast", "middle"])
+@pytest.mark.parametrize("n,with_init,with_dt,gate", [(128, True, True, "Dz"), (64, False, True, "z"), (128, False, False, "D"), (64, True, False, "Dz"),
+                                                      (128, False, True, "")])
+def test_long_pieces_with_steps_skip_and_gate(n, with_init, with_dt, gate, decay, dtype):
+    """The same with everything else that a call may have; the gate is a factor behind equal sums, so the bound stays."""
+    import workloadsuite_b200 as W
+
+    tiles, (X, A, B, C), init = _long_pieces(1, 16, n, 0, decay, dtype)
+    s, gen = X.shape[1], torch.Generator(DEV).manual_seed(n)
+    kw = dict(initial_states=init if with_init else None, return_final_state=True)
+    if with_dt:
+        kw["dt"] = (0.2 + torch.rand(1, s, 16, generator=gen, device=DEV)).to(dtype)
+    if "D" in gate:
+        kw["D"] = torch.randn(16, generator=gen, device=DEV).to(dtype)
+    if "z" in gate:
+        kw["z"] = torch.randn(1, s, 16, 64, generator=gen, device=DEV).to(dtype)
+    whole = W.ssd_forward(X, A, B, C, 1, nsegments=1, **kw)
+    for a, c in zip(W.ssd_forward(X, A, B, C, 1, **kw), whole):
+        _same_but_for_the_order(a, c, s)
+    Y = W.ssd_forward(X, A, B, C, 1, **kw, out=X)[0]     # (over an input: every tile is read once more before it is written)
+    assert Y.data_ptr() == X.data_ptr()
+    _same_but_for_the_order(Y, whole[0], s)
+
+
+@pytest.mark.parametrize("n", [64, 128])
+@pytest.mark.parametrize("gate", [False, True], ids=["plain", "gate"])
+@pytest.mark.parametrize("ragged", [0, 1], ids=["tiles", "ragged"])
+@pytest.mark.parametrize("what", ["nan_decay", "nan_decay_first", "nan_x", "inf_init", "huge_init"])
+def test_long_pieces_pass_on_what_does_not_vanish(what, ragged, gate, n):
+    """A number that is not finite where the decays leave nothing of an ordinary one, in one column of a head (a decay: in the whole head), and a
+    finite one that they leave something of: as far as uncut, to the end of the next piece at least.  What the calls of odd length have of
+    that is done again by the recurrence, uncut or not."""
+    import workloadsuite_b200 as W
+
+    tiles, (X, A, B, C), init = _long_pieces(1, 16, n, ragged, "fast")
+    s, piece = X.shape[1], 44 * 128
+    upto = s + 1
+    if what.startswith("nan_decay"):
+        A[:, s // 2 if what == "nan_decay" else 3000, 2] = float("nan")
+        init = init if what == "nan_decay" else None
+    elif what == "nan_x":
+        X[:, s // 2, 2, 5] = float("nan")
+        upto = s + 1 if ragged else (s // 2 // piece + 2) * piece
+    elif what == "inf_init":
+        init[:, 2, :, 5] = float("inf")
+        upto = s + 1 if ragged else piece
+    else:
+        A.fill_(-0.4)                  # 51.2 a tile
+        X[:, :, 2, 5] = 0.0
+        init[:, 2, :, 5] = 1e36
+    more = {}
+    if gate:
+        gen = torch.Generator(DEV).manual_seed(n)
+        more = {"z": 1.0 + torch.rand(X.shape, generator=gen, device=DEV).bfloat16()}
+    kw = dict(initial_states=init, return_final_state=True, return_logdecay=True, **more)
+    whole = W.ssd_forward(X, A, B, C, 1, nsegments=1, **kw)
+    state = None if init is None else init.clone()
+    in_place = {} if state is None else {"out_final_state": state}
+    for got in (W.ssd_forward(X, A, B, C, 1, **kw), W.ssd_forward(X, A, B, C, 1, **{**kw, "initial_states": state}, **in_place)):
+        assert torch.equal(got[2].isnan(), whole[2].isnan())
+        Y, Yw = got[0][:, :upto], whole[0][:, :upto]
+        assert torch.equal(Y.isfinite(), Yw.isfinite())
+        if upto > s:
+            assert torch.equal(got[1].isfinite(), whole[1].isfinite())
+        if what == "huge_init":
+            a, c = Y[0, :piece, 2, 5].double(), Yw[0, :piece, 2, 5].double()
+            small = (c.abs() < 1e-33) & (c.abs() > 1e-37)     # behind e^-160
+            assert small[384:].any() and ((a - c).abs()[small] / c.abs()[small]).median().item() < 2 ** -6
+        else:
+            assert not Yw.isfinite().all()
+        keep = Yw.isfinite().all(dim=3, keepdim=True).expand_as(Yw) & (torch.arange(16, device=DEV) != 2)[:, None]
+        _same_but_for_the_order(Y.where(keep, 0.0), Yw.where(keep, 0.0), Y.shape[1])
 
 
 @pytest.mark.parametrize("gate", [False, True], ids=["plain", "gate"])
@@ -261,6 +341,27 @@ def test_cut_sequences_carry_their_state_in_place(b, h, n, tiles, gate):
             state = init.clone()
             Y2, H2 = W.ssd_forward(*args, initial_states=state, return_final_state=True, out_final_state=state, nsegments=2, **more)
             assert H2.data_ptr() == state.data_ptr() and torch.equal(Y, Y2) and torch.equal(H, state)
+
+
+def test_long_pieces_are_what_is_scanned_once():
+    """That the sequences of the tests around this one take that way, unless their decays are slow or an output lies on an input: the piece behind
+    one whose state is not finite, and no other, has its bit in the scratch set (behind the ready flags) and was walked again."""
+    import ctypes
+
+    import workloadsuite_b200 as W
+    from workloadsuite_b200 import _lib, ssd
+
+    for decay, over_x in (("fast", False), ("middle", False), ("slow", False), ("fast", True)):
+        tiles, (X, A, B, C), init = _long_pieces(1, 16, 128, 0, decay)
+        X[:, X.shape[1] // 2, 2, 5] = float("nan")
+        args, Y = _lib.SsdArgs(), X if over_x else torch.empty_like(X)
+        ssd._fill(args, X, A, B, C, None, init, Y, None, None, 1, None, None, False)
+        ws = torch.zeros(_lib.load().ssd_b200_workspace_bytes(ctypes.byref(args)), dtype=torch.uint8, device=DEV)
+        args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
+        assert _lib.load().ssd_b200_forward(ctypes.byref(args), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        words = ws[296 * 128 * 64 * 4 + 1280 :].view(torch.int32)[296:301].tolist()
+        cta = tiles // 44 + tiles // 2 // 44 + 1             # of the second pair of heads
+        assert words == [(1 << cta % 32) * (cta // 32 == i and decay != "slow" and not over_x) for i in range(5)]
 
 
 @pytest.mark.parametrize("s", [3, 8, 37, 130])

@@ -91,6 +91,10 @@ bool final_on_initial(const SsdArgs* a) {
 // Y written over the gates.  A kernel that reads each gate ahead of its place in Y may do that, but not for a second time.
 bool output_on_gate(const SsdArgs* a) { return range(a, a->Z, a->z_stride, a->nheads, a->headdim, elem_size(a->dtype)).on(output(a)); }
 
+// Look-back calls of the tensor-core kernel that scan only the beginnings of long pieces first: what is walked again after all needs its
+// inputs as they were.
+bool by_beginnings(const SsdArgs* a) { return ssd::tc2_long_pieces(*a) && !outputs_on_inputs(a) && !output_on_gate(a); }
+
 // The fp32 scan of a call whose kernel is not chosen by the caller: on the tensor cores at fp32 precision where they can
 // (ssd_split.cu), unless the sequences are so short that the recurrence is through before the other kernel's pipeline has
 // filled.  Its time goes with tokens x state, bf16: 8 heads of 17, 33 and 100 tokens, n 128: 8.5, 13.6 and 33 us, there 9.3, 9.4
@@ -334,7 +338,7 @@ static int forward_impl(const SsdArgs* args, void* stream_v, bool fuse_epilogue,
     if (chain != 0) {
       pc.chain = chain;
       pc.fin_on_init = chain == 2 && !split && final_on_initial(args) ? 1 : 0;
-      pc.beginnings = chain == 2 && !pc.fin_on_init ? 1 : 0;
+      pc.beginnings = chain == 2 && (split || by_beginnings(args)) ? 1 : 0;
       pc.chain_state = reinterpret_cast<float*>(ws);
       pc.chain_ld = reinterpret_cast<float*>(ws + align_up(kSlots * np * sizeof(float), 256));
       pc.chain_flag = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(pc.chain_ld) + align_up(kSlots * sizeof(float), 256));   // (cleared by the launch)

@@ -57,7 +57,8 @@ struct ScanParams {
   float* chain_ld;        // [slot] running sum of the log-decay up to the end of the piece
   int32_t* chain_flag;    // [slot], cleared by the launch
   int fin_on_init;        // look-back: `fin` and `init` share memory: a state is written once all pieces of its sequence have read theirs
-  int beginnings;         // look-back: of long pieces only the beginning may be scanned first
+  int beginnings;         // look-back: of long pieces only the beginning may be scanned first (no output on an input)
+  int walk_again;         // the launch behind such a one: pieces that what entered them did not vanish in are walked again
   // The tensor-core kernel at fp32 precision writes a word per CTA: not 0 if the fp32 scan has to do the call again.  The scan, when
   // given them (redo_n of them), starts beside that kernel's end and leaves at once if all are 0; cut sequences' segment states and
   // log-decay sums are then in chain_state and chain_ld, [unit][segment].
@@ -139,6 +140,7 @@ bool tc2_fuses_epilogue(const SsdArgs& a);
 int64_t tc2_units(const SsdArgs& a);   // pairs of heads
 int tc_default_segments(const SsdArgs& a, int64_t units);
 int tc_chain_mode(const SsdArgs& a, int nseg, int64_t units);   // 1: chained, 2: look-back (one launch each); 0: two passes + fold
+bool tc2_long_pieces(const SsdArgs& a);   // look-back, by shape: ScanParams::beginnings, and one more launch
 int launch_tc2(const SsdArgs& a, const ScanParams& prm, cudaStream_t stream);
 int launch_clear_flags(int32_t* flags, int count, cudaStream_t stream);   // to zero, beside what is launched next
 

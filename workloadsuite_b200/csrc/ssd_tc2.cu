@@ -155,6 +155,8 @@ __device__ __forceinline__ void make_xd(uint32_t xb, uint32_t xd, const Factors&
   }
 }
 
+__device__ __forceinline__ int32_t* walk_bits(const ScanParams& sp) { return sp.chain_flag + 2 * kSms; }
+
 // EPI: apply the skip and gate of model_ref.py:116-118 to Y on its way out (sp.D / sp.Z; either may be null).
 // WIDE: Xd in fp32 arithmetic.  Groups with an odd number of heads have always had it so (bf16, final state against 64 bits:
 // 1.65e-3, with the packed products 2.23e-3); those with an even number have the reference's packed products.
@@ -189,6 +191,13 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   // (fault injection for the tests of the give-up path: the first CTA of a chained launch never publishes its
   //  hand-over, so the CTA that continues its sequence runs into the bound of its wait)
   if (sp.inject_lost_handover && sp.chain && blockIdx.x == 0) return;
+  if constexpr (LB == 1) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (sp.walk_again) {
+      grid_dependency_wait();
+      if (!(walk_bits(sp)[blockIdx.x / 32] >> blockIdx.x % 32 & 1)) return;
+    }
+  }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int32_t* status = sp.status;
 
@@ -211,6 +220,10 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     m->abort_flag = 0;
     m->wait_clocks = sp.wait_clocks;
     work_list(prm, m->work);
+    if (LB == 1 && sp.walk_again) {   // one item: the piece, from the state that enters it
+      m->work.again = m->work.npre = 0;
+      m->work.total = m->work.hi - m->work.lo;
+    }
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&m->tmem_base, 512);
@@ -224,7 +237,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   if constexpr (LB == 1) {
-    find_beginning<2>(prm, m->work, m->look, kThreads2 / 32);
+    if (!sp.walk_again) find_beginning<2>(prm, m->work, m->look, kThreads2 / 32);
     __syncthreads();
   }
   tc_fence_after();
@@ -615,7 +628,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       if (c.goes_on(wk)) return;
       asum0 = asum = acomp = 0.f;
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
-      fold = sp.chain && !from_zero && (c.t_begin > 0 || kCarry);   // (the latter: settle() is behind it)
+      fold = sp.chain && !from_zero && (c.t_begin > 0 || kCarry || (LB == 1 && wk.again == 2));   // (the latter two: settle() is to see it)
       if (sp.init && c.live(wk, h) && !from_zero && !fold && owns_state) {
         const float* I = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk) + h) * sp.init_unit_stride + c.seg * sp.init_seg_stride +
                          (int64_t)l * P;
@@ -679,15 +692,34 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         asum0 += LB ? __shfl_sync(0xffffffffu, lds, next) : ld;
         next = (next + 1) & 31;
       }
+      if (LB && asum0 != asum0) {   // (a log-decay that is NaN, in the sequence's first piece perhaps: nothing was added behind it)
+        const uint64_t nan2 = pair(asum0, asum0);
+#pragma unroll
+        for (int e = 0; e < P / 2; ++e) H[e] = nan2;
+      }
     };
-    // Where the final states lie on the initial ones, the other pieces of the sequence are told (in the upper bits of the flag: this warp has
-    // published by then, if it does) that this one has read what enters it.
+    // Look-back, behind what enters an item that produces Y.  A beginning is done again: a state that does not vanish behind it has the piece
+    // done again (a bit per CTA, see launch_tc2()).  And where the final states lie on the initial ones, the other pieces of the sequence are
+    // told (in the upper bits of the flag: this warp has published by then, if it does) that this one has read.
     auto settle = [&]() {
-      __syncwarp();
-      grid_dependency_wait();
-      if (lane == 0) {
-        const int one = 1 << kReadBit;
-        asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + 2 * blockIdx.x + h), "r"(one) : "memory");
+      if (LB == 1 && wk.again == 2) {
+        bool gone = true;
+        if (owns_state) {
+#pragma unroll
+          for (int e = 0; e < P / 2; ++e) gone = gone && vanishes(unpair(H[e]));
+        }
+        if (!__all_sync(0xffffffffu, gone) && lane == 0) {
+          grid_dependency_wait();
+          atomicOr(walk_bits(sp) + blockIdx.x / 32, 1 << blockIdx.x % 32);
+        }
+      }
+      if constexpr (kCarry) {
+        __syncwarp();
+        grid_dependency_wait();
+        if (lane == 0) {
+          const int one = 1 << kReadBit;
+          asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(sp.chain_flag + 2 * blockIdx.x + h), "r"(one) : "memory");
+        }
       }
     };
     // The state leaving an item: to this CTA's slot, or (last or only piece of the sequence) the caller's outputs.
@@ -769,7 +801,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       // D. 16-bit copy of the state for C.H
       if (__builtin_expect(fold, 0)) {
         fold_item();
-        if constexpr (kCarry) settle();
+        if constexpr (LB) settle();
         fold = false;
       }
       if (wy) {
@@ -1055,7 +1087,13 @@ int launch_typed2(const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMa
     return SSD_ERR_CUDA;
   const int nt = (prm.sp.seqlen + T - 1) / T;
   const int grid = prm.sp.chain ? dealt_grid(prm.upairs, nt, prm.sp.chain) : std::min(prm.nitems, kSms);
-  return launch_tiles(kern, grid, kThreads2, smem, prm.sp, stream, tx, tb, tc, ty, prm);
+  const int rc = launch_tiles(kern, grid, kThreads2, smem, prm.sp, stream, tx, tb, tc, ty, prm);
+  if (LB != 1 || !prm.sp.beginnings || rc != SSD_OK) return rc;
+  // What entered a piece and did not vanish (see find_beginning()): the piece again, from the states that the launch before left in scratch.
+  // 1 us where there is none.  (As one more item of the same launch, or that launch's list again, 1.5 to 3 % of every look-back call.)
+  TileParams again = prm;
+  again.sp.walk_again = 1;
+  return launch_early(kern, grid, kThreads2, smem, stream, tx, tb, tc, ty, again);
 }
 
 bool odd_groups(const SsdArgs& a) { return a.nheads / a.ngroups % 2 != 0; }
@@ -1067,6 +1105,12 @@ int64_t unit_pairs(const SsdArgs& a) { return (int64_t)a.batch * a.ngroups * ((a
 
 int64_t tc2_units(const SsdArgs& a) { return unit_pairs(a); }
 
+bool tc2_long_pieces(const SsdArgs& a) {
+  const int64_t units = unit_pairs(a), nt = (a.seqlen + T - 1) / T;
+  if (units >= kSms) return false;
+  const int64_t pieces = dealt_grid(units, (int)nt, 2) / units;
+  return dealt_grid(units, (int)nt, 2) % units == 0 && pieces > 1 && (nt + pieces - 1) / pieces >= kLeastBeginning;
+}
 
 int launch_clear_flags(int32_t* flags, int count, cudaStream_t stream) {
   return launch(clear_flags_kernel, 1, count, 0, stream, flags);

@@ -29,7 +29,8 @@ constexpr int kSms = 148;
 //    log-decays after c) F_c), skipping those whose decay factor has underflowed.
 //    Of a long piece only a beginning is scanned that way (find_beginning()): from where what enters the piece has decayed to nothing,
 //    the scan from zero is the scan, and writes Y at once (and the sequence's final state, where the piece ends it).  Then the
-//    beginning is done again, from the state that does enter.
+//    beginning is done again, from the state that does enter -- and by a launch behind this one the whole piece, if that state turns out to
+//    be one that does not decay to nothing (not finite, or of 2^67 and more).
 // Computed once per CTA (thread 0, into shared memory): the 64-bit divisions are bulky code.
 struct Work {
   int total;            // tiles of all items
@@ -160,13 +161,15 @@ struct CursorOf {
 
 // Look-back mode, all threads of a CTA, behind a barrier after work_list() and ahead of one before the list is used: how much of the
 // range's last piece needs the state that enters it.  Where the log-decays from its first token on sum to less than -150, e^-150 = 2^-216
-// has taken any entering state below 2^67 past the smallest fp32 number (2^-149): it is not there any more.  A layer's slowest heads (rate
+// has taken any entering state below 2^67 (kVanishes) past the smallest fp32 number (2^-149): it is not there any more.  A layer's slowest heads (rate
 // 1, steps of 0.03) get there after 40 tiles.  1 x 131 072 tokens, 32 heads, 114 tiles a CTA: 510 -> 432 us, bit by bit the same.
 // A piece scanned so is through with its first pass later (n - 0.6 k tile times for a beginning of k tiles) than one scanned for the state
 // only (0.4 n), and what waits for it waits longer.  So the pieces of a sequence all do it or none: if, by the sequence's first tiles, k is
 // at most 0.6 of a piece (32 768 tokens, 64 heads, each piece for itself and up to 1.0: 271 -> 298 us); and only where every range is one
 // piece, as other ranges may begin with one that waits (the same case: 270 -> 305).  A look takes 1.5 us, another where it says yes; pieces
 // of less than 40 tiles are left alone.
+constexpr float kVanishes = 0x1p67f;
+__device__ __forceinline__ bool vanishes(float2 v) { return fabsf(v.x) < kVanishes && fabsf(v.y) < kVanishes; }
 constexpr int kLookTiles = 32, kFirstTiles = 2, kLeastBeginning = 40;
 template <int kHeads>   // heads of an item
 struct Look {
@@ -342,12 +345,15 @@ inline int dealt_grid(int64_t units, int tiles, int chain) {
   return grid;
 }
 
+// Ready flags of a launch, and behind them a bit for each CTA whose piece is to be walked again.
+constexpr int kFlags = 2 * kSms + (kSms + 31) / 32;
+
 // Launches a kernel over the tiles; where sequences are cut, behind the clearing of their ready flags, which it starts beside.
 template <typename... Params, typename... Args>
 int launch_tiles(void (*kernel)(Params...), int grid, int threads, int smem, const ScanParams& sp, cudaStream_t stream,
                  const Args&... args) {
   if (!sp.chain) return launch(kernel, grid, threads, smem, stream, args...);
-  if (launch_clear_flags(sp.chain_flag, 2 * kSms, stream) != SSD_OK) return SSD_ERR_CUDA;
+  if (launch_clear_flags(sp.chain_flag, kFlags, stream) != SSD_OK) return SSD_ERR_CUDA;
   return launch_early(kernel, grid, threads, smem, stream, args...);
 }
 
