@@ -47,9 +47,8 @@ enum { SSD_DTYPE_F32 = 0, SSD_DTYPE_F16 = 1, SSD_DTYPE_BF16 = 2 };
 enum {
   SSD_KERNEL_AUTO = 0,    /* tensor-core kernel when the shape allows and the sequence is whole tiles of 128 tokens,
                              else the fp32 scan, on the tensor cores (products of 16-bit pieces that hold fp32
-                             numbers) where the shape allows that */
-  SSD_KERNEL_SCAN_F32 = 1,/* fp32 token recurrence on CUDA cores (any dtype in, fp32 math; fp32 tensors from 64 tokens on in
-                             chunked form) */
+                             numbers) where the shape allows that, fp32 tensors from 64 tokens on in chunked form */
+  SSD_KERNEL_SCAN_F32 = 1,/* fp32 token recurrence on CUDA cores (any dtype in, fp32 math) */
   SSD_KERNEL_TCGEN05 = 2  /* tcgen05/TMEM chunked kernel (f16/bf16 only, any length): faster than the scan,
                              but the masked products, the decayed X and the state's copy are rounded to 16 bits */
 };

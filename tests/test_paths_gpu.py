@@ -382,6 +382,24 @@ def test_fp32_scan_with_registers_for_more_ctas(n, units, s, dtype):
 
 
 @pytest.mark.parametrize("n", [16, 32, 64, 128])
+@pytest.mark.parametrize("cut", [70, 77, 123])
+def test_fp32_recurrence_by_name(cut, n):
+    """Token by token whatever the length: a sequence in two parts leaves the same state, bit by bit, as at once (Y's sums over the state
+    may be taken in another order)."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=2, s=200, h=4, p=64, n=n, g=2, dtype=torch.float32, init=True, seed=n, decay_scale=0.1)
+    X, A, B, C, init = (inp[k].to(DEV) for k in ("X", "A", "B", "C", "initial_states"))
+    run = lambda lo, hi, H: W.ssd_forward(X[:, lo:hi], A[:, lo:hi], B[:, lo:hi], C[:, lo:hi], 1, initial_states=H, return_final_state=True,
+                                          kernel="scan_f32", nsegments=1)
+    Y, H = run(0, 200, init)
+    Y1, H1 = run(0, cut, init)
+    Y2, H2 = run(cut, 200, H1)
+    assert torch.equal(H, H2)
+    assert (Y - torch.cat([Y1, Y2], 1)).abs().max().item() < 2 ** -20 * Y.abs().max().item()
+
+
+@pytest.mark.parametrize("n", [16, 32, 64, 128])
 @pytest.mark.parametrize("s", [64, 65, 79, 128, 129, 200])
 @pytest.mark.parametrize("decays", ["mild", "both_signs", "resets", "strong", "growth", "x_nan", "b_inf", "huge"])
 def test_fp32_tokens_side_by_side(decays, s, n):

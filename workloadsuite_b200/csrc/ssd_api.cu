@@ -223,7 +223,7 @@ bool states_aligned16(const SsdArgs* a) { return aligned16(a->initial_state) && 
 
 int launch_kernel(int kernel, const SsdArgs* a, const ssd::ScanParams& prm, cudaStream_t stream) {
   if (kernel == SSD_KERNEL_TCGEN05) return ssd::launch_tc2(*a, prm, stream);
-  return ssd::launch_scan_f32(prm, a->dtype, stream);
+  return ssd::launch_scan_f32(prm, a->dtype, stream, a->kernel != SSD_KERNEL_AUTO);
 }
 
 }  // namespace

@@ -121,7 +121,7 @@ __device__ __forceinline__ float load_skip(const ScanParams& p, int head) {
 
 // Launchers implemented in the kernel translation units.  Each returns an
 // SSD_ERR_* code and enqueues on `stream`.
-int launch_scan_f32(const ScanParams& prm, int dtype, cudaStream_t stream);
+int launch_scan_f32(const ScanParams& prm, int dtype, cudaStream_t stream, bool in_line = true);   // in_line: as the token recurrence, not chunked
 bool scan_f32_supports(int p, int n);
 int scan_f32_tile_tokens();
 

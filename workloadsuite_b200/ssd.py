@@ -187,8 +187,8 @@ def ssd_forward(
     ``kernel``: None lets the library choose.  ``"tcgen05"`` (16-bit tensors, p = 64, n = 64 or 128) runs on the tensor
     cores and rounds intermediate operands to 16 bits; it is chosen for sequences of whole tiles (multiples of 128 tokens).
     ``"scan_f32"`` computes in float32 throughout; it is chosen for everything else, where it runs on the tensor cores too
-    if the shape allows (asked for by name, it is the token-by-token recurrence, or its chunked form for float32 tensors from 64
-    tokens on).  ``kernel="tcgen05"`` takes any length where
+    if the shape allows, and for float32 tensors from 64 tokens on in chunked form (asked for by name, it is the token-by-token
+    recurrence).  ``kernel="tcgen05"`` takes any length where
     16-bit intermediates are accurate enough (relative error of Y in bfloat16 2.4e-3 instead of 1.7e-3, of the final
     state 2e-3 instead of 1e-7) at four fifths of the time.  Numbers that are not finite, log-decays above 1/32 and float16
     numbers beyond some 4 096 make the recurrence do such a call again; outputs on inputs (``out_final_state`` on
