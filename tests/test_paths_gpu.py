@@ -449,6 +449,42 @@ def test_fp32_tokens_side_by_side(decays, s, n):
     assert torch.equal(again.nan_to_num(), Y.nan_to_num())       # (Y over X)
 
 
+@pytest.mark.parametrize("n", [16, 32, 64, 128])
+@pytest.mark.parametrize("s", [64, 77, 200])
+@pytest.mark.parametrize("decays", ["even", "spikes", "resets", "up_and_down"])
+def test_fp32_strong_decays_keep_their_bits(decays, s, n):
+    """What is left behind decays that leave the range of a piece's scaling, element by element: x in every eleventh token only, so that most of Y is
+    nothing else.  Measured by the same sums of magnitudes, an element is off by the rounding of its weight (a decay e^-80 known to 2^-24 of its
+    exponent: 5e-6) and of a sum of up to 128 products (128 * 2^-24 = 8e-6 at most); and by no more than the recurrence is."""
+    import workloadsuite_b200 as W
+
+    inp = O.make_inputs(b=2, s=s, h=4, p=64, n=n, g=2, dtype=torch.float32, init=True, seed=s + n, decay_scale=0.1)
+    gen = torch.Generator().manual_seed(s)
+    dt = 0.2 + torch.rand(2, s, 4, generator=gen)
+    X, A, B, C, init = (inp[k] for k in ("X", "A", "B", "C", "initial_states"))
+    X[:, torch.arange(s) % 11 != 3] = 0.0
+    if decays == "even":
+        A = -2.6 - torch.rand(A.shape, generator=gen)
+    elif decays == "spikes":
+        A[:, 5::13] = -41.0
+    elif decays == "resets":
+        A[:, 9::16], A[:, 40:42], A[:, 15] = -float("inf"), -float("inf"), -200.0
+    elif decays == "up_and_down":
+        A[:, 2::8], A[:, 4::8] = 30.0, -30.0
+    want, Hw = O.ssd_recurrence(X, A, B, C, dt=dt, initial_states=init, return_final_state=True)
+    size, Hs = O.ssd_recurrence(X.abs(), A, B.abs(), C.abs(), dt=dt, initial_states=init.abs(), return_final_state=True)
+    d = [t.to(DEV) for t in (X, A, B, C)]
+    kw = dict(dt=dt.to(DEV), initial_states=init.to(DEV), return_final_state=True)
+    errors = []
+    for kernel in (None, "scan_f32"):
+        Y, H = W.ssd_forward(*d, 1, kernel=kernel, **kw)
+        for got, ref, terms in ((Y.cpu().double(), want, size), (H.cpu().double(), Hw, Hs)):
+            assert (got[terms == 0] == 0).all()
+            err = ((got - ref).abs() / terms)[terms > 1e-34]        # (below, fp32 has fewer bits)
+            errors += [err.square().mean().sqrt().item(), err.max().item()] if err.numel() else [0.0, 0.0]
+    assert max(errors) < 1.3e-5 and errors[0] < max(1.5 * errors[4], 1e-7) and errors[2] < max(1.5 * errors[6], 1e-7), errors
+
+
 @pytest.mark.parametrize("b,h,n,g", [(3, 6, 128, 2), (1, 4, 256, 1), (40, 6, 16, 3), (40, 6, 32, 2), (40, 6, 256, 6), (2, 1, 64, 1)])
 def test_step_reads_strided_operands_and_d_in_its_own_type(b, h, n, g):
     """Columns of a projection's output against the same values copied out: the same arithmetic, so the same bits.  CTAs of half
