@@ -6,6 +6,7 @@
 namespace ssd {
 
 bool chunk_f32_takes(const ScanParams& prm);   // fp32 tensors of this shape and alignment
+bool chunk_f32_pays(const ScanParams& prm);    // and is faster than the recurrence there
 int launch_chunk_f32(const ScanParams& prm, cudaStream_t stream);
 
 }  // namespace ssd

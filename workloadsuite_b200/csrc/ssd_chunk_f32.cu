@@ -427,6 +427,23 @@ bool chunk_f32_takes(const ScanParams& prm) {
   return prm.p == kP && (prm.n == 16 || prm.n == 32 || prm.n == 64 || prm.n == 128) && prm.vec_ok && al(prm.init) && al(prm.fin) && prm.batch <= 65535;
 }
 
+// A tile costs much the same whatever is in it, so what counts is what is left for the last one.  Times of 3 984 heads in microseconds (start,
+// tile, 16 tokens of a tile; start, 64 tokens one after the other): n 32: 65, 80, 112 and 129 tokens 221, 225, 241 and 388, the recurrence 166,
+// 194, 262 and 303; n 64: 64, 65, 96 and 129 245, 375, 393 and 594, there 279, 293, 405 and 545; n 128: 32, 34, 48 and 65 279, 369, 372 and 619,
+// there 282, 305, 409 and 543.  With up to eight heads an SM the recurrence is a tenth slower than that (not with n 128), with up to one 1.4
+// times (n 128: a tenth).
+bool chunk_f32_pays(const ScanParams& prm) {
+  struct Cost { int tokens, start, tile, piece, start_in_line, in_line; };
+  const Cost c = prm.n == 16 ? Cost{128, 2, 60, 7, 8, 83} : prm.n == 32 ? Cost{128, 20, 115, 15, 11, 144} : prm.n == 64 ? Cost{64, 20, 100, 30, 12, 262}
+                                                                                                            : Cost{64, 30, 160, 55, 25, 500};
+  const int64_t tokens = prm.seqlen < prm.seg_len ? prm.seqlen : prm.seg_len, ctas = (int64_t)prm.batch * prm.nheads * prm.nseg;
+  if (tokens < (prm.n == 128 ? 32 : 64)) return false;
+  const int64_t side_by_side = c.start + (tokens + c.tokens - 1) / c.tokens * c.tile + (tokens + kQ - 1) / kQ * c.piece;
+  const int64_t in_line = c.start_in_line + tokens * c.in_line / 64;
+  const int percent = ctas <= 148 ? (prm.n == 128 ? 110 : 140) : ctas <= 8 * 148 && prm.n != 128 ? 110 : 100;
+  return 100 * side_by_side <= percent * in_line;
+}
+
 int launch_chunk_f32(const ScanParams& prm, cudaStream_t stream) {
   switch (prm.n) {
     case 16: return launch_chunk<16, 8, 1>(prm, stream);

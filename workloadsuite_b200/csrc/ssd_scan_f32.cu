@@ -565,11 +565,8 @@ int scan_f32_tile_tokens() { return kTile; }
 
 int launch_scan_f32(const ScanParams& prm, int dtype, cudaStream_t stream, bool in_line) {
   if (!scan_f32_supports(prm.p, prm.n)) return SSD_ERR_UNSUPPORTED;
-  // fp32 tensors, unless the caller asks for this kernel by name: tokens side by side, where there are enough of them for its pieces (16 x 8 heads, n 16: 48 tokens 5.4 us either way, 64
-  // 5.6 there and 6.4 here, 128 7.3 and 9.9; n 128, 128 heads: 16 tokens 10.7 and 8.3, 32 11.4 and 12.8; 2 048 heads, n 64: 48 tokens
-  // 128 and 128, 64 138 and 161).
-  const int tokens = std::min(prm.seqlen, prm.seg_len);
-  if (!in_line && dtype == SSD_DTYPE_F32 && (tokens >= 64 || (tokens >= 32 && prm.n == 128)) && chunk_f32_takes(prm)) return launch_chunk_f32(prm, stream);
+  // fp32 tensors, unless the caller asks for this kernel by name: tokens side by side, where that is faster
+  if (!in_line && dtype == SSD_DTYPE_F32 && chunk_f32_takes(prm) && chunk_f32_pays(prm)) return launch_chunk_f32(prm, stream);
   switch (dtype) {
     case SSD_DTYPE_F32: return launch_t<float>(prm, stream);
     case SSD_DTYPE_F16: return launch_t<__half>(prm, stream);
