@@ -163,7 +163,7 @@ __device__ __forceinline__ int32_t* walk_bits(const ScanParams& sp) { return sp.
 // LB: an instance for sequences cut in look-back mode (sp.chain == 2), as what a piece's beginning takes costs the walk of the others
 // (see CursorOf).  The others keep their checks of sp.chain == 2, never true there: without them the compiler's registers spill 24 to 60
 // bytes (8 x 2048 tokens of 24 heads 52.1 -> 55.3 us).
-// (2: the final states lie on the initial ones; what that takes costs the others 0.5 us.)
+// (2: the final states lie on the initial ones; what that takes costs the others 0.5 to 1 us.)
 template <typename T16, int N, bool EPI, bool WIDE, int LB>
 __global__ void __launch_bounds__(kThreads2, 1)
 ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
@@ -236,7 +236,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (LB == 1) {
+  if constexpr (LB > 0) {   // (never with sp.fin_on_init; without the call kCarry's registers spill: 1 x 131 072 tokens of 32 heads 597 us, 510 so)
     if (!sp.walk_again) find_beginning<2>(prm, m->work, m->look, kThreads2 / 32);
     __syncthreads();
   }
