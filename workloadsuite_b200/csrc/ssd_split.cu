@@ -539,7 +539,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     float asum0 = 0.f;               // log-decay summed over the earlier pieces of the sequence
     float asum = 0.f, acomp = 0.f;   // compensated sum of the tile totals
     Cursor c;
-    bool fold = false, entered = false;
+    bool fold = false;
 
     // P of this thread's row, 32 columns.  The block is below the diagonal (weight = decay from the block's end to the row * decay
     // to the block's end, both in one product), on it (an exponential per column), or above (zero).
@@ -662,8 +662,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       if (c.goes_on(wk)) return;
       asum0 = asum = acomp = 0.f;
       const bool from_zero = sp.chain == 2 && !wy;               // (the look-back scan)
-      fold = sp.chain && c.t_begin > 0 && !from_zero;
-      entered = LB && wk.again == 2 && !from_zero;
+      fold = sp.chain && !from_zero && (c.t_begin > 0 || (LB && wk.again == 2));   // (the latter is to be looked at behind the fold)
       if (sp.init && !from_zero && !fold && owns_state) {
         const float* I = sp.init + ((int64_t)c.b * sp.nheads + c.head(wk)) * sp.init_unit_stride + (int64_t)l * P + 16 * J;
         if (prm.st32) {
@@ -691,7 +690,7 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       const bool look_back = sp.chain == 2;
       const bool init = sp.init && look_back;
       int p = (int)blockIdx.x - 1;
-      const int from = look_back ? wk.from : p;
+      const int from = !look_back ? p : LB && c.t_begin == 0 ? (int)blockIdx.x : wk.from;
       wait_published(p, from);
       float lds = 0.f;   // look-back: log-decays of 32 pieces, one in each lane (asked for one by one they are a round trip to L2 each)
       int next = 0;
@@ -764,14 +763,11 @@ ssd_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       if (__builtin_expect(fold, 0)) {
         fold_item();
         fold = false;
-      }
-      if constexpr (LB) {
-        if (__builtin_expect(entered, 0)) {   // (a beginning done again, from a state that does not vanish behind it)
+        if (LB && wk.again == 2) {   // (a beginning done again: from a state that does not vanish behind it?)
           bool gone = true;
 #pragma unroll
           for (int e = 0; e < 8; ++e) gone = gone && vanishes(unpair(H[e]));
           if (!gone) m->bad = 1;
-          entered = false;
         }
       }
       if (wy) {
