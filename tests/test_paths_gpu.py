@@ -364,6 +364,27 @@ def test_long_pieces_are_what_is_scanned_once():
         assert words == [(1 << cta % 32) * (cta // 32 == i and decay != "slow" and not over_x) for i in range(5)]
 
 
+@pytest.mark.parametrize("in_place", [False, True], ids=["by_beginnings", "state_in_place"])
+def test_a_lost_piece_of_a_long_sequence_is_reported(in_place):
+    """The first CTA leaves without publishing: those behind it give up after 3 ms, the launch that walks pieces again has nothing to do (what they
+    folded is no state), and the next forward is as ever."""
+    import time
+
+    import workloadsuite_b200 as W
+
+    tiles, (X, A, B, C), init = _long_pieces(1, 16, 128, 0, "fast")
+    run = lambda state, **kw: W.ssd_forward(X, A, B, C, 1, initial_states=state, return_final_state=True, out_final_state=state if in_place else None, **kw)
+    Y, H = run(init.clone())
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    run(init.clone(), wait_limit_ms=3, inject_lost_handover=True)
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 0.5 and W.device_status(DEV) == 6
+    again = run(init.clone())
+    torch.cuda.synchronize()
+    assert W.device_status(DEV) == 0 and torch.equal(Y, again[0]) and torch.equal(H, again[1])
+
+
 @pytest.mark.parametrize("s", [3, 8, 37, 130])
 @pytest.mark.parametrize("p,n", [(64, 16), (64, 128), (32, 32), (128, 64)])
 def test_fp32_scan_tokens_in_line_and_the_rest(s, p, n):

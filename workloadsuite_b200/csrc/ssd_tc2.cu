@@ -708,7 +708,7 @@ ssd_tc2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 #pragma unroll
           for (int e = 0; e < P / 2; ++e) gone = gone && vanishes(unpair(H[e]));
         }
-        if (!__all_sync(0xffffffffu, gone) && lane == 0) {
+        if (!__all_sync(0xffffffffu, gone) && lane == 0 && !m->abort_flag) {
           grid_dependency_wait();
           atomicOr(walk_bits(sp) + blockIdx.x / 32, 1 << blockIdx.x % 32);
         }
